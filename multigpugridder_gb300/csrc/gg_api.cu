@@ -2,7 +2,7 @@
 //
 // One handle owns one GPU's state: the resident FP32 CAS volume (plus, with
 // FP16/BF16 storage, the copy the forward projection reads: rows padded for
-// aligned vector loads), the KB table and pre-compensation vector, batch buffers and
+// TMA), the KB table and pre-compensation vector, batch buffers and
 // cached cuFFT plans.  It replaces the reference's MultiGPUGridder /
 // gpuGridder / AbstractGridder trio (src/Gridders/) for one device:
 //   * the volume is prepared on the device once per setVolume instead of on
@@ -150,10 +150,13 @@ struct gg_gridder {
     DevBuf<float> ker;
     DevBuf<double> precomp;
     DevBuf<float> cas;       // FP32 CAS volume V^3 (resident)
-    DevBuf<float> cas_fp;    // FP16/BF16 copy the forward projection reads: row pitch
-                             // fp_pitch(V) (FP16 scaled by scales[0])
-    DevBuf<float> cas_y, cas_z; // FP32: the CAS volume with y / z as the contiguous axis
-    bool cas_fp_valid = false;  // cas_fp (FP16/BF16) or cas_y/cas_z (FP32) match cas
+    DevBuf<unsigned char> cas_fp; // the copy the forward projection reads: storage `prec`, row
+                                  // pitch fp_pitch(V, prec) (FP16 scaled by scales[0])
+    DevBuf<unsigned char> fp_maps; // its tensor maps (gg_fp_tile.cu)
+    const void *fp_maps_vol = nullptr; // the copy's address and storage they were made for
+    int fp_maps_prec = -1;
+    bool cas_fp_valid = false;  // cas_fp matches cas
+    int *fault = nullptr;       // pinned: set by a kernel whose copies did not arrive
     DevBuf<float> pd;        // plane density V^3
     DevBuf<float> adj;       // CAS-volume gradient V^3 (forward-operator adjoint)
     DevBuf<float> axes;
@@ -167,7 +170,7 @@ struct gg_gridder {
         DevBuf<float> casimg, real, img;
         DevBuf<cufftComplex> spec;
         DevBuf<uint16_t> casimg_lp;
-        DevBuf<int> order; // the forward projection's direction order (grouped by copy)
+        DevBuf<unsigned char> plans; // the forward projection's box plans, one per direction
         PinBuf stage;
         cudaEvent_t ev_ready = nullptr, ev_free = nullptr;
     } slot[2];
@@ -238,7 +241,7 @@ void ensure_slot(gg_gridder *h, int s, int b, bool need_img)
     sl.spec.ensure(H * b);
     if (need_img) sl.img.ensure(NN * b);
     if (h->img_prec() != kF32) sl.casimg_lp.ensure(MM * b);
-    sl.order.ensure(b);
+    sl.plans.ensure(fp_plan_bytes(b));
     if (!sl.ev_ready) GG_CK(cudaEventCreateWithFlags(&sl.ev_ready, cudaEventDisableTiming));
     if (!sl.ev_free) {
         GG_CK(cudaEventCreateWithFlags(&sl.ev_free, cudaEventDisableTiming));
@@ -303,35 +306,27 @@ void check_axes_count(int n)
     if (n < 0) fail(GG_ERR_INVALID_ARG, "n_axes must be >= 0 (got %d)", n);
 }
 
-// Floats taken by one pitched 2-byte copy of the CAS volume (a multiple of 4,
-// so each copy starts 16-byte aligned).
-size_t fp_copy_floats(const gg_gridder *h)
-{
-    return ((size_t)fp_pitch(h->V) * h->V * h->V * prec_bytes(h->prec) + 15) / 16 * 4;
-}
-
-// Refresh the copies of the CAS volume read by the forward projection.
+// Refresh the copy of the CAS volume read by the forward projection.
 void update_fp(gg_gridder *h, cudaStream_t s)
 {
     if (h->cas_fp_valid) return;
-    if (h->prec == kF32) {
-        // FP32 taps are read one by one: the dense volume and its two transposes
-        const size_t V3 = (size_t)h->V * h->V * h->V;
-        h->cas_y.ensure(V3);
-        h->cas_z.ensure(V3);
-        GG_CK(launch_transpose_volume(h->cas.p, h->V, h->cas_y.p, 1, s));
-        GG_CK(launch_transpose_volume(h->cas.p, h->V, h->cas_z.p, 2, s));
-        h->cas_fp_valid = true;
-        return;
+    const size_t V = h->V, P = fp_pitch(h->V, h->prec);
+    h->cas_fp.ensure(P * V * V * prec_bytes(h->prec));
+    if (h->fp_maps_vol != h->cas_fp.p || h->fp_maps_prec != h->prec) {
+        h->fp_maps.ensure(fp_tile_map_bytes(h->prec));
+        h->fp_maps_prec = -1;
+        GG_CK(fp_tile_make_maps(h->cas_fp.p, h->V, (int)P, h->prec, h->fp_maps.p));
+        h->fp_maps_vol = h->cas_fp.p;
+        h->fp_maps_prec = h->prec;
     }
-    // FP16/BF16: three pitched copies with x, y and z contiguous, back to back
-    const size_t V3 = (size_t)h->V * h->V * h->V;
-    h->cas_fp.ensure(3 * fp_copy_floats(h));
-    if (h->prec == kF16) GG_CK(launch_storage_scale(h->cas.p, V3, 8192.0f, h->work.p, h->scales.p, s));
-    for (int l = 0; l < 3; l++)
-        GG_CK(launch_pitch_volume(h->cas.p, h->V, fp_pitch(h->V), h->cas_fp.p + l * fp_copy_floats(h), h->prec,
-                                  h->vol_scale(), s, l));
+    if (h->prec == kF16) GG_CK(launch_storage_scale(h->cas.p, V * V * V, 8192.0f, h->work.p, h->scales.p, s));
+    GG_CK(launch_pitch_volume(h->cas.p, h->V, (int)P, h->cas_fp.p, h->prec, h->vol_scale(), s));
     h->cas_fp_valid = true;
+}
+
+FpTiles fp_tiles(const gg_gridder *h)
+{
+    return FpTiles{h->cas_fp.p, h->prec, fp_pitch(h->V, h->prec), h->fp_maps.p, h->fault};
 }
 
 // ---- device-side pipelines (all on stream s) --------------------------------
@@ -369,12 +364,12 @@ void fp_batch(gg_gridder *h, const float *d_axes, int b, float *cas_out, float *
 {
     auto &S = h->slot[sl];
     ProfScope ps(h, s, GG_KERNEL_FORWARD);
-    const bool dense = h->prec == kF32;
-    GG_CK(launch_forward_project(dense ? h->cas.p : h->cas_fp.p, h->prec, dense ? h->V : fp_pitch(h->V), cas_out,
-                                 h->ker.p, d_axes, b, h->geom(), h->five_taps, h->vol_scale(), s,
-                                 dense ? (const void *)h->cas_y.p : (const void *)(h->cas_fp.p + fp_copy_floats(h)),
-                                 dense ? (const void *)h->cas_z.p : (const void *)(h->cas_fp.p + 2 * fp_copy_floats(h)),
-                                 S.order.p));
+    if (h->five_taps)
+        GG_CK(launch_forward_project(h->cas_fp.p, h->prec, fp_pitch(h->V, h->prec), cas_out, h->ker.p, d_axes, b,
+                                     h->geom(), true, h->vol_scale(), s));
+    else
+        GG_CK(launch_forward_project_tiled(fp_tiles(h), cas_out, h->ker.p, d_axes, b, h->geom(), h->vol_scale(), s,
+                                           S.plans.p));
     ps.done();
     if (img_out && h->fused_fft) {
         GG_CK(launch_cas_to_images_fused(cas_out, h->M, h->N, b, img_out, s));
@@ -673,6 +668,10 @@ void init_handle(gg_gridder *h)
     GG_CK(cudaMemcpy(h->scales.p, ones, sizeof(ones), cudaMemcpyHostToDevice));
     h->work.ensure(1);
     GG_CK(cudaMemset(h->work.p, 0, sizeof(unsigned int)));
+    void *fault = nullptr;
+    GG_CK(cudaHostAlloc(&fault, sizeof(int), cudaHostAllocDefault));
+    h->fault = (int *)fault;
+    *h->fault = 0;
     h->fused_fft = fft2_fused_ok(h->N, h->M);
 }
 
@@ -698,8 +697,8 @@ void destroy_handle(gg_gridder *h)
     h->precomp.release();
     h->cas.release();
     h->cas_fp.release();
-    h->cas_y.release();
-    h->cas_z.release();
+    h->fp_maps.release();
+    if (h->fault) cudaFreeHost(h->fault);
     h->pd.release();
     h->adj.release();
     h->axes.release();
@@ -728,6 +727,7 @@ template <typename F> int guarded(gg_gridder *h, F &&f)
     try {
         set_device(h);
         f();
+        if (*(volatile int *)h->fault) fail(GG_ERR_CUDA, "a forward projection's copies to shared memory did not arrive");
         h->err.clear();
         return GG_OK;
     } catch (const GGError &e) {
@@ -1450,9 +1450,9 @@ bool gg::gridder_view(gg_gridder *h, GridderView *out)
 {
     if (!h || !h->cas.p) return false;
     std::lock_guard<std::mutex> lock(h->mu);
-    const bool t = h->prec == kF32 && h->cas_fp_valid;
-    *out = GridderView{h->device, h->N, h->M, h->V, h->geom(), h->cas.p, t ? h->cas_y.p : nullptr,
-                       t ? h->cas_z.p : nullptr, h->ker.p, h->five_taps, h->fused_fft};
+    FpTiles t = fp_tiles(h);
+    if (h->prec != kF32 || !h->cas_fp_valid) t.maps = nullptr;
+    *out = GridderView{h->device, h->N, h->M, h->V, h->geom(), h->cas.p, t, h->ker.p, h->five_taps, h->fused_fft};
     return true;
 }
 

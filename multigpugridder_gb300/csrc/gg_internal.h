@@ -31,29 +31,37 @@ struct Geom {
 // kept in device memory (d_scale; NULL means 1) so no host sync is needed.
 // The forward projection multiplies every output pixel by *d_scale.
 // The volume's rows are `pitch` elements apart (planes pitch*V); the
-// reference's dense layout is pitch = V.  fp_pitch(V) rows let the 4-tap
-// kernel read each row of taps with aligned vector loads.
-// d_vol_y, d_vol_z (optional): copies of the volume, in the same storage and
-// pitch, with y and z as the contiguous axis (launch_transpose_volume for
-// dense FP32, launch_pitch_volume layouts 1 and 2 for FP16/BF16); each
-// direction then reads the copy whose contiguous axis is the most
-// perpendicular to it.  d_order (optional, n ints of scratch, used with the
-// copies): the directions then run grouped by the copy they read (a stable
-// partition computed on the device), so that one copy at a time is hot in
-// L2; each image is still written at its direction's slot.
+// reference's dense layout is pitch = V.  2-byte storage only with five_taps
+// (the 4-tap form of a gridder's own volumes is launch_forward_project_tiled).
 cudaError_t launch_forward_project(const void *d_vol, int vprec, int pitch, float *d_img, const float *d_ker,
                                    const float *d_axes, int n, const Geom &g, bool five_taps,
-                                   const float *d_scale, cudaStream_t s, const void *d_vol_y = nullptr,
-                                   const void *d_vol_z = nullptr, int *d_order = nullptr);
-// FP32 volume V^3 (x fastest) -> the same volume with y (layout 1: [z][x][y])
-// or z (layout 2: [y][x][z]) as the contiguous axis.
-cudaError_t launch_transpose_volume(const float *d_in, int V, float *d_out, int layout, cudaStream_t s);
-inline int fp_pitch(int V) { return (V + 4 + 7) / 8 * 8; }
+                                   const float *d_scale, cudaStream_t s);
+
+// ---- forward projection from staged boxes (gg_fp_tile.cu) -------------------
+// Row pitch of the copy of the CAS volume that the tiled forward projection
+// reads: rows of a multiple of 16 bytes, as TMA addresses them.
+inline int fp_pitch(int V, int prec) { return prec == kF32 ? (V + 3) / 4 * 4 : (V + 7) / 8 * 8; }
+// Such a copy with its tensor maps: `maps` is a device buffer of
+// fp_tile_map_bytes(prec), filled by fp_tile_make_maps (synchronous) for this
+// address, V, pitch and storage.  `fault` (device-accessible) is set to 1 by a
+// kernel whose copies did not arrive.
+struct FpTiles {
+    const void *vol;
+    int prec, pitch;
+    const void *maps;
+    int *fault;
+};
+size_t fp_tile_map_bytes(int prec);
+cudaError_t fp_tile_make_maps(const void *d_vol, int V, int pitch, int prec, void *d_maps);
+// Scratch of one launch of n directions.
+size_t fp_plan_bytes(int n);
+// 4-tap forward projection (zero table edges); d_plans: fp_plan_bytes(n).
+cudaError_t launch_forward_project_tiled(const FpTiles &v, float *d_img, const float *d_ker, const float *d_axes, int n,
+                                         const Geom &g, const float *d_scale, cudaStream_t s, void *d_plans);
 // FP32 CAS volume V^3 -> the same volume with row pitch P (zero-filled past
-// V) in storage `prec` (x / *d_scale for FP16), with x (layout 0: [z][y][x]),
-// y (layout 1: [z][x][y]) or z (layout 2: [y][x][z]) as the contiguous axis.
+// V) in storage `prec` (x / *d_scale for FP16).
 cudaError_t launch_pitch_volume(const float *d_cas, int V, int P, void *d_out, int prec, const float *d_scale,
-                                cudaStream_t s, int layout = 0);
+                                cudaStream_t s);
 
 // Back projection with the reference window rule, accumulated (+=) into the
 // FP32 CAS volume.  d_img holds n*M*M CAS images in storage `iprec`; when
@@ -182,7 +190,7 @@ struct GridderView {
     int device, N, M, V;
     Geom g;
     const float *cas; // FP32 CAS volume V^3
-    const float *cas_y, *cas_z; // its copies with y / z contiguous (may be null)
+    FpTiles tiles;    // its copy for the tiled forward projection (maps null if not prepared as FP32)
     const float *ker; // KB table
     bool five_taps;
     bool fused_fft;   // fft2_fused_ok(N, M)

@@ -14,8 +14,8 @@
 #include <cstring>
 #include <type_traits>
 
-#include "gg_common.cuh"
 #include "gg_internal.h"
+#include "gg_project.cuh"
 
 namespace gg {
 
@@ -23,40 +23,12 @@ namespace gg {
 // Shared pieces
 // ---------------------------------------------------------------------------
 
-// Sample point of pixel (di, dj) (offsets from the image centre) in the CAS
-// volume frame: the reference's nx*di + ny*dj + volCenter
-// (gpuForwardProject.cu:53-55) as its build evaluates it, fma(nx, di, ny*dj) +
-// vc, written with round-to-nearest intrinsics so the grouping cannot change.
-// Shared by the forward and adjoint kernels so both see identical bits.
-__device__ __forceinline__ float sample_coord(float n_x, float n_y, int di, int dj, int vc)
-{
-    return __fadd_rn(__fmaf_rn(n_x, (float)di, __fmul_rn(n_y, (float)dj)), (float)vc);
-}
-
 // A voxel's image-frame coordinate (gpuBackProject.cu:62-64),
 // fma(a2, n2, fma(a0, n0, a1*n1)); every grouping of the three products gave
 // the same results against the reference kernel, this one is fixed here.
 __device__ __forceinline__ float voxel_proj(float a0, float a1, float a2, float n0, float n1, float n2)
 {
     return __fmaf_rn(a2, n2, __fmaf_rn(a0, n0, __fmul_rn(a1, n1)));
-}
-
-// Table lookup of the reference's nearest-index KB rule,
-// ker[roundf(fma(r, kerScale, kerCenter))], as floor(fma(r, kerScale,
-// kerCenter + 1/2)): equal for every float r in [-2, 2] (checked
-// exhaustively) and one conversion instead of a roundf and a conversion.
-// Callers pass r in [-2, 2]; the clamp only keeps a NaN or infinite
-// coordinate (bad axes) inside the table.  Entry k is read at sker[k * rep]
-// (rep interleaved copies).
-__device__ __forceinline__ float kb_weight(const float *sker, float r, float kerScale, float kerCenterHalf, int kerSize,
-                                           int rep = 1)
-{
-    return sker[min(max(__float2int_rd(__fmaf_rn(r, kerScale, kerCenterHalf)), 0), kerSize - 1) * rep];
-}
-
-__device__ __forceinline__ void load_table(float *sker, const float *ker, int kerSize)
-{
-    for (int t = threadIdx.x; t < kerSize; t += blockDim.x) sker[t] = __ldg(ker + t);
 }
 
 // An attribute of the current device, cached per device ordinal (a process
@@ -94,6 +66,11 @@ static int num_sms()
 // ---------------------------------------------------------------------------
 // Forward projection
 // ---------------------------------------------------------------------------
+// The gridder's own volumes take fp_tile_kernel (gg_fp_tile.cu).  fp_kernel
+// reads the taps from global memory: for a caller's dense volume, which TMA
+// cannot address (its rows are not multiples of 16 bytes), and for KB tables
+// whose edges are not zero.
+//
 // One CTA = a 16x16 pixel tile of one direction; persistent grid-stride loop
 // over (direction, tile) items, direction-major so that the CTAs resident at
 // any time read the same few slabs of the volume.  Warps cover 8x4 pixel
@@ -107,126 +84,15 @@ static int num_sms()
 // reference's full window for tables without zero edges.
 //
 // The volume may be stored with a row pitch P >= V (plane pitch P*V; the
-// reference's dense layout is P = V).  VEC (2-byte storage, 4 taps, P a
-// multiple of 8, P >= V + 4): each row of 4 taps is read as the 8 elements from the 4-aligned
-// x at or below floor(f) - 1 in two aligned vector loads, and the 4 x weights
-// are placed at their offsets in an 8-wide weight vector (zeros elsewhere) once
-// per pixel.  The extra terms are exact zeros, so the sums are those of the
-// 4 scalar taps, bit for bit, for a finite volume.
+// reference's dense layout is P = V).
 constexpr int kFpTile = 16;
 constexpr int kFpThreads = 256;
 
-__device__ __forceinline__ void ld8(const float *p, float v[8])
-{
-    const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
-    const float4 b = __ldg(reinterpret_cast<const float4 *>(p) + 1);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-}
-
-__device__ __forceinline__ void ld8(const __half *p, float v[8])
-{
-    const uint2 a = __ldg(reinterpret_cast<const uint2 *>(p));
-    const uint2 b = __ldg(reinterpret_cast<const uint2 *>(p) + 1);
-    const unsigned w[4] = {a.x, a.y, b.x, b.y};
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w[q]));
-        v[2 * q] = f.x;
-        v[2 * q + 1] = f.y;
-    }
-}
-
-__device__ __forceinline__ void ld8(const __nv_bfloat16 *p, float v[8])
-{
-    const uint2 a = __ldg(reinterpret_cast<const uint2 *>(p));
-    const uint2 b = __ldg(reinterpret_cast<const uint2 *>(p) + 1);
-    const unsigned w[4] = {a.x, a.y, b.x, b.y};
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        v[2 * q] = __uint_as_float(w[q] << 16);
-        v[2 * q + 1] = __uint_as_float(w[q] & 0xFFFF0000u);
-    }
-}
-
-// The copy a TR forward projection reads for a direction (layout 0: x,
-// 1: y, 2: z contiguous): the one whose contiguous axis is the most
-// perpendicular to the viewing direction (ax + 6 .. ax + 8).
-__device__ __forceinline__ int fp_copy_of(const float *ax)
-{
-    const float nz0 = fabsf(__ldg(ax + 6)), nz1 = fabsf(__ldg(ax + 7)), nz2 = fabsf(__ldg(ax + 8));
-    return (nz1 < nz0 && nz1 <= nz2) ? 1 : (nz2 < nz0 && nz2 < nz1) ? 2 : 0;
-}
-
-// Directions of a TR launch grouped by the copy they read: order[] lists the
-// directions reading copy 0, then copy 1, then copy 2, each group in
-// direction order (a stable partition).  The forward projection runs its
-// work in this order, so that at any time the directions in flight read one
-// copy of the volume (72 MB at 128^3) instead of all three (216 MB, more
-// than the 126 MB L2).  One CTA: counts, then each chunk of 1,024
-// directions scattered with warp ballots and the running offsets.
-constexpr int kOrdThreads = 1024;
-
-__global__ void __launch_bounds__(kOrdThreads) fp_order_kernel(const float *__restrict__ axes, int n, int *__restrict__ order)
-{
-    __shared__ int cnt[3], base[3];
-    __shared__ int wcnt[kOrdThreads / 32][3];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x < 3) cnt[threadIdx.x] = 0;
-    __syncthreads();
-    int c[3] = {0, 0, 0};
-    for (int a = threadIdx.x; a < n; a += kOrdThreads) c[fp_copy_of(axes + 9 * (size_t)a)]++;
-#pragma unroll
-    for (int l = 0; l < 3; l++) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) c[l] += __shfl_xor_sync(0xffffffffu, c[l], o);
-        if (lane == 0) atomicAdd(&cnt[l], c[l]);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        base[0] = 0;
-        base[1] = cnt[0];
-        base[2] = cnt[0] + cnt[1];
-    }
-    __syncthreads();
-    const unsigned lt = (1u << lane) - 1u;
-    for (int c0 = 0; c0 < n; c0 += kOrdThreads) {
-        const int a = c0 + threadIdx.x;
-        const int l = a < n ? fp_copy_of(axes + 9 * (size_t)a) : 3;
-        unsigned m[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) m[k] = __ballot_sync(0xffffffffu, l == k);
-        if (lane < 3) wcnt[warp][lane] = __popc(m[lane]);
-        __syncthreads();
-        if (l < 3) {
-            int pos = base[l] + __popc(m[l] & lt);
-            for (int w = 0; w < warp; w++) pos += wcnt[w][l];
-            order[pos] = a;
-        }
-        __syncthreads();
-        if (threadIdx.x < 3) {
-            int t = 0;
-            for (int w = 0; w < kOrdThreads / 32; w++) t += wcnt[w][threadIdx.x];
-            base[threadIdx.x] += t;
-        }
-        __syncthreads();
-    }
-}
-
-// TR: two more copies of the volume with y and z as the contiguous axis
-// (volY[z][x][y], volZ[y][x][z]).  A warp's 8x4 pixels touch about
-// 32 |n . e_c| + (perimeter) distinct volume rows per gather, e_c the
-// contiguous axis and n the viewing direction, so each direction reads the
-// copy whose contiguous axis is the most perpendicular to n.  FP32 (dense
-// copies): each thread still sums its taps in the same order, so the results
-// are identical.  VEC (pitched 2-byte copies): the rows of taps are read along
-// the copy's contiguous axis, which changes only the order of the sums.
-template <typename TV, int TAPS, bool VEC, bool TR = false>
+template <typename TV, int TAPS>
 __global__ void __launch_bounds__(kFpThreads)
 fp_kernel(const TV *__restrict__ vol, int V, int P, float *__restrict__ img, int M,
           const float *__restrict__ axes, int maskR, const float *__restrict__ ker, int kerSize,
-          float kerHW, int tilesX, long long nItems, const float *__restrict__ d_scale,
-          const TV *__restrict__ volY, const TV *__restrict__ volZ, const int *__restrict__ order)
+          float kerHW, int tilesX, long long nItems, const float *__restrict__ d_scale)
 {
     const float outScale = d_scale ? *d_scale : 1.0f;
     __shared__ float sker[kMaxKerSize];
@@ -234,9 +100,8 @@ fp_kernel(const TV *__restrict__ vol, int V, int P, float *__restrict__ img, int
     __syncthreads();
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // 8x4 warp tiles (2 x 4 per CTA), or with TR 4x8 tiles (4 x 2) when the
-    // copy's contiguous axis advances more per image row than per column, so
-    // that the eight-pixel side of a warp runs along the volume's rows
+    // 8x4 warp tiles (2 x 4 per CTA)
+    const int lx = (lane & 7) | ((warp & 1) << 3), ly = (lane >> 3) | ((warp >> 1) << 2);
     const int ic = M / 2, vc = V / 2;
     const float kerCenter = ((float)kerSize - 1) / 2;
     const float kerScale = kerCenter / kerHW;
@@ -249,20 +114,9 @@ fp_kernel(const TV *__restrict__ vol, int V, int P, float *__restrict__ img, int
 
     const bool items32 = nItems <= 0x7fffffffLL; // 32-bit division per item whenever it fits
     for (long long item = blockIdx.x; item < nItems; item += gridDim.x) {
-        const int slot = items32 ? (int)((unsigned)item / (unsigned)tilesPerImg) : (int)(item / tilesPerImg);
-        const int t = (int)(item - (long long)slot * tilesPerImg);
-        const int a = order ? __ldg(order + slot) : slot; // the direction (and image) of this work slot
+        const int a = items32 ? (int)((unsigned)item / (unsigned)tilesPerImg) : (int)(item / tilesPerImg);
+        const int t = (int)(item - (long long)a * tilesPerImg);
         const float *ax = axes + 9 * (size_t)a;
-        // the copy (layout 0: x, 1: y, 2: z contiguous) whose contiguous axis
-        // is the most perpendicular to the direction
-        int lay = 0;
-        bool tall = false;
-        if (TR) {
-            lay = fp_copy_of(ax);
-            tall = fabsf(__ldg(ax + 3 + lay)) > fabsf(__ldg(ax + lay));
-        }
-        const int lx = tall ? (lane >> 3) | ((warp & 3) << 2) : (lane & 7) | ((warp & 1) << 3);
-        const int ly = tall ? (lane & 7) | ((warp >> 2) << 3) : (lane >> 3) | ((warp >> 1) << 2);
         const int i = (t % tilesX) * kFpTile + lx;
         const int j = (t / tilesX) * kFpTile + ly;
         if (i >= M || j >= M) continue;
@@ -304,55 +158,8 @@ fp_kernel(const TV *__restrict__ vol, int V, int P, float *__restrict__ img, int
         }
 
         float acc = 0.0f;
-        const bool inside = b0 >= 0 && b1 >= 0 && b2 >= 0 && b0 + TAPS <= V && b1 + TAPS <= V && b2 + TAPS <= V;
-        if (VEC && inside) {
-            // the copy's axes, fastest first
-            const int bc = lay == 0 ? b0 : lay == 1 ? b1 : b2;       // contiguous axis
-            const int bb = lay == 0 ? b1 : b0;                        // middle axis
-            const int ba = lay == 2 ? b1 : b2;                        // outer axis
-            float wc[TAPS], wb[TAPS], wa[TAPS];
-#pragma unroll
-            for (int d = 0; d < TAPS; d++) {
-                wc[d] = lay == 0 ? wi[d] : lay == 1 ? wj[d] : wk[d];
-                wb[d] = lay == 0 ? wj[d] : wi[d];
-                wa[d] = lay == 2 ? wj[d] : wk[d];
-            }
-            const int sft = bc & 3;
-            float w8[8];
-#pragma unroll
-            for (int t = 0; t < 8; t++)
-                w8[t] = t == sft ? wc[0] : t == sft + 1 ? wc[1] : t == sft + 2 ? wc[2] : t == sft + 3 ? wc[3] : 0.0f;
-            const TV *base = (lay == 0 ? vol : lay == 1 ? volY : volZ) + (size_t)ba * PV + (size_t)bb * P + (bc - sft);
-#pragma unroll
-            for (int dk = 0; dk < TAPS; dk++) {
-#pragma unroll
-                for (int dj2 = 0; dj2 < TAPS; dj2++) {
-                    float v[8];
-                    ld8(base + (size_t)dk * PV + (size_t)dj2 * P, v);
-                    float s = 0.0f;
-#pragma unroll
-                    for (int t = 0; t < 8; t++) s = fmaf(w8[t], v[t], s);
-                    acc = fmaf(wb[dj2] * wa[dk], s, acc);
-                }
-            }
-        } else if (TR && inside) {
-            // element strides of x, y, z in the chosen copy
-            const size_t sx = lay == 0 ? 1 : (size_t)V;
-            const size_t sy = lay == 0 ? (size_t)V : lay == 1 ? 1 : VV;
-            const size_t sz = lay == 2 ? 1 : VV;
-            const TV *base = (lay == 0 ? vol : lay == 1 ? volY : volZ) + b0 * sx + b1 * sy + b2 * sz;
-#pragma unroll
-            for (int dk = 0; dk < TAPS; dk++) {
-#pragma unroll
-                for (int dj2 = 0; dj2 < TAPS; dj2++) {
-                    const TV *p = base + dk * sz + dj2 * sy;
-                    float s = 0.0f;
-#pragma unroll
-                    for (int d = 0; d < TAPS; d++) s = fmaf(wi[d], ld_f32(p + d * sx), s);
-                    acc = fmaf(wj[dj2] * wk[dk], s, acc);
-                }
-            }
-        } else if (inside) {
+        const bool inside = b0 >= 0 && b1 >= 0 && b2 >= 0 && b0 <= V - TAPS && b1 <= V - TAPS && b2 <= V - TAPS;
+        if (inside) {
             const TV *base = vol + (size_t)b2 * PV + (size_t)b1 * P + b0;
 #pragma unroll
             for (int dk = 0; dk < TAPS; dk++) {
@@ -382,63 +189,33 @@ fp_kernel(const TV *__restrict__ vol, int V, int P, float *__restrict__ img, int
     }
 }
 
-template <typename TV, int TAPS, bool VEC, bool TR = false>
-static cudaError_t launch_fp_t(const TV *vol, int P, float *img, const float *ker, const float *axes, int n,
-                               const Geom &g, const float *scale, cudaStream_t s, const TV *volY = nullptr,
-                               const TV *volZ = nullptr, int *order = nullptr)
+template <typename TV, int TAPS>
+static cudaError_t launch_fp_t(const void *d_vol, int P, float *img, const float *ker, const float *axes, int n,
+                               const Geom &g, const float *scale, cudaStream_t s)
 {
     const int tilesX = (g.M + kFpTile - 1) / kFpTile;
     const long long nItems = (long long)n * tilesX * tilesX;
     if (nItems == 0) return cudaSuccess;
-    if (!TR) order = nullptr;
-    if (order) {
-        fp_order_kernel<<<1, kOrdThreads, 0, s>>>(axes, n, order);
-        count_launches(1);
-    }
     int perSm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fp_kernel<TV, TAPS, VEC, TR>, kFpThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fp_kernel<TV, TAPS>, kFpThreads, 0);
     if (perSm <= 0) perSm = 1;
     long long grid = (long long)num_sms() * perSm;
     if (grid > nItems) grid = nItems;
-    fp_kernel<TV, TAPS, VEC, TR><<<(unsigned)grid, kFpThreads, 0, s>>>(vol, g.V, P, img, g.M, axes, g.mask_radius,
-                                                                        ker, g.ker_size, g.ker_hw, tilesX, nItems,
-                                                                        scale, volY, volZ, order);
+    fp_kernel<TV, TAPS><<<(unsigned)grid, kFpThreads, 0, s>>>((const TV *)d_vol, g.V, P, img, g.M, axes, g.mask_radius,
+                                                              ker, g.ker_size, g.ker_hw, tilesX, nItems, scale);
     count_launches(1);
     return cudaGetLastError();
 }
 
-template <typename TV>
-static cudaError_t launch_fp_p(const void *d_vol, int P, float *d_img, const float *d_ker, const float *d_axes, int n,
-                               const Geom &g, bool five_taps, const float *scale, cudaStream_t s,
-                               const void *d_vol_y, const void *d_vol_z, int *d_order)
-{
-    const TV *v = (const TV *)d_vol;
-    if (five_taps) return launch_fp_t<TV, 5, false>(v, P, d_img, d_ker, d_axes, n, g, scale, s);
-    const TV *vy = (const TV *)d_vol_y, *vz = (const TV *)d_vol_z;
-    if (sizeof(TV) == 4 && vy && vz && P == g.V)
-        return launch_fp_t<TV, 4, false, true>(v, P, d_img, d_ker, d_axes, n, g, scale, s, vy, vz, d_order);
-    // 2-byte storage only: with FP32 the 8-element rows double the bytes each
-    // tap row moves through L1, which costs more than the loads it saves
-    const bool vec = sizeof(TV) == 2 && P % 8 == 0 && P >= g.V + 4 && ((size_t)d_vol & 15) == 0;
-    const bool aligned = ((size_t)vy & 15) == 0 && ((size_t)vz & 15) == 0;
-    if (vec && vy && vz && aligned)
-        return launch_fp_t<TV, 4, true, true>(v, P, d_img, d_ker, d_axes, n, g, scale, s, vy, vz, d_order);
-    if (vec) return launch_fp_t<TV, 4, true>(v, P, d_img, d_ker, d_axes, n, g, scale, s);
-    return launch_fp_t<TV, 4, false>(v, P, d_img, d_ker, d_axes, n, g, scale, s);
-}
-
 cudaError_t launch_forward_project(const void *d_vol, int vprec, int pitch, float *d_img, const float *d_ker,
                                    const float *d_axes, int n, const Geom &g, bool five_taps, const float *scale,
-                                   cudaStream_t s, const void *d_vol_y, const void *d_vol_z, int *d_order)
+                                   cudaStream_t s)
 {
-    if (vprec == kF32)
-        return launch_fp_p<float>(d_vol, pitch, d_img, d_ker, d_axes, n, g, five_taps, scale, s, d_vol_y, d_vol_z,
-                                  d_order);
-    if (vprec == kF16)
-        return launch_fp_p<__half>(d_vol, pitch, d_img, d_ker, d_axes, n, g, five_taps, scale, s, d_vol_y, d_vol_z,
-                                   d_order);
-    return launch_fp_p<__nv_bfloat16>(d_vol, pitch, d_img, d_ker, d_axes, n, g, five_taps, scale, s, d_vol_y, d_vol_z,
-                                      d_order);
+    if (vprec == kF32 && !five_taps) return launch_fp_t<float, 4>(d_vol, pitch, d_img, d_ker, d_axes, n, g, scale, s);
+    if (!five_taps) return cudaErrorInvalidValue; // 2-byte volumes with zero table edges are projected by tiles
+    if (vprec == kF32) return launch_fp_t<float, 5>(d_vol, pitch, d_img, d_ker, d_axes, n, g, scale, s);
+    if (vprec == kF16) return launch_fp_t<__half, 5>(d_vol, pitch, d_img, d_ker, d_axes, n, g, scale, s);
+    return launch_fp_t<__nv_bfloat16, 5>(d_vol, pitch, d_img, d_ker, d_axes, n, g, scale, s);
 }
 
 // ---------------------------------------------------------------------------

@@ -141,7 +141,7 @@ struct Request {
     // device buffers, allocated by the first chunk and freed by the last
     float *d_axes = nullptr, *d_cas = nullptr, *d_real = nullptr, *d_img = nullptr, *d_acc = nullptr;
     cufftComplex *d_spec = nullptr;
-    int *d_order = nullptr;
+    unsigned char *d_plans = nullptr;
     int status = GG_OK;
     std::string err;
     double t_submit = 0, t_start = 0, t_done = 0;
@@ -221,7 +221,7 @@ void plan_request(Request &r, double quantum)
     r.chunk = std::min(c, pow2ceil(std::max(r.n, 1)));
     const size_t b = (size_t)r.chunk;
     size_t bytes = (size_t)std::max(r.n, 1) * 9 * sizeof(float);
-    bytes += b * (MM * sizeof(float) + NN * sizeof(float) + sizeof(int));
+    bytes += b * (MM * sizeof(float) + NN * sizeof(float)) + fp_plan_bytes((int)b);
     if (!v.fused_fft) bytes += b * (H * sizeof(cufftComplex) + MM * sizeof(float));
     if (r.op == GG_OP_BACK) bytes += (size_t)v.V * v.V * v.V * sizeof(float);
     r.footprint = bytes;
@@ -293,12 +293,12 @@ template <typename T> T *pool_alloc(gg_server *S, size_t count, cudaStream_t s)
 // cudaFreeAsync) and clears them.
 void take_buffers(Request &r, std::vector<void *> &out)
 {
-    void *bufs[] = {r.d_acc, r.d_order, r.d_img, r.d_real, r.d_spec, r.d_cas, r.d_axes};
+    void *bufs[] = {r.d_acc, r.d_plans, r.d_img, r.d_real, r.d_spec, r.d_cas, r.d_axes};
     for (void *p : bufs)
         if (p) out.push_back(p);
     r.d_acc = r.d_cas = r.d_real = r.d_img = r.d_axes = nullptr;
     r.d_spec = nullptr;
-    r.d_order = nullptr;
+    r.d_plans = nullptr;
 }
 
 void free_buffers(Request &r, cudaStream_t s)
@@ -330,7 +330,7 @@ void enqueue_chunk(gg_server *S, Request &r)
             r.d_spec = pool_alloc<cufftComplex>(S, H * B, s);
             r.d_real = pool_alloc<float>(S, MM * B, s);
         }
-        if (r.op == GG_OP_FORWARD) r.d_order = pool_alloc<int>(S, B, s);
+        if (r.op == GG_OP_FORWARD) r.d_plans = pool_alloc<unsigned char>(S, fp_plan_bytes(B), s);
         if (r.n > 0)
             GS_CK(cudaMemcpyAsync(r.d_axes, r.axes, (size_t)r.n * 9 * sizeof(float), cudaMemcpyHostToDevice, s));
         if (r.op == GG_OP_BACK) {
@@ -348,8 +348,10 @@ void enqueue_chunk(gg_server *S, Request &r)
         }
         const float *axes = r.d_axes + (size_t)c0 * 9;
         if (r.op == GG_OP_FORWARD) {
-            GS_CK(launch_forward_project(v.cas, kF32, v.V, r.d_cas, v.ker, axes, b, v.g, v.five_taps, nullptr, s,
-                                         v.cas_y, v.cas_z, r.d_order));
+            if (v.tiles.maps && !v.five_taps)
+                GS_CK(launch_forward_project_tiled(v.tiles, r.d_cas, v.ker, axes, b, v.g, nullptr, s, r.d_plans));
+            else
+                GS_CK(launch_forward_project(v.cas, kF32, v.V, r.d_cas, v.ker, axes, b, v.g, v.five_taps, nullptr, s));
             if (v.fused_fft) {
                 GS_CK(launch_cas_to_images_fused(r.d_cas, v.M, v.N, b, r.d_img, s));
             } else {
