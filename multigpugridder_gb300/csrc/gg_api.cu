@@ -158,6 +158,7 @@ struct gg_gridder {
     bool cas_fp_valid = false;  // cas_fp matches cas
     int *fault = nullptr;       // pinned: set by a kernel whose copies did not arrive
     DevBuf<float> pd;        // plane density V^3
+    DevBuf<float> bp_part;   // sums of a split back projection's segments
     DevBuf<float> adj;       // CAS-volume gradient V^3 (forward-operator adjoint)
     DevBuf<float> axes;
     DevBuf<float> vol_io;    // N^3
@@ -382,6 +383,15 @@ void fp_batch(gg_gridder *h, const float *d_axes, int b, float *cas_out, float *
     }
 }
 
+// The split of a back projection of b directions, with room for its sums
+// (`stacks`: 2 with a density or a second image stack).
+BpSplit bp_split(gg_gridder *h, int b, int stacks)
+{
+    const int nseg = bp_segments(b, h->geom());
+    if (nseg > 1) h->bp_part.ensure((size_t)(nseg - 1) * stacks * h->V * h->V * h->V);
+    return BpSplit{nseg, h->bp_part.p};
+}
+
 // Back-project b directions: images (device, FFT path) or CAS images (device).
 // With `pd`, the plane density of the same directions is accumulated into pd
 // as well (fused into the same kernel for the reference rule).
@@ -436,10 +446,12 @@ void bp_batch(gg_gridder *h, const float *d_axes, int b, const float *img, const
     if (h->bp_mode == GG_BP_ADJOINT && !ones) {
         GG_CK(launch_back_project_adjoint(target, src, iprec, h->ker.p, d_axes, b, h->geom(), scale, !h->five_taps, s));
     } else if (pd && !ones) {
-        GG_CK(launch_back_project_ref_density(target, pd, src, iprec, h->ker.p, d_axes, b, h->geom(), scale, s));
+        GG_CK(launch_back_project_ref_density(target, pd, src, iprec, h->ker.p, d_axes, b, h->geom(), scale, s,
+                                              bp_split(h, b, 2)));
         pd = nullptr;
     } else {
-        GG_CK(launch_back_project_ref(target, src, iprec, ones, h->ker.p, d_axes, b, h->geom(), scale, s));
+        GG_CK(launch_back_project_ref(target, src, iprec, ones, h->ker.p, d_axes, b, h->geom(), scale, s, false,
+                                      bp_split(h, b, 1)));
     }
     ps.done();
     if (pd) {
@@ -473,7 +485,8 @@ void ctf_batch(gg_gridder *h, const float *d_axes, int b, const float *img, cons
     if (h->img_prec() == kF32 && h->bp_mode != GG_BP_ADJOINT) {
         // both stacks in one back-projection pass
         ProfScope ps(h, s, GG_KERNEL_BACK);
-        GG_CK(launch_back_project_ref_pair(h->cas.p, h->pd.p, S.casimg.p, S.real.p, h->ker.p, d_axes, b, h->geom(), s));
+        GG_CK(launch_back_project_ref_pair(h->cas.p, h->pd.p, S.casimg.p, S.real.p, h->ker.p, d_axes, b, h->geom(), s,
+                                           bp_split(h, b, 2)));
         ps.done();
     } else {
         bp_batch(h, d_axes, b, nullptr, S.casimg.p, h->cas.p, false, sl, s);
@@ -700,6 +713,7 @@ void destroy_handle(gg_gridder *h)
     h->fp_maps.release();
     if (h->fault) cudaFreeHost(h->fault);
     h->pd.release();
+    h->bp_part.release();
     h->adj.release();
     h->axes.release();
     h->vol_io.release();

@@ -63,6 +63,17 @@ cudaError_t launch_forward_project_tiled(const FpTiles &v, float *d_img, const f
 cudaError_t launch_pitch_volume(const float *d_cas, int V, int P, void *d_out, int prec, const float *d_scale,
                                 cudaStream_t s);
 
+// A back projection split into nseg contiguous segments of its directions, run
+// side by side: segment 0 accumulates into the volume as an unsplit launch
+// does, the others write their sums to `part` ((nseg - 1) * V^3 floats, twice
+// that with a density), and a merge adds them in order.  nseg = 1: unsplit.
+struct BpSplit {
+    int nseg;
+    float *part;
+};
+// The number of segments for n directions.
+int bp_segments(int n, const Geom &g);
+
 // Back projection with the reference window rule, accumulated (+=) into the
 // FP32 CAS volume.  d_img holds n*M*M CAS images in storage `iprec`; when
 // `ones` is set the images are taken to be all ones (plane density) and
@@ -72,19 +83,21 @@ cudaError_t launch_pitch_volume(const float *d_cas, int V, int P, void *d_out, i
 // images, the same sums bit for bit).
 cudaError_t launch_back_project_ref(float *d_vol, const void *d_img, int iprec, bool ones,
                                     const float *d_ker, const float *d_axes, int n, const Geom &g,
-                                    const float *d_scale, cudaStream_t s, bool shared = false);
+                                    const float *d_scale, cudaStream_t s, bool shared = false,
+                                    BpSplit split = {1, nullptr});
 
 // Reference-rule back projection of d_img into d_vol and, in the same pass,
 // of all-ones images (the plane density) into d_pd; both accumulated.
 cudaError_t launch_back_project_ref_density(float *d_vol, float *d_pd, const void *d_img, int iprec,
                                             const float *d_ker, const float *d_axes, int n, const Geom &g,
-                                            const float *d_scale, cudaStream_t s);
+                                            const float *d_scale, cudaStream_t s, BpSplit split = {1, nullptr});
 
 // Reference-rule back projection of two FP32 image stacks over the same
 // directions in one pass: d_img into d_vol and d_img2 into d_pd, both
 // accumulated, each equal to its own launch_back_project_ref.
 cudaError_t launch_back_project_ref_pair(float *d_vol, float *d_pd, const float *d_img, const float *d_img2,
-                                         const float *d_ker, const float *d_axes, int n, const Geom &g, cudaStream_t s);
+                                         const float *d_ker, const float *d_axes, int n, const Geom &g, cudaStream_t s,
+                                         BpSplit split = {1, nullptr});
 
 // Exact adjoint of launch_forward_project (4 taps), accumulated into d_vol.
 // zero_edges: the KB table's first and last entries are 0 (the fast path

@@ -639,31 +639,55 @@ struct BpGroupMem {
 // axis is max(|2 B i + B - 1 - 2c| - (B - 1), 0) for bricks of size B, all
 // integers, so the test is exact; along x the bricks that pass form the
 // interval |2 B i + B - 1 - 2c| <= B - 1 + t, t = isqrt(rem).
-__device__ __forceinline__ int box_dist2(int i, int B, int c)
+__host__ __device__ __forceinline__ int box_dist2(int i, int B, int c)
 {
-    return max(abs(2 * B * i + B - 1 - 2 * c) - (B - 1), 0);
+    const int d = 2 * B * i + B - 1 - 2 * c, e = (d < 0 ? -d : d) - (B - 1);
+    return e > 0 ? e : 0;
 }
 
-__device__ __forceinline__ int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
+__host__ __device__ __forceinline__ int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
-__device__ void brick_row(int j, int k, int bricksX, int c, int BZ, int reach, int &lo, int &n)
+__host__ __device__ inline void brick_row(int j, int k, int bricksX, int c, int BZ, int reach, int &lo, int &n)
 {
     const long long dy = box_dist2(j, kCBY, c), dz = box_dist2(k, BZ, c);
     const long long rem = 4 * ((long long)reach * reach + 1) - dy * dy - dz * dz;
     lo = 0;
     n = 0;
     if (rem < 0) return;
-    long long t = (long long)sqrt((double)rem);
+    long long t = (long long)sqrtf((float)rem); // a guess, corrected below
     while (t * t > rem) t--;
     while ((t + 1) * (t + 1) <= rem) t++;
     const int B = kCBX;
-    const int ilo = max(-floor_div(-(2 * c - 2 * (B - 1) - (int)t), 2 * B), 0); // ceil
-    const int ihi = min(floor_div(2 * c + (int)t, 2 * B), bricksX - 1);
+    int ilo = -floor_div(-(2 * c - 2 * (B - 1) - (int)t), 2 * B); // ceil
+    if (ilo < 0) ilo = 0;
+    int ihi = floor_div(2 * c + (int)t, 2 * B);
+    if (ihi > bricksX - 1) ihi = bricksX - 1;
     if (ihi >= ilo) {
         lo = ilo;
         n = ihi - ilo + 1;
     }
 }
+
+// Rank r of 0 .. n - 1 from the middle outwards: the bricks near the centre,
+// which the most directions reach, start first, and the light ones at the rim
+// fill the last wave (two-stack form, 1,000 images at M = 256: 7.94 -> 7.53 ms
+// a call; reconstructVol of 1,000 at M = 128: 4.81 -> 4.58 ms before the
+// segments).
+__host__ __device__ __forceinline__ int middle_out(int r, int n)
+{
+    const int c = (n - 1) / 2;
+    return r & 1 ? c + (r + 1) / 2 : c - r / 2;
+}
+
+// The CTAs of a launch, layer by layer from the middle outwards: layer rank r
+// holds the brick runs pre[r] .. pre[r + 1] - 1.  Counted on the host, so that
+// no CTA starts (and takes a whole SM) without bricks: at M = 256 the box of
+// bricks holds 6,182 runs, of which 1,900 meet the sphere (reconstructVol of
+// 1,000 images 6.99 -> 6.66 ms, of 16 images 688 -> 618 us).
+constexpr int kMaxLayers = 511; // 6,132 voxels of 12-deep bricks: 860 GB of CAS volume
+struct BpLayers {
+    int layers, pre[kMaxLayers + 1];
+};
 
 __device__ __forceinline__ void group_sync(int id)
 {
@@ -671,12 +695,13 @@ __device__ __forceinline__ void group_sync(int id)
 }
 
 template <typename TI, bool ONES, bool DENS, bool ADJ, bool DW = false, bool DEEP = false, int G = kBpGroups,
-          int TS = 0, bool LEAN = true>
+          int TS = 0, bool LEAN = true, bool SPLIT = false>
 __global__ void __launch_bounds__(kCThreads *G, G == 1 ? 3 : 1)
 bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, const TI *__restrict__ img, int M,
                       const float *__restrict__ axes, int n, int maskR, const float *__restrict__ ker, int kerSize,
                       float kerHW, int bricksX, int bricksY, BpTable tb, int zeroEdges,
-                      const float *__restrict__ d_scale, const float *__restrict__ img2, int vecImg)
+                      const float *__restrict__ d_scale, const float *__restrict__ img2, int vecImg, BpSplit split,
+                      const __grid_constant__ BpLayers lay)
 {
     static_assert(!DW || (!ONES && !DENS && !ADJ), "the second image stack is a reference-rule option");
     constexpr int W = ADJ ? 7 : 5, HALF = W / 2;
@@ -695,18 +720,27 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
     const int volCenter = (int)((float)V) / 2;
     const int imgCenter = (int)((float)M) / 2;
 
-    // The CTA's bricks: those of z-layer blockIdx.y that meet the sphere of
-    // radius `reach` (the adjoint reaches voxels up to 2*sqrt(3) beyond the
-    // mask), numbered row by row; the CTA takes the run of RUN * G numbers
-    // from RUN * G * blockIdx.x (below).  Row (y, z) holds the x interval
-    // [slo, slo + n).
+    // The CTA's bricks: those of z-layer kz that meet the sphere of radius
+    // `reach` (the adjoint reaches voxels up to 2*sqrt(3) beyond the mask),
+    // numbered row by row; the CTA takes run `run` of RUN * G numbers (below).
+    // Row (y, z) holds the x interval [slo, slo + n).
+    // SPLIT: a run's segments of the directions are neighbours in the grid.
     const int reach = ADJ ? maskR + 4 : maskR;
-    const int kz = blockIdx.y;
+    const int ns = SPLIT ? split.nseg : 1, item = SPLIT ? blockIdx.x / ns : blockIdx.x;
+    const int d0 = SPLIT ? (int)((long long)n * (blockIdx.x % ns) / ns) : 0;
+    const int d1 = SPLIT ? (int)((long long)n * (blockIdx.x % ns + 1) / ns) : n;
+    int rank = 0; // the last layer rank whose first run is <= item
+    for (int hi = lay.layers - 1; rank < hi;) {
+        const int mid = (rank + hi + 1) >> 1;
+        if (lay.pre[mid] <= item) rank = mid;
+        else hi = mid - 1;
+    }
+    const int kz = middle_out(rank, lay.layers), run = item - lay.pre[rank];
     for (int j = threadIdx.x; j < bricksY; j += blockDim.x) {
-        int lo, n;
-        brick_row(j, kz, bricksX, volCenter, kCBZ, reach, lo, n);
+        int lo, cnt;
+        brick_row(j, kz, bricksX, volCenter, kCBZ, reach, lo, cnt);
         slo[j] = lo;
-        spre[j] = n;
+        spre[j] = cnt;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -720,8 +754,14 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
     }
     __syncthreads();
     const int total = spre[bricksY];
-    if (((DEEP && G > 1) ? 2 : 1) * G * (int)blockIdx.x >= total) return; // the whole CTA
-    for (int t = threadIdx.x; t < tabWords; t += blockDim.x) bp_smem[t] = __ldg(ker + min(t / cp, kerSize - 1));
+    if (TS == 128) { // 32 copies: a warp's lanes store 16 copies of 8 entries
+        for (int t = threadIdx.x; t < tb.entries * 8; t += blockDim.x) {
+            const float w = __ldg(ker + min(t >> 3, kerSize - 1));
+            reinterpret_cast<float4 *>(bp_smem)[t] = make_float4(w, w, w, w);
+        }
+    } else {
+        for (int t = threadIdx.x; t < tabWords; t += blockDim.x) bp_smem[t] = __ldg(ker + min(t / cp, kerSize - 1));
+    }
     __syncthreads();
 
     // Group g runs brick g of the CTA's run of RUN * G bricks, and
@@ -733,7 +773,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
     constexpr int RUN = (DEEP && G > 1) ? 2 : 1;
     const int grp = threadIdx.x / kCThreads;
     for (int pass = 0; pass < RUN; pass++) {
-        const int a = RUN * G * blockIdx.x + (pass == 0 ? grp : RUN * G - 1 - grp);
+        const int a = RUN * G * run + (pass == 0 ? grp : RUN * G - 1 - grp);
         if (a >= total) break;
         int row = 0; // the last row whose prefix is <= a (it holds brick a)
         for (int hi = bricksY - 1; row < hi;) {
@@ -871,8 +911,8 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
             }
         };
 
-        for (int c0 = 0; c0 < n; c0 += kBpChunk) {
-            const int cn = min(kBpChunk, n - c0);
+        for (int c0 = d0; c0 < d1; c0 += kBpChunk) {
+            const int cn = min(kBpChunk, d1 - c0);
             group_sync(grp + 1);
             if (cn == kBpChunk) {
                 // a whole chunk: all of a thread's loads in flight before its stores
@@ -887,7 +927,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
             }
             group_sync(grp + 1);
             // cull: thread tid takes directions tid + p * kCThreads; the kept
-            // ones are listed in direction order (pass by pass, warp by warp)
+            // ones are listed in direction order (pass by pass, warp by warp).
             constexpr int kPasses = kBpChunk / kCThreads;
             unsigned ballots[kPasses];
             bool keeps[kPasses];
@@ -1215,16 +1255,43 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
         for (int s = 0; s < BD; s++) {
             if (!((inmask >> s) & 1u)) continue;
             const size_t o = (size_t)(bz + s) * V * V + (size_t)ly * V + lx;
-            vol[o] = vol[o] + wacc[lane + 32 * s] * sc;
-            if (DENS || DW) pd[o] = pd[o] + waccw[lane + 32 * s];
+            if (!SPLIT || blockIdx.x % split.nseg == 0) {
+                vol[o] = vol[o] + wacc[lane + 32 * s] * sc;
+                if (DENS || DW) pd[o] = pd[o] + waccw[lane + 32 * s];
+            } else {
+                float *const pv = split.part + (size_t)(blockIdx.x % split.nseg - 1) * (DENS || DW ? 2 : 1) * V * V * V;
+                pv[o] = wacc[lane + 32 * s] * sc;
+                if (DENS || DW) pv[(size_t)V * V * V + o] = waccw[lane + 32 * s];
+            }
         }
     }
+}
+
+// Adds the segments' sums of a split launch to the volume (and the density),
+// in segment order: (((v + s1) + s2) + ...).  Voxels of the mask sphere, which
+// every segment has written.  Bound: HBM / L2, 4 (segments + 1) bytes a voxel.
+__global__ void __launch_bounds__(256)
+bp_merge_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, int maskR, BpSplit split)
+{
+    const int x = blockIdx.x * 256 + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
+    if (x >= V) return;
+    const long long c = V / 2, dx = x - c, dy = y - c, dz = z - c;
+    if (dx * dx + dy * dy + dz * dz > (long long)maskR * maskR) return;
+    const size_t V3 = (size_t)V * V * V, o = ((size_t)z * V + y) * V + x;
+    const int per = pd ? 2 : 1;
+    float v = vol[o], d = pd ? pd[o] : 0.0f;
+    for (int s = 0; s + 1 < split.nseg; s++) {
+        v = __fadd_rn(v, split.part[s * per * V3 + o]);
+        if (pd) d = __fadd_rn(d, split.part[(s * per + 1) * V3 + o]);
+    }
+    vol[o] = v;
+    if (pd) pd[o] = d;
 }
 
 template <typename TI, bool ONES, bool DENS, bool ADJ, bool DW, bool DEEP, int G>
 static cudaError_t launch_bp_compact_g(float *vol, const TI *img, const float *ker, const float *axes, int n,
                                        const Geom &g, const float *scale, cudaStream_t s, float *pd, bool zero_edges,
-                                       const float *img2, int max_copies)
+                                       const float *img2, int max_copies, BpSplit split)
 {
     constexpr int kCBZ = BpShape<ADJ, DW, DEEP>::BZ;
     const int bx = (g.V + kCBX - 1) / kCBX, by = (g.V + kCBY - 1) / kCBY, bz = (g.V + kCBZ - 1) / kCBZ;
@@ -1240,19 +1307,44 @@ static cudaError_t launch_bp_compact_g(float *vol, const TI *img, const float *k
     // quad loads of image rows: 4 | M and the stacks aligned to 4 elements
     const size_t qa = 4 * sizeof(TI);
     const int vec = (g.M % 4 == 0) && ((size_t)img % qa == 0) && (!img2 || (size_t)img2 % 16 == 0) ? 1 : 0;
-    // CTA (x, z): bricks run x .. of z-layer z that meet the sphere
+    // one CTA for each run of RUN * G bricks of a layer that meet the sphere
     const int run = ((DEEP && G > 1) ? 2 : 1) * G;
-    const dim3 grid((unsigned)((bx * by + run - 1) / run), (unsigned)bz);
+    if (bz > kMaxLayers) return cudaErrorInvalidValue;
+    BpLayers lay;
+    lay.layers = bz;
+    lay.pre[0] = 0;
+    for (int r = 0; r < bz; r++) {
+        int bricks = 0;
+        for (int j = 0; j < by; j++) {
+            int lo, cnt;
+            brick_row(j, middle_out(r, bz), bx, (int)((float)g.V) / 2, kCBZ, ADJ ? g.mask_radius + 4 : g.mask_radius, lo,
+                      cnt);
+            bricks += cnt;
+        }
+        lay.pre[r + 1] = lay.pre[r] + (bricks + run - 1) / run;
+    }
+    const unsigned grid = (unsigned)lay.pre[bz] * (unsigned)split.nseg;
+    if (grid == 0) return cudaSuccess;
     // the table stride as a compile-time constant where the copy count gives one
     auto go = [&](auto kern) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
         if (e != cudaSuccess) return e;
         kern<<<grid, kCThreads * G, dyn, s>>>(vol, pd, g.V, img, g.M, axes, n, g.mask_radius, ker, g.ker_size,
-                                              g.ker_hw, bx, by, tb, zero_edges ? 1 : 0, scale, img2, vec);
+                                              g.ker_hw, bx, by, tb, zero_edges ? 1 : 0, scale, img2, vec, split, lay);
         count_launches(1);
+        if (split.nseg > 1) {
+            const dim3 mg((unsigned)((g.V + 255) / 256), (unsigned)g.V, (unsigned)g.V);
+            bp_merge_kernel<<<mg, 256, 0, s>>>(vol, DENS || DW ? pd : nullptr, g.V, g.mask_radius, split);
+            count_launches(1);
+        }
         return cudaGetLastError();
     };
     if constexpr (LEAN) {
+        if constexpr (!ONES && !ADJ) {
+            if (split.nseg > 1) // bp_segments splits only tables that get 32 copies
+                return tb.copies == 32 ? go(bp_ref_compact_kernel<TI, ONES, DENS, ADJ, DW, DEEP, G, 128, true, true>)
+                                       : cudaErrorInvalidValue;
+        }
         if (tb.copies == 32) return go(bp_ref_compact_kernel<TI, ONES, DENS, ADJ, DW, DEEP, G, 128, true>);
     }
     return go(bp_ref_compact_kernel<TI, ONES, DENS, ADJ, DW, DEEP, G, 0, LEAN>);
@@ -1261,7 +1353,8 @@ static cudaError_t launch_bp_compact_g(float *vol, const TI *img, const float *k
 template <typename TI, bool ONES, bool DENS = false, bool ADJ = false, bool DW = false, bool DEEP = false>
 static cudaError_t launch_bp_compact_t(float *vol, const TI *img, const float *ker, const float *axes, int n,
                                        const Geom &g, const float *scale, cudaStream_t s, float *pd = nullptr,
-                                       bool zero_edges = true, const float *img2 = nullptr, bool shared = false)
+                                       bool zero_edges = true, const float *img2 = nullptr, bool shared = false,
+                                       BpSplit split = {1, nullptr})
 {
     if (n <= 0) return cudaSuccess;
     // A GPU shared with concurrent launches (the serving lanes): one group
@@ -1272,55 +1365,85 @@ static cudaError_t launch_bp_compact_t(float *vol, const TI *img, const float *k
     if constexpr (std::is_same<TI, float>::value && !ONES && !DENS && !ADJ && !DW) {
         if (shared)
             return launch_bp_compact_g<TI, ONES, DENS, ADJ, DW, DEEP, 1>(vol, img, ker, axes, n, g, scale, s, pd,
-                                                                         zero_edges, img2, 1);
+                                                                         zero_edges, img2, 1, BpSplit{1, nullptr});
     }
     return launch_bp_compact_g<TI, ONES, DENS, ADJ, DW, DEEP, kGroupsOf<ADJ, DW, DEEP>>(vol, img, ker, axes, n, g, scale, s, pd,
-                                                                         zero_edges, img2, 32);
+                                                                         zero_edges, img2, 32, split);
 }
 
 // Reference-rule launch with the block depth chosen by the image size.
 template <typename TI, bool ONES, bool DENS>
 static cudaError_t launch_bp_ref_sized(float *vol, const TI *img, const float *ker, const float *axes, int n,
-                                       const Geom &g, const float *scale, cudaStream_t s, float *pd = nullptr,
-                                       bool shared = false)
+                                       const Geom &g, const float *scale, cudaStream_t s, float *pd, bool shared,
+                                       BpSplit split)
 {
     if (g.M >= 512)
         return launch_bp_compact_t<TI, ONES, DENS, false, false, true>(vol, img, ker, axes, n, g, scale, s, pd, true,
-                                                                        nullptr, shared);
-    return launch_bp_compact_t<TI, ONES, DENS>(vol, img, ker, axes, n, g, scale, s, pd, true, nullptr, shared);
+                                                                        nullptr, shared, split);
+    return launch_bp_compact_t<TI, ONES, DENS>(vol, img, ker, axes, n, g, scale, s, pd, true, nullptr, shared, split);
 }
 
 cudaError_t launch_back_project_ref(float *d_vol, const void *d_img, int iprec, bool ones, const float *d_ker,
                                     const float *d_axes, int n, const Geom &g, const float *scale, cudaStream_t s,
-                                    bool shared)
+                                    bool shared, BpSplit split)
 {
-    if (ones) return launch_bp_ref_sized<float, true, false>(d_vol, nullptr, d_ker, d_axes, n, g, scale, s);
+    if (ones)
+        return launch_bp_ref_sized<float, true, false>(d_vol, nullptr, d_ker, d_axes, n, g, scale, s, nullptr, false, split);
     if (iprec == kF32)
         return launch_bp_ref_sized<float, false, false>(d_vol, (const float *)d_img, d_ker, d_axes, n, g, scale, s,
-                                                        nullptr, shared);
+                                                        nullptr, shared, split);
     if (iprec == kF16)
-        return launch_bp_ref_sized<__half, false, false>(d_vol, (const __half *)d_img, d_ker, d_axes, n, g, scale, s);
+        return launch_bp_ref_sized<__half, false, false>(d_vol, (const __half *)d_img, d_ker, d_axes, n, g, scale, s,
+                                                         nullptr, false, split);
     return launch_bp_ref_sized<__nv_bfloat16, false, false>(d_vol, (const __nv_bfloat16 *)d_img, d_ker, d_axes, n, g,
-                                                            scale, s);
+                                                            scale, s, nullptr, false, split);
 }
 
 cudaError_t launch_back_project_ref_density(float *d_vol, float *d_pd, const void *d_img, int iprec, const float *d_ker,
-                                            const float *d_axes, int n, const Geom &g, const float *scale, cudaStream_t s)
+                                            const float *d_axes, int n, const Geom &g, const float *scale,
+                                            cudaStream_t s, BpSplit split)
 {
     if (iprec == kF32)
-        return launch_bp_ref_sized<float, false, true>(d_vol, (const float *)d_img, d_ker, d_axes, n, g, scale, s, d_pd);
+        return launch_bp_ref_sized<float, false, true>(d_vol, (const float *)d_img, d_ker, d_axes, n, g, scale, s, d_pd,
+                                                       false, split);
     if (iprec == kF16)
         return launch_bp_ref_sized<__half, false, true>(d_vol, (const __half *)d_img, d_ker, d_axes, n, g, scale, s,
-                                                        d_pd);
+                                                        d_pd, false, split);
     return launch_bp_ref_sized<__nv_bfloat16, false, true>(d_vol, (const __nv_bfloat16 *)d_img, d_ker, d_axes, n, g,
-                                                           scale, s, d_pd);
+                                                           scale, s, d_pd, false, split);
 }
 
 cudaError_t launch_back_project_ref_pair(float *d_vol, float *d_pd, const float *d_img, const float *d_img2,
-                                         const float *d_ker, const float *d_axes, int n, const Geom &g, cudaStream_t s)
+                                         const float *d_ker, const float *d_axes, int n, const Geom &g, cudaStream_t s,
+                                         BpSplit split)
 {
     return launch_bp_compact_t<float, false, false, false, true>(d_vol, d_img, d_ker, d_axes, n, g, nullptr, s, d_pd,
-                                                                  true, d_img2);
+                                                                  true, d_img2, false, split);
+}
+
+// How many segments.  Every direction reaches the bricks at the centre, so the
+// centre's CTA is a serial chain over all n of them (4.6 ms for 1,000) while
+// the others' work falls as 1 / radius; where the launch has few brick runs
+// (245 at M = 128) that chain is the launch's time.  Segments cut it, but each
+// pays a CTA's start (table, sums, about 10 us) and fills rounds less well, so
+// the fewer the directions, the fewer runs it takes before they cost more than
+// they give.  Measured, reconstructVol, 1 / best / next segment count in us:
+// M = 64, n = 1000: 3939 / 908 (6) / 1095 (4); M = 128, n = 1000: 4579 /
+// 2203 (3) / 2256 (4), n = 256: 1242 / 731 (2) / 781 (3), n = 16: 158 (1) /
+// 178 (2); M = 160, n = 256: 1269 / 1106 (2), n = 64: 436 (1) / 478 (2);
+// M = 200, n = 1000: 4985 / 4752 (2), n = 512: 2632 (1) / 2770 (2);
+// M = 256, n = 1000: 6657 (1) / 7055 (2).
+// The rule looks at n and the geometry only, so the plain, density and
+// two-stack forms of one call add the same partial sums.
+int bp_segments(int n, const Geom &g)
+{
+    if (g.ker_size > 513) return 1; // no room for the 32 table copies of the split form
+    const double r = g.mask_radius + 2.0;
+    const int runs = (int)(4.19 * r * r * r / (3 * kCBX * kCBY * 12)) + 1; // of three bricks in the mask's sphere
+    const int want = n < 32 ? 200 : n < 192 ? 300 : n < 512 ? 450 : 700;
+    int s = 1 + want / runs;
+    if ((n >= 128 && runs < 610) || (n >= 768 && runs < 1100)) s = std::max(s, 2);
+    return std::max(1, std::min({s, 6, n / 3}));
 }
 
 cudaError_t launch_back_project_adjoint(float *d_vol, const void *d_img, int iprec, const float *d_ker,
