@@ -159,7 +159,7 @@ struct gg_gridder {
     int *fault = nullptr;       // pinned: set by a kernel whose copies did not arrive
     DevBuf<float> pd;        // plane density V^3
     DevBuf<float> bp_part;   // sums of a split back projection's segments
-    DevBuf<float> adj;       // CAS-volume gradient V^3 (forward-operator adjoint)
+    DevBuf<float> adj;       // CAS-volume gradient, V^2 rows of fp_pitch(V, kF32) (forward-operator adjoint)
     DevBuf<float> axes;
     DevBuf<float> vol_io;    // N^3
     DevBuf<float> x3;        // M^3 real FFT input/output
@@ -444,7 +444,7 @@ void bp_batch(gg_gridder *h, const float *d_axes, int b, const float *img, const
     if (ones) iprec = kF32;
     ProfScope ps(h, s, ones ? GG_KERNEL_DENSITY : GG_KERNEL_BACK);
     if (h->bp_mode == GG_BP_ADJOINT && !ones) {
-        GG_CK(launch_back_project_adjoint(target, src, iprec, h->ker.p, d_axes, b, h->geom(), scale, !h->five_taps, s));
+        GG_CK(launch_back_project_adjoint(target, h->V, src, iprec, h->ker.p, d_axes, b, h->geom(), scale, s));
     } else if (pd && !ones) {
         GG_CK(launch_back_project_ref_density(target, pd, src, iprec, h->ker.p, d_axes, b, h->geom(), scale, s,
                                               bp_split(h, b, 2)));
@@ -459,7 +459,7 @@ void bp_batch(gg_gridder *h, const float *d_axes, int b, const float *img, const
         const size_t MM = (size_t)h->M * h->M;
         ProfScope pd_ps(h, s, GG_KERNEL_DENSITY);
         GG_CK(launch_fill(S.casimg.p, MM * b, 1.0f, s));
-        GG_CK(launch_back_project_adjoint(pd, S.casimg.p, kF32, h->ker.p, d_axes, b, h->geom(), nullptr, !h->five_taps, s));
+        GG_CK(launch_back_project_adjoint(pd, h->V, S.casimg.p, kF32, h->ker.p, d_axes, b, h->geom(), nullptr, s));
         pd_ps.done();
     }
 }
@@ -505,9 +505,11 @@ void check_ctf(const CtfParams &c)
 // images): image gradients (device, n*N*N) -> volume gradient (device, N^3).
 void forward_adjoint(gg_gridder *h, const float *d_axes, int n, const float *d_img_grad, float *d_vol_grad, cudaStream_t s)
 {
-    const size_t V3 = (size_t)h->V * h->V * h->V, NN = (size_t)h->N * h->N;
-    h->adj.ensure(V3);
-    GG_CK(cudaMemsetAsync(h->adj.p, 0, V3 * sizeof(float), s));
+    // rows of 16 bytes, for the adjoint's vector additions
+    const int P = fp_pitch(h->V, kF32);
+    const size_t PV2 = (size_t)P * h->V * h->V, NN = (size_t)h->N * h->N;
+    h->adj.ensure(PV2);
+    GG_CK(cudaMemsetAsync(h->adj.p, 0, PV2 * sizeof(float), s));
     const int B = h->max_batch;
     for (int a0 = 0; a0 < n; a0 += B) {
         const int b = std::min(B, n - a0);
@@ -523,14 +525,14 @@ void forward_adjoint(gg_gridder *h, const float *d_axes, int n, const float *d_i
             GG_CK(launch_spectrum_to_cas_images_adjoint(S.spec.p, h->M, b, S.casimg.p, s));
         }
         ProfScope ps(h, s, GG_KERNEL_BACK);
-        GG_CK(launch_back_project_adjoint(h->adj.p, S.casimg.p, kF32, h->ker.p, d_axes + (size_t)a0 * 9, b, h->geom(),
-                                          nullptr, !h->five_taps, s));
+        GG_CK(launch_back_project_adjoint(h->adj.p, P, S.casimg.p, kF32, h->ker.p, d_axes + (size_t)a0 * 9, b, h->geom(),
+                                          nullptr, s));
         ps.done();
     }
     const size_t M3 = (size_t)h->M * h->M * h->M;
     h->x3.ensure(M3);
     h->spec3.ensure((size_t)h->M * h->M * (h->M / 2 + 1));
-    GG_CK(launch_cas_volume_adjoint_input(h->adj.p, h->V, h->M, h->x3.p, s));
+    GG_CK(launch_cas_volume_adjoint_input(h->adj.p, P, h->V, h->M, h->x3.p, s));
     cufftHandle p = plan3(h, true);
     GG_CKF(cufftSetStream(p, s));
     GG_CKF(cufftExecR2C(p, h->x3.p, h->spec3.p));
@@ -1431,8 +1433,8 @@ extern "C" int gg_back_project_adjoint_kernel(float *d_cas_volume, const float *
     }
     Geom g{cas_vol_size, cas_img_size, mask_radius, kb_table_size, ker_hwidth};
     // zero table edges were checked above
-    cudaError_t e = launch_back_project_adjoint(d_cas_volume, d_cas_images, kF32, d_kb_table, d_axes, n_axes, g, nullptr,
-                                                true, (cudaStream_t)stream);
+    cudaError_t e = launch_back_project_adjoint(d_cas_volume, cas_vol_size, d_cas_images, kF32, d_kb_table, d_axes, n_axes,
+                                                g, nullptr, (cudaStream_t)stream);
     if (e != cudaSuccess) {
         g_global_err = cudaGetErrorString(e);
         return GG_ERR_CUDA;

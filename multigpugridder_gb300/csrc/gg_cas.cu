@@ -276,14 +276,14 @@ spectrum_to_cas_images_kernel(const cufftComplex *__restrict__ spec, int M, int 
 
 // Gradient of the CAS volume -> volume, first half: crop V^3 to the inner M^3
 // and fftshift (the adjoint of the zero-pad and of the output fftshift).
-__global__ void cas_volume_adjoint_input_kernel(const float *__restrict__ g, int V, int M, float *__restrict__ x)
+__global__ void cas_volume_adjoint_input_kernel(const float *__restrict__ g, int P, int V, int M, float *__restrict__ x)
 {
     const size_t total = (size_t)M * M * M;
     const int b = V / 2 - M / 2;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
         const int qi = (int)(e % M), qj = (int)((e / M) % M), qk = (int)(e / ((size_t)M * M));
         const int i = shift_idx(qi, M), j = shift_idx(qj, M), k = shift_idx(qk, M);
-        x[e] = g[((size_t)(k + b) * V + (j + b)) * V + (i + b)];
+        x[e] = g[((size_t)(k + b) * V + (j + b)) * P + (i + b)];
     }
 }
 
@@ -572,9 +572,9 @@ cudaError_t launch_spectrum_to_cas_images_adjoint(const cufftComplex *d_spec, in
     return cudaGetLastError();
 }
 
-cudaError_t launch_cas_volume_adjoint_input(const float *d_g, int V, int M, float *d_x, cudaStream_t s)
+cudaError_t launch_cas_volume_adjoint_input(const float *d_g, int pitch, int V, int M, float *d_x, cudaStream_t s)
 {
-    cas_volume_adjoint_input_kernel<<<grid_for((size_t)M * M * M, kT), kT, 0, s>>>(d_g, V, M, d_x);
+    cas_volume_adjoint_input_kernel<<<grid_for((size_t)M * M * M, kT), kT, 0, s>>>(d_g, pitch, V, M, d_x);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -99,12 +99,12 @@ cudaError_t launch_back_project_ref_pair(float *d_vol, float *d_pd, const float 
                                          const float *d_ker, const float *d_axes, int n, const Geom &g, cudaStream_t s,
                                          BpSplit split = {1, nullptr});
 
-// Exact adjoint of launch_forward_project (4 taps), accumulated into d_vol.
-// zero_edges: the KB table's first and last entries are 0 (the fast path
-// relies on it).
-cudaError_t launch_back_project_adjoint(float *d_vol, const void *d_img, int iprec, const float *d_ker,
+// Exact adjoint of the 4-tap forward projection (gg_adjoint.cu), added to
+// d_vol, rows `pitch` floats apart (planes pitch * V; dense: pitch = V).  The
+// KB table's first and last entries are 0.
+cudaError_t launch_back_project_adjoint(float *d_vol, int pitch, const void *d_img, int iprec, const float *d_ker,
                                         const float *d_axes, int n, const Geom &g, const float *d_scale,
-                                        bool zero_edges, cudaStream_t s);
+                                        cudaStream_t s);
 
 // ---- CAS / FFT stages (gg_cas.cu) ------------------------------------------
 // Volume N^3 -> real M^3 FFT input: centred zero-pad, separable precomp
@@ -138,8 +138,8 @@ cudaError_t launch_spectrum_to_cas_images(const cufftComplex *d_spec, int M, int
 // (Re+Im, first row/column zero, 1/M^2).
 cudaError_t launch_spectrum_to_cas_images_adjoint(const cufftComplex *d_spec, int M, int n, float *d_cas,
                                                   cudaStream_t s);
-// CAS-volume gradient V^3 -> R2C input M^3 (inner crop + shift).
-cudaError_t launch_cas_volume_adjoint_input(const float *d_g, int V, int M, float *d_x, cudaStream_t s);
+// CAS-volume gradient V^3 (rows `pitch` floats apart) -> R2C input M^3 (inner crop + shift).
+cudaError_t launch_cas_volume_adjoint_input(const float *d_g, int pitch, int V, int M, float *d_x, cudaStream_t s);
 // R2C spectrum -> volume gradient N^3 (Re+Im, shift, precomp, crop).
 cudaError_t launch_spectrum_to_vol_adjoint(const cufftComplex *d_spec, int M, int N, const double *d_precomp,
                                            float *d_vol, cudaStream_t s);

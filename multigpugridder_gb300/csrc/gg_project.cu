@@ -2,7 +2,6 @@
 //
 //   forward projection   CAS volume -> CAS images (pixel-driven gather)
 //   back projection      CAS images -> CAS volume, reference window rule
-//   adjoint projection   exact adjoint of the forward projection
 //
 // Conventions follow the reference kernels (src/Projection/gpuForwardProject.cu,
 // src/Projection/gpuBackProject.cu): x fastest, CAS-volume centre V/2, image
@@ -300,11 +299,9 @@ __device__ __forceinline__ void ref_window(const RefWindow &q, const float *sker
 constexpr int kCBX = 16, kCBY = 8; // brick: 2x2x2 warp blocks of 8x4xBD (BD = 6, or 8 on large images)
 constexpr int kCThreads = 256;  // threads of a group
 constexpr int kBpGroups = 3;    // groups (bricks) per CTA, one CTA per SM
-// The adjoint's and the two-stack form's 6-deep kernels run two groups per CTA: with the
-// adjoint's 24-wide footprints, or the second stack's footprints, the voxel queue's two
-// buffers fit only beside two groups (adjoint of 4,096 directions at 128^3: 67.8 ms with
-// three one-buffer groups, 62.0 ms with two queued ones).
-template <bool ADJ, bool DW, bool DEEP> constexpr int kGroupsOf = ((ADJ || DW) && !DEEP) ? 2 : kBpGroups;
+// The two-stack form's 6-deep kernel runs two groups per CTA: with the second
+// stack's footprints, the voxel queue's two buffers fit only beside two groups.
+template <bool DW, bool DEEP> constexpr int kGroupsOf = (DW && !DEEP) ? 2 : kBpGroups;
 static_assert(kBpChunk % kCThreads == 0, "the cull gives each thread kBpChunk / kCThreads directions");
 // Depth of a warp block: 6 voxels, or 8 (DEEP, reference rule) on CAS images
 // of 512^2 and more.  Deeper blocks have more active voxels per direction
@@ -312,17 +309,16 @@ static_assert(kBpChunk % kCThreads == 0, "the cull gives each thread kBpChunk / 
 // voxels, which pays most where the images are large (each staging reads from
 // L2 or DRAM); on 256^2 images 8-deep blocks measured 20% slower than 4-deep
 // ones and 6-deep ones 0.7% faster.  With 6 the footprint still fits 16
-// pixels for any orthonormal axes (2 |(3.5, 1.5, 2.5)| + 1.2 < 11), and the
-// adjoint's 7x7 windows fit 24.  The adjoint and the two-stack form had 4
-// while their 256-thread CTAs held a padded table each; with the shared table
-// copies 6-deep blocks measured faster for both (gradient step 89.6 -> 87.4
-// ms, CTF-corrected reconstructVol 88.6 -> 84.1 ms).
-template <bool ADJ, bool DW, bool DEEP>
+// pixels for any orthonormal axes (2 |(3.5, 1.5, 2.5)| + 1.2 < 11).  The
+// two-stack form had 4 while its 256-thread CTAs held a padded table each; with
+// the shared table copies 6-deep blocks measured faster (CTF-corrected
+// reconstructVol 88.6 -> 84.1 ms).
+template <bool DW, bool DEEP>
 struct BpShape {
     static constexpr int BD = DEEP ? 8 : 6;
     static constexpr int WV = 32 * BD;                         // voxels per warp block
     static constexpr int BZ = 2 * BD;                          // brick depth
-    static constexpr int FW = ADJ ? 24 : (BD == 8 ? 20 : 16);  // footprint width and height
+    static constexpr int FW = BD == 8 ? 20 : 16;  // footprint width and height
 };
 
 // The fast window.  For a voxel coordinate v and a window pixel whose
@@ -534,51 +530,6 @@ static BpTable bp_table(int kerSize, size_t other_bytes, int max_copies = 32, si
     return t;
 }
 
-// The exact adjoint of fp_kernel<., 4> for one voxel, without the fast
-// path's assumptions: every in-mask pixel whose 4^3 forward window contains
-// the voxel, with the forward weight.  Such a pixel lies within 2*sqrt(3) of
-// the voxel's projection.
-template <typename TI>
-__device__ float adjoint_window_slow(int vi, int vj, int vk, int volCenter, float nx0, float nx1, float nx2, float ny0,
-                                     float ny1, float ny2, const TI *__restrict__ img_ptr, int M, int imgCenter,
-                                     int maskR, const float *sker, int rep, float kerScale, float kerCenterHalf,
-                                     int kerSize)
-{
-    const float pi = ((float)vi - volCenter) * nx0 + ((float)vj - volCenter) * nx1 + ((float)vk - volCenter) * nx2;
-    const float pj = ((float)vi - volCenter) * ny0 + ((float)vj - volCenter) * ny1 + ((float)vk - volCenter) * ny2;
-    const int ilo = (int)ceilf(pi - 3.47f), ihi = (int)floorf(pi + 3.47f);
-    const int jlo = (int)ceilf(pj - 3.47f), jhi = (int)floorf(pj + 3.47f);
-    const long long R2 = (long long)maskR * maskR;
-    float s = 0.0f;
-    for (int dj = jlo; dj <= jhi; dj++) {
-        for (int di = ilo; di <= ihi; di++) {
-            if ((long long)di * di + (long long)dj * dj > R2) continue;
-            const int pxi = di + imgCenter, pxj = dj + imgCenter;
-            if (pxi < 0 || pxi >= M || pxj < 0 || pxj >= M) continue;
-            const float fi = sample_coord(nx0, ny0, di, dj, volCenter);
-            const float fj = sample_coord(nx1, ny1, di, dj, volCenter);
-            const float fk = sample_coord(nx2, ny2, di, dj, volCenter);
-            // membership in the forward window floor(f)-1 .. floor(f)+2
-            const int oi = vi - ((int)floorf(fi) - 1), oj = vj - ((int)floorf(fj) - 1), ok = vk - ((int)floorf(fk) - 1);
-            if ((unsigned)oi > 3u || (unsigned)oj > 3u || (unsigned)ok > 3u) continue;
-            const float w = kb_weight(sker, (float)vi - fi, kerScale, kerCenterHalf, kerSize, rep) *
-                            kb_weight(sker, (float)vj - fj, kerScale, kerCenterHalf, kerSize, rep) *
-                            kb_weight(sker, (float)vk - fk, kerScale, kerCenterHalf, kerSize, rep);
-            s = fmaf(w, ld_f32(img_ptr + (size_t)pxj * M + pxi), s);
-        }
-    }
-    return s;
-}
-
-// ADJ: the exact adjoint of fp_kernel<., 4> (gradient of the forward
-// projection) instead of the reference rule.  The same pixel positions and
-// table indices (sample_coord is the reference's pixel-position expression),
-// a 7x7 window around the voxel's projection for voxels within 2*sqrt(3) of
-// the plane, pixels outside the image or the mask staged as zero, and the
-// index of r = v - Q: floor(fma(Q, -s, h + v*s)).  With a zero-edge table
-// every pixel whose forward window misses the voxel gets weight 0, so the
-// wider window adds exact zeros (zero_edges; otherwise the slow path checks
-// window membership as the forward does).
 // DW (reference rule, FP32 images): pd accumulates the back projection of a
 // second image stack img2 (the same directions) in the same pass, with the
 // same weights and summation order as a separate back projection of img2.
@@ -592,15 +543,14 @@ struct alignas(16) BpDirMeta {
 // A warp's queue of voxel windows: entries (block voxel | footprint buffer
 // << 8) in direction order, run 32 at a time, so that rounds are full across
 // directions.  NB footprint buffers per warp: 2 where shared memory allows
-// (the 6-deep reference-rule form, and the adjoint's with two groups per CTA;
-// a direction's footprint is staged while the previous direction's last
-// voxels still wait in the queue); else 1, and each direction's active voxels
+// (the 6-deep forms; a direction's footprint is staged while the previous
+// direction's last voxels still wait in the queue); else 1, and each direction's active voxels
 // run at once from the same array (a plain list, no queue): queue rounds with
 // one buffer measured slower (per-lane direction records, spills).
-template <bool ADJ, bool DW, bool DEEP>
+template <bool DW, bool DEEP>
 struct BpQueue {
     static constexpr int NB = !DEEP ? 2 : 1;
-    static constexpr int NEED = (NB - 1) * 31 + BpShape<ADJ, DW, DEEP>::WV; // most entries held at once
+    static constexpr int NEED = (NB - 1) * 31 + BpShape<DW, DEEP>::WV; // most entries held at once
     static constexpr int CAP = NEED <= 128 ? 128 : (NEED <= 256 ? 256 : 512);
 };
 
@@ -610,10 +560,10 @@ struct BpQueue {
 // footprint rows of FW + 4 pixels from fi0 & ~3 (16-byte aligned, written by
 // vector stores).  Otherwise (the serving lanes' one-group CTAs): 16-bit
 // entries carrying the buffer bit, rows of FW + 1 pixels from fi0.
-template <bool DENS, bool ADJ, bool DW, bool DEEP, bool LEAN = true>
+template <bool DENS, bool DW, bool DEEP, bool LEAN = true>
 struct BpGroupMem {
-    using Shape = BpShape<ADJ, DW, DEEP>;
-    using Q = BpQueue<ADJ, DW, DEEP>;
+    using Shape = BpShape<DW, DEEP>;
+    using Q = BpQueue<DW, DEEP>;
     using QEnt = typename std::conditional<LEAN, unsigned char, unsigned short>::type;
     using LEnt = typename std::conditional<LEAN, unsigned short, int>::type;
     static constexpr int NW = kCThreads / 32, WV = Shape::WV,
@@ -694,23 +644,23 @@ __device__ __forceinline__ void group_sync(int id)
     asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kCThreads) : "memory");
 }
 
-template <typename TI, bool ONES, bool DENS, bool ADJ, bool DW = false, bool DEEP = false, int G = kBpGroups,
+template <typename TI, bool ONES, bool DENS, bool DW = false, bool DEEP = false, int G = kBpGroups,
           int TS = 0, bool LEAN = true, bool SPLIT = false>
 __global__ void __launch_bounds__(kCThreads *G, G == 1 ? 3 : 1)
 bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, const TI *__restrict__ img, int M,
                       const float *__restrict__ axes, int n, int maskR, const float *__restrict__ ker, int kerSize,
-                      float kerHW, int bricksX, int bricksY, BpTable tb, int zeroEdges,
+                      float kerHW, int bricksX, int bricksY, BpTable tb,
                       const float *__restrict__ d_scale, const float *__restrict__ img2, int vecImg, BpSplit split,
                       const __grid_constant__ BpLayers lay)
 {
-    static_assert(!DW || (!ONES && !DENS && !ADJ), "the second image stack is a reference-rule option");
-    constexpr int W = ADJ ? 7 : 5, HALF = W / 2;
-    using Shape = BpShape<ADJ, DW, DEEP>;
+    static_assert(!DW || (!ONES && !DENS), "the second image stack is a reference-rule option");
+    constexpr int W = 5, HALF = W / 2;
+    using Shape = BpShape<DW, DEEP>;
     constexpr int BD = Shape::BD, kWarpVox = Shape::WV, kCBZ = Shape::BZ;
     // LEAN two-buffer form: footprint rows hold the pixels from fi0 & ~3 (16-byte aligned rows)
-    constexpr bool QALIGN = LEAN && BpQueue<ADJ, DW, DEEP>::NB == 2;
+    constexpr bool QALIGN = LEAN && BpQueue<DW, DEEP>::NB == 2;
     constexpr int FW = Shape::FW, FH = FW, FS = FW + (QALIGN ? 4 : 1);
-    using Mem = BpGroupMem<DENS, ADJ, DW, DEEP, LEAN>;
+    using Mem = BpGroupMem<DENS, DW, DEEP, LEAN>;
     using QEnt = typename Mem::QEnt;
     // [table: tb.entries x tb.copies][G x Mem][row starts][row prefix]
     extern __shared__ __align__(16) float bp_smem[];
@@ -720,12 +670,10 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
     const int volCenter = (int)((float)V) / 2;
     const int imgCenter = (int)((float)M) / 2;
 
-    // The CTA's bricks: those of z-layer kz that meet the sphere of radius
-    // `reach` (the adjoint reaches voxels up to 2*sqrt(3) beyond the mask),
+    // The CTA's bricks: those of z-layer kz that meet the mask sphere,
     // numbered row by row; the CTA takes run `run` of RUN * G numbers (below).
     // Row (y, z) holds the x interval [slo, slo + n).
     // SPLIT: a run's segments of the directions are neighbours in the grid.
-    const int reach = ADJ ? maskR + 4 : maskR;
     const int ns = SPLIT ? split.nseg : 1, item = SPLIT ? blockIdx.x / ns : blockIdx.x;
     const int d0 = SPLIT ? (int)((long long)n * (blockIdx.x % ns) / ns) : 0;
     const int d1 = SPLIT ? (int)((long long)n * (blockIdx.x % ns + 1) / ns) : n;
@@ -738,7 +686,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
     const int kz = middle_out(rank, lay.layers), run = item - lay.pre[rank];
     for (int j = threadIdx.x; j < bricksY; j += blockDim.x) {
         int lo, cnt;
-        brick_row(j, kz, bricksX, volCenter, kCBZ, reach, lo, cnt);
+        brick_row(j, kz, bricksX, volCenter, kCBZ, maskR, lo, cnt);
         slo[j] = lo;
         spre[j] = cnt;
     }
@@ -791,7 +739,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
         const float *sker = bp_smem + lane % cp; // entry k at sker[k * cp]
         const unsigned stride = 4u * (unsigned)cp;
         const unsigned tab = (unsigned)__cvta_generic_to_shared(bp_smem) + 4u * (unsigned)(lane % cp) - tb.magic_bits * stride;
-        constexpr int NB = BpQueue<ADJ, DW, DEEP>::NB, QM = BpQueue<ADJ, DW, DEEP>::CAP - 1;
+        constexpr int NB = BpQueue<DW, DEEP>::NB, QM = BpQueue<DW, DEEP>::CAP - 1;
         float *const wfoot0 = sm.sfoot + warp * (NB * FH * FS);
         float *const wfoot20 = sm.sfoot2 + (DW ? warp * (NB * FH * FS) : 0);
         BpDirMeta *const wmeta = sm.smeta + warp * NB;
@@ -802,14 +750,13 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
         // this lane's voxels: x = lx, y = ly, z = bz + s
         const int lx = bx + (lane & 7), ly = by + (lane >> 3);
         const long long R2 = (long long)maskR * maskR;
-        const long long reach2 = ADJ ? (long long)(maskR + 4) * (maskR + 4) : R2;
         unsigned inmask = 0;
 #pragma unroll
         for (int s = 0; s < BD; s++) {
             const int lz = bz + s;
             const long long d2 = (long long)(lx - volCenter) * (lx - volCenter) + (long long)(ly - volCenter) * (ly - volCenter) +
                                  (long long)(lz - volCenter) * (lz - volCenter);
-            if (lx < V && ly < V && lz < V && d2 <= reach2) inmask |= 1u << s;
+            if (lx < V && ly < V && lz < V && d2 <= R2) inmask |= 1u << s;
             wacc[lane + 32 * s] = 0.0f;
             if (DENS || DW) waccw[lane + 32 * s] = 0.0f;
         }
@@ -818,9 +765,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
         const float kerCenterHalf = kerCenter + 0.5f;
         const float ax0 = (float)lx - volCenter, ay0 = (float)ly - volCenter;
         const float wcx = bx + 3.5f - volCenter, wcy = by + 1.5f - volCenter, wcz = bz + 0.5f * (BD - 1) - volCenter;
-        // slab half-thickness: kerHW for the reference rule; for the adjoint, any
-        // voxel within the 4^3 window of a sample point (|r| < 2 per axis)
-        const float slab = ADJ ? 2.0f * 1.7320508f + kCullEps : kerHW + kCullEps;
+        const float slab = kerHW + kCullEps; // half-thickness
         const int MM = M * M;
         // Directions are staged through shared memory in chunks, culled against
         // the brick (compacted in order), then against each warp's 8x4xBD block.
@@ -833,7 +778,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
         int qhead = 0, qsize = 0, nbuf = 0, nfront = 0, bfront = 0;
 
         // One voxel's window sum for one direction: the fast window from the
-        // footprint, or the reference's (or the adjoint's) window from the image.
+        // footprint, or the reference's window from the image.
         auto voxel_window = [&](const int l, const float nx0, const float nx1, const float nx2, const float ny0,
                                 const float ny1, const float ny2, const int fi0, const int fj0, const int fh,
                                 const bool foot, const TI *img_ptr, const float *img2_ptr, const float *wfoot,
@@ -847,10 +792,9 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
             const bool inside = imgi >= 2 && imgj >= 2 && imgi + 2 < M && imgj + 2 < M;
             const int ri = imgi - HALF - fi0, rj = imgj - HALF - fj0;
             if (foot && (unsigned)ri <= (unsigned)(FW - W) && (unsigned)rj <= (unsigned)(fh - W) && vi >= 4 &&
-                vj >= 4 && vk >= 4 && (ADJ || inside || !DENS)) {
-                // reference rule: index of r = Q - v; adjoint: of r = v - Q
-                const float sg = ADJ ? -kerScale : kerScale;
-                // scaled by 1/P (exact): the saturating index form
+                vj >= 4 && vk >= 4 && (inside || !DENS)) {
+                // index of r = Q - v, scaled by 1/P (exact): the saturating index form
+                const float sg = kerScale;
                 const FootWin fwin{nx0, nx1, nx2, ny0, ny1, ny2, (float)volCenter, sg * tb.scale,
                                    (kerCenterHalf - (float)vi * sg) * tb.scale,
                                    (kerCenterHalf - (float)vj * sg) * tb.scale,
@@ -859,9 +803,6 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                 const float pi0 = (float)(imgi - HALF - imgCenter), pj0 = (float)(imgj - HALF - imgCenter);
                 foot_window_x2<DENS, W, W, FS, DW, TS>(fwin, fb, tab, pi0, pj0, cs, cw,
                                                 DW ? wfoot2 + rj * FS + ri + (QALIGN ? (fi0 & 3) : 0) : nullptr);
-            } else if (ADJ) {
-                cs = adjoint_window_slow<TI>(vi, vj, vk, volCenter, nx0, nx1, nx2, ny0, ny1, ny2, img_ptr, M,
-                                             imgCenter, maskR, sker, cp, kerScale, kerCenterHalf, kerSize);
             } else {
                 const RefWindow rw{nx0, nx1, nx2, ny0, ny1, ny2, (float)vi, (float)vj, (float)vk,
                                    (float)volCenter, kerScale, kerCenterHalf};
@@ -980,27 +921,19 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                 const int al = e & (kBpChunk - 1);
                 const float *ax = sax + al * 9;
                 const float nz0 = ax[6], nz1 = ax[7], nz2 = ax[8];
-                // Adjoint, orthonormal axes: a pixel weighs non-zero only if its
-                // sample point f lies in the voxel's cube |f - v| < 2 (each axis),
-                // which the plane reaches only if |f_k| < 2 |nz|_1: a slab
-                // thinner than 2 sqrt(3) for most directions.
-                const float slabD = ADJ && (e & kBpChunk)
-                                        ? fminf(slab, 2.0f * (fabsf(nz0) + fabsf(nz1) + fabsf(nz2)) + kCullEps)
-                                        : slab;
                 {   // the warp's 8x4xBD block against the slab (uniform)
                     const float d = wcx * nz0 + wcy * nz1 + wcz * nz2;
                     const float ext = 0.5f * (7.0f * fabsf(nz0) + 3.0f * fabsf(nz1) + (float)(BD - 1) * fabsf(nz2));
                     if (fabsf(d) > slab + ext) continue;
                 }
-                // the reference's per-voxel slab test (gpuBackProject.cu:64-66), or
-                // the adjoint's reach
+                // the reference's per-voxel slab test (gpuBackProject.cu:64-66)
                 unsigned actm = 0;
                 int total = 0;
 #pragma unroll
                 for (int s = 0; s < BD; s++) {
                     const float az = (float)(bz + s) - volCenter;
                     const float fk = voxel_proj(ax0, ay0, az, nz0, nz1, nz2);
-                    const bool act = ((inmask >> s) & 1u) && (ADJ ? fabsf(fk) < slabD : fabsf(fk) <= kerHW);
+                    const bool act = ((inmask >> s) & 1u) && fabsf(fk) <= kerHW;
                     actm |= (act ? 1u : 0u) << s;
                     total += __popc(__ballot_sync(0xffffffffu, act));
                 }
@@ -1031,8 +964,8 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                     fj0 = (int)floorf(jc - hj - 0.6f) - HALF;
                     const int fw = (int)floorf(ic + hi + 0.6f) + HALF - fi0 + 1;
                     fh = (int)floorf(jc + hj + 0.6f) + HALF - fj0 + 1;
-                    foot = fw <= FW && fh <= FH && fh >= W && (!ADJ || zeroEdges);
-                    if (foot && !ADJ && !ONES && vecImg) {
+                    foot = fw <= FW && fh <= FH && fh >= W;
+                    if (foot && !ONES && vecImg) {
                         // vector loads of aligned pixel quads (rows start at
                         // multiples of 4 elements: 4 divides M, the image stacks
                         // are aligned), the linear-index rule still applied
@@ -1111,7 +1044,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                                 }
                             }
                         }
-                    } else if (foot && !ADJ && sizeof(TI) == 2 && !ONES && !(M & 1)) {
+                    } else if (foot && sizeof(TI) == 2 && !ONES && !(M & 1)) {
                         // the same with 4-byte pixel pairs when only 2 divides M
                         constexpr int NPR = FW / 2 + 1; // pairs per footprint row
                         const int base = fi0 & ~1, odd = fi0 & 1;
@@ -1132,7 +1065,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                             if (c0 >= 0 && c0 < FW) wfoot[r * FS + c0 + ash] = v0;
                             if (c0 + 1 < FW) wfoot[r * FS + c0 + 1 + ash] = v1; // c0 + 1 >= 0
                         }
-                    } else if (foot && !ADJ) {
+                    } else if (foot) {
                         // the reference's linear-index rule (gpuBackProject.cu:99)
                         for (int t = lane; t < fh * FW; t += 32) {
                             const int r = t / FW, c = t - r * FW;
@@ -1144,60 +1077,6 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                             }
                             wfoot[r * FS + c + (QALIGN ? (fi0 & 3) : 0)] = v;
                             if (DW) wfoot2[r * FS + c + (QALIGN ? (fi0 & 3) : 0)] = v2;
-                        }
-                    } else if (foot) {
-                        // the forward projection's pixels: inside the image and the mask
-                        if (vecImg && !ONES) {
-                            // aligned pixel quads (4 divides M: a quad lies wholly inside or
-                            // outside the image rows), three in flight per lane at a time;
-                            // the mask is applied pixel by pixel
-                            constexpr int NQ = FW / 4 + 1; // quads per footprint row
-                            const int base = fi0 & ~3, sh = fi0 & 3, nq = fh * NQ;
-                            for (int t0 = lane; t0 < nq; t0 += 96) {
-                                float v[3][4];
-#pragma unroll
-                                for (int u = 0; u < 3; u++) {
-                                    const int t = t0 + 32 * u;
-#pragma unroll
-                                    for (int e = 0; e < 4; e++) v[u][e] = 0.0f;
-                                    const int r = t / NQ, qq = t - r * NQ;
-                                    const int pj = fj0 + r, pi = base + 4 * qq;
-                                    if (t < nq && pj >= 0 && pj < M && pi >= 0 && pi < M) {
-                                        ld_quad(img_ptr + (size_t)pj * M + pi, v[u]);
-                                        const long long dj = pj - imgCenter;
-#pragma unroll
-                                        for (int e = 0; e < 4; e++) {
-                                            const long long di = pi + e - imgCenter;
-                                            if (di * di + dj * dj > R2) v[u][e] = 0.0f;
-                                        }
-                                    }
-                                }
-#pragma unroll
-                                for (int u = 0; u < 3; u++) {
-                                    const int t = t0 + 32 * u;
-                                    if (t < nq) {
-                                        const int r = t / NQ, qq = t - r * NQ;
-                                        const int c0 = 4 * qq - sh; // footprint column of the quad's first pixel
-                                        if (QALIGN) {
-                                            *reinterpret_cast<float4 *>(wfoot + r * FS + 4 * qq) =
-                                                make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
-                                        } else {
-#pragma unroll
-                                            for (int e = 0; e < 4; e++)
-                                                if (c0 + e >= 0 && c0 + e < FW) wfoot[r * FS + c0 + e] = v[u][e];
-                                        }
-                                    }
-                                }
-                            }
-                        } else {
-                            for (int t = lane; t < fh * FW; t += 32) {
-                                const int r = t / FW, c = t - r * FW;
-                                const int pi = fi0 + c, pj = fj0 + r, di = pi - imgCenter, dj = pj - imgCenter;
-                                float v = 0.0f;
-                                if (pi >= 0 && pi < M && pj >= 0 && pj < M && (long long)di * di + (long long)dj * dj <= R2)
-                                    v = ld_f32(img_ptr + (size_t)pj * M + pi);
-                                wfoot[r * FS + c + (QALIGN ? (fi0 & 3) : 0)] = v;
-                            }
                         }
                     }
                 }
@@ -1288,16 +1167,16 @@ bp_merge_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, int mask
     if (pd) pd[o] = d;
 }
 
-template <typename TI, bool ONES, bool DENS, bool ADJ, bool DW, bool DEEP, int G>
+template <typename TI, bool ONES, bool DENS, bool DW, bool DEEP, int G>
 static cudaError_t launch_bp_compact_g(float *vol, const TI *img, const float *ker, const float *axes, int n,
-                                       const Geom &g, const float *scale, cudaStream_t s, float *pd, bool zero_edges,
-                                       const float *img2, int max_copies, BpSplit split)
+                                       const Geom &g, const float *scale, cudaStream_t s, float *pd, const float *img2,
+                                        int max_copies, BpSplit split)
 {
-    constexpr int kCBZ = BpShape<ADJ, DW, DEEP>::BZ;
+    constexpr int kCBZ = BpShape<DW, DEEP>::BZ;
     const int bx = (g.V + kCBX - 1) / kCBX, by = (g.V + kCBY - 1) / kCBY, bz = (g.V + kCBZ - 1) / kCBZ;
     // one group per CTA (the serving lanes): the non-LEAN layout
     constexpr bool LEAN = G > 1;
-    using Mem = BpGroupMem<DENS, ADJ, DW, DEEP, LEAN>;
+    using Mem = BpGroupMem<DENS, DW, DEEP, LEAN>;
     const size_t other = G * sizeof(Mem) + (2 * (size_t)by + 1) * sizeof(int);
     // one group per CTA: three CTAs an SM (228 KB, 1 KB reserved per CTA)
     const size_t limit = G == 1 ? (size_t)(228 * 1024 / 3 - 1024) : 0;
@@ -1317,8 +1196,7 @@ static cudaError_t launch_bp_compact_g(float *vol, const TI *img, const float *k
         int bricks = 0;
         for (int j = 0; j < by; j++) {
             int lo, cnt;
-            brick_row(j, middle_out(r, bz), bx, (int)((float)g.V) / 2, kCBZ, ADJ ? g.mask_radius + 4 : g.mask_radius, lo,
-                      cnt);
+            brick_row(j, middle_out(r, bz), bx, (int)((float)g.V) / 2, kCBZ, g.mask_radius, lo, cnt);
             bricks += cnt;
         }
         lay.pre[r + 1] = lay.pre[r] + (bricks + run - 1) / run;
@@ -1330,7 +1208,7 @@ static cudaError_t launch_bp_compact_g(float *vol, const TI *img, const float *k
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
         if (e != cudaSuccess) return e;
         kern<<<grid, kCThreads * G, dyn, s>>>(vol, pd, g.V, img, g.M, axes, n, g.mask_radius, ker, g.ker_size,
-                                              g.ker_hw, bx, by, tb, zero_edges ? 1 : 0, scale, img2, vec, split, lay);
+                                              g.ker_hw, bx, by, tb, scale, img2, vec, split, lay);
         count_launches(1);
         if (split.nseg > 1) {
             const dim3 mg((unsigned)((g.V + 255) / 256), (unsigned)g.V, (unsigned)g.V);
@@ -1340,20 +1218,20 @@ static cudaError_t launch_bp_compact_g(float *vol, const TI *img, const float *k
         return cudaGetLastError();
     };
     if constexpr (LEAN) {
-        if constexpr (!ONES && !ADJ) {
+        if constexpr (!ONES) {
             if (split.nseg > 1) // bp_segments splits only tables that get 32 copies
-                return tb.copies == 32 ? go(bp_ref_compact_kernel<TI, ONES, DENS, ADJ, DW, DEEP, G, 128, true, true>)
+                return tb.copies == 32 ? go(bp_ref_compact_kernel<TI, ONES, DENS, DW, DEEP, G, 128, true, true>)
                                        : cudaErrorInvalidValue;
         }
-        if (tb.copies == 32) return go(bp_ref_compact_kernel<TI, ONES, DENS, ADJ, DW, DEEP, G, 128, true>);
+        if (tb.copies == 32) return go(bp_ref_compact_kernel<TI, ONES, DENS, DW, DEEP, G, 128, true>);
     }
-    return go(bp_ref_compact_kernel<TI, ONES, DENS, ADJ, DW, DEEP, G, 0, LEAN>);
+    return go(bp_ref_compact_kernel<TI, ONES, DENS, DW, DEEP, G, 0, LEAN>);
 }
 
-template <typename TI, bool ONES, bool DENS = false, bool ADJ = false, bool DW = false, bool DEEP = false>
+template <typename TI, bool ONES, bool DENS = false, bool DW = false, bool DEEP = false>
 static cudaError_t launch_bp_compact_t(float *vol, const TI *img, const float *ker, const float *axes, int n,
                                        const Geom &g, const float *scale, cudaStream_t s, float *pd = nullptr,
-                                       bool zero_edges = true, const float *img2 = nullptr, bool shared = false,
+                                       const float *img2 = nullptr, bool shared = false,
                                        BpSplit split = {1, nullptr})
 {
     if (n <= 0) return cudaSuccess;
@@ -1362,13 +1240,13 @@ static cudaError_t launch_bp_compact_t(float *vol, const TI *img, const float *k
     // other lanes can fill as they free (serving capacity 172 -> 195 req/s);
     // alone, three groups sharing 32 table copies (batched back projection
     // 78.5 -> 71.7 ms per 10k images).
-    if constexpr (std::is_same<TI, float>::value && !ONES && !DENS && !ADJ && !DW) {
+    if constexpr (std::is_same<TI, float>::value && !ONES && !DENS && !DW) {
         if (shared)
-            return launch_bp_compact_g<TI, ONES, DENS, ADJ, DW, DEEP, 1>(vol, img, ker, axes, n, g, scale, s, pd,
-                                                                         zero_edges, img2, 1, BpSplit{1, nullptr});
+            return launch_bp_compact_g<TI, ONES, DENS, DW, DEEP, 1>(vol, img, ker, axes, n, g, scale, s, pd,
+                                                                         img2, 1, BpSplit{1, nullptr});
     }
-    return launch_bp_compact_g<TI, ONES, DENS, ADJ, DW, DEEP, kGroupsOf<ADJ, DW, DEEP>>(vol, img, ker, axes, n, g, scale, s, pd,
-                                                                         zero_edges, img2, 32, split);
+    return launch_bp_compact_g<TI, ONES, DENS, DW, DEEP, kGroupsOf<DW, DEEP>>(vol, img, ker, axes, n, g, scale, s, pd,
+                                                                         img2, 32, split);
 }
 
 // Reference-rule launch with the block depth chosen by the image size.
@@ -1378,9 +1256,9 @@ static cudaError_t launch_bp_ref_sized(float *vol, const TI *img, const float *k
                                        BpSplit split)
 {
     if (g.M >= 512)
-        return launch_bp_compact_t<TI, ONES, DENS, false, false, true>(vol, img, ker, axes, n, g, scale, s, pd, true,
-                                                                        nullptr, shared, split);
-    return launch_bp_compact_t<TI, ONES, DENS>(vol, img, ker, axes, n, g, scale, s, pd, true, nullptr, shared, split);
+        return launch_bp_compact_t<TI, ONES, DENS, false, true>(vol, img, ker, axes, n, g, scale, s, pd, nullptr,
+                                                                 shared, split);
+    return launch_bp_compact_t<TI, ONES, DENS>(vol, img, ker, axes, n, g, scale, s, pd, nullptr, shared, split);
 }
 
 cudaError_t launch_back_project_ref(float *d_vol, const void *d_img, int iprec, bool ones, const float *d_ker,
@@ -1417,8 +1295,8 @@ cudaError_t launch_back_project_ref_pair(float *d_vol, float *d_pd, const float 
                                          const float *d_ker, const float *d_axes, int n, const Geom &g, cudaStream_t s,
                                          BpSplit split)
 {
-    return launch_bp_compact_t<float, false, false, false, true>(d_vol, d_img, d_ker, d_axes, n, g, nullptr, s, d_pd,
-                                                                  true, d_img2, false, split);
+    return launch_bp_compact_t<float, false, false, true>(d_vol, d_img, d_ker, d_axes, n, g, nullptr, s, d_pd, d_img2,
+                                                           false, split);
 }
 
 // How many segments.  Every direction reaches the bricks at the centre, so the
@@ -1444,20 +1322,6 @@ int bp_segments(int n, const Geom &g)
     int s = 1 + want / runs;
     if ((n >= 128 && runs < 610) || (n >= 768 && runs < 1100)) s = std::max(s, 2);
     return std::max(1, std::min({s, 6, n / 3}));
-}
-
-cudaError_t launch_back_project_adjoint(float *d_vol, const void *d_img, int iprec, const float *d_ker,
-                                        const float *d_axes, int n, const Geom &g, const float *scale, bool zero_edges,
-                                        cudaStream_t s)
-{
-    if (iprec == kF32)
-        return launch_bp_compact_t<float, false, false, true>(d_vol, (const float *)d_img, d_ker, d_axes, n, g, scale, s,
-                                                               nullptr, zero_edges);
-    if (iprec == kF16)
-        return launch_bp_compact_t<__half, false, false, true>(d_vol, (const __half *)d_img, d_ker, d_axes, n, g, scale,
-                                                                s, nullptr, zero_edges);
-    return launch_bp_compact_t<__nv_bfloat16, false, false, true>(d_vol, (const __nv_bfloat16 *)d_img, d_ker, d_axes, n,
-                                                                   g, scale, s, nullptr, zero_edges);
 }
 
 } // namespace gg
