@@ -148,7 +148,7 @@ struct gg_gridder {
     float ker_hw = 2.0f;
 
     DevBuf<float> ker;
-    DevBuf<double> precomp;
+    DevBuf<float2> precomp;  // FP64 factors as float pairs
     DevBuf<float> cas;       // FP32 CAS volume V^3 (resident)
     DevBuf<unsigned char> cas_fp; // the copy the forward projection reads: storage `prec`, row
                                   // pitch fp_pitch(V, prec) (FP16 scaled by scales[0])
@@ -343,16 +343,17 @@ void do_set_volume(gg_gridder *h, const float *d_vol, cudaStream_t s)
     cufftHandle p = plan3(h, true);
     GG_CKF(cufftSetStream(p, s));
     GG_CKF(cufftExecR2C(p, h->x3.p, h->spec3.p));
-    GG_CK(launch_spectrum_to_cas_volume(h->spec3.p, h->M, h->V, h->cas.p, kF32, nullptr, s));
+    GG_CK(launch_spectrum_to_cas_volume(h->spec3.p, h->M, h->V, h->cas.p, s));
     h->cas_fp_valid = false;
 }
 
-void do_get_volume(gg_gridder *h, const float *d_cas, float *d_vol, cudaStream_t s)
+// With a density the CAS volume is divided by it first, in place (+ 1e-6).
+void do_get_volume(gg_gridder *h, float *d_cas, const float *d_density, float *d_vol, cudaStream_t s)
 {
     const size_t M3 = (size_t)h->M * h->M * h->M;
     h->x3.ensure(M3);
     h->spec3.ensure((size_t)h->M * h->M * (h->M / 2 + 1));
-    GG_CK(launch_cas_volume_to_spectrum(d_cas, h->V, h->M, h->spec3.p, s));
+    GG_CK(launch_cas_volume_to_spectrum(d_cas, d_density, 1e-6f, h->V, h->M, h->spec3.p, s));
     cufftHandle p = plan3(h, false);
     GG_CKF(cufftSetStream(p, s));
     GG_CKF(cufftExecC2R(p, h->spec3.p, h->x3.p));
@@ -677,7 +678,12 @@ void init_handle(gg_gridder *h)
     h->five_taps = !(tf[0] == 0.0f && tf[h->ker_size - 1] == 0.0f);
     precomp_f64(h->M, (int)h->ker_hw, pc.data());
     h->precomp.ensure(h->M);
-    GG_CK(cudaMemcpy(h->precomp.p, pc.data(), pc.size() * sizeof(double), cudaMemcpyHostToDevice));
+    std::vector<float2> pf(h->M);
+    for (int i = 0; i < h->M; i++) {
+        pf[i].x = (float)pc[i];
+        pf[i].y = (float)(pc[i] - (double)pf[i].x);
+    }
+    GG_CK(cudaMemcpy(h->precomp.p, pf.data(), pf.size() * sizeof(float2), cudaMemcpyHostToDevice));
     h->scales.ensure(2);
     const float ones[2] = {1.0f, 1.0f};
     GG_CK(cudaMemcpy(h->scales.p, ones, sizeof(ones), cudaMemcpyHostToDevice));
@@ -1029,7 +1035,7 @@ extern "C" int gg_get_volume(gg_gridder *h, float *volume_out)
         require_volume(h);
         const size_t N3 = (size_t)h->N * h->N * h->N;
         h->vol_io.ensure(N3);
-        do_get_volume(h, h->cas.p, h->vol_io.p, h->cs);
+        do_get_volume(h, h->cas.p, nullptr, h->vol_io.p, h->cs);
         GG_CK(cudaMemcpyAsync(volume_out, h->vol_io.p, N3 * sizeof(float), cudaMemcpyDeviceToHost, h->cs));
         GG_CK(cudaStreamSynchronize(h->cs));
     });
@@ -1049,9 +1055,8 @@ extern "C" int gg_reconstruct_volume(gg_gridder *h, const float *axes, int n_axe
         // back projection of the images and, in the same pass, the plane
         // density (the same directions with all-ones CAS images)
         if (n_axes > 0) bp_host(h, axes, n_axes, images, nullptr, h->cas.p, false, h->pd.p);
-        GG_CK(launch_divide_plane_density(h->cas.p, h->pd.p, V3, 1e-6f, h->cs));
         h->vol_io.ensure(N3);
-        do_get_volume(h, h->cas.p, h->vol_io.p, h->cs);
+        do_get_volume(h, h->cas.p, h->pd.p, h->vol_io.p, h->cs);
         GG_CK(cudaMemcpyAsync(volume_out, h->vol_io.p, N3 * sizeof(float), cudaMemcpyDeviceToHost, h->cs));
         GG_CK(cudaStreamSynchronize(h->cs));
         h->cas_fp_valid = false;
@@ -1154,7 +1159,7 @@ extern "C" int gg_get_volume_dev(gg_gridder *h, float *d_volume_out, void *strea
         require_volume(h);
         cudaStream_t s = (cudaStream_t)stream;
         begin_dev(h, s);
-        do_get_volume(h, h->cas.p, d_volume_out, s);
+        do_get_volume(h, h->cas.p, nullptr, d_volume_out, s);
         end_dev(h, s);
     });
 }
@@ -1179,8 +1184,7 @@ extern "C" int gg_reconstruct_volume_dev(gg_gridder *h, const float *d_axes, int
             ensure_slot(h, 0, B, false);
             bp_batch(h, d_axes + (size_t)a0 * 9, b, d_images + (size_t)a0 * NN, nullptr, h->cas.p, false, 0, s, h->pd.p);
         }
-        GG_CK(launch_divide_plane_density(h->cas.p, h->pd.p, V3, 1e-6f, s));
-        do_get_volume(h, h->cas.p, d_volume_out, s);
+        do_get_volume(h, h->cas.p, h->pd.p, d_volume_out, s);
         h->cas_fp_valid = false;
         end_dev(h, s);
     });
@@ -1218,8 +1222,7 @@ extern "C" int gg_volume_from_sums_dev(gg_gridder *h, const float *d_sums, float
         h->cas.ensure(V3);
         GG_CK(cudaMemcpyAsync(h->cas.p, d_sums, V3 * sizeof(float), cudaMemcpyDeviceToDevice, s));
         // tmpCASVolume ./ (PlaneDensity + 1e-6) (MultiGPUGridder_Matlab_Class.m:308)
-        GG_CK(launch_divide_plane_density(h->cas.p, d_sums + V3, V3, 1e-6f, s));
-        do_get_volume(h, h->cas.p, d_volume_out, s);
+        do_get_volume(h, h->cas.p, d_sums + V3, d_volume_out, s);
         h->cas_fp_valid = false;
         end_dev(h, s);
     });
@@ -1254,8 +1257,7 @@ extern "C" int gg_reconstruct_volume_ctf_dev(gg_gridder *h, const float *d_axes,
                       d_defocus_v ? d_defocus_v + a0 : nullptr, d_astig_angle ? d_astig_angle + a0 : nullptr, c, 0,
                       s);
         }
-        GG_CK(launch_divide_plane_density(h->cas.p, h->pd.p, V3, 1e-6f, s));
-        do_get_volume(h, h->cas.p, d_volume_out, s);
+        do_get_volume(h, h->cas.p, h->pd.p, d_volume_out, s);
         h->cas_fp_valid = false;
         end_dev(h, s);
     });
@@ -1300,9 +1302,8 @@ extern "C" int gg_reconstruct_volume_ctf(gg_gridder *h, const float *axes, int n
                 ctf_batch(h, h->axes.p + (size_t)a0 * 9, b, dbuf, df.p + a0, astig ? df.p + nn + a0 : nullptr,
                           astig ? df.p + 2 * nn + a0 : nullptr, c, sl, s);
             });
-        GG_CK(launch_divide_plane_density(h->cas.p, h->pd.p, V3, 1e-6f, s));
         h->vol_io.ensure(N3);
-        do_get_volume(h, h->cas.p, h->vol_io.p, s);
+        do_get_volume(h, h->cas.p, h->pd.p, h->vol_io.p, s);
         GG_CK(cudaMemcpyAsync(volume_out, h->vol_io.p, N3 * sizeof(float), cudaMemcpyDeviceToHost, s));
         GG_CK(cudaStreamSynchronize(s));
         df.release();

@@ -31,91 +31,216 @@ static inline unsigned grid_for(size_t count, int threads)
 
 __device__ __forceinline__ int shift_idx(int q, int M) { return q + M / 2 >= M ? q + M / 2 - M : q + M / 2; }
 
-// ---- 3-D: volume -> CAS volume --------------------------------------------
+// ---- 3-D stages --------------------------------------------------------------
+// One warp per row (or pair of rows) of the 3-D arrays: row indices are divided
+// out once a row, lanes walk the columns, and the shifts turn into two
+// contiguous segments.  Bound: HBM.  The elementwise forms before them spent
+// their time on three 64-bit divisions an element and on FP64 products (2 FP64
+// lanes an SM): at N = 256, M = 512, preparing a volume took 567 + 739 us
+// around 780 us of cuFFT, now 97 + 189 us (6.0 TB/s); getVol's output stage at
+// N = 192, M = 384: 185 -> 26 us.
+//
+// Precomp factors are float pairs (hi + lo = the FP64 value to 48 bits); their
+// products keep the pair, so the one rounding to FP32 at the end is the FP64
+// product's but for ties.
+constexpr int kRows = 8; // warps (rows in flight) per block
 
-// x[q] = (zero-padded volume * precomp^3)[(q + M/2) mod M] per axis.
-__global__ void vol_to_fft_input_kernel(const float *__restrict__ vol, int N, int M,
-                                        const double *__restrict__ pc, float *__restrict__ x)
+static inline unsigned rows_grid(long long rows)
 {
-    const size_t total = (size_t)M * M * M;
-    const int b = M / 2 - N / 2;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const int qi = (int)(e % M), qj = (int)((e / M) % M), qk = (int)(e / ((size_t)M * M));
-        const int i = shift_idx(qi, M), j = shift_idx(qj, M), k = shift_idx(qk, M);
-        const int oi = i - b, oj = j - b, ok = k - b;
-        float v = 0.0f;
-        if ((unsigned)oi < (unsigned)N && (unsigned)oj < (unsigned)N && (unsigned)ok < (unsigned)N) {
-            const float f = (float)(pc[i] * pc[j] * pc[k]);
-            v = vol[(size_t)ok * N * N + (size_t)oj * N + oi] * f;
+    const long long g = (rows + kRows - 1) / kRows;
+    return (unsigned)(g < 0x7fffffffLL ? g : 0x7fffffffLL);
+}
+
+struct FF {
+    float h, l;
+};
+__device__ __forceinline__ FF ff_mul(FF a, FF b)
+{
+    const float p = __fmul_rn(a.h, b.h);
+    const float e = __fmaf_rn(a.h, b.h, -p) + (a.h * b.l + a.l * b.h);
+    const float s = __fadd_rn(p, e);
+    return FF{s, __fsub_rn(e, __fsub_rn(s, p))};
+}
+__device__ __forceinline__ FF ff_at(const float2 *__restrict__ pc, int i)
+{
+    const float2 v = __ldg(pc + i);
+    return FF{v.x, v.y};
+}
+// x * f, f a pair, rounded once
+__device__ __forceinline__ float ff_scale(float x, FF f)
+{
+    const float p = __fmul_rn(x, f.h);
+    return __fadd_rn(p, __fmaf_rn(x, f.h, -p) + x * f.l);
+}
+
+// x[q] = (zero-padded volume * precomp^3)[(q + M/2) mod M] per axis, the
+// factor rounded to FP32 before it multiplies.
+__global__ void __launch_bounds__(32 * kRows)
+vol_to_fft_input_kernel(const float *__restrict__ vol, int N, int M, const float2 *__restrict__ pc, float *__restrict__ x)
+{
+    const int lane = threadIdx.x & 31, b = M / 2 - N / 2;
+    const long long rows = (long long)M * M;
+    for (long long r = (long long)blockIdx.x * kRows + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * kRows) {
+        const int qk = (int)(r / M), qj = (int)(r - (long long)qk * M);
+        const int j = shift_idx(qj, M), k = shift_idx(qk, M);
+        float *xr = x + r * M;
+        const bool in = (unsigned)(j - b) < (unsigned)N && (unsigned)(k - b) < (unsigned)N;
+        if (!in) {
+            // rows start on 8 bytes: M is even
+            for (int q = 2 * lane; q < M; q += 64) *reinterpret_cast<float2 *>(xr + q) = make_float2(0.0f, 0.0f);
+            continue;
         }
-        x[e] = v;
+        const FF jk = ff_mul(ff_at(pc, j), ff_at(pc, k));
+        const float *vr = vol + ((size_t)(k - b) * N + (j - b)) * N - b;
+#pragma unroll 4
+        for (int q = lane; q < M; q += 32) {
+            const int i = shift_idx(q, M);
+            float v = 0.0f;
+            if ((unsigned)(i - b) < (unsigned)N) {
+                const FF f = ff_mul(ff_at(pc, i), jk);
+                v = __ldg(vr + i) * f.h;
+            }
+            xr[q] = v;
+        }
     }
 }
 
-// CAS[pad+k][pad+j][pad+i] = Re+Im of fftshift(Y)[k][j][i]; border zero.
-template <typename T>
-__global__ void spectrum_to_cas_volume_kernel(const cufftComplex *__restrict__ spec, int M, int V, T *__restrict__ cas,
-                                              const float *__restrict__ d_scale)
+// CAS[pad+k][pad+j][pad+i] = Re+Im of fftshift(Y)[k][j][i]; border zero.  A
+// warp owns a CAS row: it zeroes the row's border and sends the half-spectrum
+// row at (j, k) where its entries belong: Re+Im to the upper half of this row
+// and Re-Im to the lower half of the mirrored row (Y[-w][-v][-u] =
+// conj(Y[w][v][u])), so the spectrum is read once.
+__global__ void __launch_bounds__(32 * kRows)
+spectrum_to_cas_volume_kernel(const cufftComplex *__restrict__ spec, int M, int V, float *__restrict__ cas)
 {
-    const float inv_scale = d_scale ? 1.0f / *d_scale : 1.0f;
-    const size_t total = (size_t)V * V * V;
-    const int pad = V / 2 - M / 2;
-    const int H = M / 2 + 1;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const int ci = (int)(e % V), cj = (int)((e / V) % V), ck = (int)(e / ((size_t)V * V));
-        const int i = ci - pad, j = cj - pad, k = ck - pad;
-        float out = 0.0f;
-        if ((unsigned)i < (unsigned)M && (unsigned)j < (unsigned)M && (unsigned)k < (unsigned)M) {
-            const int u = shift_idx(i, M), v = shift_idx(j, M), w = shift_idx(k, M);
-            if (u <= M / 2) {
-                const cufftComplex c = spec[((size_t)w * M + v) * H + u];
-                out = c.x + c.y;
-            } else {  // conjugate symmetry: Y[w][v][u] = conj(Y[-w][-v][-u])
-                const int w2 = w ? M - w : 0, v2 = v ? M - v : 0, u2 = M - u;
-                const cufftComplex c = spec[((size_t)w2 * M + v2) * H + u2];
-                out = c.x - c.y;
-            }
+    const int lane = threadIdx.x & 31, pad = V / 2 - M / 2, H = M / 2 + 1;
+    const long long rows = (long long)V * V;
+    for (long long r = (long long)blockIdx.x * kRows + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * kRows) {
+        const int ck = (int)(r / V), cj = (int)(r - (long long)ck * V), j = cj - pad, k = ck - pad;
+        float *row = cas + r * V;
+        if ((unsigned)j >= (unsigned)M || (unsigned)k >= (unsigned)M) {
+            for (int c = lane; c < V; c += 32) row[c] = 0.0f;
+            continue;
         }
-        cas[e] = from_f32<T>(out * inv_scale);
+        for (int c = lane; c < pad; c += 32) row[c] = 0.0f;
+        for (int c = pad + M + lane; c < V; c += 32) row[c] = 0.0f;
+        const int v = shift_idx(j, M), w = shift_idx(k, M);
+        const int jm = shift_idx(v ? M - v : 0, M), km = shift_idx(w ? M - w : 0, M);
+        float *up = row + pad + M / 2;                                             // i = M/2 + u
+        float *down = cas + ((size_t)(km + pad) * V + (jm + pad)) * V + pad + M / 2; // i = M/2 - u
+        const cufftComplex *s = spec + ((size_t)w * M + v) * H;
+#pragma unroll 4
+        for (int u = lane; u < M / 2; u += 32) {
+            const float2 c = __ldg(reinterpret_cast<const float2 *>(s) + u);
+            up[u] = c.x + c.y;
+            if (u) down[-u] = c.x - c.y;
+        }
+        if (lane == 0) { // u = M/2 is i = 0 of this row
+            const float2 c = __ldg(reinterpret_cast<const float2 *>(s) + M / 2);
+            row[pad] = c.x + c.y;
+        }
     }
 }
 
 // ---- 3-D: CAS volume -> volume ---------------------------------------------
 
 // H[w][v][u] = FromCAS(crop(cas))[(w+M/2)%M][(v+M/2)%M][(u+M/2)%M], u <= M/2.
-__global__ void cas_volume_to_spectrum_kernel(const float *__restrict__ cas, int V, int M, cufftComplex *__restrict__ spec)
+// A warp takes a CAS row and its mirror image through the centre, which
+// together hold both spectrum rows.  DIV: the volume is divided first, in
+// place: a = a / (b + eps) over every voxel (reconstructVol's plane-density
+// division, MultiGPUGridder_Matlab_Class.m:308), borders included; one pass in
+// place of two (M = 384: 196 + 160 -> 226 us; M = 256: 59 + 50 -> 82 us).
+template <bool DIV>
+__global__ void __launch_bounds__(32 * kRows)
+cas_volume_to_spectrum_kernel(float *__restrict__ cas, const float *__restrict__ den, float eps, int V, int M,
+                              cufftComplex *__restrict__ spec)
 {
-    const int H = M / 2 + 1;
-    const size_t total = (size_t)M * M * H;
-    const int b = V / 2 - M / 2;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const int u = (int)(e % H), v = (int)((e / H) % M), w = (int)(e / ((size_t)H * M));
-        const int i = shift_idx(u, M), j = shift_idx(v, M), k = shift_idx(w, M);
-        cufftComplex c;
-        c.x = 0.0f;
-        c.y = 0.0f;
-        if (i != 0 && j != 0 && k != 0) {
-            const float r1 = cas[((size_t)(k + b) * V + (j + b)) * V + (i + b)];
-            const float r2 = cas[((size_t)(M - k + b) * V + (M - j + b)) * V + (M - i + b)];
-            c.x = 0.5f * (r1 + r2);
-            c.y = 0.5f * (r1 - r2);
+    const int lane = threadIdx.x & 31, pad = V / 2 - M / 2, H = M / 2 + 1;
+    const long long rows = (long long)V * V;
+    auto value = [&](size_t o) {
+        float a = cas[o];
+        if (DIV) a = a / (__ldg(den + o) + eps);
+        return a;
+    };
+    for (long long r = (long long)blockIdx.x * kRows + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * kRows) {
+        const int ck = (int)(r / V), cj = (int)(r - (long long)ck * V), j = cj - pad, k = ck - pad;
+        const bool inner = (unsigned)j < (unsigned)M && (unsigned)k < (unsigned)M;
+        const size_t ra = (size_t)r * V;
+        if (!inner || j == 0 || k == 0) {
+            if (DIV)
+                for (int c = lane; c < V; c += 32) cas[ra + c] = value(ra + c);
+            if (inner) { // FromCAS zeroes the first planes
+                float2 *s = reinterpret_cast<float2 *>(spec) + ((size_t)shift_idx(k, M) * M + shift_idx(j, M)) * H;
+                for (int u = lane; u < H; u += 32) s[u] = make_float2(0.0f, 0.0f);
+            }
+            continue;
         }
-        spec[e] = c;
+        const int jm = M - j, km = M - k;
+        if (k > km || (k == km && j > jm)) continue; // its mirror row's warp has both
+        const size_t rb = ((size_t)(km + pad) * V + (jm + pad)) * V;
+        if (DIV) { // the columns outside the spectrum: borders and i = 0
+            for (int t = lane; t <= V - M; t += 32) {
+                const int c = t <= pad ? t : t + M - 1; // 0 .. pad, pad + M .. V - 1
+                const float x = value(ra + c), y = value(rb + c);
+                cas[ra + c] = x;
+                cas[rb + c] = y;
+            }
+        }
+        float2 *sa = reinterpret_cast<float2 *>(spec) + ((size_t)shift_idx(k, M) * M + shift_idx(j, M)) * H;
+        float2 *sb = reinterpret_cast<float2 *>(spec) + ((size_t)shift_idx(km, M) * M + shift_idx(jm, M)) * H;
+        const size_t ca = ra + pad + M / 2, cb = rb + pad + M / 2;
+        // kU columns a lane at a time, all loaded before any is stored (the
+        // stores go to the array that is read, so the compiler keeps the order)
+        constexpr int kU = DIV ? 2 : 4;
+        for (int u0 = lane; u0 < M / 2; u0 += 32 * kU) {
+            float a[kU][4], d[kU][4];
+#pragma unroll
+            for (int q = 0; q < kU; q++) {
+                const int u = u0 + 32 * q;
+                const size_t o[4] = {ca + u, ca - u, cb + u, cb - u};
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    a[q][e] = u < M / 2 ? cas[o[e]] : 0.0f;
+                    d[q][e] = DIV && u < M / 2 ? __ldg(den + o[e]) : 0.0f;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < kU; q++) {
+                const int u = u0 + 32 * q;
+                if (u >= M / 2) break;
+                if (DIV) {
+                    const size_t o[4] = {ca + u, ca - u, cb + u, cb - u};
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        a[q][e] = a[q][e] / (d[q][e] + eps);
+                        cas[o[e]] = a[q][e];
+                    }
+                }
+                sa[u] = make_float2(0.5f * (a[q][0] + a[q][3]), 0.5f * (a[q][0] - a[q][3]));
+                sb[u] = make_float2(0.5f * (a[q][2] + a[q][1]), 0.5f * (a[q][2] - a[q][1]));
+            }
+        }
+        if (lane == 0) { // u = M/2 is i = 0
+            sa[M / 2] = make_float2(0.0f, 0.0f);
+            sb[M / 2] = make_float2(0.0f, 0.0f);
+        }
     }
 }
 
 // vol[k][j][i] = y[(k+ob+M/2)%M]... / M^3 * precomp, centred crop.
-__global__ void fft_output_to_vol_kernel(const float *__restrict__ y, int M, int N, const double *__restrict__ pc,
-                                         float *__restrict__ vol)
+__global__ void __launch_bounds__(32 * kRows)
+fft_output_to_vol_kernel(const float *__restrict__ y, int M, int N, const float2 *__restrict__ pc, FF inv,
+                         float *__restrict__ vol)
 {
-    const size_t total = (size_t)N * N * N;
-    const int ob = M / 2 - N / 2;
-    const double inv = 1.0 / ((double)M * M * M);
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const int oi = (int)(e % N), oj = (int)((e / N) % N), ok = (int)(e / ((size_t)N * N));
-        const int i = oi + ob, j = oj + ob, k = ok + ob;
-        const float val = y[((size_t)shift_idx(k, M) * M + shift_idx(j, M)) * M + shift_idx(i, M)];
-        vol[e] = (float)((double)val * inv * pc[i] * pc[j] * pc[k]);
+    const int lane = threadIdx.x & 31, ob = M / 2 - N / 2;
+    const long long rows = (long long)N * N;
+    for (long long r = (long long)blockIdx.x * kRows + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * kRows) {
+        const int ok = (int)(r / N), oj = (int)(r - (long long)ok * N), j = oj + ob, k = ok + ob;
+        const FF jk = ff_mul(inv, ff_mul(ff_at(pc, j), ff_at(pc, k)));
+        const float *yr = y + ((size_t)shift_idx(k, M) * M + shift_idx(j, M)) * M;
+#pragma unroll 4
+        for (int oi = lane; oi < N; oi += 32)
+            vol[r * N + oi] = ff_scale(__ldg(yr + shift_idx(oi + ob, M)), ff_mul(ff_at(pc, oi + ob), jk));
     }
 }
 
@@ -276,40 +401,40 @@ spectrum_to_cas_images_kernel(const cufftComplex *__restrict__ spec, int M, int 
 
 // Gradient of the CAS volume -> volume, first half: crop V^3 to the inner M^3
 // and fftshift (the adjoint of the zero-pad and of the output fftshift).
-__global__ void cas_volume_adjoint_input_kernel(const float *__restrict__ g, int P, int V, int M, float *__restrict__ x)
+__global__ void __launch_bounds__(32 * kRows)
+cas_volume_adjoint_input_kernel(const float *__restrict__ g, int P, int V, int M, float *__restrict__ x)
 {
-    const size_t total = (size_t)M * M * M;
-    const int b = V / 2 - M / 2;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const int qi = (int)(e % M), qj = (int)((e / M) % M), qk = (int)(e / ((size_t)M * M));
-        const int i = shift_idx(qi, M), j = shift_idx(qj, M), k = shift_idx(qk, M);
-        x[e] = g[((size_t)(k + b) * V + (j + b)) * P + (i + b)];
+    const int lane = threadIdx.x & 31, b = V / 2 - M / 2;
+    const long long rows = (long long)M * M;
+    for (long long r = (long long)blockIdx.x * kRows + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * kRows) {
+        const int qk = (int)(r / M), qj = (int)(r - (long long)qk * M);
+        const float *gr = g + ((size_t)(shift_idx(qk, M) + b) * V + (shift_idx(qj, M) + b)) * P + b;
+#pragma unroll 4
+        for (int q = lane; q < M; q += 32) x[r * M + q] = __ldg(gr + shift_idx(q, M));
     }
 }
 
 // Second half: Re+Im of fftshift(FFT), times the precomp, centred crop to N^3.
 // (The adjoint of ToCAS maps g to g + i g; with the unnormalised FFT's adjoint
 // M^3 * ifft of a real input equal to conj(fft), Re((1+i) conj(F)) = Re F + Im F.)
-__global__ void spectrum_to_vol_adjoint_kernel(const cufftComplex *__restrict__ spec, int M, int N,
-                                               const double *__restrict__ pc, float *__restrict__ vol)
+__global__ void __launch_bounds__(32 * kRows)
+spectrum_to_vol_adjoint_kernel(const cufftComplex *__restrict__ spec, int M, int N, const float2 *__restrict__ pc,
+                               float *__restrict__ vol)
 {
-    const size_t total = (size_t)N * N * N;
-    const int ob = M / 2 - N / 2;
-    const int H = M / 2 + 1;
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const int oi = (int)(e % N), oj = (int)((e / N) % N), ok = (int)(e / ((size_t)N * N));
-        const int i = oi + ob, j = oj + ob, k = ok + ob;
-        const int u = shift_idx(i, M), v = shift_idx(j, M), w = shift_idx(k, M);
-        float val;
-        if (u <= M / 2) {
-            const cufftComplex c = spec[((size_t)w * M + v) * H + u];
-            val = c.x + c.y;
-        } else {
-            const int w2 = w ? M - w : 0, v2 = v ? M - v : 0;
-            const cufftComplex c = spec[((size_t)w2 * M + v2) * H + (M - u)];
-            val = c.x - c.y;
+    const int lane = threadIdx.x & 31, ob = M / 2 - N / 2, H = M / 2 + 1;
+    const long long rows = (long long)N * N;
+    for (long long r = (long long)blockIdx.x * kRows + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * kRows) {
+        const int ok = (int)(r / N), oj = (int)(r - (long long)ok * N), j = oj + ob, k = ok + ob;
+        const int v = shift_idx(j, M), w = shift_idx(k, M), v2 = v ? M - v : 0, w2 = w ? M - w : 0;
+        const FF jk = ff_mul(ff_at(pc, j), ff_at(pc, k));
+        const float2 *s1 = reinterpret_cast<const float2 *>(spec) + ((size_t)w * M + v) * H;
+        const float2 *s2 = reinterpret_cast<const float2 *>(spec) + ((size_t)w2 * M + v2) * H;
+#pragma unroll 4
+        for (int oi = lane; oi < N; oi += 32) {
+            const int i = oi + ob, u = shift_idx(i, M);
+            const float2 c = u <= M / 2 ? __ldg(s1 + u) : __ldg(s2 + (M - u));
+            vol[r * N + oi] = ff_scale(u <= M / 2 ? c.x + c.y : c.x - c.y, ff_mul(ff_at(pc, i), jk));
         }
-        vol[e] = (float)((double)val * pc[i] * pc[j] * pc[k]);
     }
 }
 
@@ -491,34 +616,38 @@ __global__ void scale_from_max_kernel(unsigned int *work, float target, float *d
 
 constexpr int kT = 256;
 
-cudaError_t launch_vol_to_fft_input(const float *d_vol, int N, int M, const double *d_precomp, float *d_x, cudaStream_t s)
+cudaError_t launch_vol_to_fft_input(const float *d_vol, int N, int M, const float2 *d_precomp, float *d_x, cudaStream_t s)
 {
-    vol_to_fft_input_kernel<<<grid_for((size_t)M * M * M, kT), kT, 0, s>>>(d_vol, N, M, d_precomp, d_x);
+    vol_to_fft_input_kernel<<<rows_grid((long long)M * M), 32 * kRows, 0, s>>>(d_vol, N, M, d_precomp, d_x);
     count_launches(1);
     return cudaGetLastError();
 }
 
-cudaError_t launch_spectrum_to_cas_volume(const cufftComplex *d_spec, int M, int V, void *d_cas, int prec,
-                                          const float *d_scale, cudaStream_t s)
+cudaError_t launch_spectrum_to_cas_volume(const cufftComplex *d_spec, int M, int V, float *d_cas, cudaStream_t s)
 {
-    const unsigned g = grid_for((size_t)V * V * V, kT);
-    if (prec == kF32) spectrum_to_cas_volume_kernel<float><<<g, kT, 0, s>>>(d_spec, M, V, (float *)d_cas, d_scale);
-    else if (prec == kF16) spectrum_to_cas_volume_kernel<__half><<<g, kT, 0, s>>>(d_spec, M, V, (__half *)d_cas, d_scale);
-    else spectrum_to_cas_volume_kernel<__nv_bfloat16><<<g, kT, 0, s>>>(d_spec, M, V, (__nv_bfloat16 *)d_cas, d_scale);
+    spectrum_to_cas_volume_kernel<<<rows_grid((long long)V * V), 32 * kRows, 0, s>>>(d_spec, M, V, d_cas);
     count_launches(1);
     return cudaGetLastError();
 }
 
-cudaError_t launch_cas_volume_to_spectrum(const float *d_cas, int V, int M, cufftComplex *d_spec, cudaStream_t s)
+cudaError_t launch_cas_volume_to_spectrum(float *d_cas, const float *d_density, float eps, int V, int M,
+                                          cufftComplex *d_spec, cudaStream_t s)
 {
-    cas_volume_to_spectrum_kernel<<<grid_for((size_t)M * M * (M / 2 + 1), kT), kT, 0, s>>>(d_cas, V, M, d_spec);
+    const unsigned g = rows_grid((long long)V * V);
+    if (d_density)
+        cas_volume_to_spectrum_kernel<true><<<g, 32 * kRows, 0, s>>>(d_cas, d_density, eps, V, M, d_spec);
+    else
+        cas_volume_to_spectrum_kernel<false><<<g, 32 * kRows, 0, s>>>(d_cas, nullptr, 0.0f, V, M, d_spec);
     count_launches(1);
     return cudaGetLastError();
 }
 
-cudaError_t launch_fft_output_to_vol(const float *d_y, int M, int N, const double *d_precomp, float *d_vol, cudaStream_t s)
+cudaError_t launch_fft_output_to_vol(const float *d_y, int M, int N, const float2 *d_precomp, float *d_vol, cudaStream_t s)
 {
-    fft_output_to_vol_kernel<<<grid_for((size_t)N * N * N, kT), kT, 0, s>>>(d_y, M, N, d_precomp, d_vol);
+    const double inv = 1.0 / ((double)M * M * M);
+    const float h = (float)inv;
+    fft_output_to_vol_kernel<<<rows_grid((long long)N * N), 32 * kRows, 0, s>>>(d_y, M, N, d_precomp,
+                                                                                FF{h, (float)(inv - (double)h)}, d_vol);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -574,15 +703,15 @@ cudaError_t launch_spectrum_to_cas_images_adjoint(const cufftComplex *d_spec, in
 
 cudaError_t launch_cas_volume_adjoint_input(const float *d_g, int pitch, int V, int M, float *d_x, cudaStream_t s)
 {
-    cas_volume_adjoint_input_kernel<<<grid_for((size_t)M * M * M, kT), kT, 0, s>>>(d_g, pitch, V, M, d_x);
+    cas_volume_adjoint_input_kernel<<<rows_grid((long long)M * M), 32 * kRows, 0, s>>>(d_g, pitch, V, M, d_x);
     count_launches(1);
     return cudaGetLastError();
 }
 
-cudaError_t launch_spectrum_to_vol_adjoint(const cufftComplex *d_spec, int M, int N, const double *d_precomp, float *d_vol,
+cudaError_t launch_spectrum_to_vol_adjoint(const cufftComplex *d_spec, int M, int N, const float2 *d_precomp, float *d_vol,
                                            cudaStream_t s)
 {
-    spectrum_to_vol_adjoint_kernel<<<grid_for((size_t)N * N * N, kT), kT, 0, s>>>(d_spec, M, N, d_precomp, d_vol);
+    spectrum_to_vol_adjoint_kernel<<<rows_grid((long long)N * N), 32 * kRows, 0, s>>>(d_spec, M, N, d_precomp, d_vol);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -109,17 +109,18 @@ cudaError_t launch_back_project_adjoint(float *d_vol, int pitch, const void *d_i
 // ---- CAS / FFT stages (gg_cas.cu) ------------------------------------------
 // Volume N^3 -> real M^3 FFT input: centred zero-pad, separable precomp
 // multiply, fftshift folded into the index map.
-cudaError_t launch_vol_to_fft_input(const float *d_vol, int N, int M, const double *d_precomp,
+// d_precomp here and below: the FP64 factors as float pairs (hi, lo).
+cudaError_t launch_vol_to_fft_input(const float *d_vol, int N, int M, const float2 *d_precomp,
                                     float *d_x, cudaStream_t s);
-// R2C half spectrum [M][M][M/2+1] -> CAS volume V^3 (storage `prec`), border zeroed.
-cudaError_t launch_spectrum_to_cas_volume(const cufftComplex *d_spec, int M, int V, void *d_cas,
-                                          int prec, const float *d_scale, cudaStream_t s);
+// R2C half spectrum [M][M][M/2+1] -> FP32 CAS volume V^3, border zeroed.
+cudaError_t launch_spectrum_to_cas_volume(const cufftComplex *d_spec, int M, int V, float *d_cas, cudaStream_t s);
 // CAS volume V^3 (FP32) -> Hermitian half spectrum for C2R: crop the pad,
-// FromCAS 3-D, fftshift folded into the index map.
-cudaError_t launch_cas_volume_to_spectrum(const float *d_cas, int V, int M, cufftComplex *d_spec,
-                                          cudaStream_t s);
+// FromCAS 3-D, fftshift folded into the index map.  d_density (optional): the
+// volume is first divided in place, cas / (density + eps).
+cudaError_t launch_cas_volume_to_spectrum(float *d_cas, const float *d_density, float eps, int V, int M,
+                                          cufftComplex *d_spec, cudaStream_t s);
 // C2R output M^3 -> volume N^3: fftshift, 1/M^3, precomp, centred crop.
-cudaError_t launch_fft_output_to_vol(const float *d_y, int M, int N, const double *d_precomp,
+cudaError_t launch_fft_output_to_vol(const float *d_y, int M, int N, const float2 *d_precomp,
                                      float *d_vol, cudaStream_t s);
 // CAS images n*M*M -> Hermitian half spectra n*M*(M/2+1) (FromCAS 2-D + shift).
 cudaError_t launch_cas_images_to_spectrum(const float *d_cas, int M, int n, cufftComplex *d_spec,
@@ -141,7 +142,7 @@ cudaError_t launch_spectrum_to_cas_images_adjoint(const cufftComplex *d_spec, in
 // CAS-volume gradient V^3 (rows `pitch` floats apart) -> R2C input M^3 (inner crop + shift).
 cudaError_t launch_cas_volume_adjoint_input(const float *d_g, int pitch, int V, int M, float *d_x, cudaStream_t s);
 // R2C spectrum -> volume gradient N^3 (Re+Im, shift, precomp, crop).
-cudaError_t launch_spectrum_to_vol_adjoint(const cufftComplex *d_spec, int M, int N, const double *d_precomp,
+cudaError_t launch_spectrum_to_vol_adjoint(const cufftComplex *d_spec, int M, int N, const float2 *d_precomp,
                                            float *d_vol, cudaStream_t s);
 // d[0..count) = value.
 cudaError_t launch_fill(float *d, size_t count, float value, cudaStream_t s);
