@@ -311,6 +311,12 @@ void check_axes_count(int n)
 void update_fp(gg_gridder *h, cudaStream_t s)
 {
     if (h->cas_fp_valid) return;
+    if (!h->fault) {
+        void *p = nullptr;
+        GG_CK(cudaHostAlloc(&p, sizeof(int), cudaHostAllocDefault));
+        h->fault = (int *)p;
+        *h->fault = 0;
+    }
     const size_t V = h->V, P = fp_pitch(h->V, h->prec);
     h->cas_fp.ensure(P * V * V * prec_bytes(h->prec));
     if (h->fp_maps_vol != h->cas_fp.p || h->fp_maps_prec != h->prec) {
@@ -689,10 +695,6 @@ void init_handle(gg_gridder *h)
     GG_CK(cudaMemcpy(h->scales.p, ones, sizeof(ones), cudaMemcpyHostToDevice));
     h->work.ensure(1);
     GG_CK(cudaMemset(h->work.p, 0, sizeof(unsigned int)));
-    void *fault = nullptr;
-    GG_CK(cudaHostAlloc(&fault, sizeof(int), cudaHostAllocDefault));
-    h->fault = (int *)fault;
-    *h->fault = 0;
     h->fused_fft = fft2_fused_ok(h->N, h->M);
 }
 
@@ -749,7 +751,7 @@ template <typename F> int guarded(gg_gridder *h, F &&f)
     try {
         set_device(h);
         f();
-        if (*(volatile int *)h->fault) fail(GG_ERR_CUDA, "a forward projection's copies to shared memory did not arrive");
+        if (h->fault && *(volatile int *)h->fault) fail(GG_ERR_CUDA, "a forward projection's copies to shared memory did not arrive");
         h->err.clear();
         return GG_OK;
     } catch (const GGError &e) {

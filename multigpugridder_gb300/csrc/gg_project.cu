@@ -392,6 +392,12 @@ __device__ __forceinline__ float lds_f32(unsigned addr)
     return v;
 }
 
+__device__ __forceinline__ void cp_async16(float *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
 struct FootWin {
     float nx0, nx1, nx2, ny0, ny1, ny2;
     float vc;         // volume centre
@@ -916,35 +922,48 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
             group_sync(grp + 1);
             const int count = sm.scount;
 
-            for (int q = 0; q < count; q++) {
-                const int e = slist[q];
+            // NB = 2: a pass beyond the last chunk's list runs what is left in
+            // the queue, so that the window code is expanded once
+            const bool last = NB > 1 && c0 + kBpChunk >= d1;
+            for (int q = 0; q < count + (last ? 1 : 0); q++) {
+                const bool flush = NB > 1 && q == count;
+                const int e = flush ? 0 : slist[q];
                 const int al = e & (kBpChunk - 1);
                 const float *ax = sax + al * 9;
                 const float nz0 = ax[6], nz1 = ax[7], nz2 = ax[8];
                 {   // the warp's 8x4xBD block against the slab (uniform)
                     const float d = wcx * nz0 + wcy * nz1 + wcz * nz2;
                     const float ext = 0.5f * (7.0f * fabsf(nz0) + 3.0f * fabsf(nz1) + (float)(BD - 1) * fabsf(nz2));
-                    if (fabsf(d) > slab + ext) continue;
+                    if (!flush && fabsf(d) > slab + ext) continue;
                 }
-                // the reference's per-voxel slab test (gpuBackProject.cu:64-66)
-                unsigned actm = 0;
+                // Whole rounds, and whatever buffer b's earlier direction still
+                // has in the queue (at its front), run before b is refilled.
+                const int b = NB > 1 ? nbuf : 0;
+                if (NB > 1) {
+                    if (QALIGN && sizeof(TI) == 4 && !ONES) {
+                        asm volatile("cp.async.wait_all;" ::: "memory");
+                        __syncwarp(); // the footprints' copies are complete, for every lane
+                    }
+                    while (qsize >= 32 || (qsize > 0 && (flush || (LEAN ? bfront : (int)(wq[qhead & QM] >> 8)) == b)))
+                        run_round(min(qsize, 32));
+                    if (flush) break;
+                }
+                // the reference's per-voxel slab test (gpuBackProject.cu:64-66);
+                // the active voxels join the queue (NB = 1: the list) slot by
+                // slot in lane order
+                const int tail = NB > 1 ? qhead + qsize : 0;
                 int total = 0;
 #pragma unroll
                 for (int s = 0; s < BD; s++) {
                     const float az = (float)(bz + s) - volCenter;
                     const float fk = voxel_proj(ax0, ay0, az, nz0, nz1, nz2);
                     const bool act = ((inmask >> s) & 1u) && fabsf(fk) <= kerHW;
-                    actm |= (act ? 1u : 0u) << s;
-                    total += __popc(__ballot_sync(0xffffffffu, act));
+                    const unsigned bal = __ballot_sync(0xffffffffu, act);
+                    if (act) wq[(tail + total + __popc(bal & lt_mask)) & QM] = (QEnt)((lane + 32 * s) | (LEAN ? 0 : b << 8));
+                    total += __popc(bal);
                 }
                 if (total == 0) continue;
-                int b = 0;
-                if (NB > 1) {
-                    b = nbuf;
-                    nbuf ^= 1;
-                    // buffer b's earlier voxels (all at the front of the queue) run first
-                    while (qsize > 0 && (LEAN ? bfront : (int)(wq[qhead & QM] >> 8)) == b) run_round(min(qsize, 32));
-                }
+                if (NB > 1) nbuf ^= 1;
                 float *const wfoot = wfoot0 + b * (FH * FS);
                 float *const wfoot2 = wfoot20 + (DW ? b * (FH * FS) : 0);
                 const float nx0 = ax[0], nx1 = ax[1], nx2 = ax[2];
@@ -960,11 +979,11 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                     const float hz = 0.5f * (float)(BD - 1);
                     const float hi = 3.5f * fabsf(nx0) + 1.5f * fabsf(nx1) + hz * fabsf(nx2);
                     const float hj = 3.5f * fabsf(ny0) + 1.5f * fabsf(ny1) + hz * fabsf(ny2);
-                    fi0 = (int)floorf(ic - hi - 0.6f) - HALF;
-                    fj0 = (int)floorf(jc - hj - 0.6f) - HALF;
-                    const int fw = (int)floorf(ic + hi + 0.6f) + HALF - fi0 + 1;
-                    fh = (int)floorf(jc + hj + 0.6f) + HALF - fj0 + 1;
-                    foot = fw <= FW && fh <= FH && fh >= W;
+                    // at most 2 |(3.5, 1.5, hz)| + 1.2 apart: width and height fit FW
+                    fi0 = __float2int_rd(ic - hi - 0.6f) - HALF;
+                    fj0 = __float2int_rd(jc - hj - 0.6f) - HALF;
+                    fh = __float2int_rd(jc + hj + 0.6f) + HALF - fj0 + 1;
+                    foot = fh <= FH;
                     if (foot && !ONES && vecImg) {
                         // vector loads of aligned pixel quads (rows start at
                         // multiples of 4 elements: 4 divides M, the image stacks
@@ -972,43 +991,36 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                         // pixel by pixel
                         constexpr int NQ = FW / 4 + 1; // quads per footprint row
                         const int base = fi0 & ~3, sh = fi0 & 3;
-                        if constexpr (DW) {
-                            // two image stacks: one quad at a time (both stacks'
-                            // quads held at once would spill)
-                            for (int t = lane; t < fh * NQ; t += 32) {
-                                const int r = t / NQ, qq = t - r * NQ;
-                                const int c0 = 4 * qq - sh; // footprint column of the quad's first pixel
-                                const int lin0 = (fj0 + r) * M + base + 4 * qq;
-                                float v[4] = {0.0f, 0.0f, 0.0f, 0.0f}, v2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                                if (lin0 >= 0 && lin0 + 3 < MM) {
-                                    ld_quad(img_ptr + lin0, v);
-                                    ld_quad(img2_ptr + lin0, v2);
-                                } else {
-#pragma unroll
-                                    for (int e = 0; e < 4; e++)
-                                        if (lin0 + e >= 0 && lin0 + e < MM) {
-                                            v[e] = ld_f32(img_ptr + lin0 + e);
-                                            v2[e] = __ldg(img2_ptr + lin0 + e);
-                                        }
+                        const int first = fj0 * M + base, nq = fh * NQ;
+                        if constexpr (QALIGN && sizeof(TI) == 4) {
+                            if (first >= 0 && first + (fh - 1) * M + 4 * NQ <= MM) {
+                                // no pixel outside the image's index range: quad t of
+                                // the footprint lies at its word 4 t (FS = 4 NQ).
+                                // Copied behind the warp's back: nothing is held in
+                                // registers, and the copies are waited for when the
+                                // next direction's rounds begin
+                                for (int t = lane; t < nq; t += 32) {
+                                    const int o = first + (t / NQ) * (M - 4 * NQ) + 4 * t;
+                                    cp_async16(wfoot + 4 * t, img_ptr + o);
+                                    if (DW) cp_async16(wfoot2 + 4 * t, img2_ptr + o);
                                 }
-                                if (QALIGN) {
-                                    *reinterpret_cast<float4 *>(wfoot + r * FS + 4 * qq) = make_float4(v[0], v[1], v[2], v[3]);
-                                    *reinterpret_cast<float4 *>(wfoot2 + r * FS + 4 * qq) =
-                                        make_float4(v2[0], v2[1], v2[2], v2[3]);
-                                } else {
+                            } else {
+#pragma unroll 1
+                                for (int t = lane; t < nq; t += 32) {
+                                    const int lin0 = first + (t / NQ) * (M - 4 * NQ) + 4 * t;
 #pragma unroll
-                                    for (int e = 0; e < 4; e++)
-                                        if (c0 + e >= 0 && c0 + e < FW) {
-                                            wfoot[r * FS + c0 + e] = v[e];
-                                            wfoot2[r * FS + c0 + e] = v2[e];
-                                        }
+                                    for (int e = 0; e < 4; e++) {
+                                        const bool in = lin0 + e >= 0 && lin0 + e < MM;
+                                        wfoot[4 * t + e] = in ? ld_f32(img_ptr + lin0 + e) : 0.0f;
+                                        if (DW) wfoot2[4 * t + e] = in ? __ldg(img2_ptr + lin0 + e) : 0.0f;
+                                    }
                                 }
                             }
                         } else {
                             // a lane's quads (at most KQ) are all loaded before any is
                             // stored, so their L2 latencies overlap
+                            static_assert(!DW, "the two-stack form stages by copies");
                             constexpr int KQ = (FH * NQ + 31) / 32;
-                            const int nq = fh * NQ;
                             float v[KQ][4];
 #pragma unroll
                             for (int u = 0; u < KQ; u++) {
@@ -1083,32 +1095,13 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                 if (NB > 1) {
                     if (lane == 0)
                         wmeta[b] = BpDirMeta{nx0, nx1, nx2, ny0, ny1, ny2, fi0, fj0, fh, foot ? 1 : 0, c0 + al, 0};
-                    // the active voxels join the queue slot by slot, in lane order
-                    int pos = qhead + qsize;
-#pragma unroll
-                    for (int s = 0; s < BD; s++) {
-                        const bool act = (actm >> s) & 1u;
-                        const unsigned bal = __ballot_sync(0xffffffffu, act);
-                        if (act) wq[(pos + __popc(bal & lt_mask)) & QM] = (QEnt)((lane + 32 * s) | (LEAN ? 0 : b << 8));
-                        pos += __popc(bal);
-                    }
                     if (qsize == 0) {
                         bfront = b;
                         nfront = total;
                     }
                     qsize += total;
                     __syncwarp(); // the queue entries, the footprint and its record are complete
-                    while (qsize >= 32) run_round(32);
                 } else {
-                    // the active voxels, slot by slot in lane order, run at once
-                    int pos = 0;
-#pragma unroll
-                    for (int s = 0; s < BD; s++) {
-                        const bool act = (actm >> s) & 1u;
-                        const unsigned bal = __ballot_sync(0xffffffffu, act);
-                        if (act) wq[pos + __popc(bal & lt_mask)] = (QEnt)(lane + 32 * s);
-                        pos += __popc(bal);
-                    }
                     __syncwarp(); // the voxel list and the footprint are complete
                     for (int base = 0; base < total; base += 32) {
                         const int t = base + lane;
@@ -1126,8 +1119,6 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                 }
             }
         }
-        if (NB > 1)
-            while (qsize > 0) run_round(min(qsize, 32));
         __syncwarp();
         const float sc = d_scale ? *d_scale : 1.0f;
 #pragma unroll
