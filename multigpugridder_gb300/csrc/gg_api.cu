@@ -159,6 +159,7 @@ struct gg_gridder {
     int *fault = nullptr;       // pinned: set by a kernel whose copies did not arrive
     DevBuf<float> pd;        // plane density V^3
     DevBuf<float> bp_part;   // sums of a split back projection's segments
+    DevBuf<unsigned> bp_next; // its groups' work counter, 0 between launches
     DevBuf<float> adj;       // CAS-volume gradient, V^2 rows of fp_pitch(V, kF32) (forward-operator adjoint)
     DevBuf<float> axes;
     DevBuf<float> vol_io;    // N^3
@@ -396,7 +397,7 @@ BpSplit bp_split(gg_gridder *h, int b, int stacks)
 {
     const int nseg = bp_segments(b, h->geom());
     if (nseg > 1) h->bp_part.ensure((size_t)(nseg - 1) * stacks * h->V * h->V * h->V);
-    return BpSplit{nseg, h->bp_part.p};
+    return BpSplit{nseg, h->bp_part.p, h->bp_next.p};
 }
 
 // Back-project b directions: images (device, FFT path) or CAS images (device).
@@ -693,6 +694,8 @@ void init_handle(gg_gridder *h)
     h->scales.ensure(2);
     const float ones[2] = {1.0f, 1.0f};
     GG_CK(cudaMemcpy(h->scales.p, ones, sizeof(ones), cudaMemcpyHostToDevice));
+    h->bp_next.ensure(1);
+    GG_CK(cudaMemset(h->bp_next.p, 0, sizeof(unsigned)));
     h->work.ensure(1);
     GG_CK(cudaMemset(h->work.p, 0, sizeof(unsigned int)));
     h->fused_fft = fft2_fused_ok(h->N, h->M);
@@ -724,6 +727,7 @@ void destroy_handle(gg_gridder *h)
     if (h->fault) cudaFreeHost(h->fault);
     h->pd.release();
     h->bp_part.release();
+    h->bp_next.release();
     h->adj.release();
     h->axes.release();
     h->vol_io.release();

@@ -67,9 +67,13 @@ cudaError_t launch_pitch_volume(const float *d_cas, int V, int P, void *d_out, i
 // side by side: segment 0 accumulates into the volume as an unsplit launch
 // does, the others write their sums to `part` ((nseg - 1) * V^3 floats, twice
 // that with a density), and a merge adds them in order.  nseg = 1: unsplit.
+// next (optional): a device counter, zero between launches and used by one
+// launch at a time, from which the brick groups of a launch that owns the GPU
+// take their work.
 struct BpSplit {
-    int nseg;
-    float *part;
+    int nseg = 1;
+    float *part = nullptr;
+    unsigned *next = nullptr;
 };
 // The number of segments for n directions.
 int bp_segments(int n, const Geom &g);
@@ -84,20 +88,20 @@ int bp_segments(int n, const Geom &g);
 cudaError_t launch_back_project_ref(float *d_vol, const void *d_img, int iprec, bool ones,
                                     const float *d_ker, const float *d_axes, int n, const Geom &g,
                                     const float *d_scale, cudaStream_t s, bool shared = false,
-                                    BpSplit split = {1, nullptr});
+                                    BpSplit split = BpSplit());
 
 // Reference-rule back projection of d_img into d_vol and, in the same pass,
 // of all-ones images (the plane density) into d_pd; both accumulated.
 cudaError_t launch_back_project_ref_density(float *d_vol, float *d_pd, const void *d_img, int iprec,
                                             const float *d_ker, const float *d_axes, int n, const Geom &g,
-                                            const float *d_scale, cudaStream_t s, BpSplit split = {1, nullptr});
+                                            const float *d_scale, cudaStream_t s, BpSplit split = BpSplit());
 
 // Reference-rule back projection of two FP32 image stacks over the same
 // directions in one pass: d_img into d_vol and d_img2 into d_pd, both
 // accumulated, each equal to its own launch_back_project_ref.
 cudaError_t launch_back_project_ref_pair(float *d_vol, float *d_pd, const float *d_img, const float *d_img2,
                                          const float *d_ker, const float *d_axes, int n, const Geom &g, cudaStream_t s,
-                                         BpSplit split = {1, nullptr});
+                                         BpSplit split = BpSplit());
 
 // Exact adjoint of the 4-tap forward projection (gg_adjoint.cu), added to
 // d_vol, rows `pitch` floats apart (planes pitch * V; dense: pitch = V).  The

@@ -635,8 +635,8 @@ __host__ __device__ __forceinline__ int middle_out(int r, int n)
     return r & 1 ? c + (r + 1) / 2 : c - r / 2;
 }
 
-// The CTAs of a launch, layer by layer from the middle outwards: layer rank r
-// holds the brick runs pre[r] .. pre[r + 1] - 1.  Counted on the host, so that
+// The bricks of a launch, layer by layer from the middle outwards: layer rank r
+// holds bricks pre[r] .. pre[r + 1] - 1, row by row.  Counted on the host, so that
 // no CTA starts (and takes a whole SM) without bricks: at M = 256 the box of
 // bricks holds 6,182 runs, of which 1,900 meet the sphere (reconstructVol of
 // 1,000 images 6.99 -> 6.66 ms, of 16 images 688 -> 618 us).
@@ -644,6 +644,41 @@ constexpr int kMaxLayers = 511; // 6,132 voxels of 12-deep bricks: 860 GB of CAS
 struct BpLayers {
     int layers, pre[kMaxLayers + 1];
 };
+
+// Place (x, y, z) of a brick in its layer's rows, by a scan over the rows; the
+// whole warp calls it for one brick.  Out of line: inlined, its invariants
+// took registers through the window loops.
+__device__ __noinline__ int3 brick_at(int brick, const BpLayers &lay, int bricksX, int bricksY, int c, int BZ, int maskR)
+{
+    const int lane = threadIdx.x & 31;
+    int rank = 0; // the last layer rank whose first brick is <= brick
+    for (int hi = lay.layers - 1; rank < hi;) {
+        const int mid = (rank + hi + 1) >> 1;
+        if (lay.pre[mid] <= brick) rank = mid;
+        else hi = mid - 1;
+    }
+    int3 at = make_int3(0, 0, middle_out(rank, lay.layers));
+    for (int j0 = 0, before = lay.pre[rank]; j0 < bricksY; j0 += 32) {
+        int lo = 0, cnt = 0;
+        if (j0 + lane < bricksY) brick_row(j0 + lane, at.z, bricksX, c, BZ, maskR, lo, cnt);
+        int incl = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
+        }
+        const int first = before + incl - cnt;
+        const unsigned hit = __ballot_sync(0xffffffffu, brick >= first && brick < first + cnt);
+        if (hit) {
+            const int src = __ffs(hit) - 1;
+            at.x = __shfl_sync(0xffffffffu, lo + brick - first, src);
+            at.y = j0 + src;
+            break;
+        }
+        before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    return at;
+}
 
 __device__ __forceinline__ void group_sync(int id)
 {
@@ -668,46 +703,13 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
     constexpr int FW = Shape::FW, FH = FW, FS = FW + (QALIGN ? 4 : 1);
     using Mem = BpGroupMem<DENS, DW, DEEP, LEAN>;
     using QEnt = typename Mem::QEnt;
-    // [table: tb.entries x tb.copies][G x Mem][row starts][row prefix]
+    // [table: tb.entries x tb.copies][G x Mem]
     extern __shared__ __align__(16) float bp_smem[];
     const int cp = tb.copies, tabWords = tb.entries * cp;
     Mem *gmem = reinterpret_cast<Mem *>(bp_smem + ((tabWords + 3) & ~3)); // 16-byte aligned
-    int *slo = reinterpret_cast<int *>(gmem + G), *spre = slo + bricksY;
     const int volCenter = (int)((float)V) / 2;
     const int imgCenter = (int)((float)M) / 2;
 
-    // The CTA's bricks: those of z-layer kz that meet the mask sphere,
-    // numbered row by row; the CTA takes run `run` of RUN * G numbers (below).
-    // Row (y, z) holds the x interval [slo, slo + n).
-    // SPLIT: a run's segments of the directions are neighbours in the grid.
-    const int ns = SPLIT ? split.nseg : 1, item = SPLIT ? blockIdx.x / ns : blockIdx.x;
-    const int d0 = SPLIT ? (int)((long long)n * (blockIdx.x % ns) / ns) : 0;
-    const int d1 = SPLIT ? (int)((long long)n * (blockIdx.x % ns + 1) / ns) : n;
-    int rank = 0; // the last layer rank whose first run is <= item
-    for (int hi = lay.layers - 1; rank < hi;) {
-        const int mid = (rank + hi + 1) >> 1;
-        if (lay.pre[mid] <= item) rank = mid;
-        else hi = mid - 1;
-    }
-    const int kz = middle_out(rank, lay.layers), run = item - lay.pre[rank];
-    for (int j = threadIdx.x; j < bricksY; j += blockDim.x) {
-        int lo, cnt;
-        brick_row(j, kz, bricksX, volCenter, kCBZ, maskR, lo, cnt);
-        slo[j] = lo;
-        spre[j] = cnt;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int j = 0; j < bricksY; j++) {
-            const int c = spre[j];
-            spre[j] = acc;
-            acc += c;
-        }
-        spre[bricksY] = acc;
-    }
-    __syncthreads();
-    const int total = spre[bricksY];
     if (TS == 128) { // 32 copies: a warp's lanes store 16 copies of 8 entries
         for (int t = threadIdx.x; t < tb.entries * 8; t += blockDim.x) {
             const float w = __ldg(ker + min(t >> 3, kerSize - 1));
@@ -718,29 +720,30 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
     }
     __syncthreads();
 
-    // Group g runs brick g of the CTA's run of RUN * G bricks, and
-    // with 8-deep blocks (RUN = 2) then brick 2 G - 1 - g: along a run
-    // the work drifts (about 2/r of the directions reach a voxel at radius r),
-    // and the mirrored pairs even it out.  On 512^2 images that measured 2-3%
-    // faster; on 256^2 images 8% slower, as the groups drift apart in time and
-    // lose the L1 reuse of the neighbouring bricks' footprints.
-    constexpr int RUN = (DEEP && G > 1) ? 2 : 1;
+    // Items: the bricks that meet the mask sphere (SPLIT: times the segments of
+    // the directions, a brick's side by side), heaviest layers first.  With a
+    // counter (split.next) each group takes the next item on its own: no group
+    // waits for the others' bricks (15% of the warps' time when a CTA ended with
+    // its slowest brick) and the KB table is staged once an SM.  reconstructVol
+    // of 1,000 images at M = 256 6.39 -> 6.09 ms, of 512 at M = 512 15.24 ->
+    // 14.56 ms, of 16 at M = 256 530 -> 468 us; CTF-corrected 6.96 -> 6.55 ms.
     const int grp = threadIdx.x / kCThreads;
-    for (int pass = 0; pass < RUN; pass++) {
-        const int a = RUN * G * run + (pass == 0 ? grp : RUN * G - 1 - grp);
-        if (a >= total) break;
-        int row = 0; // the last row whose prefix is <= a (it holds brick a)
-        for (int hi = bricksY - 1; row < hi;) {
-            const int mid = (row + hi + 1) >> 1;
-            if (spre[mid] <= a) row = mid;
-            else hi = mid - 1;
-        }
+    const int ns = SPLIT ? split.nseg : 1, items = lay.pre[lay.layers] * ns;
+    // SPLIT, or few items: apart, so that an SM's groups share out the heavy
+    // ones (reconstructVol of 16 images at M = 128: 142 against 149 us); many:
+    // neighbours, which share footprints in L1 (1,000 at M = 256: 6.09 against
+    // 6.33 ms)
+    const bool apart = split.next && (SPLIT || items < 4 * (int)gridDim.x * G);
+    for (int item = apart ? grp * gridDim.x + blockIdx.x : blockIdx.x * G + grp; item < items;) {
+        const int3 at = brick_at(SPLIT ? item / ns : item, lay, bricksX, bricksY, volCenter, kCBZ, maskR);
+        const int d0 = SPLIT ? (int)((long long)n * (item % ns) / ns) : 0;
+        const int d1 = SPLIT ? (int)((long long)n * (item % ns + 1) / ns) : n;
         Mem &sm = gmem[grp];
         float *sax = sm.sax;
         typename Mem::LEnt *slist = sm.slist;
         int *swarp = sm.swarp;
         const int tid = threadIdx.x - grp * kCThreads, warp = tid >> 5, lane = tid & 31;
-        const int x0 = (slo[row] + a - spre[row]) * kCBX, y0 = row * kCBY, z0 = kz * kCBZ;
+        const int x0 = at.x * kCBX, y0 = at.y * kCBY, z0 = at.z * kCBZ;
         const int bx = x0 + (warp & 1) * 8, by = y0 + ((warp >> 1) & 1) * 4, bz = z0 + (warp >> 2) * BD;
         const float *sker = bp_smem + lane % cp; // entry k at sker[k * cp]
         const unsigned stride = 4u * (unsigned)cp;
@@ -1125,15 +1128,26 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
         for (int s = 0; s < BD; s++) {
             if (!((inmask >> s) & 1u)) continue;
             const size_t o = (size_t)(bz + s) * V * V + (size_t)ly * V + lx;
-            if (!SPLIT || blockIdx.x % split.nseg == 0) {
+            if (!SPLIT || item % ns == 0) {
                 vol[o] = vol[o] + wacc[lane + 32 * s] * sc;
                 if (DENS || DW) pd[o] = pd[o] + waccw[lane + 32 * s];
             } else {
-                float *const pv = split.part + (size_t)(blockIdx.x % split.nseg - 1) * (DENS || DW ? 2 : 1) * V * V * V;
+                float *const pv = split.part + (size_t)(item % ns - 1) * (DENS || DW ? 2 : 1) * V * V * V;
                 pv[o] = wacc[lane + 32 * s] * sc;
                 if (DENS || DW) pv[(size_t)V * V * V + o] = waccw[lane + 32 * s];
             }
         }
+        if (!split.next) return;
+        if (tid == 0) {
+            // every item is fetched or started on once: the fetch that returns
+            // items - 1 is the last, and leaves the counter at 0 for the next launch
+            const unsigned f = atomicAdd(split.next, 1u);
+            if (f == (unsigned)items - 1) atomicExch(split.next, 0u);
+            sm.scount = (int)f;
+        }
+        group_sync(grp + 1);
+        item = (int)gridDim.x * G + sm.scount;
+        group_sync(grp + 1); // read by all before the next item's culling writes it
     }
 }
 
@@ -1168,7 +1182,7 @@ static cudaError_t launch_bp_compact_g(float *vol, const TI *img, const float *k
     // one group per CTA (the serving lanes): the non-LEAN layout
     constexpr bool LEAN = G > 1;
     using Mem = BpGroupMem<DENS, DW, DEEP, LEAN>;
-    const size_t other = G * sizeof(Mem) + (2 * (size_t)by + 1) * sizeof(int);
+    const size_t other = G * sizeof(Mem);
     // one group per CTA: three CTAs an SM (228 KB, 1 KB reserved per CTA)
     const size_t limit = G == 1 ? (size_t)(228 * 1024 / 3 - 1024) : 0;
     const BpTable tb = bp_table(g.ker_size, other, max_copies, limit);
@@ -1177,8 +1191,6 @@ static cudaError_t launch_bp_compact_g(float *vol, const TI *img, const float *k
     // quad loads of image rows: 4 | M and the stacks aligned to 4 elements
     const size_t qa = 4 * sizeof(TI);
     const int vec = (g.M % 4 == 0) && ((size_t)img % qa == 0) && (!img2 || (size_t)img2 % 16 == 0) ? 1 : 0;
-    // one CTA for each run of RUN * G bricks of a layer that meet the sphere
-    const int run = ((DEEP && G > 1) ? 2 : 1) * G;
     if (bz > kMaxLayers) return cudaErrorInvalidValue;
     BpLayers lay;
     lay.layers = bz;
@@ -1190,15 +1202,17 @@ static cudaError_t launch_bp_compact_g(float *vol, const TI *img, const float *k
             brick_row(j, middle_out(r, bz), bx, (int)((float)g.V) / 2, kCBZ, g.mask_radius, lo, cnt);
             bricks += cnt;
         }
-        lay.pre[r + 1] = lay.pre[r] + (bricks + run - 1) / run;
+        lay.pre[r + 1] = lay.pre[r] + bricks;
     }
-    const unsigned grid = (unsigned)lay.pre[bz] * (unsigned)split.nseg;
-    if (grid == 0) return cudaSuccess;
+    const long long items = (long long)lay.pre[bz] * split.nseg;
+    if (items == 0) return cudaSuccess;
+    long long grid = (items + G - 1) / G;
+    if (split.next) grid = std::min<long long>(grid, num_sms()); // one CTA an SM
     // the table stride as a compile-time constant where the copy count gives one
     auto go = [&](auto kern) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
         if (e != cudaSuccess) return e;
-        kern<<<grid, kCThreads * G, dyn, s>>>(vol, pd, g.V, img, g.M, axes, n, g.mask_radius, ker, g.ker_size,
+        kern<<<(unsigned)grid, kCThreads * G, dyn, s>>>(vol, pd, g.V, img, g.M, axes, n, g.mask_radius, ker, g.ker_size,
                                               g.ker_hw, bx, by, tb, scale, img2, vec, split, lay);
         count_launches(1);
         if (split.nseg > 1) {
@@ -1223,7 +1237,7 @@ template <typename TI, bool ONES, bool DENS = false, bool DW = false, bool DEEP 
 static cudaError_t launch_bp_compact_t(float *vol, const TI *img, const float *ker, const float *axes, int n,
                                        const Geom &g, const float *scale, cudaStream_t s, float *pd = nullptr,
                                        const float *img2 = nullptr, bool shared = false,
-                                       BpSplit split = {1, nullptr})
+                                       BpSplit split = BpSplit())
 {
     if (n <= 0) return cudaSuccess;
     // A GPU shared with concurrent launches (the serving lanes): one group
@@ -1234,7 +1248,7 @@ static cudaError_t launch_bp_compact_t(float *vol, const TI *img, const float *k
     if constexpr (std::is_same<TI, float>::value && !ONES && !DENS && !DW) {
         if (shared)
             return launch_bp_compact_g<TI, ONES, DENS, DW, DEEP, 1>(vol, img, ker, axes, n, g, scale, s, pd,
-                                                                         img2, 1, BpSplit{1, nullptr});
+                                                                         img2, 1, BpSplit());
     }
     return launch_bp_compact_g<TI, ONES, DENS, DW, DEEP, kGroupsOf<DW, DEEP>>(vol, img, ker, axes, n, g, scale, s, pd,
                                                                          img2, 32, split);
@@ -1290,29 +1304,28 @@ cudaError_t launch_back_project_ref_pair(float *d_vol, float *d_pd, const float 
                                                            false, split);
 }
 
-// How many segments.  Every direction reaches the bricks at the centre, so the
-// centre's CTA is a serial chain over all n of them (4.6 ms for 1,000) while
-// the others' work falls as 1 / radius; where the launch has few brick runs
-// (245 at M = 128) that chain is the launch's time.  Segments cut it, but each
-// pays a CTA's start (table, sums, about 10 us) and fills rounds less well, so
-// the fewer the directions, the fewer runs it takes before they cost more than
-// they give.  Measured, reconstructVol, 1 / best / next segment count in us:
-// M = 64, n = 1000: 3939 / 908 (6) / 1095 (4); M = 128, n = 1000: 4579 /
-// 2203 (3) / 2256 (4), n = 256: 1242 / 731 (2) / 781 (3), n = 16: 158 (1) /
-// 178 (2); M = 160, n = 256: 1269 / 1106 (2), n = 64: 436 (1) / 478 (2);
-// M = 200, n = 1000: 4985 / 4752 (2), n = 512: 2632 (1) / 2770 (2);
-// M = 256, n = 1000: 6657 (1) / 7055 (2).
+// How many segments.  Every direction reaches the bricks at the centre, so a
+// centre brick is a serial chain over all n of them while the others' work
+// falls as 1 / radius; where a launch has few bricks (750 at M = 128 for 456
+// groups) that chain is the launch's time.  Segments cut it, but each pays a
+// brick's start and merge and fills rounds less well, so `want` items suffice,
+// the fewer the fewer the directions.  Measured, reconstructVol in us by
+// segment count: M = 64, n = 1000: 3783 (1), 682 (8), 627 (12); M = 128,
+// n = 1000: 4311 (1), 1789 (4), 1736 (6), 1762 (8), n = 256: 1195 (1), 564
+// (4), 594 (6), n = 64: 351 (1), 243 (3), 255 (4), n = 16: 142 (1), 151 (2);
+// M = 160, n = 1000: 4554 (1), 2694 (3), 2768 (6); M = 200, n = 1000: 5258
+// (1), 4112 (2), 4195 (4), n = 256: 1498 (1), 1314 (2), 1420 (4); M = 256,
+// n = 1000: 6093 (1), 6088 (2), 6201 (3).
 // The rule looks at n and the geometry only, so the plain, density and
 // two-stack forms of one call add the same partial sums.
 int bp_segments(int n, const Geom &g)
 {
     if (g.ker_size > 513) return 1; // no room for the 32 table copies of the split form
     const double r = g.mask_radius + 2.0;
-    const int runs = (int)(4.19 * r * r * r / (3 * kCBX * kCBY * 12)) + 1; // of three bricks in the mask's sphere
-    const int want = n < 32 ? 200 : n < 192 ? 300 : n < 512 ? 450 : 700;
-    int s = 1 + want / runs;
-    if ((n >= 128 && runs < 610) || (n >= 768 && runs < 1100)) s = std::max(s, 2);
-    return std::max(1, std::min({s, 6, n / 3}));
+    const int bricks = (int)(4.19 * r * r * r / (kCBX * kCBY * 12)) + 1; // in the mask's sphere
+    const int want = n < 32 ? 500 : n < 192 ? 2000 : n < 512 ? 3000 : 4500;
+    const int most = n < 32 ? n / 4 : std::min(n / 16, 12);
+    return std::max(1, std::min((want + bricks - 1) / bricks, most));
 }
 
 } // namespace gg
