@@ -68,8 +68,8 @@ cudaError_t launch_pitch_volume(const float *d_cas, int V, int P, void *d_out, i
 // does, the others write their sums to `part` ((nseg - 1) * V^3 floats, twice
 // that with a density), and a merge adds them in order.  nseg = 1: unsplit.
 // next (optional): a device counter, zero between launches and used by one
-// launch at a time, from which the brick groups of a launch that owns the GPU
-// take their work.
+// launch at a time, from which the warps of a launch that owns the GPU take
+// their work.
 struct BpSplit {
     int nseg = 1;
     float *part = nullptr;

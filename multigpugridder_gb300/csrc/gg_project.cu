@@ -220,9 +220,9 @@ cudaError_t launch_forward_project(const void *d_vol, int vprec, int pitch, floa
 // ---------------------------------------------------------------------------
 // Back projection: the reference window and shared constants
 // ---------------------------------------------------------------------------
-// Directions are staged through shared memory in chunks of kBpChunk, two per
-// thread of a brick group for the cull.
-constexpr int kBpChunk = 512;
+// Each warp takes the directions in batches of kBpBatch, one per lane for the
+// cull.
+constexpr int kBpBatch = 32;
 
 // Conservative reach of the slab test: fp32 rounding of f_imgk is far below this.
 constexpr float kCullEps = 1e-2f;
@@ -286,23 +286,23 @@ __device__ __forceinline__ void ref_window(const RefWindow &q, const float *sker
 // Back projection, reference window rule
 // ---------------------------------------------------------------------------
 // Only the voxels inside a direction's slab (|f_imgk| <= 2, a few percent of
-// the volume) run the 25-pixel window.  A group of 256 threads (8 warps) owns
-// a 16x8x(2 BD) brick and each warp an 8x4xBD block of it, BD voxels per lane:
-// block voxel l = lane + 32 s (x = l & 7, y = (l >> 3) & 3, z = l >> 5).  Per
-// direction a warp tests its 32 BD voxels against the slab, lists the active
-// ones in shared memory and runs them 32 at a time, one per lane.  Every voxel
-// still receives its directions one by one in order and its window in the
-// reference's order, so the per-voxel sums are those of the reference
-// kernel's loops, bit for bit.  A CTA holds kBpGroups groups on neighbouring
-// bricks, which share one copy of the KB table (below); each group
-// synchronises on its own named barrier.
+// the volume) run the 25-pixel window.  A warp owns an 8x4xBD block of the
+// volume, BD voxels per lane: block voxel l = lane + 32 s (x = l & 7, y =
+// (l >> 3) & 3, z = l >> 5); eight blocks make a 16x8x(2 BD) brick, the unit in
+// which the volume is numbered.  The warp culls the directions 32 at a time,
+// one per lane, and for each that reaches its block tests its 32 BD voxels
+// against the slab, lists the active ones in shared memory and runs them 32 at
+// a time, one per lane.  Every voxel still receives its directions one by one
+// in order and its window in the reference's order, so the per-voxel sums are
+// those of the reference kernel's loops, bit for bit.  A CTA holds the warps of
+// kBpGroups bricks, which share one copy of the KB table (below) and run
+// independently.
 constexpr int kCBX = 16, kCBY = 8; // brick: 2x2x2 warp blocks of 8x4xBD (BD = 6, or 8 on large images)
-constexpr int kCThreads = 256;  // threads of a group
-constexpr int kBpGroups = 3;    // groups (bricks) per CTA, one CTA per SM
-// The two-stack form's 6-deep kernel runs two groups per CTA: with the second
-// stack's footprints, the voxel queue's two buffers fit only beside two groups.
+constexpr int kCThreads = 256;  // threads of a brick's eight warps
+constexpr int kBpGroups = 3;    // bricks' worth of warps per CTA, one CTA per SM
+// The two-stack form's 6-deep kernel runs 16 warps per CTA: with the second
+// stack's footprints, 24 warps' two buffers do not fit.
 template <bool DW, bool DEEP> constexpr int kGroupsOf = (DW && !DEEP) ? 2 : kBpGroups;
-static_assert(kBpChunk % kCThreads == 0, "the cull gives each thread kBpChunk / kCThreads directions");
 // Depth of a warp block: 6 voxels, or 8 (DEEP, reference rule) on CAS images
 // of 512^2 and more.  Deeper blocks have more active voxels per direction
 // (fewer idle lanes in the last round of 32) and stage a footprint for more
@@ -560,32 +560,27 @@ struct BpQueue {
     static constexpr int CAP = NEED <= 128 ? 128 : (NEED <= 256 ? 256 : 512);
 };
 
-// One group's working set in shared memory (after the table).  LEAN (the
+// One warp's working set in shared memory (after the table).  LEAN (the
 // launches that own the GPU): 8-bit queue entries with the footprint buffer
-// tracked per warp, 16-bit direction-list entries, and in the two-buffer form
-// footprint rows of FW + 4 pixels from fi0 & ~3 (16-byte aligned, written by
-// vector stores).  Otherwise (the serving lanes' one-group CTAs): 16-bit
-// entries carrying the buffer bit, rows of FW + 1 pixels from fi0.
+// tracked per warp, and in the two-buffer form footprint rows of FW + 4 pixels
+// from fi0 & ~3 (16-byte aligned, copied in 16-byte quads).  Otherwise (the
+// serving lanes' one-brick CTAs): 16-bit entries carrying the buffer bit, rows
+// of FW + 1 pixels from fi0.
 template <bool DENS, bool DW, bool DEEP, bool LEAN = true>
-struct BpGroupMem {
+struct alignas(16) BpWarpMem {
     using Shape = BpShape<DW, DEEP>;
     using Q = BpQueue<DW, DEEP>;
     using QEnt = typename std::conditional<LEAN, unsigned char, unsigned short>::type;
-    using LEnt = typename std::conditional<LEAN, unsigned short, int>::type;
-    static constexpr int NW = kCThreads / 32, WV = Shape::WV,
-                         FP = Shape::FW * (Shape::FW + (LEAN && Q::NB == 2 ? 4 : 1));
-    BpDirMeta smeta[NW * Q::NB];
-    float sax[kBpChunk * 9];
-    LEnt slist[kBpChunk];
-    int swarp[kBpChunk / 32]; // kept directions per (pass, warp)
-    int scount;
-    // per-voxel sums [warp][block voxel]; a voxel is updated by at most one
-    // lane per direction, directions in order, so no atomics are needed
-    float sacc[NW * WV];
-    float saccw[DENS || DW ? NW * WV : 1];
-    alignas(16) float sfoot[NW * Q::NB * FP];
-    float sfoot2[DW ? NW * Q::NB * FP : 1];
-    QEnt squeue[NW * Q::CAP];
+    static constexpr int WV = Shape::WV, FP = Shape::FW * (Shape::FW + (LEAN && Q::NB == 2 ? 4 : 1));
+    float sfoot[Q::NB * FP];
+    float sfoot2[DW ? Q::NB * FP : 4];
+    BpDirMeta smeta[Q::NB];
+    float sdir[2][kBpBatch * 9]; // two batches of directions
+    // per-voxel sums; a voxel is updated by at most one lane per direction,
+    // directions in order, so no atomics are needed
+    float sacc[WV];
+    float saccw[DENS || DW ? WV : 4];
+    QEnt squeue[Q::CAP];
 };
 
 // Bricks of x-width kCBX in row (y brick j, z brick k) that meet the sphere of
@@ -680,9 +675,14 @@ __device__ __noinline__ int3 brick_at(int brick, const BpLayers &lay, int bricks
     return at;
 }
 
-__device__ __forceinline__ void group_sync(int id)
+__device__ __forceinline__ void cp_async4(float *dst, const float *src)
 {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kCThreads) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait()
+{
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 template <typename TI, bool ONES, bool DENS, bool DW = false, bool DEEP = false, int G = kBpGroups,
@@ -701,12 +701,14 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
     // LEAN two-buffer form: footprint rows hold the pixels from fi0 & ~3 (16-byte aligned rows)
     constexpr bool QALIGN = LEAN && BpQueue<DW, DEEP>::NB == 2;
     constexpr int FW = Shape::FW, FH = FW, FS = FW + (QALIGN ? 4 : 1);
-    using Mem = BpGroupMem<DENS, DW, DEEP, LEAN>;
+    using Mem = BpWarpMem<DENS, DW, DEEP, LEAN>;
     using QEnt = typename Mem::QEnt;
-    // [table: tb.entries x tb.copies][G x Mem]
+    constexpr int NW = kCThreads / 32 * G; // warps of the CTA
+    // [table: tb.entries x tb.copies][NW x Mem]
     extern __shared__ __align__(16) float bp_smem[];
     const int cp = tb.copies, tabWords = tb.entries * cp;
-    Mem *gmem = reinterpret_cast<Mem *>(bp_smem + ((tabWords + 3) & ~3)); // 16-byte aligned
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    Mem &sm = reinterpret_cast<Mem *>(bp_smem + ((tabWords + 3) & ~3))[warp]; // 16-byte aligned
     const int volCenter = (int)((float)V) / 2;
     const int imgCenter = (int)((float)M) / 2;
 
@@ -720,41 +722,36 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
     }
     __syncthreads();
 
-    // Items: the bricks that meet the mask sphere (SPLIT: times the segments of
-    // the directions, a brick's side by side), heaviest layers first.  With a
-    // counter (split.next) each group takes the next item on its own: no group
-    // waits for the others' bricks (15% of the warps' time when a CTA ended with
-    // its slowest brick) and the KB table is staged once an SM.  reconstructVol
-    // of 1,000 images at M = 256 6.39 -> 6.09 ms, of 512 at M = 512 15.24 ->
-    // 14.56 ms, of 16 at M = 256 530 -> 468 us; CTF-corrected 6.96 -> 6.55 ms.
-    const int grp = threadIdx.x / kCThreads;
-    const int ns = SPLIT ? split.nseg : 1, items = lay.pre[lay.layers] * ns;
-    // SPLIT, or few items: apart, so that an SM's groups share out the heavy
-    // ones (reconstructVol of 16 images at M = 128: 142 against 149 us); many:
-    // neighbours, which share footprints in L1 (1,000 at M = 256: 6.09 against
-    // 6.33 ms)
-    const bool apart = split.next && (SPLIT || items < 4 * (int)gridDim.x * G);
-    for (int item = apart ? grp * gridDim.x + blockIdx.x : blockIdx.x * G + grp; item < items;) {
-        const int3 at = brick_at(SPLIT ? item / ns : item, lay, bricksX, bricksY, volCenter, kCBZ, maskR);
+    // Items: the warp blocks of the bricks that meet the mask sphere (SPLIT:
+    // times the segments of the directions, a block's side by side), heaviest
+    // layers first.  With a counter (split.next) each warp takes the next item
+    // on its own: the warps share the table and nothing else.  Barriers between
+    // the eight warps of a brick (for each 512 staged directions) held them 23%
+    // of their time, and a CTA that ended with the slowest of three bricks idled
+    // 15% of its warps.  reconstructVol, before the counter / with a counter per
+    // brick group / per warp: 700 images (FP16) at M = 384 11.93 / 11.22 / 10.19
+    // ms; CTF-corrected 1,000 at M = 256 6.96 / 6.55 / 5.89 ms; 512 at M = 512
+    // 15.24 / 14.56 / 13.86 ms; 16 at M = 256 530 / 477 / 409 us.
+    const int ns = SPLIT ? split.nseg : 1, items = lay.pre[lay.layers] * 8 * ns;
+    // With a counter the first items are dealt out across the SMs, so that an
+    // SM's warps share the heavy ones with others (reconstructVol of 16 images
+    // at M = 128: 131 us against 142 for neighbouring items; no difference for
+    // large launches); without one, a CTA's warps take neighbouring items.
+    for (int item = split.next ? warp * gridDim.x + blockIdx.x : blockIdx.x * NW + warp; item < items;) {
+        const int block = SPLIT ? item / ns : item;
+        const int3 at = brick_at(block >> 3, lay, bricksX, bricksY, volCenter, kCBZ, maskR);
         const int d0 = SPLIT ? (int)((long long)n * (item % ns) / ns) : 0;
         const int d1 = SPLIT ? (int)((long long)n * (item % ns + 1) / ns) : n;
-        Mem &sm = gmem[grp];
-        float *sax = sm.sax;
-        typename Mem::LEnt *slist = sm.slist;
-        int *swarp = sm.swarp;
-        const int tid = threadIdx.x - grp * kCThreads, warp = tid >> 5, lane = tid & 31;
-        const int x0 = at.x * kCBX, y0 = at.y * kCBY, z0 = at.z * kCBZ;
-        const int bx = x0 + (warp & 1) * 8, by = y0 + ((warp >> 1) & 1) * 4, bz = z0 + (warp >> 2) * BD;
+        const int bx = at.x * kCBX + (block & 1) * 8, by = at.y * kCBY + ((block >> 1) & 1) * 4,
+                  bz = at.z * kCBZ + ((block >> 2) & 1) * BD;
         const float *sker = bp_smem + lane % cp; // entry k at sker[k * cp]
         const unsigned stride = 4u * (unsigned)cp;
         const unsigned tab = (unsigned)__cvta_generic_to_shared(bp_smem) + 4u * (unsigned)(lane % cp) - tb.magic_bits * stride;
         constexpr int NB = BpQueue<DW, DEEP>::NB, QM = BpQueue<DW, DEEP>::CAP - 1;
-        float *const wfoot0 = sm.sfoot + warp * (NB * FH * FS);
-        float *const wfoot20 = sm.sfoot2 + (DW ? warp * (NB * FH * FS) : 0);
-        BpDirMeta *const wmeta = sm.smeta + warp * NB;
-        QEnt *const wq = sm.squeue + warp * (QM + 1);
-        float *const wacc = sm.sacc + warp * kWarpVox;
-        float *const waccw = sm.saccw + (DENS || DW ? warp * kWarpVox : 0);
+        float *const wfoot0 = sm.sfoot, *const wfoot20 = sm.sfoot2;
+        BpDirMeta *const wmeta = sm.smeta;
+        QEnt *const wq = sm.squeue;
+        float *const wacc = sm.sacc, *const waccw = sm.saccw;
 
         // this lane's voxels: x = lx, y = ly, z = bz + s
         const int lx = bx + (lane & 7), ly = by + (lane >> 3);
@@ -776,10 +773,6 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
         const float wcx = bx + 3.5f - volCenter, wcy = by + 1.5f - volCenter, wcz = bz + 0.5f * (BD - 1) - volCenter;
         const float slab = kerHW + kCullEps; // half-thickness
         const int MM = M * M;
-        // Directions are staged through shared memory in chunks, culled against
-        // the brick (compacted in order), then against each warp's 8x4xBD block.
-        const float bcx = x0 + 0.5f * (kCBX - 1) - volCenter, bcy = y0 + 0.5f * (kCBY - 1) - volCenter,
-                    bcz = z0 + 0.5f * (kCBZ - 1) - volCenter;
         const unsigned lt_mask = (1u << lane) - 1u;
         // the warp's queue (uniform): qsize entries from qhead.  LEAN: the first
         // nfront belong to footprint buffer bfront, the rest to the other
@@ -861,90 +854,56 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
             }
         };
 
-        for (int c0 = d0; c0 < d1; c0 += kBpChunk) {
-            const int cn = min(kBpChunk, d1 - c0);
-            group_sync(grp + 1);
-            if (cn == kBpChunk) {
-                // a whole chunk: all of a thread's loads in flight before its stores
-                constexpr int KA = kBpChunk * 9 / kCThreads;
-                float a[KA];
+        // a batch of directions, a lane's nine floats each, copied a batch ahead
+        auto fetch = [&](const int c) {
+            if (c + lane < d1) {
 #pragma unroll
-                for (int u = 0; u < KA; u++) a[u] = __ldg(axes + (size_t)c0 * 9 + tid + u * kCThreads);
-#pragma unroll
-                for (int u = 0; u < KA; u++) sax[tid + u * kCThreads] = a[u];
-            } else {
-                for (int t = tid; t < cn * 9; t += kCThreads) sax[t] = __ldg(axes + (size_t)c0 * 9 + t);
+                for (int u = 0; u < 9; u++)
+                    cp_async4(sm.sdir[(c - d0) / kBpBatch & 1] + lane * 9 + u, axes + (size_t)(c + lane) * 9 + u);
             }
-            group_sync(grp + 1);
-            // cull: thread tid takes directions tid + p * kCThreads; the kept
-            // ones are listed in direction order (pass by pass, warp by warp).
-            constexpr int kPasses = kBpChunk / kCThreads;
-            unsigned ballots[kPasses];
-            bool keeps[kPasses];
-            int orthos[kPasses];
-#pragma unroll
-            for (int pss = 0; pss < kPasses; pss++) {
-                const int d = tid + pss * kCThreads;
-                bool keep = false;
-                int ortho = 0;
-                if (d < cn) {
-                    const float *ax = sax + d * 9;
-                    const float zx = ax[6], zy = ax[7], zz = ax[8];
-                    const float dd = bcx * zx + bcy * zy + bcz * zz;
-                    const float ext = 0.5f * ((kCBX - 1) * fabsf(zx) + (kCBY - 1) * fabsf(zy) + (kCBZ - 1) * fabsf(zz));
-                    keep = fabsf(dd) <= slab + ext;
-                    // the fast window needs orthonormal axes (they bound |Q - v|);
-                    // NaN or infinite entries fail these tests
-                    const float xx = ax[0] * ax[0] + ax[1] * ax[1] + ax[2] * ax[2];
-                    const float yy = ax[3] * ax[3] + ax[4] * ax[4] + ax[5] * ax[5];
-                    const float zz2 = zx * zx + zy * zy + zz * zz;
-                    const float xy = ax[0] * ax[3] + ax[1] * ax[4] + ax[2] * ax[5];
-                    const float xz = ax[0] * zx + ax[1] * zy + ax[2] * zz;
-                    const float yz = ax[3] * zx + ax[4] * zy + ax[5] * zz;
-                    ortho = (fabsf(xx - 1.0f) <= 1e-3f && fabsf(yy - 1.0f) <= 1e-3f && fabsf(zz2 - 1.0f) <= 1e-3f &&
-                             fabsf(xy) <= 1e-3f && fabsf(xz) <= 1e-3f && fabsf(yz) <= 1e-3f) ? kBpChunk : 0;
-                }
-                keeps[pss] = keep;
-                orthos[pss] = ortho;
-                ballots[pss] = __ballot_sync(0xffffffffu, keep);
-                if (lane == 0) swarp[pss * (kCThreads / 32) + warp] = __popc(ballots[pss]);
+        };
+        fetch(d0);
+        for (int c0 = d0; c0 < d1; c0 += kBpBatch) {
+            const float *const sdir = sm.sdir[(c0 - d0) / kBpBatch & 1];
+            cp_async_wait();
+            __syncwarp(); // the batch is here, for every lane; the other buffer is free
+            fetch(c0 + kBpBatch);
+            // cull: lane l tests direction c0 + l against the warp's 8x4xBD block
+            bool keep = false, ortho = false;
+            if (c0 + lane < d1) {
+                const float *ax = sdir + lane * 9;
+                const float zx = ax[6], zy = ax[7], zz = ax[8];
+                const float dd = wcx * zx + wcy * zy + wcz * zz;
+                const float ext = 0.5f * (7.0f * fabsf(zx) + 3.0f * fabsf(zy) + (float)(BD - 1) * fabsf(zz));
+                keep = fabsf(dd) <= slab + ext;
+                // the fast window needs orthonormal axes (they bound |Q - v|);
+                // NaN or infinite entries fail these tests
+                const float xx = ax[0] * ax[0] + ax[1] * ax[1] + ax[2] * ax[2];
+                const float yy = ax[3] * ax[3] + ax[4] * ax[4] + ax[5] * ax[5];
+                const float zz2 = zx * zx + zy * zy + zz * zz;
+                const float xy = ax[0] * ax[3] + ax[1] * ax[4] + ax[2] * ax[5];
+                const float xz = ax[0] * zx + ax[1] * zy + ax[2] * zz;
+                const float yz = ax[3] * zx + ax[4] * zy + ax[5] * zz;
+                ortho = fabsf(xx - 1.0f) <= 1e-3f && fabsf(yy - 1.0f) <= 1e-3f && fabsf(zz2 - 1.0f) <= 1e-3f &&
+                        fabsf(xy) <= 1e-3f && fabsf(xz) <= 1e-3f && fabsf(yz) <= 1e-3f;
             }
-            group_sync(grp + 1);
-            {
-                int off = 0;
-#pragma unroll
-                for (int pss = 0; pss < kPasses; pss++) {
-                    int o = off;
-                    for (int w = 0; w < warp; w++) o += swarp[pss * (kCThreads / 32) + w];
-                    if (keeps[pss])
-                        slist[o + __popc(ballots[pss] & lt_mask)] = (typename Mem::LEnt)((tid + pss * kCThreads) | orthos[pss]);
-                    for (int w = 0; w < kCThreads / 32; w++) off += swarp[pss * (kCThreads / 32) + w];
-                }
-                if (tid == kCThreads - 1) sm.scount = off;
-            }
-            group_sync(grp + 1);
-            const int count = sm.scount;
-
-            // NB = 2: a pass beyond the last chunk's list runs what is left in
+            unsigned hits = __ballot_sync(0xffffffffu, keep);
+            const unsigned orthos = __ballot_sync(0xffffffffu, ortho);
+            // NB = 2: a pass beyond the last batch's hits runs what is left in
             // the queue, so that the window code is expanded once
-            const bool last = NB > 1 && c0 + kBpChunk >= d1;
-            for (int q = 0; q < count + (last ? 1 : 0); q++) {
-                const bool flush = NB > 1 && q == count;
-                const int e = flush ? 0 : slist[q];
-                const int al = e & (kBpChunk - 1);
-                const float *ax = sax + al * 9;
+            const bool last = NB > 1 && c0 + kBpBatch >= d1;
+            while (hits || last) {
+                const bool flush = NB > 1 && hits == 0;
+                const int al = flush ? 0 : __ffs(hits) - 1;
+                hits &= hits - 1;
+                const float *ax = sdir + al * 9;
                 const float nz0 = ax[6], nz1 = ax[7], nz2 = ax[8];
-                {   // the warp's 8x4xBD block against the slab (uniform)
-                    const float d = wcx * nz0 + wcy * nz1 + wcz * nz2;
-                    const float ext = 0.5f * (7.0f * fabsf(nz0) + 3.0f * fabsf(nz1) + (float)(BD - 1) * fabsf(nz2));
-                    if (!flush && fabsf(d) > slab + ext) continue;
-                }
                 // Whole rounds, and whatever buffer b's earlier direction still
                 // has in the queue (at its front), run before b is refilled.
                 const int b = NB > 1 ? nbuf : 0;
                 if (NB > 1) {
                     if (QALIGN && sizeof(TI) == 4 && !ONES) {
-                        asm volatile("cp.async.wait_all;" ::: "memory");
+                        cp_async_wait();
                         __syncwarp(); // the footprints' copies are complete, for every lane
                     }
                     while (qsize >= 32 || (qsize > 0 && (flush || (LEAN ? bfront : (int)(wq[qhead & QM] >> 8)) == b)))
@@ -976,7 +935,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                 // this warp's footprint (uniform across the warp)
                 int fi0 = 0, fj0 = 0, fh = 0;
                 bool foot = false;
-                if (e & kBpChunk) {
+                if ((orthos >> al) & 1u) {
                     const float ic = wcx * nx0 + wcy * nx1 + wcz * nx2 + (float)imgCenter;
                     const float jc = wcx * ny0 + wcy * ny1 + wcz * ny2 + (float)imgCenter;
                     const float hz = 0.5f * (float)(BD - 1);
@@ -1138,16 +1097,14 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
             }
         }
         if (!split.next) return;
-        if (tid == 0) {
-            // every item is fetched or started on once: the fetch that returns
-            // items - 1 is the last, and leaves the counter at 0 for the next launch
-            const unsigned f = atomicAdd(split.next, 1u);
+        // every item is fetched or started on once: the fetch that returns
+        // items - 1 is the last, and leaves the counter at 0 for the next launch
+        unsigned f = 0;
+        if (lane == 0) {
+            f = atomicAdd(split.next, 1u);
             if (f == (unsigned)items - 1) atomicExch(split.next, 0u);
-            sm.scount = (int)f;
         }
-        group_sync(grp + 1);
-        item = (int)gridDim.x * G + sm.scount;
-        group_sync(grp + 1); // read by all before the next item's culling writes it
+        item = (int)gridDim.x * NW + (int)__shfl_sync(0xffffffffu, f, 0);
     }
 }
 
@@ -1181,8 +1138,9 @@ static cudaError_t launch_bp_compact_g(float *vol, const TI *img, const float *k
     const int bx = (g.V + kCBX - 1) / kCBX, by = (g.V + kCBY - 1) / kCBY, bz = (g.V + kCBZ - 1) / kCBZ;
     // one group per CTA (the serving lanes): the non-LEAN layout
     constexpr bool LEAN = G > 1;
-    using Mem = BpGroupMem<DENS, DW, DEEP, LEAN>;
-    const size_t other = G * sizeof(Mem);
+    using Mem = BpWarpMem<DENS, DW, DEEP, LEAN>;
+    constexpr int NW = kCThreads / 32 * G;
+    const size_t other = NW * sizeof(Mem);
     // one group per CTA: three CTAs an SM (228 KB, 1 KB reserved per CTA)
     const size_t limit = G == 1 ? (size_t)(228 * 1024 / 3 - 1024) : 0;
     const BpTable tb = bp_table(g.ker_size, other, max_copies, limit);
@@ -1204,9 +1162,10 @@ static cudaError_t launch_bp_compact_g(float *vol, const TI *img, const float *k
         }
         lay.pre[r + 1] = lay.pre[r] + bricks;
     }
-    const long long items = (long long)lay.pre[bz] * split.nseg;
+    const long long items = (long long)lay.pre[bz] * 8 * split.nseg;
     if (items == 0) return cudaSuccess;
-    long long grid = (items + G - 1) / G;
+    if (items > 0x40000000LL) return cudaErrorInvalidValue;
+    long long grid = (items + NW - 1) / NW;
     if (split.next) grid = std::min<long long>(grid, num_sms()); // one CTA an SM
     // the table stride as a compile-time constant where the copy count gives one
     auto go = [&](auto kern) {
@@ -1304,27 +1263,29 @@ cudaError_t launch_back_project_ref_pair(float *d_vol, float *d_pd, const float 
                                                            false, split);
 }
 
-// How many segments.  Every direction reaches the bricks at the centre, so a
-// centre brick is a serial chain over all n of them while the others' work
-// falls as 1 / radius; where a launch has few bricks (750 at M = 128 for 456
-// groups) that chain is the launch's time.  Segments cut it, but each pays a
-// brick's start and merge and fills rounds less well, so `want` items suffice,
-// the fewer the fewer the directions.  Measured, reconstructVol in us by
-// segment count: M = 64, n = 1000: 3783 (1), 682 (8), 627 (12); M = 128,
-// n = 1000: 4311 (1), 1789 (4), 1736 (6), 1762 (8), n = 256: 1195 (1), 564
-// (4), 594 (6), n = 64: 351 (1), 243 (3), 255 (4), n = 16: 142 (1), 151 (2);
-// M = 160, n = 1000: 4554 (1), 2694 (3), 2768 (6); M = 200, n = 1000: 5258
-// (1), 4112 (2), 4195 (4), n = 256: 1498 (1), 1314 (2), 1420 (4); M = 256,
-// n = 1000: 6093 (1), 6088 (2), 6201 (3).
+// How many segments.  Every direction reaches the blocks at the centre, so a
+// centre block is a serial chain over all n of them while the others' work
+// falls as 1 / radius; where a launch has few blocks (6,000 at M = 128 for
+// 3,648 warps) that chain is the launch's time.  Segments cut it, but each pays
+// a block's start and merge and fills rounds less well, so `want` bricks times
+// segments suffice, the fewer the fewer the directions.  Measured,
+// reconstructVol in us by segment count: M = 64, n = 1000: 3137 (1), 648 (8),
+// 567 (12); M = 128, n = 1000: 3698 (1), 1669 (4), 1504 (6), 1539 (8), n = 256:
+// 1011 (1), 533 (4), 537 (6), n = 64: 306 (1), 229 (3), 231 (4), n = 16: 130
+// (1), 137 (2); M = 160, n = 1000: 4155 (1), 2386 (4), 2444 (6); M = 200,
+// n = 1000: 5116 (1), 3703 (3), 3742 (4), n = 256: 1433 (1), 1162 (2), 1208
+// (3); M = 256, n = 1000: 6164 (1), 5483 (2), 5541 (3), n = 256: 1734 (1), 1743
+// (2); M = 320, n = 1000: 9276 (1), 9466 (2).
 // The rule looks at n and the geometry only, so the plain, density and
-// two-stack forms of one call add the same partial sums.
+// two-stack forms of one call add the same partial sums (the two-stack form
+// alone would stay at 1 for M = 256: 5,885 against 6,056 us).
 int bp_segments(int n, const Geom &g)
 {
     if (g.ker_size > 513) return 1; // no room for the 32 table copies of the split form
     const double r = g.mask_radius + 2.0;
     const int bricks = (int)(4.19 * r * r * r / (kCBX * kCBY * 12)) + 1; // in the mask's sphere
-    const int want = n < 32 ? 500 : n < 192 ? 2000 : n < 512 ? 3000 : 4500;
-    const int most = n < 32 ? n / 4 : std::min(n / 16, 12);
+    const int want = n < 32 ? 500 : n < 192 ? 2000 : n < 512 ? 3000 : 6000;
+    const int most = n < 32 ? n / 4 : std::min(n / 10, 12);
     return std::max(1, std::min((want + bricks - 1) / bricks, most));
 }
 
