@@ -323,7 +323,7 @@ void update_fp(gg_gridder *h, cudaStream_t s)
     if (h->fp_maps_vol != h->cas_fp.p || h->fp_maps_prec != h->prec) {
         h->fp_maps.ensure(fp_tile_map_bytes(h->prec));
         h->fp_maps_prec = -1;
-        GG_CK(fp_tile_make_maps(h->cas_fp.p, h->V, (int)P, h->prec, h->fp_maps.p));
+        GG_CK(fp_tile_make_maps(h->cas_fp.p, h->V, (int)P, h->prec, h->fp_maps.p, s));
         h->fp_maps_vol = h->cas_fp.p;
         h->fp_maps_prec = h->prec;
     }
@@ -698,6 +698,9 @@ void init_handle(gg_gridder *h)
     GG_CK(cudaMemset(h->bp_next.p, 0, sizeof(unsigned)));
     h->work.ensure(1);
     GG_CK(cudaMemset(h->work.p, 0, sizeof(unsigned int)));
+    // the copies and memsets above ran on the default stream, which the streams
+    // of later calls need not wait for
+    GG_CK(cudaStreamSynchronize(cudaStreamLegacy));
     h->fused_fft = fft2_fused_ok(h->N, h->M);
 }
 
@@ -882,6 +885,7 @@ extern "C" int gg_set_kb_table(gg_gridder *h, const float *table, int n)
         h->ker.release();
         h->ker.ensure(n);
         GG_CK(cudaMemcpy(h->ker.p, table, (size_t)n * sizeof(float), cudaMemcpyHostToDevice));
+        GG_CK(cudaStreamSynchronize(cudaStreamLegacy));
         h->ker_size = n;
         h->five_taps = !(table[0] == 0.0f && table[n - 1] == 0.0f);
     });

@@ -453,14 +453,18 @@ static cudaError_t encode_maps(const void *d_vol, int V, int P, CUtensorMapDataT
     return cudaSuccess;
 }
 
-cudaError_t fp_tile_make_maps(const void *d_vol, int V, int P, int prec, void *d_maps)
+cudaError_t fp_tile_make_maps(const void *d_vol, int V, int P, int prec, void *d_maps, cudaStream_t s)
 {
     std::vector<CUtensorMap> m(fp_tile_map_bytes(prec) / sizeof(CUtensorMap));
     cudaError_t e = prec == kF32   ? encode_maps<float>(d_vol, V, P, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, m.data())
                     : prec == kF16 ? encode_maps<__half>(d_vol, V, P, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, m.data())
                                    : encode_maps<__nv_bfloat16>(d_vol, V, P, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, m.data());
     if (e != cudaSuccess) return e;
-    return cudaMemcpy(d_maps, m.data(), m.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice);
+    // on the stream and waited for: a copy from pageable memory may otherwise
+    // still be under way when it returns, and streams of other lanes do not
+    // wait for it
+    e = cudaMemcpyAsync(d_maps, m.data(), m.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, s);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(s);
 }
 
 template <typename TV>

@@ -52,7 +52,7 @@ struct FpTiles {
     int *fault;
 };
 size_t fp_tile_map_bytes(int prec);
-cudaError_t fp_tile_make_maps(const void *d_vol, int V, int pitch, int prec, void *d_maps);
+cudaError_t fp_tile_make_maps(const void *d_vol, int V, int pitch, int prec, void *d_maps, cudaStream_t s);
 // Scratch of one launch of n directions.
 size_t fp_plan_bytes(int n);
 // 4-tap forward projection (zero table edges); d_plans: fp_plan_bytes(n).

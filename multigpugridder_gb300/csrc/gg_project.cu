@@ -791,7 +791,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
             const float f_imgj = __fadd_rn(voxel_proj(a0, a1, a2, ny0, ny1, ny2), (float)imgCenter);
             const int imgi = (int)roundf(f_imgi);
             const int imgj = (int)roundf(f_imgj);
-            const bool inside = imgi >= 2 && imgj >= 2 && imgi + 2 < M && imgj + 2 < M;
+            const bool inside = imgi >= 2 && imgj >= 2 && imgi < M - 2 && imgj < M - 2; // no sum: axes may be anything
             const int ri = imgi - HALF - fi0, rj = imgj - HALF - fj0;
             if (foot && (unsigned)ri <= (unsigned)(FW - W) && (unsigned)rj <= (unsigned)(fh - W) && vi >= 4 &&
                 vj >= 4 && vk >= 4 && (inside || !DENS)) {
