@@ -16,8 +16,9 @@
  *               of the rotation, src/Matlab/utils/get_axes_from_n_rot.m:36-37
  *
  * Host-pointer calls copy through the library; pinned host memory
- * (cudaHostAlloc / cudaHostRegister) is transferred directly, pageable memory
- * is staged through an internal pinned buffer.  *_dev calls take device
+ * (cudaHostAlloc / cudaHostRegister) is transferred directly, and so is any
+ * memory where the GPU walks the host's page tables (Grace); elsewhere pageable
+ * memory is staged through an internal pinned buffer.  *_dev calls take device
  * pointers and a cudaStream_t (passed as void*, NULL = the legacy default
  * stream) and are asynchronous with respect to the host.
  *
