@@ -18,7 +18,8 @@
 // stores suffice; the additions to the volume are the only atomics, and the
 // order of a voxel's sum is that of their arrival.
 // Measured: gradient step of 512 images at 128^3, 10,195 -> 3,420 us with this
-// kernel in the gathering one's place (8,079 us of it).
+// kernel in the gathering one's place (8,079 -> 1,854 us of it); with each
+// lane's quads of the box placed once a tile and 13 warps for 12, 1,445 us.
 #include <algorithm>
 
 #include "gg_internal.h"
@@ -27,10 +28,10 @@
 namespace gg {
 
 constexpr int kAdjTile = 8;
-constexpr int kAdjWarps = 12;    // warps a CTA, one CTA an SM
-constexpr int kAdjBox = 3648;    // floats of a warp's box (99.9% of random tiles need less, none more than 4,100)
+constexpr int kAdjWarps = 13;    // warps a CTA, one CTA an SM
+constexpr int kAdjBox = 3600;    // floats of a warp's box (99.8% of random tiles need less, none more than 4,100)
 constexpr int kAdjStage = 32 * 21; // staged pixels: 16 xy products, 4 z weights, the window's place
-constexpr int kAdjRep = 4;       // interleaved table copies
+constexpr int kAdjRep = 4;       // interleaved table copies (1 where a long table leaves no room)
 
 __device__ __forceinline__ float box_ld(unsigned a)
 {
@@ -64,7 +65,7 @@ __device__ __forceinline__ void add_quad(float *p, float4 v, int left)
 // One pixel straight into the volume: windows that leave it (their taps inside
 // it), and tiles whose box does not fit (axes far from orthonormal).
 __device__ __noinline__ void pixel_to_global(float *__restrict__ vol, int V, int P, float fi, float fj, float fk, float y,
-                                             const float *sker, float kerScale, float kerCenterHalf, int kerSize)
+                                             const float *sker, int rep, float kerScale, float kerCenterHalf, int kerSize)
 {
     const float li = floorf(fi), lj = floorf(fj), lk = floorf(fk);
     // no window of a coordinate this far (or not finite) meets the volume
@@ -74,9 +75,9 @@ __device__ __noinline__ void pixel_to_global(float *__restrict__ vol, int V, int
     for (int u = 0; u < 64; u++) {
         const int x = b0 + (u & 3), yy = b1 + ((u >> 2) & 3), z = b2 + (u >> 4);
         if ((unsigned)x >= (unsigned)V || (unsigned)yy >= (unsigned)V || (unsigned)z >= (unsigned)V) continue;
-        const float w = kb_weight(sker, (float)x - fi, kerScale, kerCenterHalf, kerSize, kAdjRep) *
-                        kb_weight(sker, (float)yy - fj, kerScale, kerCenterHalf, kerSize, kAdjRep) *
-                        kb_weight(sker, (float)z - fk, kerScale, kerCenterHalf, kerSize, kAdjRep);
+        const float w = kb_weight(sker, (float)x - fi, kerScale, kerCenterHalf, kerSize, rep) *
+                        kb_weight(sker, (float)yy - fj, kerScale, kerCenterHalf, kerSize, rep) *
+                        kb_weight(sker, (float)z - fk, kerScale, kerCenterHalf, kerSize, rep);
         atomicAdd(vol + ((size_t)z * V + yy) * P + x, w * y);
     }
 }
@@ -85,23 +86,24 @@ template <typename TI, int VW>
 __global__ void __launch_bounds__(kAdjWarps * 32, 1)
 adjoint_tile_kernel(float *__restrict__ vol, int V, int P, const TI *__restrict__ img, int M,
                     const float *__restrict__ axes, int maskR, const float *__restrict__ ker, int kerSize, float kerHW,
-                    int tilesX, long long nItems, const float *__restrict__ d_scale)
+                    int tilesX, long long nItems, const float *__restrict__ d_scale, int rep)
 {
-    // [boxes][stages][table: kerSize entries x kAdjRep copies]
+    // [boxes][stages][table: kerSize entries x rep copies]
     extern __shared__ __align__(16) float adj_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float *const box = adj_smem + warp * kAdjBox;
     float *const stage = adj_smem + kAdjWarps * kAdjBox + warp * kAdjStage;
     float *const tab = adj_smem + kAdjWarps * (kAdjBox + kAdjStage);
-    for (int t = threadIdx.x; t < kerSize * kAdjRep; t += blockDim.x) tab[t] = __ldg(ker + t / kAdjRep);
+    for (int t = threadIdx.x; t < kerSize * rep; t += blockDim.x) tab[t] = __ldg(ker + t / rep);
     for (int t = lane; t < kAdjBox / 4; t += 32) reinterpret_cast<float4 *>(box)[t] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     __syncthreads();
-    const float *sker = tab + lane % kAdjRep;
+    const float *sker = tab + lane % rep;
+    const unsigned tab_step = 4u * (unsigned)rep; // bytes between entries
     const unsigned box_addr = (unsigned)__cvta_generic_to_shared(box);
     const float scale = d_scale ? *d_scale : 1.0f;
     const int ic = M / 2, vc = V / 2, R2 = maskR * maskR;
     const float kerCenter = ((float)kerSize - 1) / 2, kerScale = kerCenter / kerHW, kerCenterHalf = kerCenter + 0.5f;
-    const unsigned tab_base = (unsigned)__cvta_generic_to_shared(sker) - __float_as_uint(12582912.0f) * (4u * kAdjRep);
+    const unsigned tab_base = (unsigned)__cvta_generic_to_shared(sker) - __float_as_uint(12582912.0f) * tab_step;
     const int per = tilesX * tilesX;
     const bool items32 = nItems <= 0x7fffffffLL;
 
@@ -157,7 +159,7 @@ adjoint_tile_kernel(float *__restrict__ vol, int V, int P, const TI *__restrict_
             RP = ex <= 12 ? 12 : 20;
             SP = RP * ey;
             SP += (16 - SP) & 31; // 16 mod 32
-            boxed = ex <= 20 && ey <= 32 && nz <= 32 && SP * nz <= kAdjBox;
+            boxed = ex <= 20 && SP <= 384 && nz <= 32 && SP * nz <= kAdjBox; // 384: three quads a lane
         }
 
 #pragma unroll
@@ -165,7 +167,7 @@ adjoint_tile_kernel(float *__restrict__ vol, int V, int P, const TI *__restrict_
             // stage the half tile's pixels, those in the box first to last
             const bool use = boxed && in[h];
             if (on[h] && !use) {
-                pixel_to_global(vol, V, P, f[h][0], f[h][1], f[h][2], val[h], sker, kerScale, kerCenterHalf, kerSize);
+                pixel_to_global(vol, V, P, f[h][0], f[h][1], f[h][2], val[h], sker, rep, kerScale, kerCenterHalf, kerSize);
             }
             const unsigned who = __ballot_sync(0xffffffffu, use);
             __syncwarp(); // the previous half's staged pixels have been read
@@ -182,7 +184,7 @@ adjoint_tile_kernel(float *__restrict__ vol, int V, int P, const TI *__restrict_
                         // kb_weight of r in (-2, 2]: floor as the low bits of a sum rounded down
                         const float r = __fsub_rn(__fadd_rn(fl, (float)(u - 1)), f[h][d]);
                         const unsigned e = __float_as_uint(__fadd_rd(__fmaf_rn(r, kerScale, kerCenterHalf), 12582912.0f));
-                        asm("ld.shared.f32 %0, [%1];" : "=f"(w[d][u]) : "r"(tab_base + e * (4u * kAdjRep)));
+                        asm("ld.shared.f32 %0, [%1];" : "=f"(w[d][u]) : "r"(tab_base + e * tab_step));
                     }
                 }
 #pragma unroll
@@ -199,6 +201,7 @@ adjoint_tile_kernel(float *__restrict__ vol, int V, int P, const TI *__restrict_
             const float *const sxy = stage + (lane & 15), *const sz = stage + 16 + (lane >> 4);
             float xy = sxy[0], z0 = sz[0], z1 = sz[2];
             unsigned at = mine + __float_as_uint(stage[20]);
+#pragma unroll 2
             for (int p = 0; p < cnt; p++) {
                 // the next pixel's terms are read while this one's voxels are
                 const int nx = 21 * min(p + 1, 31);
@@ -214,17 +217,28 @@ adjoint_tile_kernel(float *__restrict__ vol, int V, int P, const TI *__restrict_
             }
         }
 
-        // The box's nonzero quads to the volume; the box is zero again.
+        // The box's nonzero quads to the volume; the box is zero again.  A lane
+        // takes the same (at most three) quads of every slice, so their places
+        // are worked out once.
         if (boxed) {
             const int rq = RP >> 2, sq = SP >> 2, ey = hi[1] + 4 - lo[1];
-            for (int z = 0; z < nz; z++) {
-                float *const slice = vol + ((size_t)(lo[2] + z) * V + lo[1]) * P + x0;
-                float4 *const bz = reinterpret_cast<float4 *>(box + z * SP);
-                for (int q = lane; q < sq; q += 32) {
-                    const int r = rq == 3 ? q / 3 : q / 5, c = 4 * (q - r * rq);
-                    const float4 v = bz[q];
-                    bz[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    if (r < ey) add_quad<VW>(slice + (size_t)r * P + c, v, (VW == 4 ? P : V) - (x0 + c));
+            float *slice = vol + ((size_t)lo[2] * V + lo[1]) * P + x0;
+            int off[3], left[3];
+#pragma unroll
+            for (int u = 0; u < 3; u++) {
+                const int q = lane + 32 * u, r = rq == 3 ? q / 3 : q / 5, c = 4 * (q - r * rq);
+                off[u] = r * P + c;
+                left[u] = r < ey ? (VW == 4 ? P : V) - (x0 + c) : 0;
+            }
+            float4 *bz = reinterpret_cast<float4 *>(box) + lane;
+            for (int z = 0; z < nz; z++, slice += (size_t)V * P, bz += sq) {
+#pragma unroll
+                for (int u = 0; u < 3; u++) {
+                    if (lane + 32 * u < sq) {
+                        const float4 v = bz[32 * u];
+                        bz[32 * u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        add_quad<VW>(slice + off[u], v, left[u]);
+                    }
                 }
             }
         }
@@ -239,10 +253,13 @@ static cudaError_t launch_adjoint_t(float *d_vol, int P, const TI *d_img, const 
     const int tilesX = (g.M + kAdjTile - 1) / kAdjTile;
     const long long nItems = (long long)n * tilesX * tilesX;
     if (nItems <= 0) return cudaSuccess;
-    const size_t smem = ((size_t)kAdjWarps * (kAdjBox + kAdjStage) + (size_t)g.ker_size * kAdjRep) * sizeof(float);
-    int dev = 0, sms = 0;
+    int dev = 0, sms = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    const size_t boxes = (size_t)kAdjWarps * (kAdjBox + kAdjStage) * sizeof(float);
+    const int rep = boxes + (size_t)g.ker_size * kAdjRep * sizeof(float) <= (size_t)optin ? kAdjRep : 1;
+    const size_t smem = boxes + (size_t)g.ker_size * rep * sizeof(float);
     const long long grid = std::min<long long>((nItems + kAdjWarps - 1) / kAdjWarps, std::max(sms, 1));
     // vector additions where every row of the volume starts aligned for them
     const size_t at = (size_t)d_vol;
@@ -250,7 +267,7 @@ static cudaError_t launch_adjoint_t(float *d_vol, int P, const TI *d_img, const 
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         kern<<<(unsigned)grid, kAdjWarps * 32, smem, s>>>(d_vol, g.V, P, d_img, g.M, d_axes, g.mask_radius, d_ker,
-                                                         g.ker_size, g.ker_hw, tilesX, nItems, scale);
+                                                         g.ker_size, g.ker_hw, tilesX, nItems, scale, rep);
         count_launches(1);
         return cudaGetLastError();
     };
