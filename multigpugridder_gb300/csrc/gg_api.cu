@@ -149,6 +149,7 @@ struct gg_gridder {
     int verbose = 0;
     int max_batch = 1024;
     bool fused_fft = false;     // fft2_fused_ok(N, M): the 2-D FFT stages run as one kernel each
+    bool fft_passes = false;    // else fftn_ok(N, M): as two; else through cuFFT
     int nstreams_fp = 2, nstreams_bp = 2;
     int prec = kF32;            // storage of the resident CAS volume the forward projection reads
     int img_prec_set = -1;      // storage of the CAS images the back projection reads; -1: as prec
@@ -169,6 +170,7 @@ struct gg_gridder {
     int *fault = nullptr;       // pinned: set by a kernel whose copies did not arrive
     DevBuf<float> pd;        // plane density V^3
     DevBuf<float> bp_part;   // sums of a split back projection's segments
+    DevBuf<float2> tw;       // fft_passes: e^(-2 pi i k / M)
     DevBuf<unsigned> bp_next; // its groups' work counter, 0 between launches
     DevBuf<float> adj;       // CAS-volume gradient, V^2 rows of fp_pitch(V, kF32) (forward-operator adjoint)
     DevBuf<float> axes;
@@ -392,6 +394,8 @@ void fp_batch(gg_gridder *h, const float *d_axes, int b, float *cas_out, float *
     ps.done();
     if (img_out && h->fused_fft) {
         GG_CK(launch_cas_to_images_fused(cas_out, h->M, h->N, b, img_out, s));
+    } else if (img_out && h->fft_passes) {
+        GG_CK(launch_cas_to_images_passes(cas_out, h->M, h->N, b, img_out, h->tw.p, (float2 *)S.spec.p, s));
     } else if (img_out) {
         GG_CK(launch_cas_images_to_spectrum(cas_out, h->M, b, S.spec.p, s));
         cufftHandle p = plan2d(h, CUFFT_C2R, b);
@@ -436,6 +440,19 @@ void bp_batch(gg_gridder *h, const float *d_axes, int b, const float *img, const
             void *dst = ip == kF32 ? (void *)S.casimg.p : (void *)S.casimg_lp.p;
             GG_CK(launch_images_to_cas_fused(img, h->N, h->M, b, dst, ip, false, s));
             src = dst;
+        } else if (h->fft_passes && ip != kF16) {
+            void *dst = ip == kF32 ? (void *)S.casimg.p : (void *)S.casimg_lp.p;
+            GG_CK(launch_images_to_cas_passes(img, h->N, h->M, b, dst, ip, false, h->tw.p, (float2 *)S.spec.p, nullptr, s));
+            src = dst;
+        } else if (h->fft_passes) {
+            // FP16: FP32 CAS images with their largest magnitude, then the
+            // storage scale and the conversion
+            GG_CK(launch_images_to_cas_passes(img, h->N, h->M, b, S.casimg.p, kF32, false, h->tw.p, (float2 *)S.spec.p,
+                                              h->work.p, s));
+            GG_CK(launch_scale_from_max(h->work.p, 8192.0f, h->scales.p + 1, s));
+            GG_CK(launch_convert(S.casimg.p, S.casimg_lp.p, ip, MM * b, h->img_scale(), s));
+            src = S.casimg_lp.p;
+            scale = h->img_scale();
         } else if (h->fused_fft) {
             // FP16: FP32 CAS images first, then the storage scale from their
             // largest magnitude and the conversion
@@ -491,6 +508,9 @@ void ctf_batch(gg_gridder *h, const float *d_axes, int b, const float *img, cons
     auto &S = h->slot[sl];
     if (h->fused_fft) {
         GG_CK(launch_images_to_cas_fused(img, h->N, h->M, b, S.casimg.p, kF32, false, s));
+    } else if (h->fft_passes) {
+        GG_CK(launch_images_to_cas_passes(img, h->N, h->M, b, S.casimg.p, kF32, false, h->tw.p, (float2 *)S.spec.p, nullptr,
+                                          s));
     } else {
         GG_CK(launch_images_to_fft_input(img, h->N, h->M, b, S.real.p, s));
         cufftHandle p = plan2d(h, CUFFT_R2C, b);
@@ -498,7 +518,7 @@ void ctf_batch(gg_gridder *h, const float *d_axes, int b, const float *img, cons
         GG_CKF(cufftExecR2C(p, S.real.p, S.spec.p));
         GG_CK(launch_spectrum_to_cas_images(S.spec.p, h->M, b, S.casimg.p, kF32, nullptr, s));
     }
-    // CAS images *= CTF, and CTF^2 into S.real (free after the R2C), in one pass
+    // CAS images *= CTF, and CTF^2 into S.real (free by now), in one pass
     GG_CK(launch_ctf(S.casimg.p, 1, S.real.p, 2, h->M, b, d_defocus, d_defocus_v, d_astig, c, s));
     if (h->img_prec() == kF32 && h->bp_mode != GG_BP_ADJOINT) {
         // both stacks in one back-projection pass
@@ -535,6 +555,9 @@ void forward_adjoint(gg_gridder *h, const float *d_axes, int n, const float *d_i
         auto &S = h->slot[0];
         if (h->fused_fft) {
             GG_CK(launch_images_to_cas_fused(d_img_grad + (size_t)a0 * NN, h->N, h->M, b, S.casimg.p, kF32, true, s));
+        } else if (h->fft_passes) {
+            GG_CK(launch_images_to_cas_passes(d_img_grad + (size_t)a0 * NN, h->N, h->M, b, S.casimg.p, kF32, true, h->tw.p,
+                                              (float2 *)S.spec.p, nullptr, s));
         } else {
             GG_CK(launch_images_to_fft_input(d_img_grad + (size_t)a0 * NN, h->N, h->M, b, S.real.p, s));
             cufftHandle p = plan2d(h, CUFFT_R2C, b);
@@ -717,10 +740,17 @@ void init_handle(gg_gridder *h)
     GG_CK(cudaMemset(h->bp_next.p, 0, sizeof(unsigned)));
     h->work.ensure(1);
     GG_CK(cudaMemset(h->work.p, 0, sizeof(unsigned int)));
+    if (fftn_ok(h->N, h->M)) {
+        std::vector<float2> tw(h->M);
+        fftn_twiddles(h->M, tw.data());
+        h->tw.ensure(h->M);
+        GG_CK(cudaMemcpy(h->tw.p, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    }
     // the copies and memsets above ran on the default stream, which the streams
     // of later calls need not wait for
     GG_CK(cudaStreamSynchronize(cudaStreamLegacy));
     h->fused_fft = fft2_fused_ok(h->N, h->M);
+    h->fft_passes = !h->fused_fft && fftn_ok(h->N, h->M);
 }
 
 void destroy_handle(gg_gridder *h)
@@ -750,6 +780,7 @@ void destroy_handle(gg_gridder *h)
     h->pd.release();
     h->bp_part.release();
     h->bp_next.release();
+    h->tw.release();
     h->adj.release();
     h->axes.release();
     h->vol_io.release();

@@ -816,8 +816,14 @@ cudaError_t launch_storage_scale(const float *d_x, size_t count, float target, u
     unsigned g = grid_for(count, kT);
     if (g > 4096) g = 4096;
     max_abs_kernel<<<g, kT, 0, s>>>(d_x, count, d_work);
+    count_launches(1);
+    return launch_scale_from_max(d_work, target, d_scale, s);
+}
+
+cudaError_t launch_scale_from_max(unsigned int *d_work, float target, float *d_scale, cudaStream_t s)
+{
     scale_from_max_kernel<<<1, 1, 0, s>>>(d_work, target, d_scale);
-    count_launches(2);
+    count_launches(1);
     return cudaGetLastError();
 }
 

@@ -160,6 +160,8 @@ cudaError_t launch_convert(const float *d_in, void *d_out, int prec, size_t coun
 // `count` floats; d_work is one scratch unsigned int.
 cudaError_t launch_storage_scale(const float *d_x, size_t count, float target, unsigned int *d_work,
                                  float *d_scale, cudaStream_t s);
+// The same from the bits of max|x| already in *d_work (left zero again).
+cudaError_t launch_scale_from_max(unsigned int *d_work, float target, float *d_scale, cudaStream_t s);
 
 // Weak-phase CTF parameters (defocus per image, underfocus positive, Å).
 struct CtfParams {
@@ -191,6 +193,19 @@ cudaError_t launch_images_to_cas_fused(const float *d_img, int N, int M, int n, 
 // CAS images n*M*M (FP32) -> images n*N*N in one launch: FromCAS, shifts,
 // inverse 2-D FFT, crop and 1/M^2.
 cudaError_t launch_cas_to_images_fused(const float *d_cas, int M, int N, int n, float *d_img, cudaStream_t s);
+
+// ---- FFT passes for the other sizes (gg_fftn.cu) ------------------------------
+// True for N <= M <= 400, M = 2^a 3^b 5^c 7^d.
+bool fftn_ok(int N, int M);
+// e^(-2 pi i k / M), k < M, for the passes' d_tw.
+void fftn_twiddles(int M, float2 *out);
+// The two directions of the fused stages above, in two launches each through
+// d_half (n * N * (M/2 + 1) values).  top (optional, images -> CAS images): the
+// bits of the largest magnitude, added by atomicMax to a zeroed word.
+cudaError_t launch_images_to_cas_passes(const float *d_img, int N, int M, int n, void *d_cas, int prec, bool adjoint,
+                                        const float2 *d_tw, float2 *d_half, unsigned *top, cudaStream_t s);
+cudaError_t launch_cas_to_images_passes(const float *d_cas, int M, int N, int n, float *d_img, const float2 *d_tw,
+                                        float2 *d_half, cudaStream_t s);
 
 // Adds to the process-wide count of kernels launched by this library.
 void count_launches(long long n);
