@@ -1,0 +1,164 @@
+"""The size and type ranges at which the kernels change their method, against
+the oracle: FFT passes, projection tiles, segments of a back projection, the
+adjoint's boxes and the CTF's row blocks.
+
+Tolerances: relative L2 1e-5 against the oracle's FP32 restatement or its FP64
+FFT of the same CAS images (FP32 rounding of sums and transforms is about
+1e-7 times a few), 1e-3 where the oracle is FP64 (rounding can move a
+nearest-index table lookup) or the storage is reduced, 1e-6 absolute for the
+CTF (the bounds of the other parity tests).
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5
+
+
+def dptr(t):
+    return ctypes.c_void_p(t.data_ptr())
+
+
+def to_dev(a, dev):
+    import torch
+
+    return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).to(dev)
+
+
+# M = 36 (radices 3, 3, 4), 100, 140 and 196 (5 and 7; M no multiple of a
+# 16-column tile's rows), 200 through interpolation 2 and 2.5, 400 (the last)
+@pytest.mark.parametrize("N,interp", [(18, 2.0), (50, 2.0), (70, 2.0), (98, 2.0), (80, 2.5), (200, 2.0)])
+def test_fft_passes(cuda, N, interp):
+    import multigpugridder_gb300 as gg
+
+    p = O.Params(N, interp)
+    n = 5
+    rng = np.random.default_rng(N)
+    axes = O.quaternion_axes(n, seed=N).astype(np.float32)
+    imgs = rng.standard_normal((n, N, N)).astype(np.float32)
+    with gg.MultiGPUGridder(N, n, interpFactor=interp, adjustInterpFactor=False) as g:
+        g.setCASVolume(rng.standard_normal((p.V,) * 3).astype(np.float32))
+        cas = g.forwardProjectCAS(axes)
+        assert cas.shape == (n, p.M, p.M)
+        out = np.empty((n, N, N), dtype=np.float32)  # forwardProject would set the volume again
+        g._call("gg_forward_project", axes.ctypes.data, n, out.ctypes.data, None)
+        assert O.rel_l2(out, O.imgs_from_cas_imgs(cas, N)) < TOL
+        g.backProject(imgs, axes)
+        got = g.getCASVolume()
+        g.backProjectCAS(O.cas_imgs_from_imgs(imgs, p.M).astype(np.float32), axes)
+        ref = g.getCASVolume()
+    assert np.linalg.norm(ref) > 0
+    assert O.rel_l2(got, ref) < TOL
+
+
+@pytest.mark.parametrize("prec", ["bf16", "f16"])
+def test_fft_passes_reduced_storage(cuda, prec):
+    import multigpugridder_gb300 as gg
+
+    N = 50
+    p = O.Params(N)
+    axes = O.quaternion_axes(6, seed=3).astype(np.float32)
+    # beyond FP16's range before its storage scale
+    imgs = (1e5 * np.random.default_rng(4).standard_normal((6, N, N))).astype(np.float32)
+    with gg.MultiGPUGridder(N, 6, precision=prec, adjustInterpFactor=False) as g:
+        g.backProject(imgs, axes)
+        got = g.getCASVolume()
+        g.backProjectCAS(O.cas_imgs_from_imgs(imgs, p.M).astype(np.float32), axes)
+        ref = g.getCASVolume()
+    # the same storage on both sides: only values on a rounding edge differ
+    assert np.linalg.norm(ref) > 0
+    assert O.rel_l2(got, ref) < 1e-3
+
+
+# few tiles (boxes planned the quick way) and more than four a block of the
+# grid; volumes smaller than a box; M no multiple of the tile; axes that are
+# not orthonormal (boxes that do not fit, windows that leave the volume)
+@pytest.mark.parametrize("prec", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("N,n,scale", [(4, 6, 1.0), (18, 5, 1.0), (26, 700, 1.0), (32, 200, 1.0), (32, 4, 1.7), (50, 6, 0.4)])
+def test_forward_tiles(cuda, N, n, scale, prec):
+    import torch
+
+    import multigpugridder_gb300 as gg
+
+    p = O.Params(N)
+    rng = np.random.default_rng(1000 + N)
+    cas = rng.standard_normal((p.V,) * 3).astype(np.float32)
+    axes = (scale * O.quaternion_axes(n, seed=N + n)).astype(np.float32)
+    stored = cas
+    if prec != "f32":  # largest value about 5: FP16 is stored at scale 1
+        stored = torch.from_numpy(cas).to(torch.bfloat16 if prec == "bf16" else torch.float16).float().numpy()
+    ref = O.fp_ref_f32(stored, axes, p.M, p.mask_radius, p.ker)
+    with gg.MultiGPUGridder(N, n, precision=prec, adjustInterpFactor=False) as g:
+        g.setCASVolume(cas)
+        got = g.forwardProjectCAS(axes)
+    assert O.rel_l2(got, ref) < TOL
+    assert np.all(got[ref == 0] == 0)
+
+
+# fewer than 32 directions, and each range of the rule's aim, at volumes of few
+# bricks; n that the segments do not divide
+@pytest.mark.parametrize("N,n", [(64, 9), (16, 33), (18, 101), (32, 210), (16, 600)])
+def test_back_projection_segments(cuda, N, n):
+    import multigpugridder_gb300 as gg
+
+    p = O.Params(N)
+    rng = np.random.default_rng(2000 + n)
+    axes = O.quaternion_axes(n, seed=n).astype(np.float32)
+    imgs = rng.standard_normal((n, N, N)).astype(np.float32)
+    ci = O.cas_imgs_from_imgs(imgs, p.M).astype(np.float32)
+    num = O.bp_ref_f32(ci, axes, p.V, p.mask_radius, p.ker)
+    den = O.bp_ref_f32(np.ones_like(ci), axes, p.V, p.mask_radius, p.ker)
+    with gg.MultiGPUGridder(N, n, adjustInterpFactor=False) as g:
+        g.backProjectCAS(ci, axes)
+        assert O.rel_l2(g.getCASVolume(), num) < TOL
+        g.backProjectCAS(ci, axes, accumulate=True)  # the merge adds to what is there
+        assert O.rel_l2(g.getCASVolume(), 2 * num) < TOL
+        g.reconstructVol(imgs, axes)
+        assert O.rel_l2(g.getCASVolume(), num / (den + np.float32(1e-6))) < TOL
+
+
+# V = 10, 38, 106 (rows of 2 and of 4 floats), 41 (odd rows); a table too long
+# to be kept four times; boxes that do not fit and boxes of few voxels
+@pytest.mark.parametrize("N,interp,size,mask,scale",
+                         [(2, 2.0, 501, 1, 1.0), (16, 2.0, 1000, 15, 1.0), (50, 2.0, 501, 49, 1.0), (14, 2.5, 501, 16, 1.0),
+                          (16, 2.0, 501, 8, 1.7), (16, 2.0, 501, 15, 0.3)])
+def test_adjoint_boxes(cuda, gglib, N, interp, size, mask, scale):
+    import torch
+
+    p = O.Params(N, interp, table_size=size, mask_radius=mask)
+    n = 9
+    rng = np.random.default_rng(3000 + N)
+    axes = (scale * O.quaternion_axes(n, seed=N)).astype(np.float32)
+    y = rng.standard_normal((n, p.M, p.M)).astype(np.float32)
+    vol = torch.zeros((p.V,) * 3, device=cuda)
+    d_ker, d_axes, d_y = to_dev(p.ker, cuda), to_dev(axes, cuda), to_dev(y, cuda)
+    assert gglib.gg_back_project_adjoint_kernel(dptr(vol), dptr(d_y), dptr(d_ker), dptr(d_axes), 2.0, n, p.V, p.M, mask,
+                                                size, None) == 0
+    torch.cuda.synchronize()
+    ref = O.bp_adjoint_f64(y.astype(np.float64), axes, p.V, mask, p.ker)
+    assert O.rel_l2(vol.cpu().numpy(), ref) < 1e-3
+
+
+# enough images for blocks of 64 rows (1024 of them), also with a remainder, and one too few
+@pytest.mark.parametrize("M,n", [(64, 1100), (100, 520), (64, 1000)])
+def test_ctf_row_blocks(cuda, gglib, M, n):
+    import torch
+
+    kv, cs, amp = (float(np.float32(v)) for v in (300.0, 2.7, 0.1))
+    rng = np.random.default_rng(M + n)
+    du = rng.uniform(5000.0, 40000.0, n).astype(np.float32)
+    dv = (du - rng.uniform(-3000.0, 3000.0, n)).astype(np.float32)
+    ang = rng.uniform(-np.pi, np.pi, n).astype(np.float32)
+    out = torch.full((n, M, M), float("nan"), device=cuda)
+    d_u, d_v, d_a = to_dev(du, cuda), to_dev(dv, cuda), to_dev(ang, cuda)
+    for v, a, ref in ((None, None, O.ctf_cas(M, du, kv, cs, amp, 1.5)),
+                      (d_v, d_a, O.ctf_cas(M, du, kv, cs, amp, 1.5, dv, ang))):
+        assert gglib.gg_filter_apply_ctf(dptr(out), M, n, dptr(d_u), None if v is None else dptr(v),
+                                         None if a is None else dptr(a), kv, cs, amp, 1.5, 1, 1, None) == 0
+        torch.cuda.synchronize()
+        assert np.max(np.abs(out.cpu().numpy() - ref)) < 1e-6
