@@ -150,6 +150,7 @@ struct gg_gridder {
     int max_batch = 1024;
     bool fused_fft = false;     // fft2_fused_ok(N, M): the 2-D FFT stages run as one kernel each
     bool fft_passes = false;    // else fftn_ok(N, M): as two; else through cuFFT
+    bool vol_passes = false;    // fftn_volume_ok: setVolume's 3-D FFT as three pruned passes
     int nstreams_fp = 2, nstreams_bp = 2;
     int prec = kF32;            // storage of the resident CAS volume the forward projection reads
     int img_prec_set = -1;      // storage of the CAS images the back projection reads; -1: as prec
@@ -170,7 +171,7 @@ struct gg_gridder {
     int *fault = nullptr;       // pinned: set by a kernel whose copies did not arrive
     DevBuf<float> pd;        // plane density V^3
     DevBuf<float> bp_part;   // sums of a split back projection's segments
-    DevBuf<float2> tw;       // fft_passes: e^(-2 pi i k / M)
+    DevBuf<float2> tw;       // fft_passes, vol_passes: e^(-2 pi i k / M)
     DevBuf<unsigned> bp_next; // its groups' work counter, 0 between launches
     DevBuf<float> adj;       // CAS-volume gradient, V^2 rows of fp_pitch(V, kF32) (forward-operator adjoint)
     DevBuf<float> axes;
@@ -354,10 +355,18 @@ FpTiles fp_tiles(const gg_gridder *h)
 void do_set_volume(gg_gridder *h, const float *d_vol, cudaStream_t s)
 {
     const size_t V3 = (size_t)h->V * h->V * h->V;
-    const size_t M3 = (size_t)h->M * h->M * h->M;
+    const size_t M3 = (size_t)h->M * h->M * h->M, H = h->M / 2 + 1;
     h->cas.ensure(V3);
+    if (h->vol_passes) {
+        h->x3.ensure(std::max(M3, 2 * H * h->N * h->N));
+        h->spec3.ensure(H * h->M * h->M);
+        GG_CK(launch_volume_to_cas_passes(d_vol, h->N, h->M, h->V, h->precomp.p, h->cas.p, h->tw.p, (float2 *)h->x3.p,
+                                          (float2 *)h->spec3.p, s));
+        h->cas_fp_valid = false;
+        return;
+    }
     h->x3.ensure(M3);
-    h->spec3.ensure((size_t)h->M * h->M * (h->M / 2 + 1));
+    h->spec3.ensure(H * h->M * h->M);
     GG_CK(launch_vol_to_fft_input(d_vol, h->N, h->M, h->precomp.p, h->x3.p, s));
     cufftHandle p = plan3(h, true);
     GG_CKF(cufftSetStream(p, s));
@@ -740,7 +749,8 @@ void init_handle(gg_gridder *h)
     GG_CK(cudaMemset(h->bp_next.p, 0, sizeof(unsigned)));
     h->work.ensure(1);
     GG_CK(cudaMemset(h->work.p, 0, sizeof(unsigned int)));
-    if (fftn_ok(h->N, h->M)) {
+    h->vol_passes = fftn_volume_ok(h->N, h->M);
+    if (h->vol_passes || fftn_ok(h->N, h->M)) {
         std::vector<float2> tw(h->M);
         fftn_twiddles(h->M, tw.data());
         h->tw.ensure(h->M);

@@ -18,6 +18,7 @@
 
 #include "gg_common.cuh"
 #include "gg_internal.h"
+#include "gg_pair.cuh"
 #include "../../include/gg_gridder.h"
 
 namespace gg {
@@ -40,37 +41,12 @@ __device__ __forceinline__ int shift_idx(int q, int M) { return q + M / 2 >= M ?
 // around 780 us of cuFFT, now 97 + 189 us (6.0 TB/s); getVol's output stage at
 // N = 192, M = 384: 185 -> 26 us.
 //
-// Precomp factors are float pairs (hi + lo = the FP64 value to 48 bits); their
-// products keep the pair, so the one rounding to FP32 at the end is the FP64
-// product's but for ties.
 constexpr int kRows = 8; // warps (rows in flight) per block
 
 static inline unsigned rows_grid(long long rows)
 {
     const long long g = (rows + kRows - 1) / kRows;
     return (unsigned)(g < 0x7fffffffLL ? g : 0x7fffffffLL);
-}
-
-struct FF {
-    float h, l;
-};
-__device__ __forceinline__ FF ff_mul(FF a, FF b)
-{
-    const float p = __fmul_rn(a.h, b.h);
-    const float e = __fmaf_rn(a.h, b.h, -p) + (a.h * b.l + a.l * b.h);
-    const float s = __fadd_rn(p, e);
-    return FF{s, __fsub_rn(e, __fsub_rn(s, p))};
-}
-__device__ __forceinline__ FF ff_at(const float2 *__restrict__ pc, int i)
-{
-    const float2 v = __ldg(pc + i);
-    return FF{v.x, v.y};
-}
-// x * f, f a pair, rounded once
-__device__ __forceinline__ float ff_scale(float x, FF f)
-{
-    const float p = __fmul_rn(x, f.h);
-    return __fadd_rn(p, __fmaf_rn(x, f.h, -p) + x * f.l);
 }
 
 // x[q] = (zero-padded volume * precomp^3)[(q + M/2) mod M] per axis, the

@@ -1,5 +1,5 @@
-// FFT passes between images and CAS images for sizes M = 2^a 3^b 5^c 7^d up to 400
-// (sm_103a).
+// FFT passes between images and CAS images for sizes M = 2^a 3^b 5^c 7^d up to 400,
+// and from a volume to its CAS volume up to 512 (sm_103a).
 //
 // Each pass transforms tiles of C lines of length M in shared memory (Stockham
 // autosort, radices 8, 7, 5, 4, 3, 2, the two buffers swapped between stages) and does
@@ -12,6 +12,11 @@
 //     mirrored, Re-Im.
 //   CAS images -> images: the columns back along y, N rows kept; then rows in
 //     pairs along x, N pixels kept.
+//
+//   volume -> CAS volume: rows in pairs along x of the N planes, columns along
+//     y, then along z with the CAS values of a voxel and its mirror image: the
+//     zero rows and planes of the padded volume are left out of the
+//     first two (10.5 M^3 bytes for N = M/2, against about 36).
 //
 // Bound: the latency of a tile's load, stages and store at 16 warps an SM or so;
 // 9 M^2 bytes an image with N = M/2 (1 in, 2 x 2 for the half spectra between
@@ -31,6 +36,7 @@
 
 #include "gg_common.cuh"
 #include "gg_internal.h"
+#include "gg_pair.cuh"
 
 namespace gg {
 
@@ -212,6 +218,29 @@ template <int C> struct LoadRealRows {
     }
 };
 
+// The same of a volume (slice s: plane s) times the precomp factors' product.
+template <int C> struct LoadVolumeRows {
+    const float *src;
+    const float2 *pc;
+    int N, M;
+    __device__ void operator()(float2 *a, int s, int tile) const
+    {
+        constexpr int CP = C + 1;
+        const int b = M / 2 - N / 2;
+        const float *im = src + (size_t)s * N * N;
+        fn_zero_gap<C>(a, N, M);
+        float *f = reinterpret_cast<float *>(a);
+        for (int r = threadIdx.x >> 5; r < 2 * C; r += kFnThreads / 32) {
+            const int row = tile * 2 * C + r;
+            const FF jk = ff_mul(ff_at(pc, min(row, N - 1) + b), ff_at(pc, s + b));
+#pragma unroll 4
+            for (int o = threadIdx.x & 31; o < N; o += 32)
+                f[2 * (fn_wrap(o, N, M) * CP + (r >> 1)) + (r & 1)] =
+                    row < N ? __ldg(im + (size_t)row * N + o) * ff_mul(ff_at(pc, o + b), jk).h : 0.0f;
+        }
+    }
+};
+
 // Lines of row pairs -> half spectra, N rows of H a slice.
 template <int C> struct StoreHalfRows {
     float2 *dst;
@@ -336,6 +365,91 @@ template <int C, typename T, bool ADJ> struct StoreCasCols {
     }
 };
 
+// Columns of a plane -> M rows of H a plane.
+template <int C> struct StoreSpecCols {
+    float2 *dst;
+    int M;
+    __device__ void operator()(const float2 *a, int s, int tile) const
+    {
+        constexpr int CP = C + 1;
+        const int H = M / 2 + 1, c = threadIdx.x % C, u = tile * C + c;
+        if (u >= H) return;
+        float2 *g = dst + (size_t)s * M * H + u;
+        for (int v = threadIdx.x / C; v < M; v += kFnThreads / C) g[(size_t)v * H] = a[v * CP + c];
+    }
+};
+
+// N planes of M rows of H -> columns along z of row s, wrapped and padded.
+template <int C> struct LoadDepthCols {
+    const float2 *src;
+    int N, M;
+    __device__ void operator()(float2 *a, int s, int tile) const
+    {
+        constexpr int CP = C + 1;
+        const int H = M / 2 + 1, c = threadIdx.x % C, u = tile * C + c;
+        const float2 *g = src + (size_t)s * H + u;
+        fn_zero_gap<C>(a, N, M);
+#pragma unroll 4
+        for (int r = threadIdx.x / C; r < N; r += kFnThreads / C)
+            a[fn_wrap(r, N, M) * CP + c] = u < H ? __ldg(g + (size_t)r * M * H) : make_float2(0.0f, 0.0f);
+    }
+};
+
+// Columns along z of row v = s of the half spectrum -> the CAS volume: Re+Im,
+// and Re-Im at the mirror image through the centre; the rows' borders zero.
+template <int C> struct StoreCasVolume {
+    float *dst;
+    int M, V;
+    __device__ void operator()(const float2 *a, int s, int tile) const
+    {
+        constexpr int CP = C + 1;
+        const int c = threadIdx.x % C, u = tile * C + c, pad = V / 2 - M / 2;
+        const int j = fn_shift(s, M), jm = fn_shift(s ? M - s : 0, M);
+        const size_t VV = (size_t)V * V;
+        float *row = dst + pad * VV + (size_t)(j + pad) * V + pad;  // of plane pad
+        float *rowm = dst + pad * VV + (size_t)(jm + pad) * V + pad;
+        if (u <= M / 2) {
+            const int i = fn_shift(u, M), im = M / 2 - u; // of u and of M - u
+            const bool mirror = u != 0 && u != M / 2;
+            for (int w = threadIdx.x / C; w < M; w += kFnThreads / C) {
+                const float2 z = a[w * CP + c];
+                row[fn_shift(w, M) * VV + i] = z.x + z.y;
+                if (mirror) rowm[fn_shift(w ? M - w : 0, M) * VV + im] = z.x - z.y;
+            }
+        }
+        if (tile == 0) {
+            const int edge = V - M; // columns outside a row's M
+            for (int e = threadIdx.x; e < M * edge; e += kFnThreads) {
+                const int k = e / edge, x = e - k * edge;
+                row[k * VV + (x < pad ? x - pad : x - pad + M)] = 0.0f;
+            }
+        }
+    }
+};
+
+// Zeroes the rows of the CAS volume that lie outside the spectrum.
+__global__ void __launch_bounds__(256) zero_border_rows_kernel(float *__restrict__ cas, int M, int V)
+{
+    const int pad = V / 2 - M / 2, warp = threadIdx.x >> 5;
+    const int slab = (V - M) * V, rows = slab + M * (V - M); // whole planes, then rows of the others
+    for (int r = blockIdx.x * 8 + warp; r < rows; r += gridDim.x * 8) {
+        int k, j;
+        if (r < slab) {
+            k = r / V;
+            j = r - k * V;
+            if (k >= pad) k += M;
+        } else {
+            const int t = r - slab;
+            k = t / (V - M);
+            j = t - k * (V - M);
+            k += pad;
+            if (j >= pad) j += M;
+        }
+        float *row = cas + ((size_t)k * V + j) * V;
+        for (int c = threadIdx.x & 31; c < V; c += 32) row[c] = 0.0f;
+    }
+}
+
 // A CAS image -> columns of its Hermitian spectrum (FromCAS), inverse (swapped).
 template <int C> struct LoadCasCols {
     const float *src;
@@ -391,7 +505,7 @@ static bool fn_plan(int M, FnPlan &p)
     return m == 1;
 }
 
-static size_t fn_smem(int M) { return ((size_t)M + 2 * (size_t)M * (kFnC + 1)) * sizeof(float2); }
+static size_t fn_smem(int M, int C) { return ((size_t)M + 2 * (size_t)M * (C + 1)) * sizeof(float2); }
 
 // Longer lines leave room for one tile of 16 an SM or tiles of 8, and either way
 // the passes lose to the library (M = 512: 705 us against 694 for 512 images).
@@ -401,6 +515,19 @@ bool fftn_ok(int N, int M)
 {
     FnPlan p;
     return N > 0 && N <= M && (N & 1) == 0 && M <= kFnMaxM && fn_plan(M, p);
+}
+
+// A volume's three passes against the library's 3-D transform and its two stage
+// kernels (setVolume and 16 projections, us): M = 64: 41 (39), 96: 61 (63), 192:
+// 127 (142), 200: 139 (177), 256: 215 (235), 320: 354 (502), 384: 597 (789), 400: 695
+// (1166), 448: 960 (1450), 500: 1396 (1722), 512 in BF16: 1228 (1347).  Above 400 in
+// tiles of 8 lines, which leave room for two an SM.
+constexpr int kFnMinVolM = 96, kFnMaxVolM = 512;
+
+bool fftn_volume_ok(int N, int M)
+{
+    FnPlan p;
+    return N > 0 && N <= M && (N & 1) == 0 && M >= kFnMinVolM && M <= kFnMaxVolM && fn_plan(M, p);
 }
 
 void fftn_twiddles(int M, float2 *out)
@@ -437,7 +564,7 @@ static cudaError_t fn_launch(const FnPlan &p, const float2 *d_tw, int tiles, int
                              cudaStream_t s)
 {
     if (n <= 0) return cudaSuccess;
-    const size_t smem = fn_smem(p.M);
+    const size_t smem = fn_smem(p.M, C);
     auto kern = fn_pass_kernel<C, Load, Store>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -481,6 +608,32 @@ cudaError_t launch_cas_to_images_passes(const float *d_cas, int M, int N, int n,
     if (e != cudaSuccess) return e;
     return fn_launch<C>(p, d_tw, (N + 2 * C - 1) / (2 * C), n, LoadHalfRows<C>{d_half, N, M},
                         StoreRealRows<C>{d_img, N, M, 1.0f / ((float)M * (float)M)}, s);
+}
+
+template <int C>
+static cudaError_t volume_to_cas_t(const FnPlan &p, const float2 *d_tw, const float *d_vol, int N, int V, const float2 *d_pc,
+                                   float *d_cas, float2 *d_half, float2 *d_planes, cudaStream_t s)
+{
+    const int M = p.M, H = M / 2 + 1, cols = (H + C - 1) / C;
+    cudaError_t e = fn_launch<C>(p, d_tw, (N + 2 * C - 1) / (2 * C), N, LoadVolumeRows<C>{d_vol, d_pc, N, M},
+                                 StoreHalfRows<C>{d_half, N, M}, s);
+    if (e != cudaSuccess) return e;
+    e = fn_launch<C>(p, d_tw, cols, N, LoadPaddedCols<C>{d_half, N, M}, StoreSpecCols<C>{d_planes, M}, s);
+    if (e != cudaSuccess) return e;
+    e = fn_launch<C>(p, d_tw, cols, M, LoadDepthCols<C>{d_planes, N, M}, StoreCasVolume<C>{d_cas, M, V}, s);
+    if (e != cudaSuccess || V == M) return e;
+    zero_border_rows_kernel<<<(unsigned)(((V - M) * (V + M) + 7) / 8), 256, 0, s>>>(d_cas, M, V);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_volume_to_cas_passes(const float *d_vol, int N, int M, int V, const float2 *d_pc, float *d_cas,
+                                        const float2 *d_tw, float2 *d_half, float2 *d_planes, cudaStream_t s)
+{
+    FnPlan p;
+    if (!fftn_volume_ok(N, M) || !fn_plan(M, p) || V < M) return cudaErrorInvalidValue;
+    if (M <= kFnMaxM) return volume_to_cas_t<kFnC>(p, d_tw, d_vol, N, V, d_pc, d_cas, d_half, d_planes, s);
+    return volume_to_cas_t<kFnC / 2>(p, d_tw, d_vol, N, V, d_pc, d_cas, d_half, d_planes, s);
 }
 
 } // namespace gg
