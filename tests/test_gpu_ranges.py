@@ -75,6 +75,24 @@ def test_fft_passes_reduced_storage(cuda, prec):
     assert O.rel_l2(got, ref) < 1e-3
 
 
+# M = 96 (the smallest), tiles of 16 lines with and without remainders, no
+# padding at all (N = M), tiles of 8 lines (M > 400)
+@pytest.mark.parametrize("N,interp", [(48, 2.0), (70, 2.0), (80, 2.5), (100, 1.0), (200, 2.0), (210, 2.0)])
+def test_volume_passes(cuda, N, interp):
+    import multigpugridder_gb300 as gg
+
+    p = O.Params(N, interp)
+    rng = np.random.default_rng(N)
+    vol = rng.standard_normal((N,) * 3).astype(np.float32)
+    with gg.MultiGPUGridder(N, 2, interpFactor=interp, adjustInterpFactor=False) as g:
+        g.setCASVolume(np.ones((p.V,) * 3, dtype=np.float32))  # no border may be left over
+        g.setVolume(vol)
+        got = g.getCASVolume()
+    ref = O.cas_from_vol(vol.astype(np.float64), p.hw, p.interp, p.pad)
+    assert O.rel_l2(got, ref) < TOL
+    assert np.all(got[ref == 0] == 0)
+
+
 # few tiles (boxes planned the quick way) and more than four a block of the
 # grid; volumes smaller than a box; M no multiple of the tile; axes that are
 # not orthonormal (boxes that do not fit, windows that leave the volume)
