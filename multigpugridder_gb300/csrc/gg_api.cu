@@ -151,6 +151,7 @@ struct gg_gridder {
     bool fused_fft = false;     // fft2_fused_ok(N, M): the 2-D FFT stages run as one kernel each
     bool fft_passes = false;    // else fftn_ok(N, M): as two; else through cuFFT
     bool vol_passes = false;    // fftn_volume_ok: setVolume's 3-D FFT as three pruned passes
+    bool vol_back_passes = false; // fftn_volume_back_ok: getVolume's too
     int nstreams_fp = 2, nstreams_bp = 2;
     int prec = kF32;            // storage of the resident CAS volume the forward projection reads
     int img_prec_set = -1;      // storage of the CAS images the back projection reads; -1: as prec
@@ -352,14 +353,21 @@ FpTiles fp_tiles(const gg_gridder *h)
 
 // ---- device-side pipelines (all on stream s) --------------------------------
 
+// The volume passes' buffers: spectrum or planes; rows and planes.
+void ensure_vol(gg_gridder *h)
+{
+    const size_t M = h->M, N = h->N, H = M / 2 + 1;
+    h->x3.ensure(std::max(M * M * M, 2 * H * N * (N + M)));
+    h->spec3.ensure(H * M * M);
+}
+
 void do_set_volume(gg_gridder *h, const float *d_vol, cudaStream_t s)
 {
     const size_t V3 = (size_t)h->V * h->V * h->V;
     const size_t M3 = (size_t)h->M * h->M * h->M, H = h->M / 2 + 1;
     h->cas.ensure(V3);
     if (h->vol_passes) {
-        h->x3.ensure(std::max(M3, 2 * H * h->N * h->N));
-        h->spec3.ensure(H * h->M * h->M);
+        ensure_vol(h);
         GG_CK(launch_volume_to_cas_passes(d_vol, h->N, h->M, h->V, h->precomp.p, h->cas.p, h->tw.p, (float2 *)h->x3.p,
                                           (float2 *)h->spec3.p, s));
         h->cas_fp_valid = false;
@@ -378,9 +386,19 @@ void do_set_volume(gg_gridder *h, const float *d_vol, cudaStream_t s)
 // With a density the CAS volume is divided by it first, in place (+ 1e-6).
 void do_get_volume(gg_gridder *h, float *d_cas, const float *d_density, float *d_vol, cudaStream_t s)
 {
-    const size_t M3 = (size_t)h->M * h->M * h->M;
+    const size_t M3 = (size_t)h->M * h->M * h->M, H = h->M / 2 + 1;
+    if (h->vol_back_passes) {
+        // half spectra of rows, then (spec3 holds the divided volume's spectrum) those of planes
+        const size_t half = H * h->N * h->N;
+        ensure_vol(h);
+        float2 *const x = (float2 *)h->x3.p, *const sp = (float2 *)h->spec3.p;
+        if (d_density) GG_CK(launch_cas_volume_to_spectrum(d_cas, d_density, 1e-6f, h->V, h->M, h->spec3.p, s));
+        GG_CK(launch_cas_to_volume_passes(d_cas, d_density ? sp : nullptr, h->N, h->M, h->V, h->precomp.p, d_vol, h->tw.p, x,
+                                          d_density ? x + half : sp, s));
+        return;
+    }
     h->x3.ensure(M3);
-    h->spec3.ensure((size_t)h->M * h->M * (h->M / 2 + 1));
+    h->spec3.ensure(H * h->M * h->M);
     GG_CK(launch_cas_volume_to_spectrum(d_cas, d_density, 1e-6f, h->V, h->M, h->spec3.p, s));
     cufftHandle p = plan3(h, false);
     GG_CKF(cufftSetStream(p, s));
@@ -750,6 +768,7 @@ void init_handle(gg_gridder *h)
     h->work.ensure(1);
     GG_CK(cudaMemset(h->work.p, 0, sizeof(unsigned int)));
     h->vol_passes = fftn_volume_ok(h->N, h->M);
+    h->vol_back_passes = fftn_volume_back_ok(h->N, h->M);
     if (h->vol_passes || fftn_ok(h->N, h->M)) {
         std::vector<float2> tw(h->M);
         fftn_twiddles(h->M, tw.data());

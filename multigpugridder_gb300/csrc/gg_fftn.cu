@@ -1,5 +1,5 @@
 // FFT passes between images and CAS images for sizes M = 2^a 3^b 5^c 7^d up to 400,
-// and from a volume to its CAS volume up to 512 (sm_103a).
+// and between a volume and its CAS volume up to 512 (sm_103a).
 //
 // Each pass transforms tiles of C lines of length M in shared memory (Stockham
 // autosort, radices 8, 7, 5, 4, 3, 2, the two buffers swapped between stages) and does
@@ -17,6 +17,7 @@
 //     y, then along z with the CAS values of a voxel and its mirror image: the
 //     zero rows and planes of the padded volume are left out of the
 //     first two (10.5 M^3 bytes for N = M/2, against about 36).
+//   CAS volume -> volume: the same backwards; only what is kept is stored.
 //
 // Bound: the latency of a tile's load, stages and store at 16 warps an SM or so;
 // 9 M^2 bytes an image with N = M/2 (1 in, 2 x 2 for the half spectra between
@@ -427,6 +428,103 @@ template <int C> struct StoreCasVolume {
     }
 };
 
+// M planes of M rows of H -> columns along z of row s, inverse (swapped).
+template <int C> struct LoadSpecDepth {
+    const float2 *src;
+    int M;
+    __device__ void operator()(float2 *a, int s, int tile) const
+    {
+        constexpr int CP = C + 1;
+        const int H = M / 2 + 1, c = threadIdx.x % C, u = tile * C + c;
+        const float2 *g = src + (size_t)s * H + u;
+#pragma unroll 4
+        for (int w = threadIdx.x / C; w < M; w += kFnThreads / C) {
+            const float2 z = u < H ? __ldg(g + (size_t)w * M * H) : make_float2(0.0f, 0.0f);
+            a[w * CP + c] = make_float2(z.y, z.x);
+        }
+    }
+};
+
+// The same from the CAS volume itself (FromCAS over the inner M^3).
+template <int C> struct LoadCasDepth {
+    const float *src;
+    int M, V;
+    __device__ void operator()(float2 *a, int s, int tile) const
+    {
+        constexpr int CP = C + 1;
+        const int c = threadIdx.x % C, u = tile * C + c, pad = V / 2 - M / 2, j = fn_shift(s, M);
+        const size_t VV = (size_t)V * V;
+        const bool live = j != 0 && u < M / 2; // u = M/2 is column 0: zero
+        const float *g = src + pad * VV + (size_t)(j + pad) * V + pad + M / 2 + u;
+        const float *gm = src + pad * VV + (size_t)(M - j + pad) * V + pad + M / 2 - u;
+#pragma unroll 4
+        for (int w = threadIdx.x / C; w < M; w += kFnThreads / C) {
+            const int k = fn_shift(w, M);
+            const bool on = live && k != 0;
+            const float x = on ? __ldg(g + k * VV) : 0.0f, y = on ? __ldg(gm + (M - k) * VV) : 0.0f;
+            a[w * CP + c] = make_float2(0.5f * (x - y), 0.5f * (x + y));
+        }
+    }
+};
+
+// Inverse columns along z of row s -> N cropped planes of M rows of H.
+template <int C> struct StoreCroppedDepth {
+    float2 *dst;
+    int N, M;
+    __device__ void operator()(const float2 *a, int s, int tile) const
+    {
+        constexpr int CP = C + 1;
+        const int H = M / 2 + 1, c = threadIdx.x % C, u = tile * C + c;
+        if (u >= H) return;
+        float2 *g = dst + (size_t)s * H + u;
+        for (int r = threadIdx.x / C; r < N; r += kFnThreads / C) {
+            const float2 z = a[fn_wrap(r, N, M) * CP + c];
+            g[(size_t)r * M * H] = make_float2(z.y, z.x);
+        }
+    }
+};
+
+// M rows of H a plane -> columns along y, inverse (swapped).
+template <int C> struct LoadSpecCols {
+    const float2 *src;
+    int M;
+    __device__ void operator()(float2 *a, int s, int tile) const
+    {
+        constexpr int CP = C + 1;
+        const int H = M / 2 + 1, c = threadIdx.x % C, u = tile * C + c;
+        const float2 *g = src + (size_t)s * M * H + u;
+#pragma unroll 4
+        for (int v = threadIdx.x / C; v < M; v += kFnThreads / C) {
+            const float2 z = u < H ? __ldg(g + (size_t)v * H) : make_float2(0.0f, 0.0f);
+            a[v * CP + c] = make_float2(z.y, z.x);
+        }
+    }
+};
+
+// Lines of row pairs -> N cropped voxels of N rows of plane s, times the precomp
+// factors' product and `inv`, rounded once.
+template <int C> struct StoreVolumeRows {
+    float *dst;
+    const float2 *pc;
+    int N, M;
+    FF inv;
+    __device__ void operator()(const float2 *a, int s, int tile) const
+    {
+        constexpr int CP = C + 1;
+        const int b = M / 2 - N / 2;
+        const float *f = reinterpret_cast<const float *>(a);
+        float *im = dst + (size_t)s * N * N;
+        for (int r = threadIdx.x >> 5; r < 2 * C; r += kFnThreads / 32) {
+            const int row = tile * 2 * C + r;
+            if (row >= N) break;
+            const FF jk = ff_mul(inv, ff_mul(ff_at(pc, row + b), ff_at(pc, s + b)));
+            for (int o = threadIdx.x & 31; o < N; o += 32)
+                im[(size_t)row * N + o] =
+                    ff_scale(f[2 * (fn_wrap(o, N, M) * CP + (r >> 1)) + 1 - (r & 1)], ff_mul(ff_at(pc, o + b), jk));
+        }
+    }
+};
+
 // Zeroes the rows of the CAS volume that lie outside the spectrum.
 __global__ void __launch_bounds__(256) zero_border_rows_kernel(float *__restrict__ cas, int M, int V)
 {
@@ -529,6 +627,12 @@ bool fftn_volume_ok(int N, int M)
     FnPlan p;
     return N > 0 && N <= M && (N & 1) == 0 && M >= kFnMinVolM && M <= kFnMaxVolM && fn_plan(M, p);
 }
+
+// Back: the z pass reads the CAS volume (or the divided one's spectrum) in full
+// and there is less to prune.  16 images back and the volume, us: M = 96: 94
+// (99), 200: 177 (215), 384: 945 (987), 400: 1065 (1385), 420: 1133 (1327); but
+// 256: 294 (292), 512: 1976 (1850), where the library has powers of two.
+bool fftn_volume_back_ok(int N, int M) { return fftn_volume_ok(N, M) && (M & (M - 1)) != 0; }
 
 void fftn_twiddles(int M, float2 *out)
 {
@@ -634,6 +738,32 @@ cudaError_t launch_volume_to_cas_passes(const float *d_vol, int N, int M, int V,
     if (!fftn_volume_ok(N, M) || !fn_plan(M, p) || V < M) return cudaErrorInvalidValue;
     if (M <= kFnMaxM) return volume_to_cas_t<kFnC>(p, d_tw, d_vol, N, V, d_pc, d_cas, d_half, d_planes, s);
     return volume_to_cas_t<kFnC / 2>(p, d_tw, d_vol, N, V, d_pc, d_cas, d_half, d_planes, s);
+}
+
+template <int C>
+static cudaError_t cas_to_volume_t(const FnPlan &p, const float2 *d_tw, const float *d_cas, const float2 *d_spec, int N, int V,
+                                   const float2 *d_pc, float *d_vol, float2 *d_half, float2 *d_planes, cudaStream_t s)
+{
+    const int M = p.M, H = M / 2 + 1, cols = (H + C - 1) / C;
+    const double m3 = 1.0 / ((double)M * M * M);
+    const FF inv{(float)m3, (float)(m3 - (double)(float)m3)};
+    const StoreCroppedDepth<C> planes{d_planes, N, M};
+    cudaError_t e = d_spec ? fn_launch<C>(p, d_tw, cols, M, LoadSpecDepth<C>{d_spec, M}, planes, s)
+                           : fn_launch<C>(p, d_tw, cols, M, LoadCasDepth<C>{d_cas, M, V}, planes, s);
+    if (e != cudaSuccess) return e;
+    e = fn_launch<C>(p, d_tw, cols, N, LoadSpecCols<C>{d_planes, M}, StoreCroppedCols<C>{d_half, N, M}, s);
+    if (e != cudaSuccess) return e;
+    return fn_launch<C>(p, d_tw, (N + 2 * C - 1) / (2 * C), N, LoadHalfRows<C>{d_half, N, M},
+                        StoreVolumeRows<C>{d_vol, d_pc, N, M, inv}, s);
+}
+
+cudaError_t launch_cas_to_volume_passes(const float *d_cas, const float2 *d_spec, int N, int M, int V, const float2 *d_pc,
+                                        float *d_vol, const float2 *d_tw, float2 *d_half, float2 *d_planes, cudaStream_t s)
+{
+    FnPlan p;
+    if (!fftn_volume_back_ok(N, M) || !fn_plan(M, p) || V < M) return cudaErrorInvalidValue;
+    if (M <= kFnMaxM) return cas_to_volume_t<kFnC>(p, d_tw, d_cas, d_spec, N, V, d_pc, d_vol, d_half, d_planes, s);
+    return cas_to_volume_t<kFnC / 2>(p, d_tw, d_cas, d_spec, N, V, d_pc, d_vol, d_half, d_planes, s);
 }
 
 } // namespace gg

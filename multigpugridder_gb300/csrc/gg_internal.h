@@ -199,6 +199,8 @@ cudaError_t launch_cas_to_images_fused(const float *d_cas, int M, int N, int n, 
 bool fftn_ok(int N, int M);
 // The same for volumes, with 96 <= M <= 512.
 bool fftn_volume_ok(int N, int M);
+// The same back, without the powers of two.
+bool fftn_volume_back_ok(int N, int M);
 // e^(-2 pi i k / M), k < M, for the passes' d_tw.
 void fftn_twiddles(int M, float2 *out);
 // The two directions of the fused stages above, in two launches each through
@@ -211,6 +213,9 @@ cudaError_t launch_cas_to_images_passes(const float *d_cas, int M, int N, int n,
 // Volume -> CAS volume through d_half (N * N * (M/2 + 1)) and d_planes (N * M * (M/2 + 1)).
 cudaError_t launch_volume_to_cas_passes(const float *d_vol, int N, int M, int V, const float2 *d_pc, float *d_cas,
                                         const float2 *d_tw, float2 *d_half, float2 *d_planes, cudaStream_t s);
+// CAS volume -> volume, from d_spec (its half spectrum, M * M * (M/2 + 1)) if given.
+cudaError_t launch_cas_to_volume_passes(const float *d_cas, const float2 *d_spec, int N, int M, int V, const float2 *d_pc,
+                                        float *d_vol, const float2 *d_tw, float2 *d_half, float2 *d_planes, cudaStream_t s);
 
 // Adds to the process-wide count of kernels launched by this library.
 void count_launches(long long n);
