@@ -88,9 +88,27 @@ def test_volume_passes(cuda, N, interp):
         g.setCASVolume(np.ones((p.V,) * 3, dtype=np.float32))  # no border may be left over
         g.setVolume(vol)
         got = g.getCASVolume()
+        cas = rng.standard_normal((p.V,) * 3).astype(np.float32)
+        g.setCASVolume(cas)
+        back = g.getVol()
     ref = O.cas_from_vol(vol.astype(np.float64), p.hw, p.interp, p.pad)
     assert O.rel_l2(got, ref) < TOL
     assert np.all(got[ref == 0] == 0)
+    assert O.rel_l2(back, O.vol_from_cas(cas, N, p.hw, p.interp)) < TOL
+
+
+# the division's spectrum through the passes (M = 96, 200, no power of two)
+@pytest.mark.parametrize("N", [48, 100])
+def test_reconstruction_passes(cuda, N):
+    import multigpugridder_gb300 as gg
+
+    p = O.Params(N)
+    axes = O.quaternion_axes(8, seed=N).astype(np.float32)
+    imgs = np.random.default_rng(N).standard_normal((8, N, N)).astype(np.float32)
+    with gg.MultiGPUGridder(N, 8, adjustInterpFactor=False) as g:
+        vol = g.reconstructVol(imgs, axes)
+        cas = g.getCASVolume()
+    assert O.rel_l2(vol, O.vol_from_cas(cas, N, p.hw, p.interp)) < TOL
 
 
 # few tiles (boxes planned the quick way) and more than four a block of the
