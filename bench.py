@@ -678,6 +678,7 @@ def run_precision(args, kind="256"):
                                                     / torch.linalg.vector_norm(ref[k].double()))
         # reconstructVol of the subset's FP32 images (the same input for every storage type)
         rec_sub = torch.empty((N, N, N), dtype=torch.float32, device=dev)
+        stream.wait_stream(torch.cuda.current_stream())  # the subset's images are gathered there
         with torch.cuda.stream(stream):
             check(L.gg_reconstruct_volume_dev(h, vp(d_sub_axes), len(sub), vp(sub_imgs_f32), vp(rec_sub), sp), h)
         torch.cuda.synchronize()
