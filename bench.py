@@ -93,12 +93,12 @@ def workload(args, rank=0, world=1):
 FLUSH_BYTES = 512 << 20  # untimed write between steps: 4x the 126 MB L2
 
 # From a one-launch ncu capture of the fused back projection at 128^3 x 2,
-# 1,024 directions per launch (profiles/bp_ref_compact_kernel_density_128cubed_1024dirs.md):
+# 2,000 directions per launch (profiles/bp_ref_compact_kernel_density_128cubed_2000dirs.md):
 # DRAM bytes (read + write) and L2 bytes (lts__t_bytes) per direction, and the
 # fraction of cycles the schedulers issued.
-NCU_BP_DRAM_PER_DIR = 545.2e6 / 1024
-NCU_BP_LTS_PER_DIR = 5.488e9 / 1024
-NCU_BP_ISSUE_ACTIVE = 0.720
+NCU_BP_DRAM_PER_DIR = 1.696e9 / 2000
+NCU_BP_LTS_PER_DIR = 17.12e9 / 2000
+NCU_BP_ISSUE_ACTIVE = 0.852
 
 
 def sizes(args):

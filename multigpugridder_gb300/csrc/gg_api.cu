@@ -1,21 +1,22 @@
 // Host engine and C ABI of the GB300 gridder (include/gg_gridder.h).
 //
-// One handle owns one GPU's state: the resident FP32 CAS volume (plus, with
-// FP16/BF16 storage, the copy the forward projection reads: rows padded for
-// TMA), the KB table and pre-compensation vector, batch buffers and
-// cached cuFFT plans.  It replaces the reference's MultiGPUGridder /
+// One handle owns one GPU's state: the resident FP32 CAS volume and the copy
+// the forward projection reads (in the storage type, rows padded for TMA), the
+// KB table and pre-compensation vector, batch buffers, FFT twiddles and cached
+// cuFFT plans.  It replaces the reference's MultiGPUGridder /
 // gpuGridder / AbstractGridder trio (src/Gridders/) for one device:
 //   * the volume is prepared on the device once per setVolume instead of on
 //     the host (CASFromVol_Gridder.m) and re-uploaded on every forward
 //     projection (gpuGridder.cpp:194);
 //   * directions are processed in batches of max_batch (SetMaxAxesToAllocate)
-//     by one kernel launch each, with one batched cuFFT transform per batch
-//     instead of one cuFFT call per image (gpuGridder.cpp:476-482);
+//     by one kernel launch each, with the transforms of a batch in one or two
+//     kernels (or one batched cuFFT call) instead of one cuFFT call per image
+//     (gpuGridder.cpp:476-482);
 //   * host transfers run on a copy stream, double-buffered against the
 //     compute stream;
 //   * back projection accumulates into one device volume on one compute
 //     stream, so the per-GPU volume sum (MultiGPUGridder.cpp:376-411) is not
-//     needed and no atomics are used.
+//     needed; where a launch splits its directions the parts are added in order.
 #include <algorithm>
 #include <atomic>
 #include <cmath>

@@ -1201,9 +1201,9 @@ static cudaError_t launch_bp_compact_t(float *vol, const TI *img, const float *k
     if (n <= 0) return cudaSuccess;
     // A GPU shared with concurrent launches (the serving lanes): one group
     // and one table copy per CTA, three CTAs an SM, which the launches of
-    // other lanes can fill as they free (serving capacity 172 -> 195 req/s);
-    // alone, three groups sharing 32 table copies (batched back projection
-    // 78.5 -> 71.7 ms per 10k images).
+    // other lanes can fill as they free (serving capacity 172 -> 195 req/s when
+    // the rule was made); alone, 24 warps sharing 32 table copies (batched back
+    // projection 78.5 -> 71.7 ms per 10k images then, 51 now).
     if constexpr (std::is_same<TI, float>::value && !ONES && !DENS && !DW) {
         if (shared)
             return launch_bp_compact_g<TI, ONES, DENS, DW, DEEP, 1>(vol, img, ker, axes, n, g, scale, s, pd,
