@@ -90,10 +90,10 @@ int gg_set_max_axes_to_allocate(gg_gridder *h, int max_axes);       /* SetMaxAxe
 int gg_set_num_streams_fp(gg_gridder *h, int n);                    /* SetNumStreamsFP: copy/compute pipeline depth */
 int gg_set_num_streams_bp(gg_gridder *h, int n);                    /* SetNumStreamsBP */
 int gg_set_precision(gg_gridder *h, int precision);                 /* GG_PREC_*: storage of CAS volume / CAS images */
-/* Storage of the CAS images the back projection reads, apart from the CAS
+/* Rounding of the CAS images the back projection reads, apart from the CAS
    volume's: GG_PREC_* or -1 (the default) to follow gg_set_precision.
-   GG_PREC_F32 under a 2-byte volume keeps the images exact; it costs about
-   the same as 2-byte images.  No counterpart in the reference. */
+   GG_PREC_F32 under a 2-byte volume keeps the images exact; it costs no more
+   than 2-byte images.  No counterpart in the reference. */
 int gg_set_image_precision(gg_gridder *h, int precision);
 int gg_set_bp_mode(gg_gridder *h, int mode);                        /* GG_BP_REF (default) or GG_BP_ADJOINT */
 

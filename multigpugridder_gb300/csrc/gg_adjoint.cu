@@ -82,9 +82,9 @@ __device__ __noinline__ void pixel_to_global(float *__restrict__ vol, int V, int
     }
 }
 
-template <typename TI, int VW>
+template <int VW>
 __global__ void __launch_bounds__(kAdjWarps * 32, 1)
-adjoint_tile_kernel(float *__restrict__ vol, int V, int P, const TI *__restrict__ img, int M,
+adjoint_tile_kernel(float *__restrict__ vol, int V, int P, const float *__restrict__ img, int M,
                     const float *__restrict__ axes, int maskR, const float *__restrict__ ker, int kerSize, float kerHW,
                     int tilesX, long long nItems, const float *__restrict__ d_scale, int rep)
 {
@@ -117,7 +117,7 @@ adjoint_tile_kernel(float *__restrict__ vol, int V, int P, const TI *__restrict_
             if (ni * ni + nj * nj > R2) continue;
         }
         const float *ax = axes + 9 * (size_t)a;
-        const TI *im = img + (size_t)a * M * M;
+        const float *im = img + (size_t)a * M * M;
         const float nx0 = __ldg(ax), nx1 = __ldg(ax + 1), nx2 = __ldg(ax + 2);
         const float ny0 = __ldg(ax + 3), ny1 = __ldg(ax + 4), ny2 = __ldg(ax + 5);
 
@@ -246,9 +246,8 @@ adjoint_tile_kernel(float *__restrict__ vol, int V, int P, const TI *__restrict_
     }
 }
 
-template <typename TI>
-static cudaError_t launch_adjoint_t(float *d_vol, int P, const TI *d_img, const float *d_ker, const float *d_axes, int n,
-                                    const Geom &g, const float *scale, cudaStream_t s)
+cudaError_t launch_back_project_adjoint(float *d_vol, int P, const float *d_img, const float *d_ker, const float *d_axes,
+                                        int n, const Geom &g, const float *scale, cudaStream_t s)
 {
     const int tilesX = (g.M + kAdjTile - 1) / kAdjTile;
     const long long nItems = (long long)n * tilesX * tilesX;
@@ -271,17 +270,9 @@ static cudaError_t launch_adjoint_t(float *d_vol, int P, const TI *d_img, const 
         count_launches(1);
         return cudaGetLastError();
     };
-    if (P % 4 == 0 && at % 16 == 0) return go(adjoint_tile_kernel<TI, 4>);
-    if (P % 2 == 0 && g.V % 2 == 0 && at % 8 == 0) return go(adjoint_tile_kernel<TI, 2>);
-    return go(adjoint_tile_kernel<TI, 1>);
-}
-
-cudaError_t launch_back_project_adjoint(float *d_vol, int pitch, const void *d_img, int iprec, const float *d_ker,
-                                        const float *d_axes, int n, const Geom &g, const float *scale, cudaStream_t s)
-{
-    if (iprec == kF32) return launch_adjoint_t<float>(d_vol, pitch, (const float *)d_img, d_ker, d_axes, n, g, scale, s);
-    if (iprec == kF16) return launch_adjoint_t<__half>(d_vol, pitch, (const __half *)d_img, d_ker, d_axes, n, g, scale, s);
-    return launch_adjoint_t<__nv_bfloat16>(d_vol, pitch, (const __nv_bfloat16 *)d_img, d_ker, d_axes, n, g, scale, s);
+    if (P % 4 == 0 && at % 16 == 0) return go(adjoint_tile_kernel<4>);
+    if (P % 2 == 0 && g.V % 2 == 0 && at % 8 == 0) return go(adjoint_tile_kernel<2>);
+    return go(adjoint_tile_kernel<1>);
 }
 
 } // namespace gg

@@ -186,7 +186,6 @@ struct gg_gridder {
     struct Slot {
         DevBuf<float> casimg, real, img;
         DevBuf<cufftComplex> spec;
-        DevBuf<uint16_t> casimg_lp;
         DevBuf<unsigned char> plans; // the forward projection's box plans, one per direction
         PinBuf stage;
         cudaEvent_t ev_ready = nullptr, ev_free = nullptr;
@@ -257,7 +256,6 @@ void ensure_slot(gg_gridder *h, int s, int b, bool need_img)
     sl.real.ensure(MM * b);
     sl.spec.ensure(H * b);
     if (need_img) sl.img.ensure(NN * b);
-    if (h->img_prec() != kF32) sl.casimg_lp.ensure(MM * b);
     sl.plans.ensure(fp_plan_bytes(b));
     if (!sl.ev_ready) GG_CK(cudaEventCreateWithFlags(&sl.ev_ready, cudaEventDisableTiming));
     if (!sl.ev_free) {
@@ -449,9 +447,8 @@ void bp_batch(gg_gridder *h, const float *d_axes, int b, const float *img, const
               int sl, cudaStream_t s, float *pd = nullptr)
 {
     auto &S = h->slot[sl];
-    const void *src = nullptr;
-    const int ip = h->img_prec(); // storage of the CAS images read here
-    int iprec = ip;
+    const float *src = nullptr;
+    const int ip = h->img_prec(); // rounding of the CAS images read here
     const float *scale = nullptr;
     if (!ones) {
         const size_t MM = (size_t)h->M * h->M;
@@ -460,34 +457,33 @@ void bp_batch(gg_gridder *h, const float *d_axes, int b, const float *img, const
                 src = casimg;
             } else {
                 if (ip == kF16) GG_CK(launch_storage_scale(casimg, MM * b, 8192.0f, h->work.p, h->scales.p + 1, s));
-                GG_CK(launch_convert(casimg, S.casimg_lp.p, ip, MM * b, h->img_scale(), s));
-                src = S.casimg_lp.p;
+                GG_CK(launch_round(casimg, S.casimg.p, ip, MM * b, h->img_scale(), s));
+                src = S.casimg.p;
                 scale = h->img_scale();
             }
         } else if (h->fused_fft && ip != kF16) {
-            void *dst = ip == kF32 ? (void *)S.casimg.p : (void *)S.casimg_lp.p;
-            GG_CK(launch_images_to_cas_fused(img, h->N, h->M, b, dst, ip, false, s));
-            src = dst;
+            GG_CK(launch_images_to_cas_fused(img, h->N, h->M, b, S.casimg.p, ip, false, s));
+            src = S.casimg.p;
         } else if (h->fft_passes && ip != kF16) {
-            void *dst = ip == kF32 ? (void *)S.casimg.p : (void *)S.casimg_lp.p;
-            GG_CK(launch_images_to_cas_passes(img, h->N, h->M, b, dst, ip, false, h->tw.p, (float2 *)S.spec.p, nullptr, s));
-            src = dst;
+            GG_CK(launch_images_to_cas_passes(img, h->N, h->M, b, S.casimg.p, ip, false, h->tw.p, (float2 *)S.spec.p, nullptr,
+                                              s));
+            src = S.casimg.p;
         } else if (h->fft_passes) {
             // FP16: FP32 CAS images with their largest magnitude, then the
-            // storage scale and the conversion
+            // storage scale and the rounding
             GG_CK(launch_images_to_cas_passes(img, h->N, h->M, b, S.casimg.p, kF32, false, h->tw.p, (float2 *)S.spec.p,
                                               h->work.p, s));
             GG_CK(launch_scale_from_max(h->work.p, 8192.0f, h->scales.p + 1, s));
-            GG_CK(launch_convert(S.casimg.p, S.casimg_lp.p, ip, MM * b, h->img_scale(), s));
-            src = S.casimg_lp.p;
+            GG_CK(launch_round(S.casimg.p, S.casimg.p, ip, MM * b, h->img_scale(), s));
+            src = S.casimg.p;
             scale = h->img_scale();
         } else if (h->fused_fft) {
             // FP16: FP32 CAS images first, then the storage scale from their
             // largest magnitude and the conversion
             GG_CK(launch_images_to_cas_fused(img, h->N, h->M, b, S.casimg.p, kF32, false, s));
             GG_CK(launch_storage_scale(S.casimg.p, MM * b, 8192.0f, h->work.p, h->scales.p + 1, s));
-            GG_CK(launch_convert(S.casimg.p, S.casimg_lp.p, ip, MM * b, h->img_scale(), s));
-            src = S.casimg_lp.p;
+            GG_CK(launch_round(S.casimg.p, S.casimg.p, ip, MM * b, h->img_scale(), s));
+            src = S.casimg.p;
             scale = h->img_scale();
         } else {
             GG_CK(launch_images_to_fft_input(img, h->N, h->M, b, S.real.p, s));
@@ -498,22 +494,20 @@ void bp_batch(gg_gridder *h, const float *d_axes, int b, const float *img, const
                 // |Re + Im| <= 2 max(|Re|, |Im|)
                 GG_CK(launch_storage_scale((const float *)S.spec.p, (size_t)h->M * (h->M / 2 + 1) * 2 * b, 4096.0f,
                                            h->work.p, h->scales.p + 1, s));
-            void *dst = ip == kF32 ? (void *)S.casimg.p : (void *)S.casimg_lp.p;
-            GG_CK(launch_spectrum_to_cas_images(S.spec.p, h->M, b, dst, ip, h->img_scale(), s));
-            src = dst;
+            GG_CK(launch_spectrum_to_cas_images(S.spec.p, h->M, b, S.casimg.p, ip, h->img_scale(), s));
+            src = S.casimg.p;
             scale = h->img_scale();
         }
     }
-    if (ones) iprec = kF32;
     ProfScope ps(h, s, ones ? GG_KERNEL_DENSITY : GG_KERNEL_BACK);
     if (h->bp_mode == GG_BP_ADJOINT && !ones) {
-        GG_CK(launch_back_project_adjoint(target, h->V, src, iprec, h->ker.p, d_axes, b, h->geom(), scale, s));
+        GG_CK(launch_back_project_adjoint(target, h->V, src, h->ker.p, d_axes, b, h->geom(), scale, s));
     } else if (pd && !ones) {
-        GG_CK(launch_back_project_ref_density(target, pd, src, iprec, h->ker.p, d_axes, b, h->geom(), scale, s,
+        GG_CK(launch_back_project_ref_density(target, pd, src, h->ker.p, d_axes, b, h->geom(), scale, s,
                                               bp_split(h, b, 2)));
         pd = nullptr;
     } else {
-        GG_CK(launch_back_project_ref(target, src, iprec, ones, h->ker.p, d_axes, b, h->geom(), scale, s, false,
+        GG_CK(launch_back_project_ref(target, src, ones, h->ker.p, d_axes, b, h->geom(), scale, s, false,
                                       bp_split(h, b, 1)));
     }
     ps.done();
@@ -522,7 +516,7 @@ void bp_batch(gg_gridder *h, const float *d_axes, int b, const float *img, const
         const size_t MM = (size_t)h->M * h->M;
         ProfScope pd_ps(h, s, GG_KERNEL_DENSITY);
         GG_CK(launch_fill(S.casimg.p, MM * b, 1.0f, s));
-        GG_CK(launch_back_project_adjoint(pd, h->V, S.casimg.p, kF32, h->ker.p, d_axes, b, h->geom(), nullptr, s));
+        GG_CK(launch_back_project_adjoint(pd, h->V, S.casimg.p, h->ker.p, d_axes, b, h->geom(), nullptr, s));
         pd_ps.done();
     }
 }
@@ -594,7 +588,7 @@ void forward_adjoint(gg_gridder *h, const float *d_axes, int n, const float *d_i
             GG_CK(launch_spectrum_to_cas_images_adjoint(S.spec.p, h->M, b, S.casimg.p, s));
         }
         ProfScope ps(h, s, GG_KERNEL_BACK);
-        GG_CK(launch_back_project_adjoint(h->adj.p, P, S.casimg.p, kF32, h->ker.p, d_axes + (size_t)a0 * 9, b, h->geom(),
+        GG_CK(launch_back_project_adjoint(h->adj.p, P, S.casimg.p, h->ker.p, d_axes + (size_t)a0 * 9, b, h->geom(),
                                           nullptr, s));
         ps.done();
     }
@@ -796,7 +790,6 @@ void destroy_handle(gg_gridder *h)
         S.real.release();
         S.img.release();
         S.spec.release();
-        S.casimg_lp.release();
         S.stage.release();
         if (S.ev_ready) cudaEventDestroy(S.ev_ready);
         if (S.ev_free) cudaEventDestroy(S.ev_free);
@@ -1014,7 +1007,6 @@ extern "C" int gg_set_precision(gg_gridder *h, int precision)
             GG_CK(cudaStreamSynchronize(h->cs));
             h->prec = precision;
             h->cas_fp_valid = false;
-            for (auto &S : h->slot) S.casimg_lp.release();
         }
     });
 }
@@ -1027,7 +1019,6 @@ extern "C" int gg_set_image_precision(gg_gridder *h, int precision)
         if (precision != h->img_prec_set) {
             GG_CK(cudaStreamSynchronize(h->cs));
             h->img_prec_set = precision;
-            for (auto &S : h->slot) S.casimg_lp.release();
         }
     });
 }
@@ -1499,7 +1490,7 @@ extern "C" int gg_back_project_kernel(float *d_cas_volume, const float *d_cas_im
         return GG_ERR_INVALID_ARG;
     }
     Geom g{cas_vol_size, cas_img_size, mask_radius, kb_table_size, ker_hwidth};
-    cudaError_t e = launch_back_project_ref(d_cas_volume, d_cas_images, kF32, false, d_kb_table, d_axes, n_axes, g, nullptr,
+    cudaError_t e = launch_back_project_ref(d_cas_volume, d_cas_images, false, d_kb_table, d_axes, n_axes, g, nullptr,
                                             (cudaStream_t)stream);
     if (e != cudaSuccess) {
         g_global_err = cudaGetErrorString(e);
@@ -1524,7 +1515,7 @@ extern "C" int gg_back_project_adjoint_kernel(float *d_cas_volume, const float *
     }
     Geom g{cas_vol_size, cas_img_size, mask_radius, kb_table_size, ker_hwidth};
     // zero table edges were checked above
-    cudaError_t e = launch_back_project_adjoint(d_cas_volume, cas_vol_size, d_cas_images, kF32, d_kb_table, d_axes, n_axes,
+    cudaError_t e = launch_back_project_adjoint(d_cas_volume, cas_vol_size, d_cas_images, d_kb_table, d_axes, n_axes,
                                                 g, nullptr, (cudaStream_t)stream);
     if (e != cudaSuccess) {
         g_global_err = cudaGetErrorString(e);

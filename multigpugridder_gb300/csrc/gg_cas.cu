@@ -421,11 +421,11 @@ __global__ void divide_plane_density_kernel(float *__restrict__ a, const float *
 }
 
 template <typename T>
-__global__ void convert_kernel(const float *__restrict__ in, T *__restrict__ out, size_t count, const float *__restrict__ d_scale)
+__global__ void round_kernel(const float *in, float *out, size_t count, const float *__restrict__ d_scale)
 {
     const float inv_scale = d_scale ? 1.0f / *d_scale : 1.0f;
     for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < count; e += (size_t)gridDim.x * blockDim.x)
-        out[e] = from_f32<T>(in[e] * inv_scale);
+        out[e] = from_f32<Rounded<T>>(in[e] * inv_scale).v;
 }
 
 // Rows of the dense FP32 volume -> rows of pitch P (even) in storage T.  Bound:
@@ -652,18 +652,19 @@ cudaError_t launch_images_to_fft_input(const float *d_img, int N, int M, int n, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_spectrum_to_cas_images(const cufftComplex *d_spec, int M, int n, void *d_cas, int prec,
+cudaError_t launch_spectrum_to_cas_images(const cufftComplex *d_spec, int M, int n, float *d_cas, int prec,
                                           const float *d_scale, cudaStream_t s)
 {
     if (n <= 0) return cudaSuccess;
     const dim3 g = row_grid(M, n), b(kRowX, kRowY);
     if (prec == kF32)
-        spectrum_to_cas_images_kernel<float, false><<<g, b, 0, s>>>(d_spec, M, n, (float *)d_cas, d_scale, 1.0f);
+        spectrum_to_cas_images_kernel<float, false><<<g, b, 0, s>>>(d_spec, M, n, d_cas, d_scale, 1.0f);
     else if (prec == kF16)
-        spectrum_to_cas_images_kernel<__half, false><<<g, b, 0, s>>>(d_spec, M, n, (__half *)d_cas, d_scale, 1.0f);
+        spectrum_to_cas_images_kernel<Rounded<__half>, false><<<g, b, 0, s>>>(d_spec, M, n, (Rounded<__half> *)d_cas,
+                                                                              d_scale, 1.0f);
     else
-        spectrum_to_cas_images_kernel<__nv_bfloat16, false><<<g, b, 0, s>>>(d_spec, M, n, (__nv_bfloat16 *)d_cas,
-                                                                             d_scale, 1.0f);
+        spectrum_to_cas_images_kernel<Rounded<__nv_bfloat16>, false><<<g, b, 0, s>>>(
+            d_spec, M, n, (Rounded<__nv_bfloat16> *)d_cas, d_scale, 1.0f);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -712,12 +713,11 @@ cudaError_t launch_divide_plane_density(float *d_a, const float *d_b, size_t cou
     return cudaGetLastError();
 }
 
-cudaError_t launch_convert(const float *d_in, void *d_out, int prec, size_t count, const float *d_scale, cudaStream_t s)
+cudaError_t launch_round(const float *d_in, float *d_out, int prec, size_t count, const float *d_scale, cudaStream_t s)
 {
     const unsigned g = grid_for(count, kT);
-    if (prec == kF32) convert_kernel<float><<<g, kT, 0, s>>>(d_in, (float *)d_out, count, d_scale);
-    else if (prec == kF16) convert_kernel<__half><<<g, kT, 0, s>>>(d_in, (__half *)d_out, count, d_scale);
-    else convert_kernel<__nv_bfloat16><<<g, kT, 0, s>>>(d_in, (__nv_bfloat16 *)d_out, count, d_scale);
+    if (prec == kF16) round_kernel<__half><<<g, kT, 0, s>>>(d_in, d_out, count, d_scale);
+    else round_kernel<__nv_bfloat16><<<g, kT, 0, s>>>(d_in, d_out, count, d_scale);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -22,4 +22,19 @@ template <> __device__ __forceinline__ float from_f32<float>(float x) { return x
 template <> __device__ __forceinline__ __half from_f32<__half>(float x) { return __float2half_rn(x); }
 template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float x) { return __float2bfloat16_rn(x); }
 
+// A value rounded to a 2-byte type and held in FP32 (CAS images of reduced
+// precision: the back projection copies FP32 footprints asynchronously, where
+// 2-byte ones passed through registers to be widened).
+template <typename T> struct Rounded {
+    float v;
+};
+template <> __device__ __forceinline__ Rounded<__half> from_f32<Rounded<__half>>(float x)
+{
+    return Rounded<__half>{__half2float(__float2half_rn(x))};
+}
+template <> __device__ __forceinline__ Rounded<__nv_bfloat16> from_f32<Rounded<__nv_bfloat16>>(float x)
+{
+    return Rounded<__nv_bfloat16>{__bfloat162float(__float2bfloat16_rn(x))};
+}
+
 } // namespace gg

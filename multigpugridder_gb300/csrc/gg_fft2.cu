@@ -473,15 +473,15 @@ static cudaError_t launch_fwd_t(const float *d_img, int N, int n, T *d_cas, floa
 }
 
 template <int M>
-static cudaError_t launch_fwd_m(const float *d_img, int N, int n, void *d_cas, int prec, bool adjoint, cudaStream_t s)
+static cudaError_t launch_fwd_m(const float *d_img, int N, int n, float *d_cas, int prec, bool adjoint, cudaStream_t s)
 {
     const float post = 1.0f / ((float)M * (float)M);
-    if (adjoint) return launch_fwd_t<M, float, true>(d_img, N, n, (float *)d_cas, post, s);
-    if (prec == kBF16) return launch_fwd_t<M, __nv_bfloat16, false>(d_img, N, n, (__nv_bfloat16 *)d_cas, 1.0f, s);
-    return launch_fwd_t<M, float, false>(d_img, N, n, (float *)d_cas, 1.0f, s);
+    if (adjoint) return launch_fwd_t<M, float, true>(d_img, N, n, d_cas, post, s);
+    if (prec == kBF16) return launch_fwd_t<M, Rounded<__nv_bfloat16>, false>(d_img, N, n, (Rounded<__nv_bfloat16> *)d_cas, 1.0f, s);
+    return launch_fwd_t<M, float, false>(d_img, N, n, d_cas, 1.0f, s);
 }
 
-cudaError_t launch_images_to_cas_fused(const float *d_img, int N, int M, int n, void *d_cas, int prec, bool adjoint,
+cudaError_t launch_images_to_cas_fused(const float *d_img, int N, int M, int n, float *d_cas, int prec, bool adjoint,
                                        cudaStream_t s)
 {
     if (n <= 0) return cudaSuccess;

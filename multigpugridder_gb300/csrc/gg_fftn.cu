@@ -618,8 +618,8 @@ bool fftn_ok(int N, int M)
 // A volume's three passes against the library's 3-D transform and its two stage
 // kernels (setVolume and 16 projections, us): M = 64: 41 (39), 96: 61 (63), 192:
 // 127 (142), 200: 139 (177), 256: 215 (235), 320: 354 (502), 384: 597 (789), 400: 695
-// (1166), 448: 960 (1450), 500: 1396 (1722), 512 in BF16: 1228 (1347).  Above 400 in
-// tiles of 8 lines, which leave room for two an SM.
+// (1166), 448: 960 (1450), 500: 1396 (1722).  Above 400 in tiles of 8 lines,
+// which leave room for two an SM.
 constexpr int kFnMinVolM = 96, kFnMaxVolM = 512;
 
 bool fftn_volume_ok(int N, int M)
@@ -689,17 +689,17 @@ static cudaError_t images_to_cas_t(const FnPlan &p, const float2 *d_tw, const fl
                         StoreCasCols<C, T, ADJ>{d_cas, M, post, top}, s);
 }
 
-cudaError_t launch_images_to_cas_passes(const float *d_img, int N, int M, int n, void *d_cas, int prec, bool adjoint,
+cudaError_t launch_images_to_cas_passes(const float *d_img, int N, int M, int n, float *d_cas, int prec, bool adjoint,
                                         const float2 *d_tw, float2 *d_half, unsigned *top, cudaStream_t s)
 {
     FnPlan p;
     if (!fftn_ok(N, M) || !fn_plan(M, p) || prec == kF16 || (adjoint && prec != kF32)) return cudaErrorInvalidValue;
     const float post = 1.0f / ((float)M * (float)M);
-    if (adjoint) return images_to_cas_t<kFnC, float, true>(p, d_tw, d_img, N, n, (float *)d_cas, post, d_half, top, s);
+    if (adjoint) return images_to_cas_t<kFnC, float, true>(p, d_tw, d_img, N, n, d_cas, post, d_half, top, s);
     if (prec == kBF16)
-        return images_to_cas_t<kFnC, __nv_bfloat16, false>(p, d_tw, d_img, N, n, (__nv_bfloat16 *)d_cas, 1.0f, d_half, top,
-                                                           s);
-    return images_to_cas_t<kFnC, float, false>(p, d_tw, d_img, N, n, (float *)d_cas, 1.0f, d_half, top, s);
+        return images_to_cas_t<kFnC, Rounded<__nv_bfloat16>, false>(p, d_tw, d_img, N, n, (Rounded<__nv_bfloat16> *)d_cas, 1.0f,
+                                                                   d_half, top, s);
+    return images_to_cas_t<kFnC, float, false>(p, d_tw, d_img, N, n, d_cas, 1.0f, d_half, top, s);
 }
 
 cudaError_t launch_cas_to_images_passes(const float *d_cas, int M, int N, int n, float *d_img, const float2 *d_tw,

@@ -79,20 +79,19 @@ struct BpSplit {
 int bp_segments(int n, const Geom &g);
 
 // Back projection with the reference window rule, accumulated (+=) into the
-// FP32 CAS volume.  d_img holds n*M*M CAS images in storage `iprec`; when
-// `ones` is set the images are taken to be all ones (plane density) and
+// FP32 CAS volume.  d_img holds n*M*M CAS images; when `ones` is set the images are taken to be all ones (plane density) and
 // d_img is not read.
 // *d_scale multiplies each voxel's sum before it is added.  shared: the GPU
 // runs other launches concurrently (smaller CTAs that share an SM; FP32
 // images, the same sums bit for bit).
-cudaError_t launch_back_project_ref(float *d_vol, const void *d_img, int iprec, bool ones,
+cudaError_t launch_back_project_ref(float *d_vol, const float *d_img, bool ones,
                                     const float *d_ker, const float *d_axes, int n, const Geom &g,
                                     const float *d_scale, cudaStream_t s, bool shared = false,
                                     BpSplit split = BpSplit());
 
 // Reference-rule back projection of d_img into d_vol and, in the same pass,
 // of all-ones images (the plane density) into d_pd; both accumulated.
-cudaError_t launch_back_project_ref_density(float *d_vol, float *d_pd, const void *d_img, int iprec,
+cudaError_t launch_back_project_ref_density(float *d_vol, float *d_pd, const float *d_img,
                                             const float *d_ker, const float *d_axes, int n, const Geom &g,
                                             const float *d_scale, cudaStream_t s, BpSplit split = BpSplit());
 
@@ -106,7 +105,7 @@ cudaError_t launch_back_project_ref_pair(float *d_vol, float *d_pd, const float 
 // Exact adjoint of the 4-tap forward projection (gg_adjoint.cu), added to
 // d_vol, rows `pitch` floats apart (planes pitch * V; dense: pitch = V).  The
 // KB table's first and last entries are 0.
-cudaError_t launch_back_project_adjoint(float *d_vol, int pitch, const void *d_img, int iprec, const float *d_ker,
+cudaError_t launch_back_project_adjoint(float *d_vol, int pitch, const float *d_img, const float *d_ker,
                                         const float *d_axes, int n, const Geom &g, const float *d_scale,
                                         cudaStream_t s);
 
@@ -135,8 +134,8 @@ cudaError_t launch_fft_output_to_images(const float *d_y, int M, int N, int n, f
 // Images n*N*N -> R2C inputs n*M*M (centred zero-pad, shift).
 cudaError_t launch_images_to_fft_input(const float *d_img, int N, int M, int n, float *d_x,
                                        cudaStream_t s);
-// R2C half spectra n*M*(M/2+1) -> CAS images n*M*M (shift, Re+Im) in storage `prec`.
-cudaError_t launch_spectrum_to_cas_images(const cufftComplex *d_spec, int M, int n, void *d_cas,
+// R2C half spectra n*M*(M/2+1) -> CAS images n*M*M (shift, Re+Im) rounded to `prec`.
+cudaError_t launch_spectrum_to_cas_images(const cufftComplex *d_spec, int M, int n, float *d_cas,
                                           int prec, const float *d_scale, cudaStream_t s);
 // Adjoint of the whole forward operator (volume -> images), by stage:
 // R2C half spectra of padded, shifted image gradients -> CAS-image gradients
@@ -153,9 +152,9 @@ cudaError_t launch_fill(float *d, size_t count, float value, cudaStream_t s);
 // a = a / (b + eps) over `count` elements (reconstructVol's plane-density division).
 cudaError_t launch_divide_plane_density(float *d_a, const float *d_b, size_t count, float eps,
                                         cudaStream_t s);
-// FP32 -> storage conversion (count elements): out = in / *d_scale.
-cudaError_t launch_convert(const float *d_in, void *d_out, int prec, size_t count, const float *d_scale,
-                           cudaStream_t s);
+// out = in / *d_scale rounded to the 2-byte type prec, in FP32 (count elements;
+// out may be in).
+cudaError_t launch_round(const float *d_in, float *d_out, int prec, size_t count, const float *d_scale, cudaStream_t s);
 // *d_scale = smallest power of two >= max|x| / target (at least 1) over
 // `count` floats; d_work is one scratch unsigned int.
 cudaError_t launch_storage_scale(const float *d_x, size_t count, float target, unsigned int *d_work,
@@ -184,11 +183,11 @@ cudaError_t launch_ctf(float *d_mul, int mul_power, float *d_gen, int gen_power,
 // True when N, M take the fused kernels: M in {64, 128, 256}, N <= M/2, N a
 // multiple of M/16, and the shared memory fits.
 bool fft2_fused_ok(int N, int M);
-// Images n*N*N -> CAS images n*M*M in storage `prec` (FP32 or BF16; FP16
+// Images n*N*N -> CAS images n*M*M rounded to `prec` (FP32 or BF16; FP16
 // needs the spectrum's scale first and is refused), in one launch: the pad,
 // shifts, forward 2-D FFT and Re+Im of the path above.  adjoint: the gradient
 // form of launch_spectrum_to_cas_images_adjoint (FP32 only).
-cudaError_t launch_images_to_cas_fused(const float *d_img, int N, int M, int n, void *d_cas, int prec, bool adjoint,
+cudaError_t launch_images_to_cas_fused(const float *d_img, int N, int M, int n, float *d_cas, int prec, bool adjoint,
                                        cudaStream_t s);
 // CAS images n*M*M (FP32) -> images n*N*N in one launch: FromCAS, shifts,
 // inverse 2-D FFT, crop and 1/M^2.
@@ -206,7 +205,7 @@ void fftn_twiddles(int M, float2 *out);
 // The two directions of the fused stages above, in two launches each through
 // d_half (n * N * (M/2 + 1) values).  top (optional, images -> CAS images): the
 // bits of the largest magnitude, added by atomicMax to a zeroed word.
-cudaError_t launch_images_to_cas_passes(const float *d_img, int N, int M, int n, void *d_cas, int prec, bool adjoint,
+cudaError_t launch_images_to_cas_passes(const float *d_img, int N, int M, int n, float *d_cas, int prec, bool adjoint,
                                         const float2 *d_tw, float2 *d_half, unsigned *top, cudaStream_t s);
 cudaError_t launch_cas_to_images_passes(const float *d_cas, int M, int N, int n, float *d_img, const float2 *d_tw,
                                         float2 *d_half, cudaStream_t s);

@@ -80,7 +80,7 @@ extern "C" int gg_back_project_normalized_noalloc(float *d_cas_volume_out, const
     cudaError_t e = launch_fill(pd, V3, 0.0f, s);
     if (e == cudaSuccess) e = launch_fill(d_cas_volume_out, V3, 0.0f, s);
     if (e == cudaSuccess && n_axes > 0)
-        e = launch_back_project_ref_density(d_cas_volume_out, pd, d_cas_images, kF32, d_kb_table, d_axes, n_axes, g,
+        e = launch_back_project_ref_density(d_cas_volume_out, pd, d_cas_images, d_kb_table, d_axes, n_axes, g,
                                             nullptr, s);
     // tmpCASVolume ./ (PlaneDensity + 1e-6) (MultiGPUGridder_Matlab_Class.m:308)
     if (e == cudaSuccess) e = launch_divide_plane_density(d_cas_volume_out, pd, V3, 1e-6f, s);

@@ -252,8 +252,8 @@ __device__ __forceinline__ float ref_pixel_pos(float pi, float pj, float n_x, fl
 // linear-index test always passes.  Table entry k is read at sker[k * rep].
 // DW: cumW sums img2 * w (a second image back-projected in the same pass,
 // fused as cumSum is) instead of w.
-template <typename TI, bool ONES, bool DENS, bool INSIDE, bool DW = false>
-__device__ __forceinline__ void ref_window(const RefWindow &q, const float *sker, int rep, const TI *__restrict__ img_ptr,
+template <bool ONES, bool DENS, bool INSIDE, bool DW = false>
+__device__ __forceinline__ void ref_window(const RefWindow &q, const float *sker, int rep, const float *__restrict__ img_ptr,
                                            int M, int imgi, int imgj, int imgCenter, float &cumSum, float &cumW,
                                            const float *__restrict__ img2_ptr = nullptr)
 {
@@ -357,16 +357,7 @@ struct BpTable {
     unsigned magic_bits; // its bits: entry floor(P y) sits at bits(y + magic) - magic_bits
 };
 
-// A 2-byte value held in the low 16 bits of u, widened to FP32 exactly.
-template <typename T> __device__ __forceinline__ float widen16(unsigned u);
-template <> __device__ __forceinline__ float widen16<__nv_bfloat16>(unsigned u) { return __uint_as_float(u << 16); }
-template <> __device__ __forceinline__ float widen16<__half>(unsigned u)
-{
-    return __half2float(__ushort_as_half((unsigned short)u));
-}
-template <> __device__ __forceinline__ float widen16<float>(unsigned u) { return __uint_as_float(u); }
-
-// Four consecutive values from a 4-element-aligned address, as FP32.
+// Four consecutive values from a 4-element-aligned address.
 __device__ __forceinline__ void ld_quad(const float *p, float (&v)[4])
 {
     const float4 q = __ldg(reinterpret_cast<const float4 *>(p));
@@ -375,16 +366,6 @@ __device__ __forceinline__ void ld_quad(const float *p, float (&v)[4])
     v[2] = q.z;
     v[3] = q.w;
 }
-template <typename T>
-__device__ __forceinline__ void ld_quad(const T *p, float (&v)[4])
-{
-    const uint2 w = __ldg(reinterpret_cast<const uint2 *>(p));
-    v[0] = widen16<T>(w.x & 0xffffu);
-    v[1] = widen16<T>(w.x >> 16);
-    v[2] = widen16<T>(w.y & 0xffffu);
-    v[3] = widen16<T>(w.y >> 16);
-}
-
 __device__ __forceinline__ float lds_f32(unsigned addr)
 {
     float v;
@@ -685,10 +666,10 @@ __device__ __forceinline__ void cp_async_wait()
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-template <typename TI, bool ONES, bool DENS, bool DW = false, bool DEEP = false, int G = kBpGroups,
+template <bool ONES, bool DENS, bool DW = false, bool DEEP = false, int G = kBpGroups,
           int TS = 0, bool LEAN = true, bool SPLIT = false>
 __global__ void __launch_bounds__(kCThreads *G, G == 1 ? 3 : 1)
-bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, const TI *__restrict__ img, int M,
+bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, const float *__restrict__ img, int M,
                       const float *__restrict__ axes, int n, int maskR, const float *__restrict__ ker, int kerSize,
                       float kerHW, int bricksX, int bricksY, BpTable tb,
                       const float *__restrict__ d_scale, const float *__restrict__ img2, int vecImg, BpSplit split,
@@ -783,7 +764,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
         // footprint, or the reference's window from the image.
         auto voxel_window = [&](const int l, const float nx0, const float nx1, const float nx2, const float ny0,
                                 const float ny1, const float ny2, const int fi0, const int fj0, const int fh,
-                                const bool foot, const TI *img_ptr, const float *img2_ptr, const float *wfoot,
+                                const bool foot, const float *img_ptr, const float *img2_ptr, const float *wfoot,
                                 const float *wfoot2, float &cs, float &cw) {
             const int vi = bx + (l & 7), vj = by + ((l >> 3) & 3), vk = bz + (l >> 5);
             const float a0 = (float)vi - volCenter, a1 = (float)vj - volCenter, a2 = (float)vk - volCenter;
@@ -809,10 +790,10 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                 const RefWindow rw{nx0, nx1, nx2, ny0, ny1, ny2, (float)vi, (float)vj, (float)vk,
                                    (float)volCenter, kerScale, kerCenterHalf};
                 if (inside)
-                    ref_window<TI, ONES, DENS, true, DW>(rw, sker, cp, img_ptr, M, imgi, imgj, imgCenter, cs, cw,
+                    ref_window<ONES, DENS, true, DW>(rw, sker, cp, img_ptr, M, imgi, imgj, imgCenter, cs, cw,
                                                          img2_ptr);
                 else
-                    ref_window<TI, ONES, DENS, false, DW>(rw, sker, cp, img_ptr, M, imgi, imgj, imgCenter, cs, cw,
+                    ref_window<ONES, DENS, false, DW>(rw, sker, cp, img_ptr, M, imgi, imgj, imgCenter, cs, cw,
                                                           img2_ptr);
             }
         };
@@ -902,7 +883,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                 // has in the queue (at its front), run before b is refilled.
                 const int b = NB > 1 ? nbuf : 0;
                 if (NB > 1) {
-                    if (QALIGN && sizeof(TI) == 4 && !ONES) {
+                    if (QALIGN && !ONES) {
                         cp_async_wait();
                         __syncwarp(); // the footprints' copies are complete, for every lane
                     }
@@ -930,7 +911,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                 float *const wfoot2 = wfoot20 + (DW ? b * (FH * FS) : 0);
                 const float nx0 = ax[0], nx1 = ax[1], nx2 = ax[2];
                 const float ny0 = ax[3], ny1 = ax[4], ny2 = ax[5];
-                const TI *img_ptr = img + (size_t)(c0 + al) * MM;
+                const float *img_ptr = img + (size_t)(c0 + al) * MM;
                 const float *img2_ptr = DW ? img2 + (size_t)(c0 + al) * MM : nullptr;
                 // this warp's footprint (uniform across the warp)
                 int fi0 = 0, fj0 = 0, fh = 0;
@@ -954,7 +935,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                         constexpr int NQ = FW / 4 + 1; // quads per footprint row
                         const int base = fi0 & ~3, sh = fi0 & 3;
                         const int first = fj0 * M + base, nq = fh * NQ;
-                        if constexpr (QALIGN && sizeof(TI) == 4) {
+                        if constexpr (QALIGN) {
                             if (first >= 0 && first + (fh - 1) * M + 4 * NQ <= MM) {
                                 // no pixel outside the image's index range: quad t of
                                 // the footprint lies at its word 4 t (FS = 4 NQ).
@@ -1007,37 +988,11 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                                 if (t < nq) {
                                     const int r = t / NQ, qq = t - r * NQ;
                                     const int c0 = 4 * qq - sh; // footprint column of the quad's first pixel
-                                    if (QALIGN) {
-                                        *reinterpret_cast<float4 *>(wfoot + r * FS + 4 * qq) =
-                                            make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
-                                    } else {
 #pragma unroll
-                                        for (int e = 0; e < 4; e++)
-                                            if (c0 + e >= 0 && c0 + e < FW) wfoot[r * FS + c0 + e] = v[u][e];
-                                    }
+                                    for (int e = 0; e < 4; e++)
+                                        if (c0 + e >= 0 && c0 + e < FW) wfoot[r * FS + c0 + e] = v[u][e];
                                 }
                             }
-                        }
-                    } else if (foot && sizeof(TI) == 2 && !ONES && !(M & 1)) {
-                        // the same with 4-byte pixel pairs when only 2 divides M
-                        constexpr int NPR = FW / 2 + 1; // pairs per footprint row
-                        const int base = fi0 & ~1, odd = fi0 & 1;
-                        for (int t = lane; t < fh * NPR; t += 32) {
-                            const int r = t / NPR, pp = t - r * NPR;
-                            const int c0 = 2 * pp - odd; // footprint column of the pair's first pixel
-                            const int lin0 = (fj0 + r) * M + base + 2 * pp;
-                            float v0 = 0.0f, v1 = 0.0f;
-                            if (lin0 >= 0 && lin0 + 1 < MM) {
-                                const unsigned w = __ldg(reinterpret_cast<const unsigned *>(img_ptr + lin0));
-                                v0 = widen16<TI>(w & 0xffffu);
-                                v1 = widen16<TI>(w >> 16);
-                            } else {
-                                if (lin0 >= 0 && lin0 < MM) v0 = ld_f32(img_ptr + lin0);
-                                if (lin0 + 1 >= 0 && lin0 + 1 < MM) v1 = ld_f32(img_ptr + lin0 + 1);
-                            }
-                            const int ash = QALIGN ? (fi0 & 3) : 0;
-                            if (c0 >= 0 && c0 < FW) wfoot[r * FS + c0 + ash] = v0;
-                            if (c0 + 1 < FW) wfoot[r * FS + c0 + 1 + ash] = v1; // c0 + 1 >= 0
                         }
                     } else if (foot) {
                         // the reference's linear-index rule (gpuBackProject.cu:99)
@@ -1129,8 +1084,8 @@ bp_merge_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, int mask
     if (pd) pd[o] = d;
 }
 
-template <typename TI, bool ONES, bool DENS, bool DW, bool DEEP, int G>
-static cudaError_t launch_bp_compact_g(float *vol, const TI *img, const float *ker, const float *axes, int n,
+template <bool ONES, bool DENS, bool DW, bool DEEP, int G>
+static cudaError_t launch_bp_compact_g(float *vol, const float *img, const float *ker, const float *axes, int n,
                                        const Geom &g, const float *scale, cudaStream_t s, float *pd, const float *img2,
                                         int max_copies, BpSplit split)
 {
@@ -1147,7 +1102,7 @@ static cudaError_t launch_bp_compact_g(float *vol, const TI *img, const float *k
     if (tb.copies == 0) return cudaErrorInvalidValue; // a KB table too long for shared memory
     const size_t dyn = (((size_t)tb.entries * tb.copies + 3) & ~(size_t)3) * sizeof(float) + other;
     // quad loads of image rows: 4 | M and the stacks aligned to 4 elements
-    const size_t qa = 4 * sizeof(TI);
+    const size_t qa = 4 * sizeof(float);
     const int vec = (g.M % 4 == 0) && ((size_t)img % qa == 0) && (!img2 || (size_t)img2 % 16 == 0) ? 1 : 0;
     if (bz > kMaxLayers) return cudaErrorInvalidValue;
     BpLayers lay;
@@ -1184,16 +1139,16 @@ static cudaError_t launch_bp_compact_g(float *vol, const TI *img, const float *k
     if constexpr (LEAN) {
         if constexpr (!ONES) {
             if (split.nseg > 1) // bp_segments splits only tables that get 32 copies
-                return tb.copies == 32 ? go(bp_ref_compact_kernel<TI, ONES, DENS, DW, DEEP, G, 128, true, true>)
+                return tb.copies == 32 ? go(bp_ref_compact_kernel<ONES, DENS, DW, DEEP, G, 128, true, true>)
                                        : cudaErrorInvalidValue;
         }
-        if (tb.copies == 32) return go(bp_ref_compact_kernel<TI, ONES, DENS, DW, DEEP, G, 128, true>);
+        if (tb.copies == 32) return go(bp_ref_compact_kernel<ONES, DENS, DW, DEEP, G, 128, true>);
     }
-    return go(bp_ref_compact_kernel<TI, ONES, DENS, DW, DEEP, G, 0, LEAN>);
+    return go(bp_ref_compact_kernel<ONES, DENS, DW, DEEP, G, 0, LEAN>);
 }
 
-template <typename TI, bool ONES, bool DENS = false, bool DW = false, bool DEEP = false>
-static cudaError_t launch_bp_compact_t(float *vol, const TI *img, const float *ker, const float *axes, int n,
+template <bool ONES, bool DENS = false, bool DW = false, bool DEEP = false>
+static cudaError_t launch_bp_compact_t(float *vol, const float *img, const float *ker, const float *axes, int n,
                                        const Geom &g, const float *scale, cudaStream_t s, float *pd = nullptr,
                                        const float *img2 = nullptr, bool shared = false,
                                        BpSplit split = BpSplit())
@@ -1204,62 +1159,47 @@ static cudaError_t launch_bp_compact_t(float *vol, const TI *img, const float *k
     // other lanes can fill as they free (serving capacity 172 -> 195 req/s when
     // the rule was made); alone, 24 warps sharing 32 table copies (batched back
     // projection 78.5 -> 71.7 ms per 10k images then, 51 now).
-    if constexpr (std::is_same<TI, float>::value && !ONES && !DENS && !DW) {
+    if constexpr (!ONES && !DENS && !DW) {
         if (shared)
-            return launch_bp_compact_g<TI, ONES, DENS, DW, DEEP, 1>(vol, img, ker, axes, n, g, scale, s, pd,
+            return launch_bp_compact_g<ONES, DENS, DW, DEEP, 1>(vol, img, ker, axes, n, g, scale, s, pd,
                                                                          img2, 1, BpSplit());
     }
-    return launch_bp_compact_g<TI, ONES, DENS, DW, DEEP, kGroupsOf<DW, DEEP>>(vol, img, ker, axes, n, g, scale, s, pd,
+    return launch_bp_compact_g<ONES, DENS, DW, DEEP, kGroupsOf<DW, DEEP>>(vol, img, ker, axes, n, g, scale, s, pd,
                                                                          img2, 32, split);
 }
 
 // Reference-rule launch with the block depth chosen by the image size.
-template <typename TI, bool ONES, bool DENS>
-static cudaError_t launch_bp_ref_sized(float *vol, const TI *img, const float *ker, const float *axes, int n,
+template <bool ONES, bool DENS>
+static cudaError_t launch_bp_ref_sized(float *vol, const float *img, const float *ker, const float *axes, int n,
                                        const Geom &g, const float *scale, cudaStream_t s, float *pd, bool shared,
                                        BpSplit split)
 {
     if (g.M >= 512)
-        return launch_bp_compact_t<TI, ONES, DENS, false, true>(vol, img, ker, axes, n, g, scale, s, pd, nullptr,
+        return launch_bp_compact_t<ONES, DENS, false, true>(vol, img, ker, axes, n, g, scale, s, pd, nullptr,
                                                                  shared, split);
-    return launch_bp_compact_t<TI, ONES, DENS>(vol, img, ker, axes, n, g, scale, s, pd, nullptr, shared, split);
+    return launch_bp_compact_t<ONES, DENS>(vol, img, ker, axes, n, g, scale, s, pd, nullptr, shared, split);
 }
 
-cudaError_t launch_back_project_ref(float *d_vol, const void *d_img, int iprec, bool ones, const float *d_ker,
-                                    const float *d_axes, int n, const Geom &g, const float *scale, cudaStream_t s,
-                                    bool shared, BpSplit split)
+cudaError_t launch_back_project_ref(float *d_vol, const float *d_img, bool ones, const float *d_ker, const float *d_axes,
+                                    int n, const Geom &g, const float *scale, cudaStream_t s, bool shared, BpSplit split)
 {
     if (ones)
-        return launch_bp_ref_sized<float, true, false>(d_vol, nullptr, d_ker, d_axes, n, g, scale, s, nullptr, false, split);
-    if (iprec == kF32)
-        return launch_bp_ref_sized<float, false, false>(d_vol, (const float *)d_img, d_ker, d_axes, n, g, scale, s,
-                                                        nullptr, shared, split);
-    if (iprec == kF16)
-        return launch_bp_ref_sized<__half, false, false>(d_vol, (const __half *)d_img, d_ker, d_axes, n, g, scale, s,
-                                                         nullptr, false, split);
-    return launch_bp_ref_sized<__nv_bfloat16, false, false>(d_vol, (const __nv_bfloat16 *)d_img, d_ker, d_axes, n, g,
-                                                            scale, s, nullptr, false, split);
+        return launch_bp_ref_sized<true, false>(d_vol, nullptr, d_ker, d_axes, n, g, scale, s, nullptr, false, split);
+    return launch_bp_ref_sized<false, false>(d_vol, d_img, d_ker, d_axes, n, g, scale, s, nullptr, shared, split);
 }
 
-cudaError_t launch_back_project_ref_density(float *d_vol, float *d_pd, const void *d_img, int iprec, const float *d_ker,
+cudaError_t launch_back_project_ref_density(float *d_vol, float *d_pd, const float *d_img, const float *d_ker,
                                             const float *d_axes, int n, const Geom &g, const float *scale,
                                             cudaStream_t s, BpSplit split)
 {
-    if (iprec == kF32)
-        return launch_bp_ref_sized<float, false, true>(d_vol, (const float *)d_img, d_ker, d_axes, n, g, scale, s, d_pd,
-                                                       false, split);
-    if (iprec == kF16)
-        return launch_bp_ref_sized<__half, false, true>(d_vol, (const __half *)d_img, d_ker, d_axes, n, g, scale, s,
-                                                        d_pd, false, split);
-    return launch_bp_ref_sized<__nv_bfloat16, false, true>(d_vol, (const __nv_bfloat16 *)d_img, d_ker, d_axes, n, g,
-                                                           scale, s, d_pd, false, split);
+    return launch_bp_ref_sized<false, true>(d_vol, d_img, d_ker, d_axes, n, g, scale, s, d_pd, false, split);
 }
 
 cudaError_t launch_back_project_ref_pair(float *d_vol, float *d_pd, const float *d_img, const float *d_img2,
                                          const float *d_ker, const float *d_axes, int n, const Geom &g, cudaStream_t s,
                                          BpSplit split)
 {
-    return launch_bp_compact_t<float, false, false, true>(d_vol, d_img, d_ker, d_axes, n, g, nullptr, s, d_pd, d_img2,
+    return launch_bp_compact_t<false, false, true>(d_vol, d_img, d_ker, d_axes, n, g, nullptr, s, d_pd, d_img2,
                                                            false, split);
 }
 

@@ -158,6 +158,25 @@ def test_back_projection_segments(cuda, N, n):
         assert O.rel_l2(g.getCASVolume(), num / (den + np.float32(1e-6))) < TOL
 
 
+# CAS images rounded to 2 bytes and read as FP32: M a multiple of 4 and not
+@pytest.mark.parametrize("prec", ["bf16", "f16"])
+@pytest.mark.parametrize("N,interp", [(32, 2.0), (44, 1.5)])
+def test_reduced_cas_images(cuda, N, interp, prec):
+    import torch
+
+    import multigpugridder_gb300 as gg
+
+    p = O.Params(N, interp)
+    axes = O.quaternion_axes(7, seed=N).astype(np.float32)
+    ci = np.random.default_rng(N).standard_normal((7, p.M, p.M)).astype(np.float32)
+    # largest value about 5: FP16 is stored at scale 1
+    stored = torch.from_numpy(ci).to(torch.bfloat16 if prec == "bf16" else torch.float16).float().numpy()
+    ref = O.bp_ref_f32(stored, axes, p.V, p.mask_radius, p.ker)
+    with gg.MultiGPUGridder(N, 7, interpFactor=interp, precision=prec, adjustInterpFactor=False) as g:
+        g.backProjectCAS(ci, axes)
+        assert O.rel_l2(g.getCASVolume(), ref) < TOL
+
+
 # V = 10, 38, 106 (rows of 2 and of 4 floats), 41 (odd rows); a table too long
 # to be kept four times; boxes that do not fit and boxes of few voxels
 @pytest.mark.parametrize("N,interp,size,mask,scale",
