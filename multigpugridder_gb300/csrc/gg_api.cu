@@ -151,7 +151,7 @@ struct gg_gridder {
     int max_batch = 1024;
     bool fused_fft = false;     // fft2_fused_ok(N, M): the 2-D FFT stages run as one kernel each
     bool fft_passes = false;    // else fftn_ok(N, M): as two; else through cuFFT
-    bool vol_passes = false;    // fftn_volume_ok: setVolume's 3-D FFT as three pruned passes
+    bool vol_passes = false;    // fftn_volume_ok: setVolume's 3-D FFT as three pruned passes (FP32 storage)
     bool vol_back_passes = false; // fftn_volume_back_ok: getVolume's too
     int nstreams_fp = 2, nstreams_bp = 2;
     int prec = kF32;            // storage of the resident CAS volume the forward projection reads
@@ -365,7 +365,10 @@ void do_set_volume(gg_gridder *h, const float *d_vol, cudaStream_t s)
     const size_t V3 = (size_t)h->V * h->V * h->V;
     const size_t M3 = (size_t)h->M * h->M * h->M, H = h->M / 2 + 1;
     h->cas.ensure(V3);
-    if (h->vol_passes) {
+    // A 2-byte volume keeps the library's transform: few of its values carry the
+    // images, and one of them that falls the other way for another transform's
+    // last bit moves them by up to 3e-5 (BF16, 108 random cases; 9e-6 in FP16).
+    if (h->vol_passes && h->prec == kF32) {
         ensure_vol(h);
         GG_CK(launch_volume_to_cas_passes(d_vol, h->N, h->M, h->V, h->precomp.p, h->cas.p, h->tw.p, (float2 *)h->x3.p,
                                           (float2 *)h->spec3.p, s));
@@ -464,13 +467,15 @@ void bp_batch(gg_gridder *h, const float *d_axes, int b, const float *img, const
         } else if (h->fused_fft && ip != kF16) {
             GG_CK(launch_images_to_cas_fused(img, h->N, h->M, b, S.casimg.p, ip, false, s));
             src = S.casimg.p;
-        } else if (h->fft_passes && ip != kF16) {
+        } else if (h->fft_passes && ip == kF32) {
             GG_CK(launch_images_to_cas_passes(img, h->N, h->M, b, S.casimg.p, ip, false, h->tw.p, (float2 *)S.spec.p, nullptr,
                                               s));
             src = S.casimg.p;
-        } else if (h->fft_passes) {
-            // FP16: FP32 CAS images with their largest magnitude, then the
-            // storage scale and the rounding
+        } else if (h->fft_passes && ip == kF16) {
+            // FP32 CAS images with their largest magnitude, then the storage
+            // scale and the rounding.  BF16 images keep the library's transform:
+            // of values this coarsely rounded, some 1 in 5,000 lies where another
+            // transform's last bit decides (1.8e-5 of a reconstruction; FP16 6e-6)
             GG_CK(launch_images_to_cas_passes(img, h->N, h->M, b, S.casimg.p, kF32, false, h->tw.p, (float2 *)S.spec.p,
                                               h->work.p, s));
             GG_CK(launch_scale_from_max(h->work.p, 8192.0f, h->scales.p + 1, s));
@@ -1007,6 +1012,8 @@ extern "C" int gg_set_precision(gg_gridder *h, int precision)
             GG_CK(cudaStreamSynchronize(h->cs));
             h->prec = precision;
             h->cas_fp_valid = false;
+            // setVolume now needs the plan that its passes did without
+            if (precision != kF32 && h->vol_passes && h->x3.p) plan3(h, true);
         }
     });
 }
