@@ -101,7 +101,8 @@ adjoint_tile_kernel(float *__restrict__ vol, int V, int P, const float *__restri
     const unsigned tab_step = 4u * (unsigned)rep; // bytes between entries
     const unsigned box_addr = (unsigned)__cvta_generic_to_shared(box);
     const float scale = d_scale ? *d_scale : 1.0f;
-    const int ic = M / 2, vc = V / 2, R2 = maskR * maskR;
+    const int ic = M / 2, vc = V / 2;
+    const long long R2 = (long long)maskR * maskR; // a caller's radius may be any int
     const float kerCenter = ((float)kerSize - 1) / 2, kerScale = kerCenter / kerHW, kerCenterHalf = kerCenter + 0.5f;
     const unsigned tab_base = (unsigned)__cvta_generic_to_shared(sker) - __float_as_uint(12582912.0f) * tab_step;
     const int per = tilesX * tilesX;
@@ -114,7 +115,7 @@ adjoint_tile_kernel(float *__restrict__ vol, int V, int P, const float *__restri
         {   // the tile's nearest pixel to the centre is outside the mask: none is inside
             const int dia = i0 - ic, dib = dia + kAdjTile - 1, dja = j0 - ic, djb = dja + kAdjTile - 1;
             const int ni = dia > 0 ? dia : dib < 0 ? dib : 0, nj = dja > 0 ? dja : djb < 0 ? djb : 0;
-            if (ni * ni + nj * nj > R2) continue;
+            if ((long long)ni * ni + (long long)nj * nj > R2) continue;
         }
         const float *ax = axes + 9 * (size_t)a;
         const float *im = img + (size_t)a * M * M;
@@ -128,7 +129,7 @@ adjoint_tile_kernel(float *__restrict__ vol, int V, int P, const float *__restri
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const int i = i0 + (lane & 7), j = j0 + (lane >> 3) + 4 * h, di = i - ic, dj = j - ic;
-            on[h] = i < M && j < M && di * di + dj * dj <= R2;
+            on[h] = i < M && j < M && (long long)di * di + (long long)dj * dj <= R2;
             val[h] = on[h] ? ld_f32(im + (size_t)j * M + i) * scale : 0.0f;
             f[h][0] = sample_coord(nx0, ny0, di, dj, vc);
             f[h][1] = sample_coord(nx1, ny1, di, dj, vc);

@@ -199,6 +199,27 @@ def test_adjoint_boxes(cuda, gglib, N, interp, size, mask, scale):
     assert O.rel_l2(vol.cpu().numpy(), ref) < 1e-3
 
 
+# radii meant as "no mask": the square fits 31 bits for 46340 and not for the
+# others (65536 squared is 0 in 32 bits, 2^31 - 1 squared 1)
+@pytest.mark.parametrize("radius", [32, 46340, 46341, 60000, 65536, 2**31 - 1])
+def test_adjoint_large_radius(cuda, gglib, radius):
+    import torch
+
+    p = O.Params(16)
+    n = 5
+    axes = O.quaternion_axes(n, seed=7).astype(np.float32)
+    y = np.random.default_rng(8).standard_normal((n, p.M, p.M)).astype(np.float32)
+    d = np.arange(p.M) - p.M // 2
+    y[:, d[:, None]**2 + d**2 > p.mask_radius**2] = 0  # windows that stay in the volume
+    vol = torch.zeros((p.V,) * 3, device=cuda)
+    d_ker, d_axes, d_y = to_dev(p.ker, cuda), to_dev(axes, cuda), to_dev(y, cuda)
+    assert gglib.gg_back_project_adjoint_kernel(dptr(vol), dptr(d_y), dptr(d_ker), dptr(d_axes), 2.0, n, p.V, p.M, radius,
+                                                len(p.ker), None) == 0
+    torch.cuda.synchronize()
+    ref = O.bp_adjoint_f64(y.astype(np.float64), axes, p.V, p.mask_radius, p.ker)
+    assert O.rel_l2(vol.cpu().numpy(), ref) < 1e-3
+
+
 # enough images for blocks of 64 rows (1024 of them), also with a remainder, and one too few
 @pytest.mark.parametrize("M,n", [(64, 1100), (100, 520), (64, 1000)])
 def test_ctf_row_blocks(cuda, gglib, M, n):
