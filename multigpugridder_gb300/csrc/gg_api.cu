@@ -164,12 +164,15 @@ struct gg_gridder {
     DevBuf<float> ker;
     DevBuf<float2> precomp;  // FP64 factors as float pairs
     DevBuf<float> cas;       // FP32 CAS volume V^3 (resident)
-    DevBuf<unsigned char> cas_fp; // the copy the forward projection reads: storage `prec`, row
-                                  // pitch fp_pitch(V, prec) (FP16 scaled by scales[0])
-    DevBuf<unsigned char> fp_maps; // its tensor maps (gg_fp_tile.cu)
-    const void *fp_maps_vol = nullptr; // the copy's address and storage they were made for
-    int fp_maps_prec = -1;
-    bool cas_fp_valid = false;  // cas_fp matches cas
+    // The copies the forward projection reads, by element size: FP32, and the
+    // 2-byte types (FP16 scaled by scales[0]); row pitch fp_pitch(V, prec).  Each
+    // keeps its place and its tensor maps (gg_fp_tile.cu) for the handle's
+    // life: maps that a launch has used are never written again.
+    struct FpCopy {
+        DevBuf<unsigned char> vol, maps;
+        bool mapped = false;
+    } fp_copy[2];
+    bool cas_fp_valid = false;  // the copy of storage `prec` matches cas
     int *fault = nullptr;       // pinned: set by a kernel whose copies did not arrive
     DevBuf<float> pd;        // plane density V^3
     DevBuf<float> bp_part;   // sums of a split back projection's segments
@@ -206,6 +209,8 @@ struct gg_gridder {
     cufftHandle plan3_r2c = 0, plan3_c2r = 0;
     bool have3_r2c = false, have3_c2r = false;
 
+    FpCopy &fp() { return fp_copy[prec == kF32 ? 0 : 1]; }
+    const FpCopy &fp() const { return fp_copy[prec == kF32 ? 0 : 1]; }
     Geom geom() const { return Geom{V, M, mask_radius, ker_size, ker_hw}; }
     const float *vol_scale() const { return prec == kF16 ? scales.p : nullptr; }
     int img_prec() const { return img_prec_set < 0 ? prec : img_prec_set; }
@@ -332,22 +337,21 @@ void update_fp(gg_gridder *h, cudaStream_t s)
         *h->fault = 0;
     }
     const size_t V = h->V, P = fp_pitch(h->V, h->prec);
-    h->cas_fp.ensure(P * V * V * prec_bytes(h->prec));
-    if (h->fp_maps_vol != h->cas_fp.p || h->fp_maps_prec != h->prec) {
-        h->fp_maps.ensure(fp_tile_map_bytes(h->prec));
-        h->fp_maps_prec = -1;
-        GG_CK(fp_tile_make_maps(h->cas_fp.p, h->V, (int)P, h->prec, h->fp_maps.p, s));
-        h->fp_maps_vol = h->cas_fp.p;
-        h->fp_maps_prec = h->prec;
+    auto &c = h->fp();
+    c.vol.ensure(P * V * V * prec_bytes(h->prec));
+    if (!c.mapped) {
+        c.maps.ensure(fp_tile_map_bytes(h->prec));
+        GG_CK(fp_tile_make_maps(c.vol.p, h->V, (int)P, h->prec, c.maps.p, s));
+        c.mapped = true;
     }
     if (h->prec == kF16) GG_CK(launch_storage_scale(h->cas.p, V * V * V, 8192.0f, h->work.p, h->scales.p, s));
-    GG_CK(launch_pitch_volume(h->cas.p, h->V, (int)P, h->cas_fp.p, h->prec, h->vol_scale(), s));
+    GG_CK(launch_pitch_volume(h->cas.p, h->V, (int)P, c.vol.p, h->prec, h->vol_scale(), s));
     h->cas_fp_valid = true;
 }
 
 FpTiles fp_tiles(const gg_gridder *h)
 {
-    return FpTiles{h->cas_fp.p, h->prec, fp_pitch(h->V, h->prec), h->fp_maps.p, h->fault};
+    return FpTiles{h->fp().vol.p, h->prec, fp_pitch(h->V, h->prec), h->fp().maps.p, h->fault};
 }
 
 // ---- device-side pipelines (all on stream s) --------------------------------
@@ -415,7 +419,7 @@ void fp_batch(gg_gridder *h, const float *d_axes, int b, float *cas_out, float *
     auto &S = h->slot[sl];
     ProfScope ps(h, s, GG_KERNEL_FORWARD);
     if (h->five_taps)
-        GG_CK(launch_forward_project(h->cas_fp.p, h->prec, fp_pitch(h->V, h->prec), cas_out, h->ker.p, d_axes, b,
+        GG_CK(launch_forward_project(h->fp().vol.p, h->prec, fp_pitch(h->V, h->prec), cas_out, h->ker.p, d_axes, b,
                                      h->geom(), true, h->vol_scale(), s));
     else
         GG_CK(launch_forward_project_tiled(fp_tiles(h), cas_out, h->ker.p, d_axes, b, h->geom(), h->vol_scale(), s,
@@ -802,8 +806,10 @@ void destroy_handle(gg_gridder *h)
     h->ker.release();
     h->precomp.release();
     h->cas.release();
-    h->cas_fp.release();
-    h->fp_maps.release();
+    for (auto &c : h->fp_copy) {
+        c.vol.release();
+        c.maps.release();
+    }
     if (h->fault) cudaFreeHost(h->fault);
     h->pd.release();
     h->bp_part.release();

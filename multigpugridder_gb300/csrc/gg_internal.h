@@ -43,7 +43,8 @@ cudaError_t launch_forward_project(const void *d_vol, int vprec, int pitch, floa
 inline int fp_pitch(int V, int prec) { return prec == kF32 ? (V + 3) / 4 * 4 : (V + 7) / 8 * 8; }
 // Such a copy with its tensor maps: `maps` is a device buffer of
 // fp_tile_map_bytes(prec), filled by fp_tile_make_maps (synchronous) for this
-// address, V, pitch and storage.  `fault` (device-accessible) is set to 1 by a
+// address, V, pitch and element size, once: maps that a launch has used may
+// not be written again, as no later launch fences them.  `fault` (device-accessible) is set to 1 by a
 // kernel whose copies did not arrive.
 struct FpTiles {
     const void *vol;

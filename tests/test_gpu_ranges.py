@@ -136,6 +136,31 @@ def test_forward_tiles(cuda, N, n, scale, prec):
     assert np.all(got[ref == 0] == 0)
 
 
+# one handle through every storage type and back (with the 4-tap tiles and with
+# five taps), against a handle that has known no other; the volume is replaced on the way
+@pytest.mark.parametrize("edge", [0.0, 0.25])
+@pytest.mark.parametrize("N", [18, 50])
+def test_precision_switches(cuda, N, edge):
+    import multigpugridder_gb300 as gg
+
+    p = O.Params(N)
+    rng = np.random.default_rng(4000 + N)
+    axes = O.quaternion_axes(40, seed=N).astype(np.float32)
+    table = p.ker.copy()
+    table[0] = edge
+    with gg.MultiGPUGridder(N, 40, adjustInterpFactor=False) as g:
+        g.setKBTable(table)
+        for prec in ("f32", "bf16", "f32", "f16", "bf16", "f16", "f32"):
+            cas = rng.standard_normal((p.V,) * 3).astype(np.float32)
+            g.set_precision(prec)
+            g.setCASVolume(cas)
+            got = g.forwardProjectCAS(axes)
+            with gg.MultiGPUGridder(N, 40, precision=prec, adjustInterpFactor=False) as f:
+                f.setKBTable(table)
+                f.setCASVolume(cas)
+                assert np.array_equal(got, f.forwardProjectCAS(axes)), prec
+
+
 # fewer than 32 directions, and each range of the rule's aim, at volumes of few
 # bricks; n that the segments do not divide
 @pytest.mark.parametrize("N,n", [(64, 9), (16, 33), (18, 101), (32, 210), (16, 600)])
