@@ -52,6 +52,16 @@ struct FpTiles {
     const void *maps;
     int *fault;
 };
+// Host side of a fault word: whether it was set; it is clear again, so that a
+// fault is reported once.
+inline bool take_fault(int *word)
+{
+    volatile int *const w = word;
+    if (!w || !*w) return false;
+    *w = 0;
+    return true;
+}
+constexpr const char *kFaultMessage = "a forward projection's copies to shared memory did not arrive";
 size_t fp_tile_map_bytes(int prec);
 cudaError_t fp_tile_make_maps(const void *d_vol, int V, int pitch, int prec, void *d_maps, cudaStream_t s);
 // Scratch of one launch of n directions.
@@ -259,3 +269,8 @@ void kb_table_f64(int hw, int size, double *out);
 void precomp_f64(int M, int hw, double *out);
 
 } // namespace gg
+
+// ---- for tests: sets the fault words as a kernel would whose copies did not
+// arrive (a host store; nothing fails on the device) ---------------------------
+struct gg_server;
+extern "C" void gg_server_mark_copy_fault(gg_server *S);

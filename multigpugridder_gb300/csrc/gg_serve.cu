@@ -164,6 +164,7 @@ struct Lane {
     std::map<std::tuple<int, int, int>, cufftHandle> plans; // (type, M, batch)
     void *work = nullptr;                                   // shared cuFFT work area
     size_t work_bytes = 0;
+    int *fault = nullptr; // pinned: set by the chunk in flight if a projection's copies did not arrive
 };
 
 } // namespace
@@ -184,6 +185,7 @@ struct gg_server {
     int active = 0;            // admitted, not yet retired
     cudaMemPool_t pool = nullptr;
     std::vector<Lane> lanes;
+    int *faults = nullptr; // the lanes' fault words
     std::map<int, Volume> volumes;
     int next_vol = 1;
     long long next_req = 1;
@@ -348,8 +350,10 @@ void enqueue_chunk(gg_server *S, Request &r)
         }
         const float *axes = r.d_axes + (size_t)c0 * 9;
         if (r.op == GG_OP_FORWARD) {
-            if (v.tiles.maps && !v.five_taps)
-                GS_CK(launch_forward_project_tiled(v.tiles, r.d_cas, v.ker, axes, b, v.g, nullptr, s, r.d_plans));
+            FpTiles tiles = v.tiles;
+            tiles.fault = L.fault; // the chunk's own, so that another request's failure is not its own
+            if (tiles.maps && !v.five_taps)
+                GS_CK(launch_forward_project_tiled(tiles, r.d_cas, v.ker, axes, b, v.g, nullptr, s, r.d_plans));
             else
                 GS_CK(launch_forward_project(v.cas, kF32, v.V, r.d_cas, v.ker, axes, b, v.g, v.five_taps, nullptr, s));
             if (v.fused_fft) {
@@ -431,6 +435,10 @@ void worker_main(gg_server *S)
             if (r->cuda_status != cudaSuccess && r->status == GG_OK) {
                 r->status = GG_ERR_CUDA;
                 r->err = cudaGetErrorString(r->cuda_status);
+            }
+            if (take_fault(L.fault) && r->status == GG_OK) {
+                r->status = GG_ERR_CUDA;
+                r->err = kFaultMessage;
             }
             if (r->status != GG_OK || r->next >= r->n) {
                 retire(S, r, frees);
@@ -577,8 +585,13 @@ extern "C" int gg_server_create(int device, double hbm_budget_gb, int lanes, gg_
         GS_CK(cudaMemPoolSetAttribute(S->pool, cudaMemPoolAttrReleaseThreshold, &keep));
         int least = 0, greatest = 0;
         GS_CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        void *words = nullptr;
+        GS_CK(cudaHostAlloc(&words, (size_t)lanes * sizeof(int), cudaHostAllocDefault));
+        S->faults = (int *)words;
         S->lanes.resize(lanes);
         for (auto &L : S->lanes) {
+            L.fault = S->faults + (&L - S->lanes.data());
+            *L.fault = 0;
             GS_CK(cudaStreamCreateWithPriority(&L.lo, cudaStreamNonBlocking, least));
             GS_CK(cudaStreamCreateWithPriority(&L.hi, cudaStreamNonBlocking, greatest));
         }
@@ -613,8 +626,15 @@ extern "C" void gg_server_destroy(gg_server *S)
         if (L.hi) cudaStreamDestroy(L.hi);
     }
     for (auto &kv : S->volumes) gg_destroy(kv.second.h);
+    if (S->faults) cudaFreeHost(S->faults);
     if (S->pool) cudaMemPoolDestroy(S->pool);
     delete S;
+}
+
+extern "C" void gg_server_mark_copy_fault(gg_server *S)
+{
+    std::lock_guard<std::mutex> lock(S->mu);
+    for (auto &L : S->lanes) *(volatile int *)L.fault = 1;
 }
 
 extern "C" const char *gg_server_last_error(const gg_server *S) { return S ? S->err.c_str() : "null server handle"; }

@@ -229,3 +229,25 @@ def test_default_quantum_chunks_equal_plain_path(cuda, gglib):
     assert np.array_equal(back, back_alone)
     assert O.rel_l2(back, _plain(gglib, v, "back", axes, imgs)) < 1e-6
     assert O.rel_l2(fwd, _plain(gglib, v, "forward", axes, None)) < 1e-6
+
+
+def test_copy_fault_fails_the_request(cuda, gglib):
+    """A chunk whose box copies did not arrive fails its request, and that one
+    only.  The word the kernel would set is set from the host."""
+    import multigpugridder_gb300 as gg
+    from multigpugridder_gb300._lib import GG_ERR_CUDA
+    from multigpugridder_gb300.serve import Server
+
+    mark = gglib.gg_server_mark_copy_fault
+    mark.argtypes, mark.restype = [ctypes.c_void_p], None
+    axes = O.quaternion_axes(8, 5).astype(np.float32)
+    with Server(lanes=1) as srv:
+        vid = srv.add_volume(O.blob_volume(16, 10, seed=6))
+        good = srv.wait(srv.submit(vid, "forward", axes))[0].copy()
+        srv.reset_stats()
+        mark(srv._h)
+        with pytest.raises(gg.GridderError) as e:
+            srv.wait(srv.submit(vid, "forward", axes))
+        assert e.value.code == GG_ERR_CUDA and "did not arrive" in str(e.value)
+        assert np.array_equal(srv.wait(srv.submit(vid, "forward", axes))[0], good)
+        assert srv.stats()["completed"] == 1
