@@ -133,7 +133,11 @@ int gg_get_volume(gg_gridder *h, float *volume_out);
 int gg_reconstruct_volume(gg_gridder *h, const float *axes, int n_axes,
                           const float *images, float *volume_out);
 
-/* Device-pointer forms of the calls above. */
+/* Device-pointer forms of the calls above.  Errors of work that has not run
+   when a call returns are reported, once, by a later call on the handle: CUDA's
+   own, and GG_ERR_CUDA where a forward projection's copies to shared memory did
+   not arrive (the images of that call are then not complete).  The host forms
+   report both themselves. */
 int gg_set_volume_dev(gg_gridder *h, const float *d_volume, void *stream);
 int gg_set_cas_volume_dev(gg_gridder *h, const float *d_cas_volume, void *stream);
 int gg_get_cas_volume_dev(gg_gridder *h, float *d_cas_volume_out, void *stream);

@@ -842,7 +842,7 @@ template <typename F> int guarded(gg_gridder *h, F &&f)
     try {
         set_device(h);
         f();
-        if (h->fault && *(volatile int *)h->fault) fail(GG_ERR_CUDA, "a forward projection's copies to shared memory did not arrive");
+        if (take_fault(h->fault)) fail(GG_ERR_CUDA, "%s", kFaultMessage);
         h->err.clear();
         return GG_OK;
     } catch (const GGError &e) {
@@ -878,6 +878,13 @@ void check_cube(const int *dims, int want, const char *what)
 // =============================================================================
 // C ABI
 // =============================================================================
+
+extern "C" int gg_mark_copy_fault(gg_gridder *h)
+{
+    if (!h || !h->fault) return GG_ERR_STATE;
+    *(volatile int *)h->fault = 1;
+    return GG_OK;
+}
 
 extern "C" int gg_version(void) { return GG_ABI_VERSION; }
 

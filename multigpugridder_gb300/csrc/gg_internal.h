@@ -273,4 +273,5 @@ void precomp_f64(int M, int hw, double *out);
 // ---- for tests: sets the fault words as a kernel would whose copies did not
 // arrive (a host store; nothing fails on the device) ---------------------------
 struct gg_server;
+extern "C" int gg_mark_copy_fault(gg_gridder *h); // GG_ERR_STATE before the first projection
 extern "C" void gg_server_mark_copy_fault(gg_server *S);

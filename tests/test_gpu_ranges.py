@@ -161,6 +161,26 @@ def test_precision_switches(cuda, N, edge):
                 assert np.array_equal(got, f.forwardProjectCAS(axes)), prec
 
 
+# the word that a kernel whose copies did not arrive would set, set from the
+# host: the call that finds it reports it, and the next one is as before
+def test_copy_fault_is_reported_once(cuda, gglib):
+    import multigpugridder_gb300 as gg
+    from multigpugridder_gb300._lib import GG_ERR_CUDA
+
+    mark = gglib.gg_mark_copy_fault
+    mark.argtypes = [ctypes.c_void_p]
+    axes = O.quaternion_axes(5, seed=1).astype(np.float32)
+    with gg.MultiGPUGridder(16, 5, adjustInterpFactor=False) as g:
+        g.setVolume(O.blob_volume(16, 10, seed=6))
+        assert mark(g.handle) != 0  # no projection yet
+        good = g.forwardProjectCAS(axes)
+        assert mark(g.handle) == 0
+        with pytest.raises(gg.GridderError) as e:
+            g.forwardProjectCAS(axes)
+        assert e.value.code == GG_ERR_CUDA and "did not arrive" in str(e.value)
+        assert np.array_equal(g.forwardProjectCAS(axes), good)
+
+
 # fewer than 32 directions, and each range of the rule's aim, at volumes of few
 # bricks; n that the segments do not divide
 @pytest.mark.parametrize("N,n", [(64, 9), (16, 33), (18, 101), (32, 210), (16, 600)])
