@@ -97,6 +97,27 @@ template <typename T> struct DevBuf {
     }
 };
 
+// Room for `count` elements in scratch that a call on stream s can do without.
+// False: it cannot be had (no memory, or growing would allocate while s is
+// being captured, which is not allowed).
+template <typename T> bool try_ensure(DevBuf<T> &b, size_t count, cudaStream_t s)
+{
+    if (b.p && count <= b.n) return true;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    try {
+        b.ensure(count);
+    } catch (const GGError &e) {
+        if (e.code != GG_ERR_OUT_OF_MEMORY) throw;
+        cudaGetLastError();
+        return false;
+    }
+    return true;
+}
+
 struct PinBuf {
     float *p = nullptr;
     size_t n = 0;
@@ -439,12 +460,19 @@ void fp_batch(gg_gridder *h, const float *d_axes, int b, float *cas_out, float *
 }
 
 // The split of a back projection of b directions, with room for its sums
-// (`stacks`: 2 with a density or a second image stack).
-BpSplit bp_split(gg_gridder *h, int b, int stacks)
+// (`stacks`: 2 with a density or a second image stack): at most 140 MB, as
+// bp_segments wants at most 6,000 bricks in all, whatever V.  Where the room
+// cannot be had the launch stays unsplit: it needs none then.
+BpSplit bp_split(gg_gridder *h, int b, int stacks, cudaStream_t s)
 {
-    const int nseg = bp_segments(b, h->geom());
-    if (nseg > 1) h->bp_part.ensure((size_t)(nseg - 1) * stacks * h->V * h->V * h->V);
-    return BpSplit{nseg, h->bp_part.p, h->bp_next.p};
+    BpSplit sp;
+    sp.next = h->bp_next.p;
+    sp.nseg = bp_segments(b, h->geom());
+    bp_part_box(h->geom(), sp.lo, sp.edge);
+    const size_t E = sp.edge;
+    if (sp.nseg > 1 && !try_ensure(h->bp_part, (size_t)(sp.nseg - 1) * stacks * E * E * E, s)) sp.nseg = 1;
+    sp.part = h->bp_part.p;
+    return sp;
 }
 
 // Back-project b directions: images (device, FFT path) or CAS images (device).
@@ -513,11 +541,11 @@ void bp_batch(gg_gridder *h, const float *d_axes, int b, const float *img, const
         GG_CK(launch_back_project_adjoint(target, h->V, src, h->ker.p, d_axes, b, h->geom(), scale, s));
     } else if (pd && !ones) {
         GG_CK(launch_back_project_ref_density(target, pd, src, h->ker.p, d_axes, b, h->geom(), scale, s,
-                                              bp_split(h, b, 2)));
+                                              bp_split(h, b, 2, s)));
         pd = nullptr;
     } else {
         GG_CK(launch_back_project_ref(target, src, ones, h->ker.p, d_axes, b, h->geom(), scale, s, false,
-                                      bp_split(h, b, 1)));
+                                      bp_split(h, b, 1, s)));
     }
     ps.done();
     if (pd) {
@@ -555,7 +583,7 @@ void ctf_batch(gg_gridder *h, const float *d_axes, int b, const float *img, cons
         // both stacks in one back-projection pass
         ProfScope ps(h, s, GG_KERNEL_BACK);
         GG_CK(launch_back_project_ref_pair(h->cas.p, h->pd.p, S.casimg.p, S.real.p, h->ker.p, d_axes, b, h->geom(), s,
-                                           bp_split(h, b, 2)));
+                                           bp_split(h, b, 2, s)));
         ps.done();
     } else {
         bp_batch(h, d_axes, b, nullptr, S.casimg.p, h->cas.p, false, sl, s);

@@ -76,18 +76,27 @@ cudaError_t launch_pitch_volume(const float *d_cas, int V, int P, void *d_out, i
 
 // A back projection split into nseg contiguous segments of its directions, run
 // side by side: segment 0 accumulates into the volume as an unsplit launch
-// does, the others write their sums to `part` ((nseg - 1) * V^3 floats, twice
-// that with a density), and a merge adds them in order.  nseg = 1: unsplit.
+// does, the others write their sums to `part`, and a merge adds them in order.
+// part: (nseg - 1) boxes of `edge`^3 floats (twice that with a density) that
+// hold the mask's sphere, from voxel `lo` along each axis (bp_part_box).
+// nseg = 1: unsplit.
 // next (optional): a device counter, zero between launches and used by one
 // launch at a time, from which the warps of a launch that owns the GPU take
 // their work.
 struct BpSplit {
-    int nseg = 1;
+    int nseg = 1, lo = 0, edge = 0;
     float *part = nullptr;
     unsigned *next = nullptr;
 };
 // The number of segments for n directions.
 int bp_segments(int n, const Geom &g);
+// The voxels lo .. lo + edge - 1 of each axis hold the mask's sphere.
+inline void bp_part_box(const Geom &g, int &lo, int &edge)
+{
+    const int c = g.V / 2, top = g.mask_radius < g.V - 1 - c ? c + g.mask_radius : g.V - 1;
+    lo = g.mask_radius < c ? c - g.mask_radius : 0;
+    edge = top - lo + 1;
+}
 
 // Back projection with the reference window rule, accumulated (+=) into the
 // FP32 CAS volume.  d_img holds n*M*M CAS images; when `ones` is set the images are taken to be all ones (plane density) and

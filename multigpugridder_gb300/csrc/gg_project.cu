@@ -1041,14 +1041,16 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
 #pragma unroll
         for (int s = 0; s < BD; s++) {
             if (!((inmask >> s) & 1u)) continue;
-            const size_t o = (size_t)(bz + s) * V * V + (size_t)ly * V + lx;
             if (!SPLIT || item % ns == 0) {
+                const size_t o = (size_t)(bz + s) * V * V + (size_t)ly * V + lx;
                 vol[o] = vol[o] + wacc[lane + 32 * s] * sc;
                 if (DENS || DW) pd[o] = pd[o] + waccw[lane + 32 * s];
             } else {
-                float *const pv = split.part + (size_t)(item % ns - 1) * (DENS || DW ? 2 : 1) * V * V * V;
-                pv[o] = wacc[lane + 32 * s] * sc;
-                if (DENS || DW) pv[(size_t)V * V * V + o] = waccw[lane + 32 * s];
+                const size_t E = split.edge, E3 = E * E * E;
+                float *const pv = split.part + (size_t)(item % ns - 1) * (DENS || DW ? 2 : 1) * E3 +
+                                  ((size_t)(bz + s - split.lo) * E + (ly - split.lo)) * E + (lx - split.lo);
+                pv[0] = wacc[lane + 32 * s] * sc;
+                if (DENS || DW) pv[E3] = waccw[lane + 32 * s];
             }
         }
         if (!split.next) return;
@@ -1065,20 +1067,22 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
 
 // Adds the segments' sums of a split launch to the volume (and the density),
 // in segment order: (((v + s1) + s2) + ...).  Voxels of the mask sphere, which
-// every segment has written.  Bound: HBM / L2, 4 (segments + 1) bytes a voxel.
+// every segment has written; the grid covers the sphere's box.  Bound: HBM /
+// L2, 4 (segments + 1) bytes a voxel.
 __global__ void __launch_bounds__(256)
 bp_merge_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, int maskR, BpSplit split)
 {
     const int x = blockIdx.x * 256 + threadIdx.x, y = blockIdx.y, z = blockIdx.z;
-    if (x >= V) return;
-    const long long c = V / 2, dx = x - c, dy = y - c, dz = z - c;
+    if (x >= split.edge) return;
+    const long long c = V / 2 - split.lo, dx = x - c, dy = y - c, dz = z - c;
     if (dx * dx + dy * dy + dz * dz > (long long)maskR * maskR) return;
-    const size_t V3 = (size_t)V * V * V, o = ((size_t)z * V + y) * V + x;
+    const size_t E = split.edge, E3 = E * E * E, q = ((size_t)z * E + y) * E + x;
+    const size_t o = ((size_t)(z + split.lo) * V + (y + split.lo)) * V + (x + split.lo);
     const int per = pd ? 2 : 1;
     float v = vol[o], d = pd ? pd[o] : 0.0f;
     for (int s = 0; s + 1 < split.nseg; s++) {
-        v = __fadd_rn(v, split.part[s * per * V3 + o]);
-        if (pd) d = __fadd_rn(d, split.part[(s * per + 1) * V3 + o]);
+        v = __fadd_rn(v, split.part[s * per * E3 + q]);
+        if (pd) d = __fadd_rn(d, split.part[(s * per + 1) * E3 + q]);
     }
     vol[o] = v;
     if (pd) pd[o] = d;
@@ -1130,7 +1134,7 @@ static cudaError_t launch_bp_compact_g(float *vol, const float *img, const float
                                               g.ker_hw, bx, by, tb, scale, img2, vec, split, lay);
         count_launches(1);
         if (split.nseg > 1) {
-            const dim3 mg((unsigned)((g.V + 255) / 256), (unsigned)g.V, (unsigned)g.V);
+            const dim3 mg((unsigned)((split.edge + 255) / 256), (unsigned)split.edge, (unsigned)split.edge);
             bp_merge_kernel<<<mg, 256, 0, s>>>(vol, DENS || DW ? pd : nullptr, g.V, g.mask_radius, split);
             count_launches(1);
         }

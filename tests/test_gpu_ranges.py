@@ -203,6 +203,57 @@ def test_back_projection_segments(cuda, N, n):
         assert O.rel_l2(g.getCASVolume(), num / (den + np.float32(1e-6))) < TOL
 
 
+# a small mask in a large volume, where the rule wants the most segments (and
+# the 8-deep blocks of M = 512): the scratch holds the mask's box, not the volume
+@pytest.mark.parametrize("N,mask,n", [(128, 20, 512), (256, 24, 40), (32, 0, 40), (32, 64, 40)])
+def test_back_projection_small_mask(cuda, N, mask, n):
+    import torch
+
+    import multigpugridder_gb300 as gg
+
+    p = O.Params(N, mask_radius=mask)
+    rng = np.random.default_rng(5000 + N + mask)
+    axes = O.quaternion_axes(n, seed=n).astype(np.float32)
+    ci = rng.standard_normal((n, p.M, p.M), dtype=np.float32)
+    num = O.bp_ref_f32(ci, axes, p.V, mask, p.ker)
+    with gg.MultiGPUGridder(N, n, adjustInterpFactor=False) as g:
+        g.setMaskRadius(mask)
+        g.backProjectCAS(ci[:8], axes[:8])  # the handle's other buffers
+        before = torch.cuda.mem_get_info()[0]
+        g.backProjectCAS(ci, axes)
+        assert before - torch.cuda.mem_get_info()[0] < 140e6
+        assert O.rel_l2(g.getCASVolume(), num) < TOL
+        imgs = rng.standard_normal((n, N, N), dtype=np.float32)
+        g.reconstructVol(imgs, axes)
+        got = g.getCASVolume()
+    ci = O.cas_imgs_from_imgs(imgs, p.M).astype(np.float32)
+    num = O.bp_ref_f32(ci, axes, p.V, mask, p.ker)
+    den = O.bp_ref_f32(np.ones_like(ci), axes, p.V, mask, p.ker)
+    assert O.rel_l2(got, num / (den + np.float32(1e-6))) < TOL
+
+
+# under capture the scratch of a split cannot grow: the launch stays unsplit
+def test_back_projection_split_under_capture(cuda, gglib):
+    import torch
+
+    import multigpugridder_gb300 as gg
+
+    N, n = 32, 300
+    p = O.Params(N)
+    axes = O.quaternion_axes(n, seed=n).astype(np.float32)
+    ci = np.random.default_rng(6).standard_normal((n, p.M, p.M)).astype(np.float32)
+    d_axes, d_ci = to_dev(axes, cuda), to_dev(ci, cuda)
+    with gg.MultiGPUGridder(N, n, adjustInterpFactor=False) as g:
+        g.backProjectCAS(ci[:8], axes[:8])  # the handle's other buffers
+        s, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            rc = gglib.gg_back_project_dev(g.handle, dptr(d_axes), n, None, dptr(d_ci), 0, ctypes.c_void_p(s.cuda_stream))
+        assert rc == 0
+        graph.replay()
+        torch.cuda.synchronize()
+        assert O.rel_l2(g.getCASVolume(), O.bp_ref_f32(ci, axes, p.V, p.mask_radius, p.ker)) < TOL
+
+
 # CAS images rounded to 2 bytes and read as FP32: M a multiple of 4 and not
 @pytest.mark.parametrize("prec", ["bf16", "f16"])
 @pytest.mark.parametrize("N,interp", [(32, 2.0), (44, 1.5)])
