@@ -25,6 +25,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -219,6 +220,7 @@ struct gg_gridder {
     cudaEvent_t ev_dev = nullptr; // end of the last *_dev call (serialises scratch use across streams)
     bool dev_pending = false;
     std::map<std::pair<int, int>, cufftHandle> plans2d;
+    std::set<int> pass_batches; // batch sizes that the passes have transformed without a plan
     // profiling: events around projection-kernel launches
     struct ProfRec {
         cudaEvent_t a, b;
@@ -377,12 +379,35 @@ FpTiles fp_tiles(const gg_gridder *h)
 
 // ---- device-side pipelines (all on stream s) --------------------------------
 
-// The volume passes' buffers: spectrum or planes; rows and planes.
-void ensure_vol(gg_gridder *h)
+// The volume passes' buffers: spectrum or planes; rows and planes.  For N
+// beyond 0.73 M they take more than the library's transform does, which then
+// runs where the room cannot be had.
+bool ensure_vol(gg_gridder *h, cudaStream_t s)
 {
     const size_t M = h->M, N = h->N, H = M / 2 + 1;
-    h->x3.ensure(std::max(M * M * M, 2 * H * N * (N + M)));
-    h->spec3.ensure(H * M * M);
+    return try_ensure(h->x3, std::max(M * M * M, 2 * H * N * (N + M)), s) && try_ensure(h->spec3, H * M * M, s);
+}
+
+// The plans of the library's transforms that a handle's passes have done
+// without: a change of storage may need them, and a captured call cannot make
+// them.  What cannot be made here is made at its first use.
+void make_plans(gg_gridder *h)
+{
+    try {
+        if (h->prec != kF32 && h->vol_passes && h->x3.p) plan3(h, true);
+        if (h->img_prec() == kBF16)
+            for (int b : h->pass_batches) plan2d(h, CUFFT_R2C, b);
+    } catch (const GGError &) {
+        cudaGetLastError();
+    }
+}
+
+// Images -> FP32 CAS images by the passes (fftn_ok).
+void images_to_cas_passes(gg_gridder *h, const float *img, int b, bool adjoint, unsigned *top, int sl, cudaStream_t s)
+{
+    auto &S = h->slot[sl];
+    if (h->pass_batches.size() < 6) h->pass_batches.insert(b);
+    GG_CK(launch_images_to_cas_passes(img, h->N, h->M, b, S.casimg.p, kF32, adjoint, h->tw.p, (float2 *)S.spec.p, top, s));
 }
 
 void do_set_volume(gg_gridder *h, const float *d_vol, cudaStream_t s)
@@ -393,8 +418,7 @@ void do_set_volume(gg_gridder *h, const float *d_vol, cudaStream_t s)
     // A 2-byte volume keeps the library's transform: few of its values carry the
     // images, and one of them that falls the other way for another transform's
     // last bit moves them by up to 3e-5 (BF16, 108 random cases; 9e-6 in FP16).
-    if (h->vol_passes && h->prec == kF32) {
-        ensure_vol(h);
+    if (h->vol_passes && h->prec == kF32 && ensure_vol(h, s)) {
         GG_CK(launch_volume_to_cas_passes(d_vol, h->N, h->M, h->V, h->precomp.p, h->cas.p, h->tw.p, (float2 *)h->x3.p,
                                           (float2 *)h->spec3.p, s));
         h->cas_fp_valid = false;
@@ -414,10 +438,9 @@ void do_set_volume(gg_gridder *h, const float *d_vol, cudaStream_t s)
 void do_get_volume(gg_gridder *h, float *d_cas, const float *d_density, float *d_vol, cudaStream_t s)
 {
     const size_t M3 = (size_t)h->M * h->M * h->M, H = h->M / 2 + 1;
-    if (h->vol_back_passes) {
+    if (h->vol_back_passes && ensure_vol(h, s)) {
         // half spectra of rows, then (spec3 holds the divided volume's spectrum) those of planes
         const size_t half = H * h->N * h->N;
-        ensure_vol(h);
         float2 *const x = (float2 *)h->x3.p, *const sp = (float2 *)h->spec3.p;
         if (d_density) GG_CK(launch_cas_volume_to_spectrum(d_cas, d_density, 1e-6f, h->V, h->M, h->spec3.p, s));
         GG_CK(launch_cas_to_volume_passes(d_cas, d_density ? sp : nullptr, h->N, h->M, h->V, h->precomp.p, d_vol, h->tw.p, x,
@@ -500,16 +523,14 @@ void bp_batch(gg_gridder *h, const float *d_axes, int b, const float *img, const
             GG_CK(launch_images_to_cas_fused(img, h->N, h->M, b, S.casimg.p, ip, false, s));
             src = S.casimg.p;
         } else if (h->fft_passes && ip == kF32) {
-            GG_CK(launch_images_to_cas_passes(img, h->N, h->M, b, S.casimg.p, ip, false, h->tw.p, (float2 *)S.spec.p, nullptr,
-                                              s));
+            images_to_cas_passes(h, img, b, false, nullptr, sl, s);
             src = S.casimg.p;
         } else if (h->fft_passes && ip == kF16) {
             // FP32 CAS images with their largest magnitude, then the storage
             // scale and the rounding.  BF16 images keep the library's transform:
             // of values this coarsely rounded, some 1 in 5,000 lies where another
             // transform's last bit decides (1.8e-5 of a reconstruction; FP16 6e-6)
-            GG_CK(launch_images_to_cas_passes(img, h->N, h->M, b, S.casimg.p, kF32, false, h->tw.p, (float2 *)S.spec.p,
-                                              h->work.p, s));
+            images_to_cas_passes(h, img, b, false, h->work.p, sl, s);
             GG_CK(launch_scale_from_max(h->work.p, 8192.0f, h->scales.p + 1, s));
             GG_CK(launch_round(S.casimg.p, S.casimg.p, ip, MM * b, h->img_scale(), s));
             src = S.casimg.p;
@@ -568,8 +589,7 @@ void ctf_batch(gg_gridder *h, const float *d_axes, int b, const float *img, cons
     if (h->fused_fft) {
         GG_CK(launch_images_to_cas_fused(img, h->N, h->M, b, S.casimg.p, kF32, false, s));
     } else if (h->fft_passes) {
-        GG_CK(launch_images_to_cas_passes(img, h->N, h->M, b, S.casimg.p, kF32, false, h->tw.p, (float2 *)S.spec.p, nullptr,
-                                          s));
+        images_to_cas_passes(h, img, b, false, nullptr, sl, s);
     } else {
         GG_CK(launch_images_to_fft_input(img, h->N, h->M, b, S.real.p, s));
         cufftHandle p = plan2d(h, CUFFT_R2C, b);
@@ -615,8 +635,7 @@ void forward_adjoint(gg_gridder *h, const float *d_axes, int n, const float *d_i
         if (h->fused_fft) {
             GG_CK(launch_images_to_cas_fused(d_img_grad + (size_t)a0 * NN, h->N, h->M, b, S.casimg.p, kF32, true, s));
         } else if (h->fft_passes) {
-            GG_CK(launch_images_to_cas_passes(d_img_grad + (size_t)a0 * NN, h->N, h->M, b, S.casimg.p, kF32, true, h->tw.p,
-                                              (float2 *)S.spec.p, nullptr, s));
+            images_to_cas_passes(h, d_img_grad + (size_t)a0 * NN, b, true, nullptr, 0, s);
         } else {
             GG_CK(launch_images_to_fft_input(d_img_grad + (size_t)a0 * NN, h->N, h->M, b, S.real.p, s));
             cufftHandle p = plan2d(h, CUFFT_R2C, b);
@@ -1053,8 +1072,7 @@ extern "C" int gg_set_precision(gg_gridder *h, int precision)
             GG_CK(cudaStreamSynchronize(h->cs));
             h->prec = precision;
             h->cas_fp_valid = false;
-            // setVolume now needs the plan that its passes did without
-            if (precision != kF32 && h->vol_passes && h->x3.p) plan3(h, true);
+            make_plans(h);
         }
     });
 }
@@ -1067,6 +1085,7 @@ extern "C" int gg_set_image_precision(gg_gridder *h, int precision)
         if (precision != h->img_prec_set) {
             GG_CK(cudaStreamSynchronize(h->cs));
             h->img_prec_set = precision;
+            make_plans(h);
         }
     });
 }

@@ -254,6 +254,48 @@ def test_back_projection_split_under_capture(cuda, gglib):
         assert O.rel_l2(g.getCASVolume(), O.bp_ref_f32(ci, axes, p.V, p.mask_radius, p.ker)) < TOL
 
 
+# the calls that the passes took over run under capture after the calls that
+# used to leave their plans and buffers behind: BF16 images after FP32 ones
+# (M = 100), setVolume after an adjoint (N = M, where the passes take more room)
+@pytest.mark.parametrize("kind", ["bf16_images", "set_volume"])
+def test_passes_under_capture(cuda, gglib, kind):
+    import torch
+
+    import multigpugridder_gb300 as gg
+
+    N, interp, n = (50, 2.0, 6) if kind == "bf16_images" else (100, 1.0, 2)
+    p = O.Params(N, interp)
+    rng = np.random.default_rng(7)
+    axes = O.quaternion_axes(n, seed=n).astype(np.float32)
+    imgs = rng.standard_normal((n, N, N)).astype(np.float32)
+    vol = rng.standard_normal((N,) * 3).astype(np.float32)
+    d_axes, d_imgs, d_vol = to_dev(axes, cuda), to_dev(imgs, cuda), to_dev(vol, cuda)
+    s, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    sp = ctypes.c_void_p(s.cuda_stream)
+    with gg.MultiGPUGridder(N, n, interpFactor=interp, adjustInterpFactor=False) as g:
+        if kind == "bf16_images":
+            g.backProject(imgs, axes)
+            g.set_image_precision("bf16")
+        else:
+            g.resetVolume()
+            grad = np.empty((N,) * 3, dtype=np.float32)
+            g._call("gg_forward_project_adjoint", axes.ctypes.data, n, imgs.ctypes.data, grad.ctypes.data)
+        with torch.cuda.graph(graph, stream=s):
+            if kind == "bf16_images":
+                rc = gglib.gg_back_project_dev(g.handle, dptr(d_axes), n, dptr(d_imgs), None, 0, sp)
+            else:
+                rc = gglib.gg_set_volume_dev(g.handle, dptr(d_vol), sp)
+        assert rc == 0
+        graph.replay()
+        torch.cuda.synchronize()
+        got = g.getCASVolume()
+    if kind == "bf16_images":
+        stored = torch.from_numpy(O.cas_imgs_from_imgs(imgs, p.M).astype(np.float32)).bfloat16().float().numpy()
+        assert O.rel_l2(got, O.bp_ref_f32(stored, axes, p.V, p.mask_radius, p.ker)) < 1e-3  # values on a rounding edge
+    else:
+        assert O.rel_l2(got, O.cas_from_vol(vol.astype(np.float64), p.hw, p.interp, p.pad)) < TOL
+
+
 # CAS images rounded to 2 bytes and read as FP32: M a multiple of 4 and not
 @pytest.mark.parametrize("prec", ["bf16", "f16"])
 @pytest.mark.parametrize("N,interp", [(32, 2.0), (44, 1.5)])
