@@ -501,77 +501,74 @@ BpSplit bp_split(gg_gridder *h, int b, int stacks, cudaStream_t s)
 // Back-project b directions: images (device, FFT path) or CAS images (device).
 // With `pd`, the plane density of the same directions is accumulated into pd
 // as well (fused into the same kernel for the reference rule).
-void bp_batch(gg_gridder *h, const float *d_axes, int b, const float *img, const float *casimg, float *target, bool ones,
-              int sl, cudaStream_t s, float *pd = nullptr)
+void bp_batch(gg_gridder *h, const float *d_axes, int b, const float *img, const float *casimg, float *target, int sl,
+              cudaStream_t s, float *pd = nullptr)
 {
     auto &S = h->slot[sl];
     const float *src = nullptr;
     const int ip = h->img_prec(); // rounding of the CAS images read here
     const float *scale = nullptr;
-    if (!ones) {
-        const size_t MM = (size_t)h->M * h->M;
-        if (casimg) {
-            if (ip == kF32) {
-                src = casimg;
-            } else {
-                if (ip == kF16) GG_CK(launch_storage_scale(casimg, MM * b, 8192.0f, h->work.p, h->scales.p + 1, s));
-                GG_CK(launch_round(casimg, S.casimg.p, ip, MM * b, h->img_scale(), s));
-                src = S.casimg.p;
-                scale = h->img_scale();
-            }
-        } else if (h->fused_fft && ip != kF16) {
-            GG_CK(launch_images_to_cas_fused(img, h->N, h->M, b, S.casimg.p, ip, false, s));
-            src = S.casimg.p;
-        } else if (h->fft_passes && ip == kF32) {
-            images_to_cas_passes(h, img, b, false, nullptr, sl, s);
-            src = S.casimg.p;
-        } else if (h->fft_passes && ip == kF16) {
-            // FP32 CAS images with their largest magnitude, then the storage
-            // scale and the rounding.  BF16 images keep the library's transform:
-            // of values this coarsely rounded, some 1 in 5,000 lies where another
-            // transform's last bit decides (1.8e-5 of a reconstruction; FP16 6e-6)
-            images_to_cas_passes(h, img, b, false, h->work.p, sl, s);
-            GG_CK(launch_scale_from_max(h->work.p, 8192.0f, h->scales.p + 1, s));
-            GG_CK(launch_round(S.casimg.p, S.casimg.p, ip, MM * b, h->img_scale(), s));
-            src = S.casimg.p;
-            scale = h->img_scale();
-        } else if (h->fused_fft) {
-            // FP16: FP32 CAS images first, then the storage scale from their
-            // largest magnitude and the conversion
-            GG_CK(launch_images_to_cas_fused(img, h->N, h->M, b, S.casimg.p, kF32, false, s));
-            GG_CK(launch_storage_scale(S.casimg.p, MM * b, 8192.0f, h->work.p, h->scales.p + 1, s));
-            GG_CK(launch_round(S.casimg.p, S.casimg.p, ip, MM * b, h->img_scale(), s));
-            src = S.casimg.p;
-            scale = h->img_scale();
+    const size_t MM = (size_t)h->M * h->M;
+    if (casimg) {
+        if (ip == kF32) {
+            src = casimg;
         } else {
-            GG_CK(launch_images_to_fft_input(img, h->N, h->M, b, S.real.p, s));
-            cufftHandle p = plan2d(h, CUFFT_R2C, b);
-            GG_CKF(cufftSetStream(p, s));
-            GG_CKF(cufftExecR2C(p, S.real.p, S.spec.p));
-            if (ip == kF16)
-                // |Re + Im| <= 2 max(|Re|, |Im|)
-                GG_CK(launch_storage_scale((const float *)S.spec.p, (size_t)h->M * (h->M / 2 + 1) * 2 * b, 4096.0f,
-                                           h->work.p, h->scales.p + 1, s));
-            GG_CK(launch_spectrum_to_cas_images(S.spec.p, h->M, b, S.casimg.p, ip, h->img_scale(), s));
+            if (ip == kF16) GG_CK(launch_storage_scale(casimg, MM * b, 8192.0f, h->work.p, h->scales.p + 1, s));
+            GG_CK(launch_round(casimg, S.casimg.p, ip, MM * b, h->img_scale(), s));
             src = S.casimg.p;
             scale = h->img_scale();
         }
+    } else if (h->fused_fft && ip != kF16) {
+        GG_CK(launch_images_to_cas_fused(img, h->N, h->M, b, S.casimg.p, ip, false, s));
+        src = S.casimg.p;
+    } else if (h->fft_passes && ip == kF32) {
+        images_to_cas_passes(h, img, b, false, nullptr, sl, s);
+        src = S.casimg.p;
+    } else if (h->fft_passes && ip == kF16) {
+        // FP32 CAS images with their largest magnitude, then the storage
+        // scale and the rounding.  BF16 images keep the library's transform:
+        // of values this coarsely rounded, some 1 in 5,000 lies where another
+        // transform's last bit decides (1.8e-5 of a reconstruction; FP16 6e-6)
+        images_to_cas_passes(h, img, b, false, h->work.p, sl, s);
+        GG_CK(launch_scale_from_max(h->work.p, 8192.0f, h->scales.p + 1, s));
+        GG_CK(launch_round(S.casimg.p, S.casimg.p, ip, MM * b, h->img_scale(), s));
+        src = S.casimg.p;
+        scale = h->img_scale();
+    } else if (h->fused_fft) {
+        // FP16: FP32 CAS images first, then the storage scale from their
+        // largest magnitude and the conversion
+        GG_CK(launch_images_to_cas_fused(img, h->N, h->M, b, S.casimg.p, kF32, false, s));
+        GG_CK(launch_storage_scale(S.casimg.p, MM * b, 8192.0f, h->work.p, h->scales.p + 1, s));
+        GG_CK(launch_round(S.casimg.p, S.casimg.p, ip, MM * b, h->img_scale(), s));
+        src = S.casimg.p;
+        scale = h->img_scale();
+    } else {
+        GG_CK(launch_images_to_fft_input(img, h->N, h->M, b, S.real.p, s));
+        cufftHandle p = plan2d(h, CUFFT_R2C, b);
+        GG_CKF(cufftSetStream(p, s));
+        GG_CKF(cufftExecR2C(p, S.real.p, S.spec.p));
+        if (ip == kF16)
+            // |Re + Im| <= 2 max(|Re|, |Im|)
+            GG_CK(launch_storage_scale((const float *)S.spec.p, (size_t)h->M * (h->M / 2 + 1) * 2 * b, 4096.0f,
+                                       h->work.p, h->scales.p + 1, s));
+        GG_CK(launch_spectrum_to_cas_images(S.spec.p, h->M, b, S.casimg.p, ip, h->img_scale(), s));
+        src = S.casimg.p;
+        scale = h->img_scale();
     }
-    ProfScope ps(h, s, ones ? GG_KERNEL_DENSITY : GG_KERNEL_BACK);
-    if (h->bp_mode == GG_BP_ADJOINT && !ones) {
+    ProfScope ps(h, s, GG_KERNEL_BACK);
+    if (h->bp_mode == GG_BP_ADJOINT) {
         GG_CK(launch_back_project_adjoint(target, h->V, src, h->ker.p, d_axes, b, h->geom(), scale, s));
-    } else if (pd && !ones) {
+    } else if (pd) {
         GG_CK(launch_back_project_ref_density(target, pd, src, h->ker.p, d_axes, b, h->geom(), scale, s,
                                               bp_split(h, b, 2, s)));
         pd = nullptr;
     } else {
-        GG_CK(launch_back_project_ref(target, src, ones, h->ker.p, d_axes, b, h->geom(), scale, s, false,
+        GG_CK(launch_back_project_ref(target, src, h->ker.p, d_axes, b, h->geom(), scale, s, false,
                                       bp_split(h, b, 1, s)));
     }
     ps.done();
     if (pd) {
         // adjoint rule: the plane density is the adjoint applied to all-ones CAS images
-        const size_t MM = (size_t)h->M * h->M;
         ProfScope pd_ps(h, s, GG_KERNEL_DENSITY);
         GG_CK(launch_fill(S.casimg.p, MM * b, 1.0f, s));
         GG_CK(launch_back_project_adjoint(pd, h->V, S.casimg.p, h->ker.p, d_axes, b, h->geom(), nullptr, s));
@@ -606,8 +603,8 @@ void ctf_batch(gg_gridder *h, const float *d_axes, int b, const float *img, cons
                                            bp_split(h, b, 2, s)));
         ps.done();
     } else {
-        bp_batch(h, d_axes, b, nullptr, S.casimg.p, h->cas.p, false, sl, s);
-        bp_batch(h, d_axes, b, nullptr, S.real.p, h->pd.p, false, sl, s);
+        bp_batch(h, d_axes, b, nullptr, S.casimg.p, h->cas.p, sl, s);
+        bp_batch(h, d_axes, b, nullptr, S.real.p, h->pd.p, sl, s);
     }
 }
 
@@ -779,14 +776,14 @@ void host_batches(gg_gridder *h, int n, const float *src, size_t per, bool casim
 }
 
 void bp_host(gg_gridder *h, const float *axes, int n, const float *images, const float *casimgs, float *target,
-             bool ones, float *pd = nullptr)
+             float *pd = nullptr)
 {
     upload_axes(h, axes, n, h->cs);
     const size_t MM = (size_t)h->M * h->M, NN = (size_t)h->N * h->N;
-    const float *src = ones ? nullptr : (casimgs ? casimgs : images);
+    const float *src = casimgs ? casimgs : images;
     host_batches(h, n, src, casimgs ? MM : NN, casimgs != nullptr, [&](int a0, int b, int sl, float *dbuf) {
-        bp_batch(h, h->axes.p + (size_t)a0 * 9, b, casimgs ? nullptr : dbuf, casimgs ? dbuf : nullptr, target, ones,
-                 sl, h->cs, pd);
+        bp_batch(h, h->axes.p + (size_t)a0 * 9, b, casimgs ? nullptr : dbuf, casimgs ? dbuf : nullptr, target, sl,
+                 h->cs, pd);
     });
 }
 
@@ -1170,7 +1167,7 @@ extern "C" int gg_back_project(gg_gridder *h, const float *axes, int n_axes, con
         const size_t V3 = (size_t)h->V * h->V * h->V;
         h->cas.ensure(V3);
         if (!accumulate) GG_CK(cudaMemsetAsync(h->cas.p, 0, V3 * sizeof(float), h->cs));
-        if (n_axes > 0) bp_host(h, axes, n_axes, images, cas_images, h->cas.p, false);
+        if (n_axes > 0) bp_host(h, axes, n_axes, images, cas_images, h->cas.p);
         GG_CK(cudaStreamSynchronize(h->cs));
         h->cas_fp_valid = false;
     });
@@ -1202,7 +1199,7 @@ extern "C" int gg_reconstruct_volume(gg_gridder *h, const float *axes, int n_axe
         GG_CK(cudaMemsetAsync(h->pd.p, 0, V3 * sizeof(float), h->cs));
         // back projection of the images and, in the same pass, the plane
         // density (the same directions with all-ones CAS images)
-        if (n_axes > 0) bp_host(h, axes, n_axes, images, nullptr, h->cas.p, false, h->pd.p);
+        if (n_axes > 0) bp_host(h, axes, n_axes, images, nullptr, h->cas.p, h->pd.p);
         h->vol_io.ensure(N3);
         do_get_volume(h, h->cas.p, h->pd.p, h->vol_io.p, h->cs);
         GG_CK(cudaMemcpyAsync(volume_out, h->vol_io.p, N3 * sizeof(float), cudaMemcpyDeviceToHost, h->cs));
@@ -1293,7 +1290,7 @@ extern "C" int gg_back_project_dev(gg_gridder *h, const float *d_axes, int n_axe
             const int b = std::min(B, n_axes - a0);
             ensure_slot(h, 0, B, false);
             bp_batch(h, d_axes + (size_t)a0 * 9, b, d_images ? d_images + (size_t)a0 * NN : nullptr,
-                     d_cas_images ? d_cas_images + (size_t)a0 * MM : nullptr, h->cas.p, false, 0, s);
+                     d_cas_images ? d_cas_images + (size_t)a0 * MM : nullptr, h->cas.p, 0, s);
         }
         h->cas_fp_valid = false;
         end_dev(h, s);
@@ -1330,7 +1327,7 @@ extern "C" int gg_reconstruct_volume_dev(gg_gridder *h, const float *d_axes, int
         for (int a0 = 0; a0 < n_axes; a0 += B) {
             const int b = std::min(B, n_axes - a0);
             ensure_slot(h, 0, B, false);
-            bp_batch(h, d_axes + (size_t)a0 * 9, b, d_images + (size_t)a0 * NN, nullptr, h->cas.p, false, 0, s, h->pd.p);
+            bp_batch(h, d_axes + (size_t)a0 * 9, b, d_images + (size_t)a0 * NN, nullptr, h->cas.p, 0, s, h->pd.p);
         }
         do_get_volume(h, h->cas.p, h->pd.p, d_volume_out, s);
         h->cas_fp_valid = false;
@@ -1353,7 +1350,7 @@ extern "C" int gg_back_project_sums_dev(gg_gridder *h, const float *d_axes, int 
         for (int a0 = 0; a0 < n_axes; a0 += B) {
             const int b = std::min(B, n_axes - a0);
             ensure_slot(h, 0, B, false);
-            bp_batch(h, d_axes + (size_t)a0 * 9, b, d_images + (size_t)a0 * NN, nullptr, d_sums, false, 0, s,
+            bp_batch(h, d_axes + (size_t)a0 * 9, b, d_images + (size_t)a0 * NN, nullptr, d_sums, 0, s,
                      d_sums + V3);
         }
         end_dev(h, s);
@@ -1557,7 +1554,7 @@ extern "C" int gg_back_project_kernel(float *d_cas_volume, const float *d_cas_im
         return GG_ERR_INVALID_ARG;
     }
     Geom g{cas_vol_size, cas_img_size, mask_radius, kb_table_size, ker_hwidth};
-    cudaError_t e = launch_back_project_ref(d_cas_volume, d_cas_images, false, d_kb_table, d_axes, n_axes, g, nullptr,
+    cudaError_t e = launch_back_project_ref(d_cas_volume, d_cas_images, d_kb_table, d_axes, n_axes, g, nullptr,
                                             (cudaStream_t)stream);
     if (e != cudaSuccess) {
         g_global_err = cudaGetErrorString(e);

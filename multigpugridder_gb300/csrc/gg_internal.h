@@ -99,12 +99,11 @@ inline void bp_part_box(const Geom &g, int &lo, int &edge)
 }
 
 // Back projection with the reference window rule, accumulated (+=) into the
-// FP32 CAS volume.  d_img holds n*M*M CAS images; when `ones` is set the images are taken to be all ones (plane density) and
-// d_img is not read.
+// FP32 CAS volume.  d_img holds n*M*M CAS images.
 // *d_scale multiplies each voxel's sum before it is added.  shared: the GPU
 // runs other launches concurrently (smaller CTAs that share an SM; FP32
 // images, the same sums bit for bit).
-cudaError_t launch_back_project_ref(float *d_vol, const float *d_img, bool ones,
+cudaError_t launch_back_project_ref(float *d_vol, const float *d_img,
                                     const float *d_ker, const float *d_axes, int n, const Geom &g,
                                     const float *d_scale, cudaStream_t s, bool shared = false,
                                     BpSplit split = BpSplit());

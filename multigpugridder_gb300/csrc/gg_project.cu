@@ -252,7 +252,7 @@ __device__ __forceinline__ float ref_pixel_pos(float pi, float pj, float n_x, fl
 // linear-index test always passes.  Table entry k is read at sker[k * rep].
 // DW: cumW sums img2 * w (a second image back-projected in the same pass,
 // fused as cumSum is) instead of w.
-template <bool ONES, bool DENS, bool INSIDE, bool DW = false>
+template <bool DENS, bool INSIDE, bool DW = false>
 __device__ __forceinline__ void ref_window(const RefWindow &q, const float *sker, int rep, const float *__restrict__ img_ptr,
                                            int M, int imgi, int imgj, int imgCenter, float &cumSum, float &cumW,
                                            const float *__restrict__ img2_ptr = nullptr)
@@ -274,7 +274,7 @@ __device__ __forceinline__ void ref_window(const RefWindow &q, const float *sker
             const int lin = j1 * M + i1;
             if (INSIDE || (lin < M * M && lin >= 0)) {
                 // cumSum += img * w, fused as the reference's build fuses it
-                cumSum = __fmaf_rn(ONES ? 1.0f : ld_f32(img_ptr + lin), w, cumSum);
+                cumSum = __fmaf_rn(ld_f32(img_ptr + lin), w, cumSum);
                 if (DENS) cumW = __fadd_rn(cumW, w);
                 if (DW) cumW = __fmaf_rn(__ldg(img2_ptr + lin), w, cumW);
             }
@@ -666,7 +666,7 @@ __device__ __forceinline__ void cp_async_wait()
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-template <bool ONES, bool DENS, bool DW = false, bool DEEP = false, int G = kBpGroups,
+template <bool DENS, bool DW = false, bool DEEP = false, int G = kBpGroups,
           int TS = 0, bool LEAN = true, bool SPLIT = false>
 __global__ void __launch_bounds__(kCThreads *G, G == 1 ? 3 : 1)
 bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, const float *__restrict__ img, int M,
@@ -675,7 +675,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                       const float *__restrict__ d_scale, const float *__restrict__ img2, int vecImg, BpSplit split,
                       const __grid_constant__ BpLayers lay)
 {
-    static_assert(!DW || (!ONES && !DENS), "the second image stack is a reference-rule option");
+    static_assert(!DW || !DENS, "the second image stack is a reference-rule option");
     constexpr int W = 5, HALF = W / 2;
     using Shape = BpShape<DW, DEEP>;
     constexpr int BD = Shape::BD, kWarpVox = Shape::WV, kCBZ = Shape::BZ;
@@ -790,10 +790,10 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                 const RefWindow rw{nx0, nx1, nx2, ny0, ny1, ny2, (float)vi, (float)vj, (float)vk,
                                    (float)volCenter, kerScale, kerCenterHalf};
                 if (inside)
-                    ref_window<ONES, DENS, true, DW>(rw, sker, cp, img_ptr, M, imgi, imgj, imgCenter, cs, cw,
+                    ref_window<DENS, true, DW>(rw, sker, cp, img_ptr, M, imgi, imgj, imgCenter, cs, cw,
                                                          img2_ptr);
                 else
-                    ref_window<ONES, DENS, false, DW>(rw, sker, cp, img_ptr, M, imgi, imgj, imgCenter, cs, cw,
+                    ref_window<DENS, false, DW>(rw, sker, cp, img_ptr, M, imgi, imgj, imgCenter, cs, cw,
                                                           img2_ptr);
             }
         };
@@ -883,7 +883,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                 // has in the queue (at its front), run before b is refilled.
                 const int b = NB > 1 ? nbuf : 0;
                 if (NB > 1) {
-                    if (QALIGN && !ONES) {
+                    if (QALIGN) {
                         cp_async_wait();
                         __syncwarp(); // the footprints' copies are complete, for every lane
                     }
@@ -927,7 +927,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                     fj0 = __float2int_rd(jc - hj - 0.6f) - HALF;
                     fh = __float2int_rd(jc + hj + 0.6f) + HALF - fj0 + 1;
                     foot = fh <= FH;
-                    if (foot && !ONES && vecImg) {
+                    if (foot && vecImg) {
                         // vector loads of aligned pixel quads (rows start at
                         // multiples of 4 elements: 4 divides M, the image stacks
                         // are aligned), the linear-index rule still applied
@@ -1001,7 +1001,7 @@ bp_ref_compact_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, co
                             const int lin = (fj0 + r) * M + (fi0 + c);
                             float v = 0.0f, v2 = 0.0f;
                             if (lin >= 0 && lin < MM) {
-                                v = ONES ? 1.0f : ld_f32(img_ptr + lin);
+                                v = ld_f32(img_ptr + lin);
                                 if (DW) v2 = __ldg(img2_ptr + lin);
                             }
                             wfoot[r * FS + c + (QALIGN ? (fi0 & 3) : 0)] = v;
@@ -1088,7 +1088,7 @@ bp_merge_kernel(float *__restrict__ vol, float *__restrict__ pd, int V, int mask
     if (pd) pd[o] = d;
 }
 
-template <bool ONES, bool DENS, bool DW, bool DEEP, int G>
+template <bool DENS, bool DW, bool DEEP, int G>
 static cudaError_t launch_bp_compact_g(float *vol, const float *img, const float *ker, const float *axes, int n,
                                        const Geom &g, const float *scale, cudaStream_t s, float *pd, const float *img2,
                                         int max_copies, BpSplit split)
@@ -1141,17 +1141,14 @@ static cudaError_t launch_bp_compact_g(float *vol, const float *img, const float
         return cudaGetLastError();
     };
     if constexpr (LEAN) {
-        if constexpr (!ONES) {
-            if (split.nseg > 1) // bp_segments splits only tables that get 32 copies
-                return tb.copies == 32 ? go(bp_ref_compact_kernel<ONES, DENS, DW, DEEP, G, 128, true, true>)
-                                       : cudaErrorInvalidValue;
-        }
-        if (tb.copies == 32) return go(bp_ref_compact_kernel<ONES, DENS, DW, DEEP, G, 128, true>);
+        if (split.nseg > 1) // bp_segments splits only tables that get 32 copies
+            return tb.copies == 32 ? go(bp_ref_compact_kernel<DENS, DW, DEEP, G, 128, true, true>) : cudaErrorInvalidValue;
+        if (tb.copies == 32) return go(bp_ref_compact_kernel<DENS, DW, DEEP, G, 128, true>);
     }
-    return go(bp_ref_compact_kernel<ONES, DENS, DW, DEEP, G, 0, LEAN>);
+    return go(bp_ref_compact_kernel<DENS, DW, DEEP, G, 0, LEAN>);
 }
 
-template <bool ONES, bool DENS = false, bool DW = false, bool DEEP = false>
+template <bool DENS, bool DW = false, bool DEEP = false>
 static cudaError_t launch_bp_compact_t(float *vol, const float *img, const float *ker, const float *axes, int n,
                                        const Geom &g, const float *scale, cudaStream_t s, float *pd = nullptr,
                                        const float *img2 = nullptr, bool shared = false,
@@ -1163,47 +1160,45 @@ static cudaError_t launch_bp_compact_t(float *vol, const float *img, const float
     // other lanes can fill as they free (serving capacity 172 -> 195 req/s when
     // the rule was made); alone, 24 warps sharing 32 table copies (batched back
     // projection 78.5 -> 71.7 ms per 10k images then, 51 now).
-    if constexpr (!ONES && !DENS && !DW) {
+    if constexpr (!DENS && !DW) {
         if (shared)
-            return launch_bp_compact_g<ONES, DENS, DW, DEEP, 1>(vol, img, ker, axes, n, g, scale, s, pd,
+            return launch_bp_compact_g<DENS, DW, DEEP, 1>(vol, img, ker, axes, n, g, scale, s, pd,
                                                                          img2, 1, BpSplit());
     }
-    return launch_bp_compact_g<ONES, DENS, DW, DEEP, kGroupsOf<DW, DEEP>>(vol, img, ker, axes, n, g, scale, s, pd,
+    return launch_bp_compact_g<DENS, DW, DEEP, kGroupsOf<DW, DEEP>>(vol, img, ker, axes, n, g, scale, s, pd,
                                                                          img2, 32, split);
 }
 
 // Reference-rule launch with the block depth chosen by the image size.
-template <bool ONES, bool DENS>
+template <bool DENS>
 static cudaError_t launch_bp_ref_sized(float *vol, const float *img, const float *ker, const float *axes, int n,
                                        const Geom &g, const float *scale, cudaStream_t s, float *pd, bool shared,
                                        BpSplit split)
 {
     if (g.M >= 512)
-        return launch_bp_compact_t<ONES, DENS, false, true>(vol, img, ker, axes, n, g, scale, s, pd, nullptr,
+        return launch_bp_compact_t<DENS, false, true>(vol, img, ker, axes, n, g, scale, s, pd, nullptr,
                                                                  shared, split);
-    return launch_bp_compact_t<ONES, DENS>(vol, img, ker, axes, n, g, scale, s, pd, nullptr, shared, split);
+    return launch_bp_compact_t<DENS>(vol, img, ker, axes, n, g, scale, s, pd, nullptr, shared, split);
 }
 
-cudaError_t launch_back_project_ref(float *d_vol, const float *d_img, bool ones, const float *d_ker, const float *d_axes,
-                                    int n, const Geom &g, const float *scale, cudaStream_t s, bool shared, BpSplit split)
+cudaError_t launch_back_project_ref(float *d_vol, const float *d_img, const float *d_ker, const float *d_axes, int n,
+                                    const Geom &g, const float *scale, cudaStream_t s, bool shared, BpSplit split)
 {
-    if (ones)
-        return launch_bp_ref_sized<true, false>(d_vol, nullptr, d_ker, d_axes, n, g, scale, s, nullptr, false, split);
-    return launch_bp_ref_sized<false, false>(d_vol, d_img, d_ker, d_axes, n, g, scale, s, nullptr, shared, split);
+    return launch_bp_ref_sized<false>(d_vol, d_img, d_ker, d_axes, n, g, scale, s, nullptr, shared, split);
 }
 
 cudaError_t launch_back_project_ref_density(float *d_vol, float *d_pd, const float *d_img, const float *d_ker,
                                             const float *d_axes, int n, const Geom &g, const float *scale,
                                             cudaStream_t s, BpSplit split)
 {
-    return launch_bp_ref_sized<false, true>(d_vol, d_img, d_ker, d_axes, n, g, scale, s, d_pd, false, split);
+    return launch_bp_ref_sized<true>(d_vol, d_img, d_ker, d_axes, n, g, scale, s, d_pd, false, split);
 }
 
 cudaError_t launch_back_project_ref_pair(float *d_vol, float *d_pd, const float *d_img, const float *d_img2,
                                          const float *d_ker, const float *d_axes, int n, const Geom &g, cudaStream_t s,
                                          BpSplit split)
 {
-    return launch_bp_compact_t<false, false, true>(d_vol, d_img, d_ker, d_axes, n, g, nullptr, s, d_pd, d_img2,
+    return launch_bp_compact_t<false, true>(d_vol, d_img, d_ker, d_axes, n, g, nullptr, s, d_pd, d_img2,
                                                            false, split);
 }
 

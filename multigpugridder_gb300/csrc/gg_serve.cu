@@ -375,7 +375,7 @@ void enqueue_chunk(gg_server *S, Request &r)
                 GS_CKF(cufftExecR2C(p, r.d_real, r.d_spec));
                 GS_CK(launch_spectrum_to_cas_images(r.d_spec, v.M, b, r.d_cas, kF32, nullptr, s));
             }
-            GS_CK(launch_back_project_ref(r.d_acc, r.d_cas, false, v.ker, axes, b, v.g, nullptr, s, true));
+            GS_CK(launch_back_project_ref(r.d_acc, r.d_cas, v.ker, axes, b, v.g, nullptr, s, true));
         }
     }
     r.next = c0 + std::max(b, 0);
