@@ -407,7 +407,7 @@ void images_to_cas_passes(gg_gridder *h, const float *img, int b, bool adjoint, 
 {
     auto &S = h->slot[sl];
     if (h->pass_batches.size() < 6) h->pass_batches.insert(b);
-    GG_CK(launch_images_to_cas_passes(img, h->N, h->M, b, S.casimg.p, kF32, adjoint, h->tw.p, (float2 *)S.spec.p, top, s));
+    GG_CK(launch_images_to_cas_passes(img, h->N, h->M, b, S.casimg.p, adjoint, h->tw.p, (float2 *)S.spec.p, top, s));
 }
 
 void do_set_volume(gg_gridder *h, const float *d_vol, cudaStream_t s)

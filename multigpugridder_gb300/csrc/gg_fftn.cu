@@ -329,11 +329,11 @@ template <int C> struct LoadPaddedCols {
     }
 };
 
-// Columns of an image's spectrum -> its CAS image (Re+Im, and Re-Im mirrored)
-// in storage T.  ADJ: the adjoint form (first row and column zero, times post).
+// Columns of an image's spectrum -> its CAS image (Re+Im, and Re-Im mirrored).
+// ADJ: the adjoint form (first row and column zero, times post).
 // top (optional): the largest magnitude's bits (atomicMax).
-template <int C, typename T, bool ADJ> struct StoreCasCols {
-    T *dst;
+template <int C, bool ADJ> struct StoreCasCols {
+    float *dst;
     int M;
     float post;
     unsigned *top;
@@ -341,7 +341,7 @@ template <int C, typename T, bool ADJ> struct StoreCasCols {
     {
         constexpr int CP = C + 1;
         const int c = threadIdx.x % C, u = tile * C + c;
-        T *cas = dst + (size_t)s * M * M;
+        float *cas = dst + (size_t)s * M * M;
         float most = 0.0f;
         if (u <= M / 2) {
             const int i = fn_shift(u, M), im = M / 2 - u; // of u and of M - u
@@ -354,8 +354,8 @@ template <int C, typename T, bool ADJ> struct StoreCasCols {
                     d = (i == 0 || j == 0) ? 0.0f : d * post;
                     e = (im == 0 || jm == 0) ? 0.0f : e * post;
                 }
-                cas[(size_t)j * M + i] = from_f32<T>(d);
-                if (mirror) cas[(size_t)jm * M + im] = from_f32<T>(e);
+                cas[(size_t)j * M + i] = d;
+                if (mirror) cas[(size_t)jm * M + im] = e;
                 most = fmaxf(most, fmaxf(fabsf(d), fabsf(e)));
             }
         }
@@ -677,8 +677,8 @@ static cudaError_t fn_launch(const FnPlan &p, const float2 *d_tw, int tiles, int
     return cudaGetLastError();
 }
 
-template <int C, typename T, bool ADJ>
-static cudaError_t images_to_cas_t(const FnPlan &p, const float2 *d_tw, const float *d_img, int N, int n, T *d_cas,
+template <int C, bool ADJ>
+static cudaError_t images_to_cas_t(const FnPlan &p, const float2 *d_tw, const float *d_img, int N, int n, float *d_cas,
                                    float post, float2 *d_half, unsigned *top, cudaStream_t s)
 {
     const int M = p.M, H = M / 2 + 1;
@@ -686,20 +686,17 @@ static cudaError_t images_to_cas_t(const FnPlan &p, const float2 *d_tw, const fl
                                  StoreHalfRows<C>{d_half, N, M}, s);
     if (e != cudaSuccess) return e;
     return fn_launch<C>(p, d_tw, (H + C - 1) / C, n, LoadPaddedCols<C>{d_half, N, M},
-                        StoreCasCols<C, T, ADJ>{d_cas, M, post, top}, s);
+                        StoreCasCols<C, ADJ>{d_cas, M, post, top}, s);
 }
 
-cudaError_t launch_images_to_cas_passes(const float *d_img, int N, int M, int n, float *d_cas, int prec, bool adjoint,
+cudaError_t launch_images_to_cas_passes(const float *d_img, int N, int M, int n, float *d_cas, bool adjoint,
                                         const float2 *d_tw, float2 *d_half, unsigned *top, cudaStream_t s)
 {
     FnPlan p;
-    if (!fftn_ok(N, M) || !fn_plan(M, p) || prec == kF16 || (adjoint && prec != kF32)) return cudaErrorInvalidValue;
+    if (!fftn_ok(N, M) || !fn_plan(M, p)) return cudaErrorInvalidValue;
     const float post = 1.0f / ((float)M * (float)M);
-    if (adjoint) return images_to_cas_t<kFnC, float, true>(p, d_tw, d_img, N, n, d_cas, post, d_half, top, s);
-    if (prec == kBF16)
-        return images_to_cas_t<kFnC, Rounded<__nv_bfloat16>, false>(p, d_tw, d_img, N, n, (Rounded<__nv_bfloat16> *)d_cas, 1.0f,
-                                                                   d_half, top, s);
-    return images_to_cas_t<kFnC, float, false>(p, d_tw, d_img, N, n, d_cas, 1.0f, d_half, top, s);
+    if (adjoint) return images_to_cas_t<kFnC, true>(p, d_tw, d_img, N, n, d_cas, post, d_half, top, s);
+    return images_to_cas_t<kFnC, false>(p, d_tw, d_img, N, n, d_cas, 1.0f, d_half, top, s);
 }
 
 cudaError_t launch_cas_to_images_passes(const float *d_cas, int M, int N, int n, float *d_img, const float2 *d_tw,

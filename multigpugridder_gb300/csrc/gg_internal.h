@@ -221,10 +221,10 @@ bool fftn_volume_ok(int N, int M);
 bool fftn_volume_back_ok(int N, int M);
 // e^(-2 pi i k / M), k < M, for the passes' d_tw.
 void fftn_twiddles(int M, float2 *out);
-// The two directions of the fused stages above, in two launches each through
-// d_half (n * N * (M/2 + 1) values).  top (optional, images -> CAS images): the
+// The two directions of the fused stages above in FP32, in two launches each
+// through d_half (n * N * (M/2 + 1) values).  top (optional, images -> CAS images): the
 // bits of the largest magnitude, added by atomicMax to a zeroed word.
-cudaError_t launch_images_to_cas_passes(const float *d_img, int N, int M, int n, float *d_cas, int prec, bool adjoint,
+cudaError_t launch_images_to_cas_passes(const float *d_img, int N, int M, int n, float *d_cas, bool adjoint,
                                         const float2 *d_tw, float2 *d_half, unsigned *top, cudaStream_t s);
 cudaError_t launch_cas_to_images_passes(const float *d_cas, int M, int N, int n, float *d_img, const float2 *d_tw,
                                         float2 *d_half, cudaStream_t s);
