@@ -136,6 +136,28 @@ def test_forward_tiles(cuda, N, n, scale, prec):
     assert np.all(got[ref == 0] == 0)
 
 
+# axes longer than one: some boxes fit and some do not; most windows leave the
+# volume; windows far outside it; columns scaled apart
+@pytest.mark.parametrize("prec", ["f32", "bf16"])
+@pytest.mark.parametrize("N,n,scale", [(50, 30, (1.08, 1.08)), (32, 100, (1.3, 0.9)), (18, 6, (2.5, 2.5)), (16, 4, (40.0, 9.0))])
+def test_forward_tiles_long_axes(cuda, N, n, scale, prec):
+    import torch
+
+    import multigpugridder_gb300 as gg
+
+    p = O.Params(N)
+    cas = np.random.default_rng(6000 + N).standard_normal((p.V,) * 3).astype(np.float32)
+    axes = O.quaternion_axes(n, seed=N).astype(np.float32)
+    axes = (axes.reshape(n, 3, 3) * np.float32(scale + (1.0,))[None, :, None]).reshape(n, 9)
+    stored = cas if prec == "f32" else torch.from_numpy(cas).bfloat16().float().numpy()
+    ref = O.fp_ref_f32(stored, axes, p.M, p.mask_radius, p.ker)
+    with gg.MultiGPUGridder(N, n, precision=prec, adjustInterpFactor=False) as g:
+        g.setCASVolume(cas)
+        got = g.forwardProjectCAS(axes)
+    assert O.rel_l2(got, ref) < TOL
+    assert np.all(got[ref == 0] == 0)
+
+
 # one handle through every storage type and back (with the 4-tap tiles and with
 # five taps), against a handle that has known no other; the volume is replaced on the way
 @pytest.mark.parametrize("edge", [0.0, 0.25])
