@@ -95,7 +95,14 @@ int gg_set_precision(gg_gridder *h, int precision);                 /* GG_PREC_*
    GG_PREC_F32 under a 2-byte volume keeps the images exact; it costs no more
    than 2-byte images.  No counterpart in the reference. */
 int gg_set_image_precision(gg_gridder *h, int precision);
-int gg_set_bp_mode(gg_gridder *h, int mode);                        /* GG_BP_REF (default) or GG_BP_ADJOINT */
+/* GG_BP_REF (default) or GG_BP_ADJOINT.  The reference rule adds a voxel's
+   directions in a fixed order: the same call gives the same bits.  How the sum is
+   grouped depends on the directions per batch (gg_set_max_axes_to_allocate)
+   and, on small volumes, on segments chosen from their number, the volume and the
+   mask, so other batch sizes agree to FP32 rounding.  The adjoint rule adds in
+   the order the GPU gets to: two runs of the same call agree to FP32 rounding
+   (relative L2 below 1e-6), not bit for bit. */
+int gg_set_bp_mode(gg_gridder *h, int mode);
 
 /* setVolume + the CAS preparation of forwardProject
    (MultiGPUGridder_Matlab_Class.m:272-275, :226-227; CASFromVol_Gridder.m:25-60),
@@ -163,7 +170,8 @@ int gg_reconstruct_volume_dev(gg_gridder *h, const float *d_axes, int n_axes,
    (one all-reduce or reduce of 2*V^3 floats).
    gg_volume_from_sums_dev: summed d_sums -> CAS volume sums[0] ./ (sums[1] +
    1e-6), left resident, then getVol into d_volume_out (N^3).  With one GPU
-   the two calls give gg_reconstruct_volume_dev's result bit for bit. */
+   the two calls give gg_reconstruct_volume_dev's result, under GG_BP_REF bit
+   for bit. */
 int gg_back_project_sums_dev(gg_gridder *h, const float *d_axes, int n_axes, const float *d_images,
                              float *d_sums, void *stream);
 int gg_volume_from_sums_dev(gg_gridder *h, const float *d_sums, float *d_volume_out, void *stream);
@@ -196,7 +204,9 @@ int gg_reconstruct_volume_ctf_dev(gg_gridder *h, const float *d_axes, int n_axes
    followed by forwardProject to images): image gradients n*N*N -> volume
    gradient N^3 (written, not accumulated).  Uses the exact-adjoint back
    projection whatever gg_set_bp_mode says and leaves the resident CAS volume
-   untouched.  No counterpart in the reference, which has no gradient. */
+   untouched.  Two runs agree to FP32 rounding (relative L2 below 1e-6), not bit
+   for bit: see gg_set_bp_mode.  No counterpart in the reference, which has no
+   gradient. */
 int gg_forward_project_adjoint(gg_gridder *h, const float *axes, int n_axes, const float *image_grads,
                                float *volume_grad_out);
 int gg_forward_project_adjoint_dev(gg_gridder *h, const float *d_axes, int n_axes, const float *d_image_grads,
@@ -221,7 +231,8 @@ int gg_back_project_kernel(float *d_cas_volume, const float *d_cas_images, const
                            void *stream);
 
 /* Exact adjoint of gg_forward_project_kernel (same weights, every pair the
-   forward gather reads).  No counterpart in the reference. */
+   forward gather reads inside the volume), added to d_cas_volume in no fixed
+   order (two runs agree to FP32 rounding).  No counterpart in the reference. */
 int gg_back_project_adjoint_kernel(float *d_cas_volume, const float *d_cas_images, const float *d_kb_table,
                                    const float *d_axes, float ker_hwidth, int n_axes, int cas_vol_size,
                                    int cas_img_size, int mask_radius, int kb_table_size, void *stream);

@@ -6,7 +6,9 @@ the CAS preparation of setVolume, the forward projection and the CAS-image to
 image path.  Its backward is the exact adjoint of that whole linear map
 (`gg_forward_project_adjoint_dev`, built on the exact-adjoint back-projection
 kernel with the forward kernel's pair set and weights), so gradients agree
-with finite differences of the forward operator.  The reference has no
+with finite differences of the forward operator.  The adjoint adds with atomics:
+two backward passes over the same inputs agree to FP32 rounding (relative L2
+below 1e-6), not bit for bit; the images are the same bits.  The reference has no
 gradient; its back projection (the window rule of gpuBackProject.cu) is not
 the adjoint of its forward projection at general orientations.
 

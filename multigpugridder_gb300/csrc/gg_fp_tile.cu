@@ -193,7 +193,7 @@ __device__ __forceinline__ void tap_weights(const TileTable &t, float f, float f
 }
 
 // A window inside the volume, read from global memory, for tiles without a box
-// (axes 1.04 times orthonormal and longer miss it more and more often); p: its
+// (axes longer than one by 2% or more begin to miss it); p: its
 // first tap, rows P and planes PV elements apart.  Out of line, as the next one:
 // neither takes registers from the box's path.  Both have the 12 weights at hand
 // and their taps unrolled: 1,000 CAS images at M = 256 from axes 1.2 times as

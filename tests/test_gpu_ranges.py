@@ -380,6 +380,37 @@ def test_adjoint_large_radius(cuda, gglib, radius):
     assert O.rel_l2(vol.cpu().numpy(), ref) < 1e-3
 
 
+# Repeated calls.  The reference rule: the same bits, split (n = 300) and not.  The
+# adjoint adds in any order: a voxel's few hundred terms of either sign, each order
+# rounding by 6e-8 a step, spread by some 1e-7 of the sum; 1e-6 bounds it.
+def test_repeated_calls(cuda):
+    import torch
+
+    import multigpugridder_gb300 as gg
+    from multigpugridder_gb300.autograd import ForwardProjector
+
+    N, n = 32, 300
+    axes = O.quaternion_axes(n, seed=9).astype(np.float32)
+    imgs = np.random.default_rng(9).standard_normal((n, N, N)).astype(np.float32)
+    runs = {}
+    for mode in ("ref", "adjoint"):
+        with gg.MultiGPUGridder(N, n, bp_mode=mode, adjustInterpFactor=False) as g:
+            for k in range(4):
+                g.backProject(imgs, axes)
+                runs[mode, k] = g.getCASVolume()
+                g.backProject(imgs[:20], axes[:20])
+                runs[mode, k, 20] = g.getCASVolume()
+    proj = ForwardProjector(N)
+    for k in range(4):
+        runs["grad", k] = proj.adjoint(to_dev(imgs, cuda), to_dev(axes, cuda)).cpu().numpy()
+    for k in range(1, 4):
+        assert np.array_equal(runs["ref", 0], runs["ref", k])
+        assert np.array_equal(runs["ref", 0, 20], runs["ref", k, 20])
+        for key in (("adjoint",), ("grad",)):
+            assert O.rel_l2(runs[key + (k,)], runs[key + (0,)]) < 1e-6
+        assert O.rel_l2(runs["adjoint", k, 20], runs["adjoint", 0, 20]) < 1e-6
+
+
 # enough images for blocks of 64 rows (1024 of them), also with a remainder, and one too few
 @pytest.mark.parametrize("M,n", [(64, 1100), (100, 520), (64, 1000)])
 def test_ctf_row_blocks(cuda, gglib, M, n):
