@@ -462,7 +462,9 @@ void fp_batch(gg_gridder *h, const float *d_axes, int b, float *cas_out, float *
 {
     auto &S = h->slot[sl];
     ProfScope ps(h, s, GG_KERNEL_FORWARD);
-    if (h->five_taps)
+    if (h->five_taps && h->prec == kF32) // five taps read the dense rows faster (200 images at M = 128: 310 us, pitched 319)
+        GG_CK(launch_forward_project(h->cas.p, kF32, h->V, cas_out, h->ker.p, d_axes, b, h->geom(), true, nullptr, s));
+    else if (h->five_taps)
         GG_CK(launch_forward_project(h->fp().vol.p, h->prec, fp_pitch(h->V, h->prec), cas_out, h->ker.p, d_axes, b,
                                      h->geom(), true, h->vol_scale(), s));
     else
