@@ -587,7 +587,7 @@ void ctf_batch(gg_gridder *h, const float *d_axes, int b, const float *img, cons
     auto &S = h->slot[sl];
     if (h->fused_fft) {
         GG_CK(launch_images_to_cas_fused(img, h->N, h->M, b, S.casimg.p, kF32, false, s));
-    } else if (h->fft_passes) {
+    } else if (h->fft_passes && h->img_prec() != kBF16) { // as bp_batch: BF16 images keep the library's transform
         images_to_cas_passes(h, img, b, false, nullptr, sl, s);
     } else {
         GG_CK(launch_images_to_fft_input(img, h->N, h->M, b, S.real.p, s));

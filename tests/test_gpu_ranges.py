@@ -411,6 +411,23 @@ def test_repeated_calls(cuda):
         assert O.rel_l2(runs["adjoint", k, 20], runs["adjoint", 0, 20]) < 1e-6
 
 
+# a CTF of -1 everywhere gives minus the plain reconstruction, bit for bit: the
+# images take the same transform in both, also where they are rounded (M = 100
+# through the passes or the library, M = 64 in one kernel)
+@pytest.mark.parametrize("prec", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("N", [32, 50])
+def test_ctf_of_minus_one(cuda, N, prec):
+    import multigpugridder_gb300 as gg
+
+    n = 20
+    axes = O.quaternion_axes(n, seed=N).astype(np.float32)
+    imgs = np.random.default_rng(N).standard_normal((n, N, N)).astype(np.float32)
+    with gg.MultiGPUGridder(N, n, precision=prec, adjustInterpFactor=False) as g:
+        plain = g.reconstructVol(imgs, axes).copy()
+        ctf = g.reconstructVolCTF(imgs, axes, np.zeros(n, dtype=np.float32), cs_mm=0.0, amp_contrast=1.0)
+    assert np.array_equal(ctf, -plain)
+
+
 # enough images for blocks of 64 rows (1024 of them), also with a remainder, and one too few
 @pytest.mark.parametrize("M,n", [(64, 1100), (100, 520), (64, 1000)])
 def test_ctf_row_blocks(cuda, gglib, M, n):
