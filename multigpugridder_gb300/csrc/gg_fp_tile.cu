@@ -492,10 +492,12 @@ static cudaError_t encode_maps(const void *d_vol, int V, int P, CUtensorMapDataT
 // Orders the maps' bytes, written by a copy, before every later launch that
 // reads them through the tensor-map proxy: the address may have held another
 // handle's maps.  Once a buffer, so that no launch pays for it (a fence for
-// every map at the projection's own start: 26 -> 72 us for 16 directions).
-__global__ void __launch_bounds__(256) fence_maps_kernel(const CUtensorMap *__restrict__ maps, int n)
+// every map at the projection's own start: 26 -> 72 us for 16 directions); by
+// one block, which every later launch comes after (10 us of a handle's first
+// projection; a block an SM 30).
+__global__ void __launch_bounds__(1024) fence_maps_kernel(const CUtensorMap *__restrict__ maps, int n)
 {
-    for (int t = threadIdx.x; t < n; t += 256)
+    for (int t = threadIdx.x; t < n; t += blockDim.x)
         asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(maps + t) : "memory");
 }
 
@@ -510,10 +512,7 @@ cudaError_t fp_tile_make_maps(const void *d_vol, int V, int P, int prec, void *d
     // wait for it
     e = cudaMemcpyAsync(d_maps, m.data(), m.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return e;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    fence_maps_kernel<<<(unsigned)std::max(sms, 1), 256, 0, s>>>((const CUtensorMap *)d_maps, (int)m.size());
+    fence_maps_kernel<<<1, 1024, 0, s>>>((const CUtensorMap *)d_maps, (int)m.size());
     count_launches(1);
     e = cudaGetLastError();
     return e != cudaSuccess ? e : cudaStreamSynchronize(s);
