@@ -11,7 +11,8 @@
 // plane summed a 7x7 pixel window, of which 22% carry weight, with three table
 // lookups per pixel (about 150 warp instructions a pixel).  Scattered, the
 // weights of a pixel are separable (12 lookups) and every product counts: 15
-// warp instructions a pixel and 9 shared-memory wavefronts, which bound it.
+// warp instructions a pixel and 12.5 shared-memory wavefronts in all (ncu),
+// which bound it: 4 its taps' reads and writes, 4 the broadcasts of its terms.
 // The lanes of a half window are 4 x 4 x 2 taps: with a row pitch of 12 or 20
 // words and a slice pitch of 16 mod 32 their addresses fall in 32 different
 // banks from any start.  The box is private to the warp, so plain loads and

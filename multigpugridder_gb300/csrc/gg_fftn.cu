@@ -19,7 +19,7 @@
 //     first two (10.5 M^3 bytes for N = M/2, against about 36).
 //   CAS volume -> volume: the same backwards; only what is kept is stored.
 //
-// Bound: the latency of a tile's load, stages and store at 16 warps an SM or so;
+// Bound: the latency of a tile's load, stages and store at 16 to 32 warps an SM;
 // 9 M^2 bytes an image with N = M/2 (1 in, 2 x 2 for the half spectra between
 // the passes, 4 out), where the library's batched transforms with a stage
 // kernel on either side moved about 29 M^2.  Measured: 300 images at M = 200

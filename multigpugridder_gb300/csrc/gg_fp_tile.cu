@@ -12,9 +12,9 @@
 // per distinct 128-byte line; three transposed copies of the volume were kept
 // to get there), from a box with a fixed slice pitch 3.0 and with the pitch
 // and the warp's shape chosen per direction 2.2 (a CPU model over random
-// directions).  fp_plan_kernel makes that choice.  Measured, 1,000 directions
-// at M = 256: kernel 2,176 -> 1,488 us, shared-memory pipe 75% busy; whole call
-// 2,389 -> 1,697 us, images the same bit for bit (FP32).  The two transposed
+// directions).  fp_plan_kernel makes that choice.  Measured at M = 256: kernel
+// for 1,024 directions 2,270 -> 1,452 us (ncu), shared-memory pipe 75% busy;
+// whole call for 1,000 2,389 -> 1,638 us, images the same bit for bit (FP32).  The two transposed
 // copies (175 us a volume at 128^3, 1,700 us of BF16 ones at 256^3) went away.
 #include <cuda.h>
 

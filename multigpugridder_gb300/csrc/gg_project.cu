@@ -400,42 +400,13 @@ __device__ __forceinline__ float fma_sat(float a, float b, float c)
 // rows FS apart); table entry floor(P y) is read at
 // tab + bits(y + q.mg) * stride.  Sums row by row, as the reference.  TS: the
 // stride in bytes when known at compile time (128 for 32 interleaved table
-// copies, 4 for one), so the address is a shift-add on the integer pipe
-// rather than a multiply on the FMA pipe; 0: q.stride.
-template <bool DENS, int WI, int WJ, int FS, bool DW = false, int TS = 0>
-__device__ __forceinline__ void foot_window(const FootWin &q, const float *fbase, unsigned tab, float pi0, float pj0,
-                                            float &cumSum, float &cumW, const float *fbase2 = nullptr)
-{
-    const unsigned st = TS ? (unsigned)TS : q.stride;
-#pragma unroll
-    for (int jo = 0; jo < WJ; jo++) {
-        const float pj = pj0 + (float)jo;
-        const float py0 = __fmul_rn(pj, q.ny0), py1 = __fmul_rn(pj, q.ny1), py2 = __fmul_rn(pj, q.ny2);
-#pragma unroll
-        for (int io = 0; io < WI; io++) {
-            const float pi = pi0 + (float)io;
-            const float q0 = __fadd_rn(__fmaf_rn(pi, q.nx0, py0), q.vc);
-            const float q1 = __fadd_rn(__fmaf_rn(pi, q.nx1, py1), q.vc);
-            const float q2 = __fadd_rn(__fmaf_rn(pi, q.nx2, py2), q.vc);
-            const unsigned b0 = __float_as_uint(__fadd_rd(fma_sat(q0, q.s, q.c0), q.mg));
-            const unsigned b1 = __float_as_uint(__fadd_rd(fma_sat(q1, q.s, q.c1), q.mg));
-            const unsigned b2 = __float_as_uint(__fadd_rd(fma_sat(q2, q.s, q.c2), q.mg));
-            float w = lds_f32(tab + b0 * st);
-            w = __fmul_rn(w, lds_f32(tab + b1 * st));
-            w = __fmul_rn(w, lds_f32(tab + b2 * st));
-            cumSum = __fmaf_rn(fbase[jo * FS + io], w, cumSum);
-            if (DENS) cumW = __fadd_rn(cumW, w);
-            if (DW) cumW = __fmaf_rn(fbase2[jo * FS + io], w, cumW);
-        }
-    }
-}
-
-// foot_window with adjacent pixels of a row taken in pairs by the packed
-// FP32x2 instructions (sm_100+): the pixel positions, the table addresses and
-// the weight products of two pixels per instruction (the saturating index fma
-// has no packed form).  Each lane of a packed instruction rounds as the scalar
-// instruction does, so every weight, and every sum (accumulated one pixel at a
-// time in the same order), is bit-identical to foot_window's.
+// copies), so the address is a shift-add on the integer pipe rather than a
+// multiply on the FMA pipe; 0: q.stride.  Adjacent pixels of a row go in pairs
+// through the packed FP32x2 instructions (sm_100+): the pixel positions, the table
+// addresses and the weight products of two pixels per instruction (the
+// saturating index fma has no packed form).  Each lane of a packed instruction
+// rounds as the scalar instruction does and the sums take one pixel at a time,
+// in order, so every weight and sum has the scalar form's bits.
 __device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
 
 template <bool DENS, int WI, int WJ, int FS, bool DW = false, int TS = 0>

@@ -105,9 +105,11 @@ int chunk_cap(int M)
 }
 
 // Estimated device seconds of one direction, for ranking requests and bounding
-// the backlog: one GB300 runs the forward projection with its 2-D stage in
-// about 34 ps and the serving back projection in about 120 ps per CAS-image
-// pixel (2.2 and 7.9 ms per 1,000 directions at M = 256).
+// the backlog: one GB300 runs the forward projection with its 2-D stage and
+// copies in about 34 ps and the serving back projection in about 120 ps per
+// CAS-image pixel (measured on one lane, ps: M = 128 39 / 297, 256 32 / 110,
+// 384 40 / 119, 512 35 / 121; a small volume's back projection fills the GPU
+// only with other lanes' beside it).
 double dir_seconds(int op, int M)
 {
     return (double)M * M * (op == GG_OP_FORWARD ? 3.4e-11 : 1.2e-10);
