@@ -93,9 +93,9 @@ def workload(args, rank=0, world=1):
 FLUSH_BYTES = 512 << 20  # untimed write between steps: 4x the 126 MB L2
 
 # From a one-launch ncu capture of the fused back projection at 128^3 x 2,
-# 2,000 directions per launch (profiles/bp_ref_compact_kernel_density_128cubed_2000dirs.md):
-# DRAM bytes (read + write) and L2 bytes (lts__t_bytes) per direction, and the
-# fraction of cycles the schedulers issued.
+# 2,000 directions per launch (its summary is in profiles/): DRAM bytes (read +
+# write) and L2 bytes (lts__t_bytes) per direction, and the fraction of cycles
+# the schedulers issued.
 NCU_BP_DRAM_PER_DIR = 1.696e9 / 2000
 NCU_BP_LTS_PER_DIR = 17.12e9 / 2000
 NCU_BP_ISSUE_ACTIVE = 0.852
@@ -342,7 +342,7 @@ def run_gb300(args):
     except (OSError, ValueError):
         pass
     hbm = peaks.get("hbm_gbs") or 6800.0
-    # the L2 read bandwidth of this GPU, measured here (the bound SURVEY-style
+    # the L2 read bandwidth of this GPU, measured here (the bound that byte
     # accounting names for 128^3: the 72 MB CAS volume stays in the 126 MB L2)
     l2 = ctypes.c_double()
     check(L.gg_measure_l2_read_gbs(10, ctypes.byref(l2)))
