@@ -274,7 +274,8 @@ __device__ __forceinline__ TileAt tile_at(long long item, int tilesX, bool items
     return TileAt{a, i0, j0, i0 - ic, min(i0 + kTile, M) - 1 - ic, j0 - ic, min(j0 + kTile, M) - 1 - ic};
 }
 // Whether any pixel of the tile is in the mask (the nearest one to the centre
-// is).  32-bit: M^2 stays below 2^31 for any volume that fits the GPU.
+// is).  32-bit: a handle's radius is at most M, and M^2 stays below 2^31 for any
+// volume that fits the GPU.
 __device__ __forceinline__ bool tile_live(const TileAt &t, int R2)
 {
     const int ni = t.dia > 0 ? t.dia : t.dib < 0 ? t.dib : 0, nj = t.dja > 0 ? t.dja : t.djb < 0 ? t.djb : 0;
